@@ -78,7 +78,7 @@ def sequence_job():
 
 def experts_job():
     """Kernels of feed-forwards made of experts (built when a model first asks for them)."""
-    return {"name": "sb_moe", "sources": ["routed_experts.cu"]}
+    return {"name": "sb_moe", "sources": ["routed_experts.cu", "experts_tcgen05.cu"]}
 
 
 def projection_job():
@@ -1139,7 +1139,8 @@ class CudaKernels:
         ff, n, k = w_down.shape[2], w_down.shape[1], h.shape[1]
         pairs = t * top
         dev = h.device
-        tile_rows = lib.sb_moe_tile_rows(_DT[h.dtype], k, ff, h.stride(0))     # 64 on the tensor-core kernels, else 32
+        tensor_rows = lib.sb_moe_tensor_rows(_DT[h.dtype], k, ff, h.stride(0), t)      # 0: not on the tensor cores
+        tile_rows = tensor_rows or lib.sb_moe_tile_rows()
         max_tiles = pairs // tile_rows + min(e, pairs)
         ints = torch.empty(2 * pairs + e + 1 + 2 * max_tiles + 1, dtype=torch.int32, device=dev)
         idx, order = ints[:pairs], ints[pairs: 2 * pairs]
@@ -1158,12 +1159,19 @@ class CudaKernels:
                    "expert choice")
         _check(lib.sb_moe_sort(_p(idx), pairs, e, tile_rows, _p(offsets), _p(order), _p(tiles), _p(n_tiles), s), "grouping by expert")
         act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
-        _check(lib.sb_moe_gate_up(_p(h), h.stride(0), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs,
-                                  e, k, ff, 1 if scale_input else 0, {"swiglu": 0, "clamped_swish": 1}[activation],
-                                  ctypes.c_float(limit), ctypes.c_float(alpha), _p(act), _DT[h.dtype], s), "experts, gate and up")
+        kind = {"swiglu": 0, "clamped_swish": 1}[activation]
+        if tensor_rows:
+            xg = torch.empty((pairs, k), dtype=h.dtype, device=dev)          # the pairs' tokens in grouped order
+            self.launches += 1
+            _check(lib.sb_moe_gate_up_tensor(_p(h), h.stride(0), t, _p(xg), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top,
+                                             pairs, e, k, ff, 1, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha),
+                                             _p(act), tile_rows, self._wait_flag(), s), "experts, gate and up")
+        else:
+            _check(lib.sb_moe_gate_up(_p(h), h.stride(0), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs,
+                                      e, k, ff, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha), _p(act),
+                                      _DT[h.dtype], s), "experts, gate and up")
         parts = out if (top == 1 and not more) else torch.empty((pairs, n), dtype=torch.float32, device=dev)
-        _check(lib.sb_moe_down(_p(act), _p(w_down), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), pairs, e, ff, n,
-                               0 if scale_input else 1, _p(parts), _DT[h.dtype], _DT[parts.dtype], tile_rows, s), "experts, down")
+        self._experts_down(lib, act, w_down, order, offsets, tiles, n_tiles, wts, 0 if scale_input else 1, parts, tensor_rows, s)
         if more:
             self.launches += 1
             gate = logits[:, outputs:] if shared_gated else None
@@ -1172,6 +1180,16 @@ class CudaKernels:
         elif top > 1:
             self.launches += 1
             _check(lib.sb_moe_combine(_p(parts), top, t, n, _p(out), _DT[out.dtype], s), "sum over a token's experts")
+
+    def _experts_down(self, lib, act, w_down, order, offsets, tiles, n_tiles, wts, scale_output, parts, tensor_rows, s) -> None:
+        e, n, ff = w_down.shape
+        pairs = act.shape[0]
+        if tensor_rows:
+            _check(lib.sb_moe_down_tensor(_p(act), _p(w_down), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), pairs, e, ff, n, scale_output,
+                                          _p(parts), _DT[parts.dtype], tensor_rows, self._wait_flag(), s), "experts, down")
+        else:
+            _check(lib.sb_moe_down(_p(act), _p(w_down), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), pairs, e, ff, n, scale_output,
+                                   _p(parts), _DT[act.dtype], _DT[parts.dtype], s), "experts, down")
 
     def table_experts(self, h, tokens, last_token, table, w_up, w_down, top: int, out, activation: str = "relu_squared") -> None:
         """out[t] = (1 / top) * sum over the experts e = table[token[t], :] of w_down[e] act(w_up[e] h[t]), act = relu squared:
@@ -1184,7 +1202,8 @@ class CudaKernels:
         n = w_down.shape[1]
         pairs = t * top
         dev = h.device
-        tile_rows = lib.sb_moe_tile_rows(_DT[h.dtype], k, ff, h.stride(0))
+        tensor_rows = lib.sb_moe_tensor_rows(_DT[h.dtype], k, ff, h.stride(0), t)
+        tile_rows = tensor_rows or lib.sb_moe_tile_rows()
         max_tiles = pairs // tile_rows + min(e, pairs)
         ints = torch.empty(2 * pairs + e + 1 + 2 * max_tiles + 1, dtype=torch.int32, device=dev)
         idx, order = ints[:pairs], ints[pairs: 2 * pairs]
@@ -1198,11 +1217,17 @@ class CudaKernels:
                                       table.shape[0], e, top, t, _p(idx), _p(wts), _p(self.errors_tensor()), s), "expert choice by table")
         _check(lib.sb_moe_sort(_p(idx), pairs, e, tile_rows, _p(offsets), _p(order), _p(tiles), _p(n_tiles), s), "grouping by expert")
         act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
-        _check(lib.sb_moe_up(_p(h), h.stride(0), _p(w_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs, e, k, ff,
-                             _p(act), _DT[h.dtype], s), "experts, up")
+        if tensor_rows:
+            xg = torch.empty((pairs, k), dtype=h.dtype, device=dev)
+            self.launches += 1
+            _check(lib.sb_moe_gate_up_tensor(_p(h), h.stride(0), t, _p(xg), _p(w_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top,
+                                             pairs, e, k, ff, 0, 0, 0, ctypes.c_float(0.0), ctypes.c_float(0.0), _p(act), tile_rows,
+                                             self._wait_flag(), s), "experts, up")
+        else:
+            _check(lib.sb_moe_up(_p(h), h.stride(0), _p(w_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs, e, k, ff,
+                                 _p(act), _DT[h.dtype], s), "experts, up")
         parts = out if top == 1 else torch.empty((pairs, n), dtype=torch.float32, device=dev)
-        _check(lib.sb_moe_down(_p(act), _p(w_down), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), pairs, e, ff, n, 1, _p(parts),
-                               _DT[h.dtype], _DT[parts.dtype], tile_rows, s), "experts, down")
+        self._experts_down(lib, act, w_down, order, offsets, tiles, n_tiles, wts, 1, parts, tensor_rows, s)
         if top > 1:
             self.launches += 1
             _check(lib.sb_moe_combine(_p(parts), top, t, n, _p(out), _DT[out.dtype], s), "sum over a token's experts")

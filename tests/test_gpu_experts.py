@@ -1,0 +1,84 @@
+"""The experts' tensor-core products at the edges of their tiles: runs of 1 to more than 256 tokens an expert, counts that are no
+multiple of 16, 64 or 128, outputs that end inside a unit, k that ends inside a stage, experts without tokens, every epilogue."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+E, TOP = 5, 2
+
+
+def _reference(x, logits, w_gu, w_down, kind):
+    x, w_gu, w_down = x.double(), w_gu.double(), w_down.double()
+    ff = w_down.shape[2]
+    score = torch.softmax(logits.double(), -1) if kind == "swiglu" else torch.sigmoid(logits.double())
+    w, idx = score.sort(dim=-1, descending=True, stable=True)
+    out = torch.zeros((x.shape[0], w_down.shape[1]), dtype=torch.float64, device=x.device)
+    most = torch.zeros_like(out)                            # the same sums of absolute values
+    for j in range(TOP):
+        for e in range(E):
+            t = (idx[:, j] == e).nonzero()[:, 0]
+            wt = w[t, j][:, None]
+            h = x[t] * wt if kind == "clamped_swish" else x[t]
+            g, u = h @ w_gu[e, :ff].T, h @ w_gu[e, ff:].T
+            if kind == "clamped_swish":
+                g = g.clamp(max=1.5)
+                a = g * torch.sigmoid(1.702 * g) * (u.clamp(-1.5, 1.5) + 1)
+            else:
+                a = g * torch.sigmoid(g) * u
+            wt = 1.0 if kind == "clamped_swish" else wt
+            out.index_add_(0, t, (a @ w_down[e].T) * wt)
+            most.index_add_(0, t, (a.abs() @ w_down[e].abs().T) * wt)
+    return out, most
+
+
+def _bound(want, most):
+    """Two roundings to bfloat16 (8 significant bits: by at most 2^-8 of the value): of the activations, so a sum moves by 2^-8 of its
+    absolute terms, and of the output; the float sums add less than 2^-15 of the absolute terms."""
+    first = (2.0 ** -8 + 2.0 ** -15) * most
+    return first + 2.0 ** -8 * (want.abs() + first) + 1e-30
+
+
+@pytest.mark.parametrize("kind", ["swiglu", "clamped_swish"])
+@pytest.mark.parametrize("tokens,k,ff,n", [(1, 64, 32, 40), (7, 96, 160, 64), (16, 2080, 96, 200), (17, 64, 128, 136), (33, 160, 64, 129), (65, 128, 416, 128),
+                                           (129, 32, 96, 257), (200, 64, 64, 64), (257, 96, 32, 72), (700, 128, 224, 300)])
+def test_expert_products(tokens, k, ff, n, kind):
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    g = torch.Generator(device="cuda").manual_seed(tokens * 1000 + ff)
+    draw = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x = draw(tokens, k).bfloat16()
+    logits = draw(tokens, E)
+    logits[:, 0] += 2.0                                     # a crowded expert
+    logits[:, 3] -= 50.0                                    # and one that nobody chooses
+    w_gu, w_down = (draw(E, 2 * ff, k) / k ** 0.5).bfloat16(), (draw(E, n, ff) / ff ** 0.5).bfloat16()
+    out = torch.full((tokens, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    kernels.routed_experts(x, logits, w_gu, w_down, TOP, out, score="softmax" if kind == "swiglu" else "sigmoid", scale_input=kind != "swiglu",
+                           activation=kind, limit=1.5, alpha=1.702)
+    kernels.check_errors()
+    want, most = _reference(x, logits, w_gu, w_down, kind)
+    assert ((out.double() - want).abs() <= _bound(want, most)).all()
+
+
+@pytest.mark.parametrize("tokens,k,ff,n", [(3, 64, 32, 48), (20, 96, 160, 130), (300, 64, 96, 72)])
+def test_ungated_expert_products(tokens, k, ff, n):
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    draw = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x = draw(tokens, k).bfloat16()
+    w_up, w_down = (draw(E, ff, k) / k ** 0.5).bfloat16(), (draw(E, n, ff) / ff ** 0.5).bfloat16()
+    ids = torch.arange(tokens, device="cuda", dtype=torch.int32)
+    table = torch.stack([torch.zeros(tokens, device="cuda"), 1 + torch.arange(tokens, device="cuda") % 3], 1).to(torch.int32).contiguous()
+    out = torch.full((tokens, n), float("nan"), device="cuda", dtype=torch.bfloat16)
+    kernels.table_experts(x, ids, None, table, w_up, w_down, 2, out)
+    kernels.check_errors()
+    want, most = (torch.zeros((tokens, n), dtype=torch.float64, device="cuda") for _ in range(2))
+    for t in range(tokens):
+        for e in table[t].tolist():
+            a = (x[t].double() @ w_up[e].double().T).clamp(min=0).square()
+            want[t] += 0.5 * (a @ w_down[e].double().T)
+            most[t] += 0.5 * (a @ w_down[e].double().abs().T)
+    assert ((out.double() - want).abs() <= _bound(want, most)).all()
