@@ -1,4 +1,5 @@
-// Paged causal attention for prompt portions on the fifth-generation tensor cores (head_dim 64 or 128, bfloat16).
+// Paged causal attention for prompt portions on the fifth-generation tensor cores (head_dim 64 or 128, and rows of 256 that are
+// keys and values at once, bfloat16), over all keys or behind a window that may keep the sequence's first keys.
 //
 // Work is cut as in attention_mma.cu: per (request, kv head), with the G = H / Hkv query heads that share the kv
 // head folded into the row dimension: row m stands for (token m / G, head hk*G + m % G). A CTA owns 128 such
@@ -21,7 +22,13 @@
 // At head_dim 128 an operand row is two 128-byte swizzle atoms: queries, keys and values arrive as two TMA boxes of 64
 // elements each, the first product walks over both atoms of Q and K, the second product covers the 128 output
 // columns in one instruction (the descriptor's leading byte offset names the distance between the atoms of V);
-// shared memory then holds one CTA per SM.
+// shared memory then holds one CTA per SM. (Two CTAs with two stages and one buffer of probabilities each, 112 KB, fit too:
+// 2,048 tokens, 24/8 heads, 81.3 us against 77.7.)
+// At head_dim 256 keys and values are the same rows (latent attention), so a tile is loaded once for both products; with its
+// 256 output columns and two score buffers the kernel holds all of tensor memory.
+// Behind a window only the tiles that a row of the CTA can see are walked. 2,048 tokens, window 1,024: 16/4 heads of 128 95.2 us on
+// mma.sync -> 38.2; 16 heads over one row of 256 172.3 -> 51.5 (bound by the softmax threads: a warp a scheduler, about 1.3 us a tile
+// against 0.55 us of products).
 // The recurrences are those of serve/kernels/attn_prefill.py:58-72 with exp2 and a folded log2(e)
 // (attn_prefill.py:330-331); probabilities are rounded to bfloat16 before the second product (attn_prefill.py:71).
 // Every wait is bounded; a wait that runs out raises *error and the CTA still frees its tensor memory.
@@ -29,7 +36,7 @@
 
 #include "common.cuh"
 
-#if SB_HEAD_DIM == 64 || SB_HEAD_DIM == 128
+#if SB_HEAD_DIM == 64 || SB_HEAD_DIM == 128 || SB_HEAD_DIM == 256
 
 using namespace sb;
 typedef __nv_bfloat16 bf16;
@@ -38,18 +45,20 @@ namespace {
 
 constexpr int D = SB_HEAD_DIM;
 constexpr int KA = D / 64;            // 128-byte swizzle atoms (64 elements) per operand row
+constexpr bool SHARED = D == 256;     // keys are the values (latent attention): one load a tile serves both products
 constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;
 constexpr int BM = 128;              // rows per CTA
 constexpr int BN = 64;               // keys per tile (one 128-byte row of probabilities: one k-block of P)
 constexpr int NS = 3;                // key/value stages
+constexpr int NP = 2;                // buffers of probabilities
 constexpr int BT_CACHE = 1024;       // block-table entries kept in shared memory
 constexpr int THREADS = 192;
-constexpr uint32_t TMEM_COLS = 256;  // S0, S1 (BN columns each), O (64), rounded up to a power of two; two CTAs share an SM
+constexpr uint32_t TMEM_COLS = D == 256 ? 512 : 256;  // S0, S1 (BN columns each), O (D), rounded up to a power of two
 constexpr unsigned WAIT_LIMIT = 1u << 26;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int Q_BYTES = BM * D * 2, KV_BYTES = BN * D * 2, P_BYTES = BM * BN * 2;
-constexpr int TILE_BYTES = Q_BYTES + 2 * NS * KV_BYTES + 2 * P_BYTES;  // 96 KB at head_dim 64, 160 KB at 128
-constexpr int SMEM_BYTES = TILE_BYTES + 256 + BT_CACHE * 4;             // + barriers + table entries; two CTAs fit an SM
+constexpr int TILE_BYTES = Q_BYTES + (SHARED ? 1 : 2) * NS * KV_BYTES + NP * P_BYTES;  // 96, 160 and 192 KB at head_dim 64, 128 and 256
+constexpr int SMEM_BYTES = TILE_BYTES + 256 + BT_CACHE * 4;             // + barriers + table entries; two CTAs fit an SM at head_dim 64
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
@@ -156,6 +165,8 @@ struct TcParams {
   // softmax's denominator once per row (no key, no value).
   float softcap_in, cap_over_scale;
   const float* sinks;
+  int window, keep;     // window > 0: a query sees the last ``window`` keys up to its own and the sequence's first ``keep``
+  int deep_group;       // requests of at most 16 rows with this many query heads a kv head are the deep shape's
 };
 
 // tanh on the special-function unit, as the exponentials (relative error about 2^-11)
@@ -177,7 +188,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   const int G = p.G;
   const int M = qn * G;
   // (a block with nothing to do still waits for the kernel before this one: see attention_deep_kernel)
-  if (M <= 16) { pdl_wait(); return; }                  // the deep shape takes this request
+  if (qn * p.deep_group <= 16) { pdl_wait(); return; }                  // the deep shape takes this request
   const int tok_per_tile = BM / G;
   const int n_mtiles = (qn + tok_per_tile - 1) / tok_per_tile;
   if (bx >= n_mtiles) { pdl_wait(); return; }
@@ -187,7 +198,13 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   const int p0 = L - qn;                                // position of the request's first query
   const int tok_last = min(tok0 + tok_per_tile, qn) - 1;
   const int hi = p0 + tok_last + 1;                     // keys [0, hi) are seen by some row of the tile
-  const int n_tiles = (hi + BN - 1) / BN;
+  // The tiles of keys to walk: all of them, or, behind a window, the n_kept tiles of the kept first keys and then those from
+  // the window of the first row on. Step j reads the keys from key_of(j) on.
+  const int behind = p.window > 0 ? max(0, p0 + tok0 - p.window + 1) / BN : 0;
+  const int n_kept = p.window > 0 ? min((p.keep + BN - 1) / BN, behind) : 0;
+  const int skipped = behind - n_kept;
+  const int n_tiles = (hi + BN - 1) / BN - skipped;
+  auto key_of = [&](int j) { return (j < n_kept ? j : j + skipped) * BN; };
 
   // all shared memory is dynamic, so that the tiles start at the CTA's (1024-byte aligned) window base: the
   // 128-byte swizzle needs that alignment, and a padded request would not let two CTAs share an SM
@@ -195,16 +212,16 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   unsigned char* base = smem;
   unsigned char* Qs = base;
   unsigned char* Ks = Qs + Q_BYTES;                     // NS stages
-  unsigned char* Vs = Ks + NS * KV_BYTES;               // NS stages
-  unsigned char* Ps = Vs + NS * KV_BYTES;               // 2 buffers of [128 rows][128 bytes]
+  unsigned char* Vs = SHARED ? Ks : Ks + NS * KV_BYTES; // NS stages
+  unsigned char* Ps = Vs + NS * KV_BYTES;               // NP buffers of [128 rows][128 bytes]
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + TILE_BYTES);
   uint64_t& q_full = bars[0];
   uint64_t* kv_full = bars + 1;                         // NS: a stage's keys and values have landed
   uint64_t* kv_empty = bars + 1 + NS;                   // NS: the products that read the stage have finished
   uint64_t* s_full = bars + 1 + 2 * NS;                 // 2: a score buffer is complete
   uint64_t* s_empty = bars + 3 + 2 * NS;                // 2: the softmax threads hold it in registers
-  uint64_t* p_full = bars + 5 + 2 * NS;                 // 2: a buffer of probabilities is written
-  uint64_t* p_empty = bars + 7 + 2 * NS;                // 2: the second product that read it has finished
+  uint64_t* p_full = bars + 5 + 2 * NS;                 // NP: a buffer of probabilities is written
+  uint64_t* p_empty = bars + 7 + 2 * NS;                // NP: the second product that read it has finished
   uint32_t& tmem_base_s = *reinterpret_cast<uint32_t*>(bars + 9 + 2 * NS);
   int* bt_s = reinterpret_cast<int*>(base + TILE_BYTES + 256);
   if ((smem_u32(base) & 1023u) != 0) {                  // never seen; refuse rather than compute with a wrong swizzle
@@ -261,17 +278,18 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % NS;
         if (!mbar_wait(&kv_empty[s], ((j / NS) & 1) ^ 1)) { failed = true; break; }
-        const int kt = j * BN, blk0 = j * pages_per_tile;   // pages tile the stage: no division in this thread's loop
+        const int kt = key_of(j), blk0 = (kt / BN) * pages_per_tile;   // pages tile the stage: no division in this thread's loop
+        if (big_pages && j == n_kept && skipped > 0) { big_blk = kt / p.ps; big_at = kt - big_blk * p.ps; }
         if (big_pages) {
           const bool there = kt < hi && big_blk < p.bt_width;
-          mbar_expect_tx(&kv_full[s], there ? (unsigned)(BN * D * 2 * 2) : 0u);
+          mbar_expect_tx(&kv_full[s], there ? (unsigned)(BN * D * 2 * (SHARED ? 1 : 2)) : 0u);
           if (there) {
             const int page = bt[big_blk];
 #pragma unroll
             for (int a = 0; a < KA; ++a) {
               const size_t off = (size_t)s * KV_BYTES + (size_t)a * BN * 128;
               tma_load_4d(Ks + off, &map_k, &kv_full[s], a * 64, big_at, hk, page);
-              tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, big_at, hk, page);
+              if (!SHARED) tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, big_at, hk, page);
             }
           }
           big_at += BN;
@@ -281,15 +299,15 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
         int n_pages = 0;
         for (int i = 0; i < pages_per_tile; ++i)
           if (kt + i * p.ps < hi && blk0 + i < p.bt_width) ++n_pages;
-        mbar_expect_tx(&kv_full[s], (unsigned)(n_pages * p.ps * D * 2 * 2));
+        mbar_expect_tx(&kv_full[s], (unsigned)(n_pages * p.ps * D * 2 * (SHARED ? 1 : 2)));
         for (int i = 0; i < n_pages; ++i) {
-          const int page = bt[blk0 + i];
+          const int page = bt[blk0 + i];                  // (-1, a page the window has passed: outside the map, zeros)
 #pragma unroll
           for (int a = 0; a < KA; ++a) {
             // atom a of a stage: 64 keys x 128 bytes; the page's keys at their rows of it
             const size_t off = (size_t)s * KV_BYTES + (size_t)a * BN * 128 + (size_t)i * p.ps * 128;
             tma_load_4d(Ks + off, &map_k, &kv_full[s], a * 64, 0, hk, page);
-            tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, 0, hk, page);
+            if (!SHARED) tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, 0, hk, page);
           }
         }
       }
@@ -316,7 +334,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
         tc_fence_after();
         issue_s(0);
         for (int j = 0; j < n_tiles; ++j) {
-          const int b = j & 1;
+          const int b = j % NP;
           if (j + 1 < n_tiles) {
             // the next tile's scores, as soon as its keys are there and its score buffer has been read
             const int t = j + 1;
@@ -324,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
             tc_fence_after();
             issue_s(t);
           }
-          if (!mbar_wait(&p_full[b], (j >> 1) & 1)) { failed = true; break; }
+          if (!mbar_wait(&p_full[b], (j / NP) & 1)) { failed = true; break; }
           tc_fence_after();
           // O += P V: P is K-major (one block of 64 keys); V is MN-major, 16 keys = 2048 bytes further per step
           const uint32_t pa = smem_u32(Ps + (size_t)b * P_BYTES), va = smem_u32(Vs + (size_t)(j % NS) * KV_BYTES);
@@ -354,10 +372,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
     const int first_pos = p0 + tok0;                     // smallest position of the tile's rows
 
     for (int j = 0; j < n_tiles && !failed; ++j) {
-      const int b = j & 1, kt = j * BN;
+      const int b = j & 1, kt = key_of(j);
       if (!mbar_wait(&s_full[b], (j >> 1) & 1)) { failed = true; break; }
       tc_fence_after();
-      const bool masked = kt + BN - 1 > first_pos;       // the tile reaches beyond what the first row may see
+      // the tile reaches beyond what the first row may see, or behind the last row's window
+      const bool masked = kt + BN - 1 > first_pos || (p.window > 0 && kt <= p0 + tok_last - p.window);
       float sv[BN];
 #pragma unroll
       for (int c = 0; c < BN / 32; ++c) tc_load32(lane_addr + (uint32_t)(b * BN + c * 32), sv + c * 32);
@@ -372,6 +391,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       if (masked) {
 #pragma unroll
         for (int i = 0; i < BN; ++i) sv[i] = (kt + i <= pos) ? sv[i] : -INFINITY;
+        if (p.window > 0) {
+          const int from = pos - p.window + 1;            // the row's first key, the kept ones aside
+#pragma unroll
+          for (int i = 0; i < BN; ++i) sv[i] = (kt + i >= from || kt + i < p.keep) ? sv[i] : -INFINITY;
+        }
       }
       float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
 #pragma unroll
@@ -383,29 +407,29 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       const bool moved = m_tile > m_ref + 8.0f;           // false for m_tile = -inf; true for m_ref = -inf, m_tile finite
       if (__any_sync(0xffffffffu, moved && m_ref != -INFINITY)) {
         // rare: rescale the accumulator in tensor memory, once the products issued so far (up to tile j-1) are done
-        const int pb = (j - 1) & 1;
-        if (!mbar_wait(&p_empty[pb], ((j - 1) >> 1) & 1)) { failed = true; break; }
+        if (!mbar_wait(&p_empty[(j - 1) % NP], ((j - 1) / NP) & 1)) { failed = true; break; }
         tc_fence_after();
         const float f = (moved && m_ref != -INFINITY) ? ex2(m_ref - m_tile) : 1.f;
-        float ov[D];
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          float ov[32];
+          tc_load32(o_addr + (uint32_t)(c * 32), ov);
+          tc_wait_ld();
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) tc_load32(o_addr + (uint32_t)(c * 32), ov + c * 32);
-        tc_wait_ld();
-#pragma unroll
-        for (int i = 0; i < D; ++i) ov[i] *= f;
-#pragma unroll
-        for (int c = 0; c < D / 32; ++c) tc_store32(o_addr + (uint32_t)(c * 32), ov + c * 32);
+          for (int i = 0; i < 32; ++i) ov[i] *= f;
+          tc_store32(o_addr + (uint32_t)(c * 32), ov);
+        }
         tc_wait_st();
         l_run *= f;
       }
       if (moved) m_ref = m_tile;                         // (with no reference yet, accumulator and sum are still zero)
       const float use = (m_ref == -INFINITY) ? 0.f : m_ref;
-      // the buffer of probabilities must have been read by the product of two tiles ago
-      if (j >= 2 && !mbar_wait(&p_empty[b], ((j - 2) >> 1) & 1)) { failed = true; break; }
+      // the buffer of probabilities must have been read by the product of NP tiles ago
+      if (j >= NP && !mbar_wait(&p_empty[j % NP], ((j - NP) / NP) & 1)) { failed = true; break; }
       // probabilities -> shared memory (bfloat16, the swizzled K-major layout of the second product);
       // ex2(-inf) = 0 takes care of masked entries
       float sum0 = 0.f, sum1 = 0.f;
-      unsigned char* prow = Ps + (size_t)b * P_BYTES + (size_t)row * 128;
+      unsigned char* prow = Ps + (size_t)(j % NP) * P_BYTES + (size_t)row * 128;
 #pragma unroll
       for (int c = 0; c < BN / 8; ++c) {                 // 16-byte pieces of 8 keys
         uint32_t pk[4];
@@ -435,12 +459,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       tc_fence_before();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[b]);
+      if (lane == 0) mbar_arrive(&p_full[j % NP]);
     }
     if (!failed) {
       // all products have finished when the last one has
-      const int pb = (n_tiles - 1) & 1;
-      if (!mbar_wait(&p_empty[pb], ((n_tiles - 1) >> 1) & 1)) failed = true;
+      if (!mbar_wait(&p_empty[(n_tiles - 1) % NP], ((n_tiles - 1) / NP) & 1)) failed = true;
       tc_fence_after();
       if (!failed) {
         if (p.sinks != nullptr && row_ok) {
@@ -450,17 +473,20 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
           l_run += (m_ref == -INFINITY) ? 1.f : exp2f(sk - m_ref);
         }
         const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        float ov[D];
+        bf16* dst = p.out + (size_t)(q0 + tok) * p.H * D + (size_t)head * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 64; ++c) {
+          float ov[64];
+          tc_load32(o_addr + (uint32_t)(c * 64), ov);
+          tc_load32(o_addr + (uint32_t)(c * 64 + 32), ov + 32);
+          tc_wait_ld();
+          if (row_ok) {
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) tc_load32(o_addr + (uint32_t)(c * 32), ov + c * 32);
-        tc_wait_ld();
-        if (row_ok) {
-          bf16* dst = p.out + (size_t)(q0 + tok) * p.H * D + (size_t)head * D;
-#pragma unroll
-          for (int i = 0; i < D / 8; ++i)
-            *reinterpret_cast<uint4*>(dst + i * 8) =
-                make_uint4(pack_bf16(ov[8 * i] * inv, ov[8 * i + 1] * inv), pack_bf16(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv),
-                           pack_bf16(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv), pack_bf16(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv));
+            for (int i = 0; i < 8; ++i)
+              *reinterpret_cast<uint4*>(dst + c * 64 + i * 8) =
+                  make_uint4(pack_bf16(ov[8 * i] * inv, ov[8 * i + 1] * inv), pack_bf16(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv),
+                             pack_bf16(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv), pack_bf16(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv));
+          }
         }
       }
     }
@@ -495,14 +521,14 @@ int encode4(CUtensorMap* map, const void* basep, const cuuint64_t dims[4], const
 
 }  // namespace
 
-// 1 if sb_attention_tc takes this geometry (else the caller uses the mma.sync kernel).
-SB_EXPORT int sb_attention_tc_supports(int H, int Hkv, int ps, int window, int q_stride) {
+// 1 if sb_attention_tc takes this geometry (else the caller uses the mma.sync kernel). shared: keys and values are one tensor.
+SB_EXPORT int sb_attention_tc_supports(int H, int Hkv, int ps, int shared, int q_stride) {
   if (H <= 0 || Hkv <= 0 || H % Hkv) return 0;
   const int G = H / Hkv;
   if (G > 128) return 0;                                // a tile holds whole tokens: 128 / G of them (rows beyond stay unused)
   if (ps < 8) return 0;
   if (ps <= BN ? (BN % ps) != 0 : ((ps % BN) != 0 || ps > 256)) return 0;   // pages tile a stage of keys (in whole swizzle atoms), or stages tile a page
-  if (window > 0) return 0;
+  if (SHARED && !shared) return 0;
   if (q_stride % 8) return 0;
   return 1;
 }
@@ -510,13 +536,13 @@ SB_EXPORT int sb_attention_tc_supports(int H, int Hkv, int ps, int window, int q
 // The wide shape of sb_attention_mma (requests with more than 16 rows) on tcgen05; arguments as there.
 // n_tokens: rows of qkv; num_pages: pages of kc / vc. rows (may be null): the n_rows requests to cover, so that a
 // step of hundreds of decoding requests and a few prompt portions launches blocks for the portions only.
-// softcap (0: none) and sinks (float [H] or null): see TcParams.
+// softcap (0: none), sinks (float [H] or null), window (0: none), keep and deep_group: see TcParams.
 SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, const void* kc, const void* vc, const int* block_table,
                                    int bt_width, const int* cu_q, const int* kv_len, int H, int Hkv, int ps, int num_pages, float scale,
                                    void* out, int n_rows, int max_q, const int* rows, int* error, float softcap, const float* sinks,
-                                   cudaStream_t stream) {
+                                   int window, int keep, int deep_group, cudaStream_t stream) {
   if (n_rows <= 0 || max_q <= 0) return 0;
-  if (!sb_attention_tc_supports(H, Hkv, ps, 0, q_stride)) return SB_ERR_SHAPE;
+  if (!sb_attention_tc_supports(H, Hkv, ps, kc == vc, q_stride) || window < 0 || keep < 0 || deep_group <= 0) return SB_ERR_SHAPE;
   if (Hkv > 65535 || n_rows > 65535) return SB_ERR_LIMIT;
   if (!aligned16(qkv) || !aligned16(kc) || !aligned16(vc) || !aligned16(out) || !error) return SB_ERR_ALIGN;
   const int G = H / Hkv;
@@ -541,6 +567,7 @@ SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, 
   p.block_table = block_table; p.bt_width = bt_width; p.cu_q = cu_q; p.kv_len = kv_len;
   p.H = H; p.Hkv = Hkv; p.G = G; p.ps = ps; p.scale_log2 = scale * LOG2E; p.out = (bf16*)out; p.error = error; p.rows = rows;
   p.softcap_in = softcap > 0.f ? scale / softcap : 0.f; p.cap_over_scale = softcap > 0.f ? softcap / scale : 0.f; p.sinks = sinks;
+  p.window = window; p.keep = window > 0 ? keep : 0; p.deep_group = deep_group;
   const int tok_per_tile = BM / G;
   const int m_tiles = (max_q + tok_per_tile - 1) / tok_per_tile;
   auto k = attention_tc_kernel;
@@ -555,7 +582,7 @@ SB_EXPORT int sb_attention_tc(const void* qkv, int q_stride, int n_tokens, const
                               int bt_width, const int* cu_q, const int* kv_len, int H, int Hkv, int ps, int num_pages, float scale,
                               void* out, int n_rows, int max_q, const int* rows, int* error, cudaStream_t stream) {
   return sb_attention_tc_opts(qkv, q_stride, n_tokens, kc, vc, block_table, bt_width, cu_q, kv_len, H, Hkv, ps, num_pages, scale, out,
-                              n_rows, max_q, rows, error, 0.f, nullptr, stream);
+                              n_rows, max_q, rows, error, 0.f, nullptr, 0, 0, H / Hkv, stream);
 }
 
 #else

@@ -716,7 +716,7 @@ class CudaKernels:
         # that each count as a kv head reading the same rows. A decoding request is then several (request, kv head) pairs of
         # few rows, which the deep shape spreads over the SMs with its key splits; as one pair of 32 rows it would be a single
         # block of the wide shape walking all keys alone. For prompt portions the grouping changes neither work nor traffic.
-        kv_div = 1
+        kv_div, all_kv_heads = 1, kv_heads
         if k_cache is v_cache:
             # (a step of single tokens takes smaller groups: measured at batch 8 after 2,048 tokens, groups of 4 against 8 give
             # 29 against 38 us a launch with 8 heads and 31 against 39 us with 16)
@@ -751,15 +751,18 @@ class CudaKernels:
             if num_splits > 1:
                 scratch = self._scratch_buffer(lib, shape.rows, kv_heads, num_splits)
                 tickets = self._ticket_buffer(shape.rows * kv_heads)
-        by_distance = slopes is not None or chunk > 0 or softcap > 0.0 or sinks is not None
-        if (which & 1) and slopes is None and not chunk and not keep_first and kv_div == 1 and self.use_tcgen05_attention and self._tc_attention_takes(lib, heads, kv_heads, head_dim, page_size, window, qkv.shape[1]):
+        # Behind a window the tensor-memory kernel walks the window's tiles and those of the kept first keys; a cap behind a window, which
+        # no design has, stays with the exact tanh of the mma.sync kernel. 2,048 tokens, window 1,024: 95 -> 38 us at head size 128, and
+        # 172 -> 52 us for shared rows of 256, all heads of a token in one tile (any grouping of them there would load the rows again).
+        if ((which & 1) and slopes is None and not chunk and not (window and softcap > 0.0) and self.use_tcgen05_attention
+                and self._tc_attention_takes(lib, heads, all_kv_heads, head_dim, page_size, k_cache is v_cache, qkv.stride(0))):
             # prompt portions on the tensor-memory path; what is left (decoding rows) goes to the deep shape below
             self.launches += 1
             _check(lib.sb_attention_tc_opts(
-                _p(qkv), qkv.shape[1], qkv.shape[0], _p(k_cache), _p(v_cache), _p(block_table), block_table.shape[1], _p(cu_q),
-                _p(kv_len), heads, kv_heads, page_size, k_cache.shape[0], ctypes.c_float(scale), _p(out),
+                _p(qkv), qkv.stride(0), qkv.shape[0], _p(k_cache), _p(v_cache), _p(block_table), block_table.shape[1], _p(cu_q),
+                _p(kv_len), heads, all_kv_heads, page_size, k_cache.shape[0], ctypes.c_float(scale), _p(out),
                 n_wide if wide_rows is not None else shape.rows, shape.max_q, _p(wide_rows), self._wait_flag(),
-                ctypes.c_float(softcap), _p(sinks), self._s()), "tcgen05 attention")
+                ctypes.c_float(softcap), _p(sinks), int(window or 0), keep_first, group, self._s()), "tcgen05 attention")
             which &= ~1
             if not which:
                 return
@@ -818,11 +821,11 @@ class CudaKernels:
                 _p(wide_rows), n_wide, n_splits, _p(part), _p(tickets), t, self._wait_flag(), 1 if self.use_tcgen05_attention else 0, _DT[q.dtype],
                 self._s()), "attention with mixed heads")
 
-    def _tc_attention_takes(self, lib, heads, kv_heads, head_dim, page_size, window, stride) -> bool:
-        key = (heads, kv_heads, head_dim, page_size, window, stride)
+    def _tc_attention_takes(self, lib, heads, kv_heads, head_dim, page_size, shared, stride) -> bool:
+        key = (heads, kv_heads, head_dim, page_size, shared, stride)
         ok = self._tc_attention_ok.get(key)
         if ok is None:
-            ok = self._tc_attention_ok[key] = bool(lib.sb_attention_tc_supports(heads, kv_heads, page_size, window, stride))
+            ok = self._tc_attention_ok[key] = bool(lib.sb_attention_tc_supports(heads, kv_heads, page_size, 1 if shared else 0, stride))
         return ok
 
     def _scratch_buffer(self, lib, rows: int, kv_heads: int, num_splits: int) -> torch.Tensor:

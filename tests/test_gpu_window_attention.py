@@ -1,0 +1,58 @@
+"""Prompt portions on the tensor-memory attention behind a window (with kept first keys and a sink), and over one cached row for all
+heads: against the mma.sync kernel's neighbourhood of the torch version, with given-back pages missing and unwritten rows poisoned."""
+import math
+
+import pytest
+import torch
+
+from tests.test_gpu_kernels import DEV, E, K, _paged_setup  # noqa: F401  (K: the fixture)
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # heads, kv, page, q_lens, kv_lens, window, keep
+    (4, 1, 64, [300], [300], 64, 0),                       # a window of one tile
+    (4, 1, 64, [300], [300], 100, 4),
+    (8, 2, 16, [130, 1, 40], [400, 700, 333], 50, 20),     # small pages: kept and passed ones in one tile
+    (8, 8, 32, [65, 17], [600, 17], 129, 70),              # kept keys over two tiles
+    (16, 4, 128, [257], [1000], 200, 4),                   # pages of two tiles
+    (12, 3, 256, [70, 300], [900, 300], 65, 130),          # pages of four tiles
+    (6, 2, 64, [200], [200], 1024, 4),                     # a window longer than the sequence
+    (16, 1, 64, [70, 2, 1], [333, 500, 90], 90, 0),        # a portion of two tokens beside a decoded one
+    (4, 2, 8, [33], [201], 1, 1),                          # a query that sees itself and the first key
+]
+
+
+@pytest.mark.parametrize("d,shared", [(64, False), (128, False), (128, True), (256, True)])
+@pytest.mark.parametrize("case", CASES, ids=[f"h{c[0]}kv{c[1]}p{c[2]}w{c[5]}k{c[6]}" for c in CASES])
+def test_window_on_the_tensor_memory_path(K, case, d, shared):  # noqa: F811
+    heads, kv_heads, page, q_lens, kv_lens, window, keep = case
+    if shared:
+        kv_heads = 1
+    s = _paged_setup("bfloat16", heads, kv_heads, d, page, q_lens, kv_lens)
+    assert K._attention_lib(d).sb_attention_tc_supports(heads, kv_heads, page, 1 if shared else 0, s["qkv"].stride(0)) == 1
+    if shared:
+        s["vc"] = s["kc"]
+    for r, (n, L) in enumerate(zip(q_lens, kv_lens)):
+        b = (L - 1) // page
+        if L % page:                                       # rows of the last page beyond the sequence
+            s["kc"][int(s["bt"][r, b]), :, L % page:] = float("nan")
+            s["vc"][int(s["bt"][r, b]), :, L % page:] = float("nan")
+        for blk in range(-(-keep // page), max(0, L - n - window + 1) // page):      # pages the window has passed: given back, reused
+            s["kc"][int(s["bt"][r, blk])] = float("nan")
+            s["vc"][int(s["bt"][r, blk])] = float("nan")
+            s["bt"][r, blk] = -1
+    sinks = torch.randn(heads, device=DEV)
+    scale = 1.0 / math.sqrt(d)
+    t = sum(q_lens)
+    out = torch.full((t, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    want = torch.empty_like(out)
+    args = (s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, scale, window)
+    K.attention(s["qkv"], *args, out, s["shape"], sinks=sinks, keep_first=keep)
+    K.check_errors()
+    E.attention(s["qkv"], *args, want, s["shape"], sinks=sinks, keep_first=keep)
+    assert bool(torch.isfinite(out).all()), "a row was not written, or NaN"
+    # probabilities are rounded to bfloat16 (2^-8 of each): a sum of p v moves by 2^-8 of sum p |v|, at most 2^-8 max |v|; plus the output's
+    # own rounding on both sides
+    top = float(torch.nan_to_num(s["vc"].float(), 0.0).abs().max())
+    torch.testing.assert_close(out.float(), want.float(), atol=2.0 ** -8 * top, rtol=2.0 ** -7)
