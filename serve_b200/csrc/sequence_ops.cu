@@ -8,6 +8,7 @@
 // are float [max_slots, ...] and are zero when a slot is handed out, so "zeros before the start" needs no
 // special case: a request's first portion reads the zeros, every later portion what the one before left.
 // Everything that enters a recurrence is float, in both dtypes; activations read and written are T.
+#include "chunked_recurrence.h"
 #include "common.cuh"
 
 using namespace sb;
@@ -186,6 +187,7 @@ struct RecArgs {
   int rot_dims;
   float k_scale;
   const int* token_row; int max_walk;                // max_walk > 0: rows that bring more tokens are left to other kernels
+  int prepare_all;                                   // (which read what the first kernel makes of their tokens too)
   float rate_scale;                                  // GLA: the exponent of the sigmoid (one over the temperature)
   // float work space, made by the first kernel: qf, kf [T, Hqk, dkp]; af [T, H, dkp] (DELTA, WKV, GLA); vf [T, H, dvp]; sc, dec [T, H]
   float *qf, *kf, *af, *vf, *sc, *dec;
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(REC_THREADS) recurrence_prep_kernel(RecArgs a)
   const long long wid = (long long)blockIdx.x * (REC_THREADS / 32) + (threadIdx.x >> 5);
   if (wid >= (long long)a.n_tokens * heads) return;      // (a whole warp leaves together; nothing below waits for the block)
   const int t = (int)(wid / heads), h = (int)(wid - (long long)t * heads), tid = threadIdx.x & 31;
-  if (a.max_walk > 0) {
+  if (a.max_walk > 0 && !a.prepare_all) {
     const int r = a.token_row[t];
     if (a.cu_q[r + 1] - a.cu_q[r] > a.max_walk) return;
   }
@@ -459,8 +461,16 @@ static inline long long rec_work_floats(int mode, int n_tokens, int H, int Hqk, 
   return (long long)n_tokens * ((long long)2 * Hqk * dkp + ((mode == MODE_DELTA || mode == MODE_WKV || mode == MODE_GLA) ? (long long)H * dkp : 0) + (long long)H * dvp + 2 * H) + 16;
 }
 
+// Requests of more than a.max_walk tokens go through the kernels of chunked_recurrence.cu if there is work space for them.
+struct Chunked {
+  const int* rows;             // the requests by falling number of tokens, or null; n_list of them are looked at
+  int n_list, max_q, chunks;
+  float* work;                 // null: every request is walked
+  int walk_too;                // some requests are short
+};
+
 template <typename T, int MODE>
-int launch_recurrence(RecArgs a, float* work, int n_rows, cudaStream_t stream) {
+int launch_recurrence(RecArgs a, float* work, int n_rows, const Chunked& ch, cudaStream_t stream) {
   const int P = rec_lanes(a.dk);
   if (P > 32) return SB_ERR_LIMIT;
   a.P = P;
@@ -478,8 +488,21 @@ int launch_recurrence(RecArgs a, float* work, int n_rows, cudaStream_t stream) {
   const long long prep_warps = (long long)a.n_tokens * (a.H > a.Hqk ? a.H : a.Hqk);
   const long long prep_blocks = (prep_warps + REC_THREADS / 32 - 1) / (REC_THREADS / 32);
   if (prep_blocks > 0x7fffffffLL) return SB_ERR_LIMIT;
+  a.prepare_all = ch.work != nullptr;
   recurrence_prep_kernel<T, MODE><<<(unsigned)prep_blocks, REC_THREADS, 0, stream>>>(a);
   SB_LAUNCH_CHECK();
+  if (ch.work) {
+    SbChunkedWalk c = {};
+    c.qf = a.qf; c.kf = a.kf; c.af = a.af; c.vf = a.vf; c.sc = a.sc; c.dec = a.dec;
+    c.n_tokens = a.n_tokens; c.H = a.H; c.Hqk = a.Hqk; c.dk = a.dk; c.dv = a.dv; c.dkp = a.dkp; c.dvp = a.dvp;
+    c.mode = MODE; c.head_rate = MODE == MODE_DELTA && a.rate_per_head;
+    c.skip = a.d_skip; c.skip_dtype = a.par_dtype;
+    c.state = a.state; c.state_stride = a.state_stride; c.slots = a.slots; c.cu_q = a.cu_q;
+    c.rows = ch.rows; c.n_list = ch.n_list; c.max_q = ch.max_q; c.min_tokens = a.max_walk;
+    c.out = a.out; c.out_stride = a.out_stride; c.work = ch.work;
+    const int rc = sb_chunked_walk(c, ch.chunks, stream);
+    if (rc || !ch.walk_too) return rc;
+  }
   const int per_tok = ((MODE == MODE_DELTA || MODE == MODE_WKV || MODE == MODE_GLA) ? 3 : 2) * a.dkp + VC;
   const size_t smem = (size_t)2 * (REC_TS * per_tok + 2 * REC_TS) * sizeof(float);
   dim3 grid(a.dvp / VC, a.H, n_rows);
@@ -776,6 +799,13 @@ SB_EXPORT int sb_causal_conv(const void* x, int x_stride, const void* w, const v
 }
 
 // Floats of work space sb_linear_recurrence needs for a step of n_tokens tokens.
+// Floats of chunk_work, or -1 if requests of these sizes are walked.
+SB_EXPORT long long sb_linear_recurrence_chunk_floats(int mode, int n_tokens, int chunks, int H, int dk, int dv) {
+  if (dk <= 0 || dk > 128 || dv <= 0) return -1;
+  const int VC = REC_THREADS / rec_lanes(dk);
+  return sb_chunked_walk_floats(mode, n_tokens, chunks, H, dk, (dv + VC - 1) / VC * VC);
+}
+
 SB_EXPORT long long sb_linear_recurrence_work_floats(int mode, int n_tokens, int H, int Hqk, int dk, int dv) {
   if (dk <= 0 || dk > 32 * REC_RPT) return -1;
   return rec_work_floats(mode, n_tokens, H, Hqk, dk, dv);
@@ -785,7 +815,9 @@ SB_EXPORT long long sb_linear_recurrence_work_floats(int mode, int n_tokens, int
 // rate per row of the state or, with rate_per_head, per head; 3: decay per key channel with a bonus [H, dk] for the
 // current token, read out before the update; 4: decay per key channel, read out after it; 5: fixed decay per head on q, k, v as
 // projected, q and k rotated by ``positions`` and ``inv_freq``, k times k_scale). With max_walk > 0 (and token_row) rows that bring
-// more tokens are passed over. See RecArgs for what each pointer is; unused ones are null. ``rate`` has a
+// more tokens are passed over, or, with chunk_work (16-byte aligned, sb_linear_recurrence_chunk_floats for ``chunks``, the sum of their
+// tokens / 32, each rounded up), run 32 tokens at a time; rows (or null), n_list, max_q: the requests to look at for that; walk_too: some
+// have at most max_walk tokens. See RecArgs for what each pointer is; unused ones are null. ``rate`` has a
 // dtype of its own (rate_dtype). out is float [T, H * dv]; work: 16-byte aligned floats,
 // as many as sb_linear_recurrence_work_floats says.
 SB_EXPORT int sb_linear_recurrence(int mode, const void* q, int q_stride, const void* k, int k_stride, const void* v, int v_stride,
@@ -794,7 +826,7 @@ SB_EXPORT int sb_linear_recurrence(int mode, const void* q, int q_stride, const 
                                    const int* slots, const int* cu_q, float* out, int out_stride, int H, int Hqk, int dk, int dv,
                                    float q_scale, int n_rows, int n_tokens, float* work, long long state_stride, int dtype, float rate_scale,
                                    const int* positions, const float* inv_freq, int rot_dims, float k_scale, const int* token_row, int max_walk,
-                                   cudaStream_t stream) {
+                                   const int* rows, int n_list, int max_q, int chunks, float* chunk_work, int walk_too, cudaStream_t stream) {
   if (n_rows <= 0 || n_tokens <= 0) return 0;
   if (!work || !aligned16(work)) return SB_ERR_ALIGN;
   if (H <= 0 || Hqk <= 0 || H % Hqk || dk <= 0 || dv <= 0) return SB_ERR_SHAPE;
@@ -810,22 +842,23 @@ SB_EXPORT int sb_linear_recurrence(int mode, const void* q, int q_stride, const 
   a.a_log = a_log; a.dt_bias = dt_bias; a.d_skip = d_skip; a.par_dtype = par_dtype; a.state = state; a.state_stride = state_stride; a.slots = slots; a.cu_q = cu_q;
   a.out = out; a.out_stride = out_stride; a.H = H; a.Hqk = Hqk; a.dk = dk; a.dv = dv; a.P = 1; a.dkp = a.dvp = 0; a.n_tokens = n_tokens;
   a.positions = positions; a.inv_freq = inv_freq; a.rot_dims = rot_dims; a.k_scale = k_scale;
-  a.token_row = token_row; a.max_walk = token_row ? max_walk : 0;
+  a.token_row = token_row; a.max_walk = token_row ? max_walk : 0; a.prepare_all = 0;
   a.q_scale = q_scale; a.rate_scale = rate_scale; a.qf = a.kf = a.af = a.vf = a.sc = a.dec = nullptr;
+  const Chunked ch = {rows, n_list, max_q, chunks, a.max_walk > 0 ? chunk_work : nullptr, walk_too};
   if (dtype == SB_DTYPE_F32) {
-    if (mode == MODE_DECAY) return launch_recurrence<float, MODE_DECAY>(a, work, n_rows, stream);
-    if (mode == MODE_SSM) return launch_recurrence<float, MODE_SSM>(a, work, n_rows, stream);
-    if (mode == MODE_DELTA) return launch_recurrence<float, MODE_DELTA>(a, work, n_rows, stream);
-    if (mode == MODE_WKV) return launch_recurrence<float, MODE_WKV>(a, work, n_rows, stream);
-    if (mode == MODE_GLA) return launch_recurrence<float, MODE_GLA>(a, work, n_rows, stream);
-    if (mode == MODE_RET) return launch_recurrence<float, MODE_RET>(a, work, n_rows, stream);
+    if (mode == MODE_DECAY) return launch_recurrence<float, MODE_DECAY>(a, work, n_rows, ch, stream);
+    if (mode == MODE_SSM) return launch_recurrence<float, MODE_SSM>(a, work, n_rows, ch, stream);
+    if (mode == MODE_DELTA) return launch_recurrence<float, MODE_DELTA>(a, work, n_rows, ch, stream);
+    if (mode == MODE_WKV) return launch_recurrence<float, MODE_WKV>(a, work, n_rows, ch, stream);
+    if (mode == MODE_GLA) return launch_recurrence<float, MODE_GLA>(a, work, n_rows, ch, stream);
+    if (mode == MODE_RET) return launch_recurrence<float, MODE_RET>(a, work, n_rows, ch, stream);
   } else if (dtype == SB_DTYPE_BF16) {
-    if (mode == MODE_DECAY) return launch_recurrence<__nv_bfloat16, MODE_DECAY>(a, work, n_rows, stream);
-    if (mode == MODE_SSM) return launch_recurrence<__nv_bfloat16, MODE_SSM>(a, work, n_rows, stream);
-    if (mode == MODE_DELTA) return launch_recurrence<__nv_bfloat16, MODE_DELTA>(a, work, n_rows, stream);
-    if (mode == MODE_WKV) return launch_recurrence<__nv_bfloat16, MODE_WKV>(a, work, n_rows, stream);
-    if (mode == MODE_GLA) return launch_recurrence<__nv_bfloat16, MODE_GLA>(a, work, n_rows, stream);
-    if (mode == MODE_RET) return launch_recurrence<__nv_bfloat16, MODE_RET>(a, work, n_rows, stream);
+    if (mode == MODE_DECAY) return launch_recurrence<__nv_bfloat16, MODE_DECAY>(a, work, n_rows, ch, stream);
+    if (mode == MODE_SSM) return launch_recurrence<__nv_bfloat16, MODE_SSM>(a, work, n_rows, ch, stream);
+    if (mode == MODE_DELTA) return launch_recurrence<__nv_bfloat16, MODE_DELTA>(a, work, n_rows, ch, stream);
+    if (mode == MODE_WKV) return launch_recurrence<__nv_bfloat16, MODE_WKV>(a, work, n_rows, ch, stream);
+    if (mode == MODE_GLA) return launch_recurrence<__nv_bfloat16, MODE_GLA>(a, work, n_rows, ch, stream);
+    if (mode == MODE_RET) return launch_recurrence<__nv_bfloat16, MODE_RET>(a, work, n_rows, ch, stream);
   } else {
     return SB_ERR_DTYPE;
   }

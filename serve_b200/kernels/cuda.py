@@ -73,7 +73,7 @@ def core_jobs():
 
 def sequence_job():
     """Kernels of the mixers with recurrent state (built when a model first asks for them)."""
-    return {"name": "sb_seq", "sources": ["sequence_ops.cu", "chunked_retention.cu"]}
+    return {"name": "sb_seq", "sources": ["sequence_ops.cu", "chunked_recurrence.cu", "chunked_retention.cu"]}
 
 
 def experts_job():
@@ -1034,8 +1034,9 @@ class CudaKernels:
         "gla": S = diag(a) S + k v^T, o = S^T (q_scale q), a = sigmoid(rate + dt_bias)^rate_scale per row (rate [T, heads * dk]);
         "retention": S = decay_h S + k v^T on q, k, v as they are, the first rot_dims elements of q and k rotated by the tokens'
         positions (pairs i, i + rot_dims / 2; inv_freq float [rot_dims / 2]), k times k_scale.
-        out: float [T, heads * dv]. In bfloat16, requests that bring more than CHUNKED_FROM tokens run "retention" chunk by chunk on
-        the tensor cores (csrc/chunked_retention.cu), the others token by token."""
+        out: float [T, heads * dv]. Requests that bring more than CHUNKED_FROM tokens run chunk by chunk: "retention" in bfloat16 on the
+        tensor cores (csrc/chunked_retention.cu), states of at most 128 rows otherwise in 32-bit arithmetic (csrc/chunked_recurrence.cu). The
+        others are walked token by token."""
         max_walk = 0
         if mode == "retention" and self._chunked_retention(q, k, v, state, ctx, out, heads, dk, dv, decay, inv_freq, rot_dims, k_scale):
             if getattr(ctx.shape, "min_q", 1) > self.CHUNKED_FROM:
@@ -1050,6 +1051,16 @@ class CudaKernels:
             raise KernelError(f"linear recurrence: a state of {dk} rows is beyond the kernel's 512")
         work = torch.empty(need, dtype=torch.float32, device=q.device)       # what the first kernel leaves for the second
         self.launches += 2
+        shape = ctx.shape
+        rows, n_list, chunks, chunk_work, walk_too = None, shape.rows, 0, None, 1
+        if not max_walk and self.use_chunked_recurrence and shape.max_q > self.CHUNKED_FROM:
+            n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32)
+            lib.sb_linear_recurrence_chunk_floats.restype = ctypes.c_longlong
+            floats = lib.sb_linear_recurrence_chunk_floats(code, q.shape[0], chunks, heads, dk, dv)
+            if 0 < floats <= self.CHUNK_SCRATCH_FLOATS:
+                chunk_work = torch.empty(floats, dtype=torch.float32, device=q.device)
+                max_walk, walk_too = self.CHUNKED_FROM, 1 if getattr(shape, "min_q", 1) <= self.CHUNKED_FROM else 0
+                self.launches += 1 + walk_too
         _check(lib.sb_linear_recurrence(
             code, _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0),
             _p(aux), aux.stride(0) if aux is not None else 0, _p(rate), rate.stride(0) if rate is not None else 0,
@@ -1057,10 +1068,21 @@ class CudaKernels:
             _p(a_log), _p(dt_bias), _p(d_skip), _DT[par.dtype] if par is not None else 0, _p(state), _p(ctx.slots), _p(ctx.cu_q),
             _p(out), out.stride(0), heads, qk_heads, dk, dv, ctypes.c_float(q_scale), ctx.shape.rows, q.shape[0], _p(work),
             ctypes.c_longlong(state.stride(0)), _DT[v.dtype], ctypes.c_float(rate_scale), _p(ctx.positions), _p(inv_freq), int(rot_dims),
-            ctypes.c_float(k_scale), _p(ctx.token_row), max_walk, self._s()), "linear recurrence")
+            ctypes.c_float(k_scale), _p(ctx.token_row), max_walk, _p(rows), n_list, int(shape.max_q), chunks, _p(chunk_work), walk_too,
+            self._s()), "linear recurrence")
 
     # Requests with more tokens than this go through the chunked kernels, where those take the layout.
     CHUNKED_FROM = 32
+    CHUNK_SCRATCH_FLOATS = 1 << 28           # work space of the 32-bit chunked kernels at most (a GB); a larger step is walked
+    use_chunked_recurrence = True            # tests: False keeps every request on the walking kernel
+
+    def _chunk_list(self, shape, tokens: int, size: int):
+        """(entries, the list or None, chunks) of the requests that bring more than CHUNKED_FROM tokens, in chunks of ``size``."""
+        neg_q = getattr(shape, "neg_q_sorted", None)
+        if neg_q is None or getattr(shape, "rows_by_q", None) is None:
+            return shape.rows, None, tokens // size + shape.rows
+        n = bisect.bisect_left(neg_q, -self.CHUNKED_FROM)
+        return n, shape.rows_by_q, sum(-(q // size) for q in neg_q[:n])
     use_chunked_retention = True             # tests: False keeps every request on the walking kernel
 
     def _chunked_retention(self, q, k, v, state, ctx, out, heads, dk, dv, decay, inv_freq, rot_dims, k_scale) -> bool:
@@ -1075,11 +1097,7 @@ class CudaKernels:
             ok = self._routes[key] = int(lib.sb_chunked_retention_supports(dk, dv, rot_dims, q.stride(0), k.stride(0), v.stride(0)))
         if not ok or any(x.data_ptr() % 8 for x in (q, k, v)):
             return False
-        rows, n_list, chunks = None, shape.rows, q.shape[0] // 64 + shape.rows
-        neg_q = getattr(shape, "neg_q_sorted", None)
-        if neg_q is not None and getattr(shape, "rows_by_q", None) is not None:
-            n_list = bisect.bisect_left(neg_q, -self.CHUNKED_FROM)
-            rows, chunks = shape.rows_by_q, sum(-(n // 64) for n in neg_q[:n_list])
+        n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 64)
         if n_list * heads > 65535:
             return False
         angles = None
