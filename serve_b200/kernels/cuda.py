@@ -1034,9 +1034,9 @@ class CudaKernels:
         "gla": S = diag(a) S + k v^T, o = S^T (q_scale q), a = sigmoid(rate + dt_bias)^rate_scale per row (rate [T, heads * dk]);
         "retention": S = decay_h S + k v^T on q, k, v as they are, the first rot_dims elements of q and k rotated by the tokens'
         positions (pairs i, i + rot_dims / 2; inv_freq float [rot_dims / 2]), k times k_scale.
-        out: float [T, heads * dv]. Requests that bring more than CHUNKED_FROM tokens run chunk by chunk: "retention" in bfloat16 on the
-        tensor cores (csrc/chunked_retention.cu), states of at most 128 rows otherwise in 32-bit arithmetic (csrc/chunked_recurrence.cu). The
-        others are walked token by token."""
+        out: float [T, heads * dv]. Long requests run chunk by chunk: "retention" in bfloat16 on the tensor cores
+        (csrc/chunked_retention.cu, more than CHUNKED_FROM tokens), otherwise a few requests of more than CHUNKS_FROM tokens with states
+        of at most 128 rows in 32-bit arithmetic (csrc/chunked_recurrence.cu). The others are walked token by token."""
         max_walk = 0
         if mode == "retention" and self._chunked_retention(q, k, v, state, ctx, out, heads, dk, dv, decay, inv_freq, rot_dims, k_scale):
             if getattr(ctx.shape, "min_q", 1) > self.CHUNKED_FROM:
@@ -1053,13 +1053,14 @@ class CudaKernels:
         self.launches += 2
         shape = ctx.shape
         rows, n_list, chunks, chunk_work, walk_too = None, shape.rows, 0, None, 1
-        if not max_walk and self.use_chunked_recurrence and shape.max_q > self.CHUNKED_FROM:
-            n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32)
+        if not max_walk and self.use_chunked_recurrence and shape.max_q > self.CHUNKS_FROM:
+            n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, self.CHUNKS_FROM)
+        if chunks and n_list * heads <= self.CHUNKS_PAIRS:
             lib.sb_linear_recurrence_chunk_floats.restype = ctypes.c_longlong
             floats = lib.sb_linear_recurrence_chunk_floats(code, q.shape[0], chunks, heads, dk, dv)
             if 0 < floats <= self.CHUNK_SCRATCH_FLOATS:
                 chunk_work = torch.empty(floats, dtype=torch.float32, device=q.device)
-                max_walk, walk_too = self.CHUNKED_FROM, 1 if getattr(shape, "min_q", 1) <= self.CHUNKED_FROM else 0
+                max_walk, walk_too = self.CHUNKS_FROM, 1 if getattr(shape, "min_q", 1) <= self.CHUNKS_FROM else 0
                 self.launches += 1 + walk_too
         _check(lib.sb_linear_recurrence(
             code, _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0),
@@ -1073,15 +1074,21 @@ class CudaKernels:
 
     # Requests with more tokens than this go through the chunked kernels, where those take the layout.
     CHUNKED_FROM = 32
+    # The 32-bit chunked kernels shorten the chain of a long request; where many (request, head) pairs fill the SMs anyway the walk does
+    # fewer operations. Chunked | walked, a layer at width 2,048 (16 heads of 128 x 128), fixed decay and gated delta rule: one request of
+    # 64 tokens 47 | 49 and 57 | 53 us, of 128 54 | 67 and 65 | 76, of 1,000 167 | 308 and 218 | 411; 3 of 1,000 (48 pairs) 416 | 474 and
+    # 549 | 651; 8 of 256 (128 pairs) 263 | 287 and 392 | 396; 16 of 190 378 | 390 and 556 | 545.
+    CHUNKS_FROM = 96
+    CHUNKS_PAIRS = 48
     CHUNK_SCRATCH_FLOATS = 1 << 28           # work space of the 32-bit chunked kernels at most (a GB); a larger step is walked
     use_chunked_recurrence = True            # tests: False keeps every request on the walking kernel
 
-    def _chunk_list(self, shape, tokens: int, size: int):
-        """(entries, the list or None, chunks) of the requests that bring more than CHUNKED_FROM tokens, in chunks of ``size``."""
+    def _chunk_list(self, shape, tokens: int, size: int, more_than: int):
+        """(entries, the list or None, chunks) of the requests that bring more tokens than ``more_than``, in chunks of ``size``."""
         neg_q = getattr(shape, "neg_q_sorted", None)
         if neg_q is None or getattr(shape, "rows_by_q", None) is None:
             return shape.rows, None, tokens // size + shape.rows
-        n = bisect.bisect_left(neg_q, -self.CHUNKED_FROM)
+        n = bisect.bisect_left(neg_q, -more_than)
         return n, shape.rows_by_q, sum(-(q // size) for q in neg_q[:n])
     use_chunked_retention = True             # tests: False keeps every request on the walking kernel
 
@@ -1097,7 +1104,7 @@ class CudaKernels:
             ok = self._routes[key] = int(lib.sb_chunked_retention_supports(dk, dv, rot_dims, q.stride(0), k.stride(0), v.stride(0)))
         if not ok or any(x.data_ptr() % 8 for x in (q, k, v)):
             return False
-        n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 64)
+        n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 64, self.CHUNKED_FROM)
         if n_list * heads > 65535:
             return False
         angles = None

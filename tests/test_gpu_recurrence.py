@@ -68,12 +68,13 @@ def _run(kernels, c, chunked=True, out_dtype=torch.float32):
     c.ctx.memo.clear()
     before = getattr(kernels, "use_chunked_recurrence", None)
     if before is not None:
-        kernels.use_chunked_recurrence, kernels.use_chunked_retention = chunked, False
+        kernels.use_chunked_recurrence, kernels.use_chunked_retention, kernels.CHUNKS_FROM = chunked, False, 32
     try:
         kernels.linear_recurrence(c.mode, *c.args, state, c.ctx, out, heads, qk_heads, dk, dv, **c.kw)
     finally:
         if before is not None:
             kernels.use_chunked_recurrence, kernels.use_chunked_retention = before, True
+            del kernels.CHUNKS_FROM                       # (the class's again)
     return out, pool
 
 
