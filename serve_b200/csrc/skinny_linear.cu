@@ -274,77 +274,92 @@ int launch_mt(const void* a, const void* w, void* out, int M, int N, int K, cuda
 
 // The same product in true 32-bit arithmetic (plain fused multiply-adds, no tensor-core mode), for the float32 path's
 // decoding steps: a warp owns NC output columns and MB activation rows, its lanes share K out among themselves in
-// steps of four values, partial sums meet by a shuffle tree of fixed order. The weights are read once from memory at
-// streaming speed (KU steps' loads per column go out together); the activation rows come from the L1 cache. NC is chosen
-// so that there are blocks for every SM (narrow outputs: one column a warp). A row's result does not depend on the other rows.
-constexpr int F32_MB = 8, F32_WARPS = 8;
+// steps of four values, partial sums meet by a shuffle tree of fixed order. The weights are read once from memory: every lane's
+// come through a ring of f32_stages cp.async stages that only it reads and writes (64 KB under way in an SM with two columns a warp;
+// as register loads one step ahead the warps waited for memory three quarters of the time). The activation rows are shared by the
+// block's warps, 512 k-values at a time in two buffers. NC is chosen so that there are blocks for every SM (narrow outputs: one column
+// a warp). A row's result does not depend on the other rows. 8 rows: [16384, 2048] (134 MB) 57.5 -> 34.2 us, [3072, 2048] and [2048, 2048]
+// 31.2 -> 21.0 us together; 20 rows of [28672, 4096] and [4096, 14336] 602 -> 388 us.
+constexpr int F32_MB = 8, F32_WARPS = 8, F32_KC = 512;
+constexpr int F32_STEPS = F32_KC / 128;         // steps of 128 k-values in a buffer of activations
+__host__ __device__ constexpr int f32_stages(int nc) { return nc == 4 ? 4 : 5; }       // at most F32_STEPS + 1: see the waits
+__host__ __device__ constexpr int f32_smem(int nc) { return (2 * F32_MB * F32_KC + f32_stages(nc) * nc * F32_WARPS * 32 * 4) * 4; }
 
-__device__ __forceinline__ float4 ld_stream_f4(const float* p) {
-  float4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
-  return v;
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+  const int n = valid ? 16 : 0;                 // 0: nothing is read, zeros are written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(n) : "memory");
 }
 
-template <int NC, int KU>
+template <int NC>
 __global__ void __launch_bounds__(F32_WARPS * 32, 2) skinny_linear_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
                                                                                float* __restrict__ out, int M, int N, int K) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int ST = f32_stages(NC);
+  extern __shared__ __align__(16) float f32_sm[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float* acts = f32_sm;                                              // [2][F32_MB][F32_KC]
+  float* ring = f32_sm + 2 * F32_MB * F32_KC + tid * 4;              // [ST][NC][thread][4]
   const int n0 = (blockIdx.x * F32_WARPS + warp) * NC;
   const int m0 = blockIdx.y * F32_MB;
   const float* wp[NC];
-  const float* ap[F32_MB];
 #pragma unroll
   for (int c = 0; c < NC; ++c) wp[c] = w + (size_t)min(n0 + c, N - 1) * K;      // clamped: computed and dropped
+  const int steps = (K + 127) / 128;
+  auto fetch = [&](int step) {                                       // (always a group, also an empty one)
+    const int k = step * 128 + lane * 4;
+    if (step < steps) {
 #pragma unroll
-  for (int i = 0; i < F32_MB; ++i) ap[i] = a + (size_t)min(m0 + i, M - 1) * K;
+      for (int c = 0; c < NC; ++c)
+        cp_async16(ring + (size_t)((step % ST) * NC + c) * F32_WARPS * 32 * 4, wp[c] + (k < K ? k : 0), k < K && n0 < N);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto fetch_acts = [&](int chunk) {                                 // (joins the group of the next fetch)
+    float* dst = acts + (size_t)(chunk & 1) * F32_MB * F32_KC;
+#pragma unroll
+    for (int u = 0; u < F32_MB * F32_KC / 4 / (F32_WARPS * 32); ++u) {
+      const int e = (u * F32_WARPS * 32 + tid) * 4, row = e / F32_KC, k = chunk * F32_KC + (e - row * F32_KC);
+      const bool valid = m0 + row < M && k < K;
+      cp_async16(dst + e, a + (valid ? (size_t)(m0 + row) * K + k : 0), valid);
+    }
+  };
   float acc[NC][F32_MB];
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
     for (int i = 0; i < F32_MB; ++i) acc[c][i] = 0.f;
   // the weights do not depend on the kernel before this one: their first loads go out before the wait
-  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 wv[KU][NC];
-  const int k_first = lane * 4;
 #pragma unroll
-  for (int u = 0; u < KU; ++u)
-#pragma unroll
-    for (int c = 0; c < NC; ++c) wv[u][c] = (k_first + u * 128 < K && n0 < N) ? ld_stream_f4(wp[c] + k_first + u * 128) : zero4;
+  for (int u = 0; u < ST - 1; ++u) fetch(u);
   pdl_launch_dependents();
   pdl_wait();
-  if (n0 >= N) return;
-  for (int k = k_first; k < K; k += 128 * KU) {
-    float4 wn[KU][NC];
+  fetch_acts(0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int step = 0; step < steps; ++step) {
+    // a buffer of activations goes out with the group of its predecessor's first step, F32_STEPS groups before it is read
+    if (step == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+    if (step % F32_STEPS == 0) {
+      __syncthreads();                                               // this buffer is there for all, the other one has been read by all
+      if (step + F32_STEPS < steps) fetch_acts(step / F32_STEPS + 1);
+    }
+    fetch(step + ST - 1);
+    float4 wv[NC];
 #pragma unroll
-    for (int u = 0; u < KU; ++u)
+    for (int c = 0; c < NC; ++c) wv[c] = *reinterpret_cast<const float4*>(ring + (size_t)((step % ST) * NC + c) * F32_WARPS * 32 * 4);
+    const float* av = acts + (size_t)((step / F32_STEPS) & 1) * F32_MB * F32_KC + (step % F32_STEPS) * 128 + lane * 4;
+#pragma unroll
+    for (int i = 0; i < F32_MB; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(av + i * F32_KC);
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        const int kn = k + 128 * KU + u * 128;
-        wn[u][c] = kn < K ? ld_stream_f4(wp[c] + kn) : zero4;
-      }
-#pragma unroll
-    for (int u = 0; u < KU; ++u) {
-      const int ku = k + u * 128;
-      if (ku < K) {
-        float4 av[F32_MB];
-#pragma unroll
-        for (int i = 0; i < F32_MB; ++i) av[i] = __ldg(reinterpret_cast<const float4*>(ap[i] + ku));
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-#pragma unroll
-          for (int i = 0; i < F32_MB; ++i) {
-            acc[c][i] = fmaf(wv[u][c].x, av[i].x, acc[c][i]);
-            acc[c][i] = fmaf(wv[u][c].y, av[i].y, acc[c][i]);
-            acc[c][i] = fmaf(wv[u][c].z, av[i].z, acc[c][i]);
-            acc[c][i] = fmaf(wv[u][c].w, av[i].w, acc[c][i]);
-          }
+        acc[c][i] = fmaf(wv[c].x, x.x, acc[c][i]);
+        acc[c][i] = fmaf(wv[c].y, x.y, acc[c][i]);
+        acc[c][i] = fmaf(wv[c].z, x.z, acc[c][i]);
+        acc[c][i] = fmaf(wv[c].w, x.w, acc[c][i]);
       }
     }
-#pragma unroll
-    for (int u = 0; u < KU; ++u)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) wv[u][c] = wn[u][c];
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
@@ -352,6 +367,14 @@ __global__ void __launch_bounds__(F32_WARPS * 32, 2) skinny_linear_f32_kernel(co
       const float s = warp_sum(acc[c][i]);
       if (lane == 0 && n0 + c < N && m0 + i < M) out[(size_t)(m0 + i) * N + n0 + c] = s;
     }
+}
+
+template <int NC>
+cudaError_t launch_f32(const float* a, const float* w, float* out, int M, int N, int K, cudaStream_t stream) {
+  auto k = skinny_linear_f32_kernel<NC>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem(NC));
+  return launch_pdl(k, dim3((N + F32_WARPS * NC - 1) / (F32_WARPS * NC), (M + F32_MB - 1) / F32_MB), dim3(F32_WARPS * 32), (size_t)f32_smem(NC),
+                    stream, a, w, out, M, N, K);
 }
 
 }  // namespace
@@ -370,17 +393,11 @@ SB_EXPORT int sb_skinny_linear_f32(const void* a, const void* w, void* out, int 
   const int want = 2 * sm_count();                     // two blocks fit an SM
   const float *af = (const float*)a, *wf = (const float*)w;
   float* of = (float*)out;
-  // columns per warp: as many as still leave blocks for every SM
-  if ((long long)((N + F32_WARPS * 4 - 1) / (F32_WARPS * 4)) * mt >= want) {
-    SB_PDL_CHECK(launch_pdl(skinny_linear_f32_kernel<4, 1>, dim3((N + F32_WARPS * 4 - 1) / (F32_WARPS * 4), mt), dim3(F32_WARPS * 32), 0,
-                            stream, af, wf, of, M, N, K));
-  } else if ((long long)((N + F32_WARPS * 2 - 1) / (F32_WARPS * 2)) * mt >= want) {
-    SB_PDL_CHECK(launch_pdl(skinny_linear_f32_kernel<2, 2>, dim3((N + F32_WARPS * 2 - 1) / (F32_WARPS * 2), mt), dim3(F32_WARPS * 32), 0,
-                            stream, af, wf, of, M, N, K));
-  } else {
-    SB_PDL_CHECK(launch_pdl(skinny_linear_f32_kernel<1, 4>, dim3((N + F32_WARPS - 1) / F32_WARPS, mt), dim3(F32_WARPS * 32), 0, stream,
-                            af, wf, of, M, N, K));
-  }
+  // columns per warp: four or two if that still leaves a block for every SM
+  const long long cols = (long long)N * mt / F32_WARPS;
+  if (cols >= 4 * want) SB_PDL_CHECK(launch_f32<4>(af, wf, of, M, N, K, stream));
+  else if (cols >= 2 * sm_count()) SB_PDL_CHECK(launch_f32<2>(af, wf, of, M, N, K, stream));
+  else SB_PDL_CHECK(launch_f32<1>(af, wf, of, M, N, K, stream));
   return 0;
 }
 

@@ -675,25 +675,24 @@ class CudaKernels:
             return self._attention_mma(lib, qkv, k_cache, v_cache, block_table, cu_q, kv_len, heads, kv_heads, head_dim,
                                        page_size, scale, window, out, shape, slopes=slopes, chunk=int(chunk), softcap=softcap, sinks=sinks,
                                        keep_first=keep_first)
-        if opts:
-            group = heads // kv_heads
-            self.launches += (1 if group <= 16 else 0) + (1 if group > 16 or shape.max_q * group > 16 else 0)
-            _check(lib.sb_attention_simt_keep(
-                _p(qkv), qkv.stride(0), _p(k_cache), _p(v_cache), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_len),
-                heads, kv_heads, page_size, k_cache.shape[0], ctypes.c_float(scale), window, _p(out), shape.rows, shape.max_q,
-                _DT[qkv.dtype], _p(slopes), int(chunk), ctypes.c_float(softcap), _p(sinks), keep_first, self._s()),
-                "attention with score options")
-            return
-        if qkv.dtype == torch.bfloat16 and not self.force_simt_attention:
+        if not opts and qkv.dtype == torch.bfloat16 and not self.force_simt_attention:
             return self._attention_mma(lib, qkv, k_cache, v_cache, block_table, cu_q, kv_len, heads, kv_heads, head_dim,
                                        page_size, scale, window, out, shape)
         group = heads // kv_heads
-        # requests of at most 16 rows run in the decoding shape, the others in tiles: one launch each, as needed
-        self.launches += (1 if group <= 16 else 0) + (1 if group > 16 or shape.max_q * group > 16 else 0)
-        _check(lib.sb_attention_simt(
-            _p(qkv), qkv.shape[1], _p(k_cache), _p(v_cache), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_len),
+        # requests of at most 16 rows run in the decoding shape, the others in tiles: one launch each, as needed. The keys of the
+        # former are shared out so that two blocks fit every SM.
+        decoding = group <= 16 and getattr(shape, "min_q", 1) * group <= 16
+        n_splits, scratch = 1, None
+        if decoding:
+            keys = min(shape.max_kv, window + keep_first + 16) if window else shape.max_kv
+            n_splits = max(1, min(2 * self.TARGET_BLOCKS // (shape.rows * kv_heads), -(-keys // 128), self.MAX_SPLITS))
+            if n_splits > 1:
+                scratch = torch.empty(shape.rows * kv_heads * n_splits * 16 * (head_dim + 2), dtype=torch.float32, device=qkv.device)
+        self.launches += (1 if group <= 16 else 0) + (1 if group > 16 or shape.max_q * group > 16 else 0) + (1 if scratch is not None else 0)
+        _check(lib.sb_attention_simt_keep(
+            _p(qkv), qkv.stride(0), _p(k_cache), _p(v_cache), _p(block_table), block_table.shape[1], _p(cu_q), _p(kv_len),
             heads, kv_heads, page_size, k_cache.shape[0], ctypes.c_float(scale), window, _p(out), shape.rows, shape.max_q,
-            _DT[qkv.dtype], self._s()), "attention")
+            _DT[qkv.dtype], _p(slopes), int(chunk), ctypes.c_float(softcap), _p(sinks), keep_first, n_splits, _p(scratch), self._s()), "attention")
 
     # Thread blocks of the deep shape that the key splits of a batch should fill: one per SM (set from the device's
     # SM count when the kernels are loaded; 148 on a B200).
