@@ -389,6 +389,45 @@ __global__ void __launch_bounds__(256) add_bias_kernel(float* __restrict__ x, co
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) x[i] += bias[i % cols];
 }
 
+// ------------------------------------------------------------- a few rows of many short products
+// out[m, b] = a[m, b] w[b]^T for up to 16 rows m and short k (the per-head products of latent attention in a decoding step:
+// 128 x 192 a head): a warp takes eight columns of one b, mma.sync m16n8k16 with the rows as the 16-row operand. All of a
+// warp's weights are fetched before the wait for the kernel before this one. The work is nothing (1 MB of weights), so what counts
+// is the launch: about 3 us of host time against 12 for the library's batched product, which also chooses a kernel each time.
+constexpr int BATCHED_K = 256;
+__global__ void __launch_bounds__(128) few_rows_batched_kernel(const __nv_bfloat16* __restrict__ a, int lda, long long a_batch,
+                                                               const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ out, int ldc,
+                                                               long long c_batch, int M, int N, int K) {
+  const int lane = threadIdx.x & 31, n0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8, b = blockIdx.y;
+  const int g = lane >> 2, c2 = (lane & 3) * 2;
+  const bool mine = n0 < N;
+  uint32_t wv[BATCHED_K / 16][2];
+  const __nv_bfloat16* wr = w + ((size_t)b * N + (mine ? n0 : 0) + g) * K + c2;
+#pragma unroll
+  for (int s = 0; s < BATCHED_K / 16; ++s) {
+    const bool in = mine && s * 16 < K;
+    wv[s][0] = in ? __ldg(reinterpret_cast<const uint32_t*>(wr + s * 16)) : 0u;
+    wv[s][1] = in ? __ldg(reinterpret_cast<const uint32_t*>(wr + s * 16 + 8)) : 0u;
+  }
+  pdl_launch_dependents();
+  pdl_wait();
+  if (!mine) return;
+  const __nv_bfloat16* r0 = a + (size_t)g * lda + b * a_batch + c2;
+  const __nv_bfloat16* r1 = r0 + (size_t)8 * lda;
+  float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int s = 0; s < BATCHED_K / 16; ++s) {
+    if (s * 16 >= K) break;
+    const uint32_t a0 = g < M ? *reinterpret_cast<const uint32_t*>(r0 + s * 16) : 0u, a1 = g + 8 < M ? *reinterpret_cast<const uint32_t*>(r1 + s * 16) : 0u;
+    const uint32_t a2 = g < M ? *reinterpret_cast<const uint32_t*>(r0 + s * 16 + 8) : 0u, a3 = g + 8 < M ? *reinterpret_cast<const uint32_t*>(r1 + s * 16 + 8) : 0u;
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(wv[s][0]), "r"(wv[s][1]));
+  }
+  __nv_bfloat16* o = out + (size_t)g * ldc + b * c_batch + n0 + c2;
+  if (g < M) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(c[0], c[1]);
+  if (g + 8 < M) *reinterpret_cast<__nv_bfloat162*>(o + (size_t)8 * ldc) = __floats2bfloat162_rn(c[2], c[3]);
+}
+
 // ------------------------------------------------------------- bias, whole-projection norm, partial rotation, cache write
 // sums float [T, (H + 2 G) * D] (row stride given): the float sums of the fused query | key | value projection, heads padded
 // to D with zeros (G = 0: queries only). Per token, one block: add the bias; divide all queries together (and all keys
@@ -400,6 +439,104 @@ __global__ void __launch_bounds__(256) add_bias_kernel(float* __restrict__ x, co
 // instead divided, after its rotation, by its own root mean square over its dim true elements, without a weight. With
 // keys_are_values the row ends with the keys, [T, (H + G) * D], and the value pages take the keys as projected, before norm and
 // rotation.
+// The same for rows of whole 16-byte pieces (D a multiple of 8, rot of 8 and rot - D too) without a norm of single heads: an
+// item is eight elements of a head, four rotated ones and their four partners or eight plain ones, so a thread turns what it
+// has loaded itself and the row never goes through shared memory; the block meets once, for the two sums and the angles. ITEMS
+// a thread (all their loads are under way together). What bounds it is the memory: 3,072 float sums a token in, as many
+// bfloat16 numbers out. 2,048 tokens of 16/4 heads of 128 (38 MB): 36.1 us as an element a lane with the row in shared memory,
+// 14.7 so; 8 tokens: 12 -> 3.3.
+template <typename T, int ITEMS>
+__global__ void __launch_bounds__(512) qk_prepare_vec_kernel(
+    const float* __restrict__ sums, int stride, const float* __restrict__ bias, const int* __restrict__ positions,
+    const int* __restrict__ token_row, int H, int G, int D, int dim, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+    float eps, const float* __restrict__ inv_freq, int rot, T* __restrict__ q_out, int q_stride, T* __restrict__ kc, T* __restrict__ vc,
+    const int* __restrict__ block_table, int bt_width, int ps, int num_pages, int* __restrict__ errors, int keys_are_values) {
+  __shared__ float red[2][16];
+  extern __shared__ __align__(16) float angles[];      // [half] cosines, [half] sines
+  const int t = blockIdx.x, half = rot >> 1, nq = H * D, nk = G * D;
+  const int per_head = D >> 3, pairs = half >> 2, items = (H + (keys_are_values ? 1 : 2) * G) * per_head;
+  const float* row = sums + (size_t)t * stride;
+  const int pos = positions[t];
+  float4 x[ITEMS], y[ITEMS];
+  int at[ITEMS], partner[ITEMS];                       // columns of the item's two pieces
+  float sq = 0.f, sk = 0.f;
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) {
+    const int i = threadIdx.x + u * blockDim.x;
+    const int head = i / per_head, j = i - head * per_head;
+    const bool turns = j < pairs && head < H + G;
+    at[u] = head * D + (turns ? j * 4 : (head < H + G ? rot + (j - pairs) * 8 : j * 8));
+    partner[u] = turns ? half : 4;
+    x[u] = y[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < items) {
+      x[u] = *reinterpret_cast<const float4*>(row + at[u]);
+      y[u] = *reinterpret_cast<const float4*>(row + at[u] + partner[u]);
+    }
+  }
+  if ((int)threadIdx.x < half) sincosf((float)pos * inv_freq[threadIdx.x], &angles[half + threadIdx.x], &angles[threadIdx.x]);
+  if (bias) {
+#pragma unroll
+    for (int u = 0; u < ITEMS; ++u) {
+      if (threadIdx.x + u * blockDim.x >= items) continue;
+      const float4 a = *reinterpret_cast<const float4*>(bias + at[u]), b = *reinterpret_cast<const float4*>(bias + at[u] + partner[u]);
+      x[u].x += a.x; x[u].y += a.y; x[u].z += a.z; x[u].w += a.w;
+      y[u].x += b.x; y[u].y += b.y; y[u].z += b.z; y[u].w += b.w;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) {
+    const float ss = (x[u].x * x[u].x + x[u].y * x[u].y + x[u].z * x[u].z + x[u].w * x[u].w) +
+                     (y[u].x * y[u].x + y[u].y * y[u].y + y[u].z * y[u].z + y[u].w * y[u].w);
+    if (at[u] < nq) sq += ss;
+    else if (at[u] < nq + nk) sk += ss;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  sq = warp_sum(sq);
+  sk = warp_sum(sk);
+  if (lane == 0) { red[0][warp] = sq; red[1][warp] = sk; }
+  __syncthreads();
+  sq = sk = 0.f;
+  for (int w = 0; w < n_warps; ++w) { sq += red[0][w]; sk += red[1][w]; }
+  const float inv_q = q_weight ? 1.0f / sqrtf(sq / (float)(H * dim) + eps) : 1.f;
+  const float inv_k = k_weight && G > 0 ? 1.0f / sqrtf(sk / (float)(G * dim) + eps) : 1.f;
+  const int blk = ps > 0 ? pos / ps : 0;
+  const int page = (G > 0 && pos >= 0 && blk < bt_width) ? block_table[(size_t)token_row[t] * bt_width + blk] : -1;
+  const bool page_ok = page >= 0 && page < num_pages;
+  if (G > 0 && !page_ok && threadIdx.x == 0) atomicAdd(errors, 1);
+  const int within = pos - blk * ps;
+#pragma unroll
+  for (int u = 0; u < ITEMS; ++u) {
+    const int i = threadIdx.x + u * blockDim.x;
+    if (i >= items) continue;
+    const int head = i / per_head, d = at[u] - head * D, d2 = d + partner[u];
+    const bool is_q = head < H, is_k = !is_q && head < H + G;
+    if (!is_q && !page_ok) continue;
+    const size_t cell = is_q ? 0 : (((size_t)page * G + (is_k ? head - H : head - H - G)) * ps + within) * D;
+    if (!is_q && (!is_k || keys_are_values)) {         // values, or keys as they are projected
+      store4f<T>(vc + cell + d, x[u]);
+      store4f<T>(vc + cell + d2, y[u]);
+      if (!is_k) continue;
+    }
+    const float* w = is_q ? q_weight : k_weight;
+    if (w) {
+      const float inv = is_q ? inv_q : inv_k;
+      const float* wr = w + (is_q ? at[u] : at[u] - nq);
+      const float4 a = *reinterpret_cast<const float4*>(wr), b = *reinterpret_cast<const float4*>(wr + partner[u]);
+      x[u].x *= inv * a.x; x[u].y *= inv * a.y; x[u].z *= inv * a.z; x[u].w *= inv * a.w;
+      y[u].x *= inv * b.x; y[u].y *= inv * b.y; y[u].z *= inv * b.z; y[u].w *= inv * b.w;
+    }
+    if (d < half) {
+      const float4 c = *reinterpret_cast<const float4*>(angles + d), sn = *reinterpret_cast<const float4*>(angles + half + d);
+      const float4 v = x[u], o = y[u];
+      x[u] = make_float4(v.x * c.x - o.x * sn.x, v.y * c.y - o.y * sn.y, v.z * c.z - o.z * sn.z, v.w * c.w - o.w * sn.w);
+      y[u] = make_float4(o.x * c.x + v.x * sn.x, o.y * c.y + v.y * sn.y, o.z * c.z + v.z * sn.z, o.w * c.w + v.w * sn.w);
+    }
+    T* dst = is_q ? q_out + (size_t)t * q_stride + head * D : kc + cell;
+    store4f<T>(dst + d, x[u]);
+    store4f<T>(dst + d2, y[u]);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512) qk_prepare_kernel(
     const float* __restrict__ sums, int stride, const float* __restrict__ bias, const int* __restrict__ positions,
@@ -677,6 +814,34 @@ SB_EXPORT int sb_qk_prepare(const float* sums, int stride, const float* bias, co
 #undef SB_HEAD_NORM
     return 0;
   }
+  const int items = n_all / 8;
+  if (head_norm == 0 && D % 8 == 0 && rot % 8 == 0 && (D - rot) % 8 == 0 && items <= 8 * 512 && stride % 4 == 0 && q_stride % 4 == 0 && aligned16(sums) &&
+      aligned16(q_out) && (!bias || aligned16(bias)) && (!q_weight || aligned16(q_weight)) && (!k_weight || aligned16(k_weight)) &&
+      (G == 0 || (aligned16(kc) && aligned16(vc)))) {
+    // few tokens: an item a thread; many: more items a thread and smaller blocks, whose starts and ends overlap
+    const int per = n_tokens >= 2 * sm_count() ? (items > 1024 ? 8 : 4) : (items <= 512 ? 1 : (items <= 1024 ? 2 : 8));
+    const int least = ((rot / 2 > (items + per - 1) / per ? rot / 2 : (items + per - 1) / per) + 31) & ~31;
+    if (least <= 512) {
+#define SB_QK_VEC(T, N)                                                                                                                        \
+  qk_prepare_vec_kernel<T, N><<<n_tokens, least, (size_t)(rot > 0 ? rot : 2) * sizeof(float), stream>>>(                                        \
+      sums, stride, bias, positions, token_row, H, G, D, dim, q_weight, k_weight, eps, inv_freq, rot, (T*)q_out, q_stride, (T*)kc, (T*)vc,       \
+      block_table, bt_width, ps, num_pages, errors, keys_are_values)
+#define SB_QK_VEC_N(T)                                                                                                                         \
+  do {                                                                                                                                         \
+    if (per == 1) SB_QK_VEC(T, 1);                                                                                                              \
+    else if (per == 2) SB_QK_VEC(T, 2);                                                                                                         \
+    else if (per == 4) SB_QK_VEC(T, 4);                                                                                                         \
+    else SB_QK_VEC(T, 8);                                                                                                                       \
+  } while (0)
+      if (dtype == SB_DTYPE_F32) SB_QK_VEC_N(float);
+      else if (dtype == SB_DTYPE_BF16) SB_QK_VEC_N(__nv_bfloat16);
+      else return SB_ERR_DTYPE;
+#undef SB_QK_VEC_N
+#undef SB_QK_VEC
+      SB_LAUNCH_CHECK();
+      return 0;
+    }
+  }
   const size_t smem = ((size_t)(rot > 0 ? rot : 2) + (size_t)n_all) * sizeof(float);
   if (smem > 200 * 1024) return SB_ERR_LIMIT;
   const int threads = n_all >= 2048 ? 512 : 256;
@@ -695,6 +860,23 @@ SB_EXPORT int sb_qk_prepare(const float* sums, int stride, const float* bias, co
   else
     return SB_ERR_DTYPE;
   SB_LAUNCH_CHECK();
+  return 0;
+}
+
+// 1 if sb_few_rows_batched takes these sizes and strides (the pointers 4-byte aligned), all in bfloat16.
+SB_EXPORT int sb_few_rows_batched_supports(int M, int N, int K, int lda, long long a_batch, int ldc, long long c_batch) {
+  return M >= 1 && M <= 16 && N >= 8 && N % 8 == 0 && K >= 16 && K % 16 == 0 && K <= BATCHED_K && lda % 2 == 0 && a_batch % 2 == 0 && ldc % 2 == 0 &&
+         c_batch % 2 == 0;
+}
+
+// out[m, b, :] = a[m, b, :] w[b]^T: a rows lda and batches a_batch apart, w [batch, N, K], out rows ldc and batches c_batch apart.
+SB_EXPORT int sb_few_rows_batched(const void* a, int lda, long long a_batch, const void* w, void* out, int ldc, long long c_batch, int M, int N,
+                                  int K, int batch, cudaStream_t stream) {
+  if (batch <= 0) return 0;
+  if (!sb_few_rows_batched_supports(M, N, K, lda, a_batch, ldc, c_batch) || batch > 65535) return SB_ERR_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out)) & 3) return SB_ERR_ALIGN;
+  SB_PDL_CHECK(launch_pdl(few_rows_batched_kernel, dim3((N + 31) / 32, batch), dim3(128), 0, stream, (const __nv_bfloat16*)a, lda, a_batch,
+                          (const __nv_bfloat16*)w, (__nv_bfloat16*)out, ldc, c_batch, M, N, K));
   return 0;
 }
 

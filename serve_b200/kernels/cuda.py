@@ -454,12 +454,26 @@ class CudaKernels:
 
     def linear_batched(self, a, w, out) -> None:
         """out[:, b] = a[:, b] @ w[b]^T for every b: a [M, B, K] and out [M, B, N] may be views of wider buffers (unit stride
-        along the last axis), w [B, N, K] is whole. One batched library product."""
+        along the last axis), w [B, N, K] is whole. In bfloat16 a few rows of short products run on a kernel of this engine, the
+        others are one batched library product."""
         m, b, k = a.shape
         n = w.shape[1]
         if (w.shape[0] != b or w.shape[2] != k or tuple(out.shape) != (m, b, n) or a.dtype != w.dtype or a.stride(2) != 1
                 or out.stride(2) != 1 or not w.is_contiguous()):
             raise KernelError(f"linear_batched: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)} do not fit")
+        if a.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and m <= 16 and self.use_skinny_linear and b <= 65535:
+            lda, step, ldc, cstep = a.stride(0), a.stride(1), out.stride(0), out.stride(1)
+            key = ("few_rows_batched", m, n, k, lda, step, ldc, cstep)
+            ok = self._routes.get(key)
+            if ok is None:
+                ok = self._routes[key] = int(self._prep_lib().sb_few_rows_batched_supports(m, n, k, lda, ctypes.c_longlong(step), ldc,
+                                                                                          ctypes.c_longlong(cstep)))
+            pa, pw, po = a.data_ptr(), w.data_ptr(), out.data_ptr()
+            if ok and not (pa | pw | po) & 3:
+                self.launches += 1
+                _check(self._prep_lib().sb_few_rows_batched(ctypes.c_void_p(pa), lda, ctypes.c_longlong(step), ctypes.c_void_p(pw), ctypes.c_void_p(po),
+                                                            ldc, ctypes.c_longlong(cstep), m, n, k, b, self._s()), "batched few-rows product")
+                return
         self.library_calls += 1
         _check(self._gemm.sb_linear_batched(_p(a), a.stride(0), ctypes.c_longlong(a.stride(1)), _p(w), _p(out), out.stride(0),
                                             ctypes.c_longlong(out.stride(1)), m, n, k, b, _DT[a.dtype], _DT[out.dtype], self._s()),
