@@ -1,4 +1,4 @@
-// The linear recurrences of sequence_ops.cu for prompt portions, 32 tokens at a time, in plain 32-bit arithmetic.
+// The linear recurrences of sequence_ops.cu for prompt portions, 32 tokens at a time.
 //
 // The walk's time is a chain: a token's read-out and update wait for the token before (0.09 us for a fixed decay to 0.34 us for
 // the delta rule a token, with one warp a scheduler). A chunk of tokens 0 .. 31 with the state S before it obeys
@@ -8,31 +8,115 @@
 // update, so its Q' uses G_(t-1)), K''_s = (c / G_s) k_s, c the product of all, P_ts = q_t . (G_t / G_s) k_s for s <= t and A_ts = b_t k_t .
 // (G_t / G_s) k_s for s < t. Ratios of products are never formed by division: G_t / G_s is the product of the decays s + 1 .. t, so a
 // decay that underflows is simply zero.
-//   chunk_prep_kernel: a block a (chunk, head), all chunks at once: P, Q', K'', c; for the delta rule W = (I + A)^-1 diag(b) K' and
+//   chunk_prep_*_kernel: a block a (chunk, head), all chunks at once: P, Q', K'', c; for the delta rule W = (I + A)^-1 diag(b) K' and
 //     V' = (I + A)^-1 diag(b) V by forward substitution, a thread a column, so that U = V' - W S.
 //   chunk_walk_kernel: a block a (request, head, 16 columns of S), a chain of tokens / 32 steps: [W; Q'] S, then U, then O and the
-//     next S. The tiles come through a two-stage cp.async ring; S lives in registers and, for the first product, in shared memory.
-// Multiply-adds per token and head are 1.25 times the walk's, but 32 tokens wide, so the FMA units and not a latency are the bound.
-// 2,048 tokens, 16 heads of 128 x 128 (B200): see the launcher. All sums are float in a fixed order.
+//     next S. The matrices come through a ring of two stages; S lives in the accumulator layout in registers.
+//
+// All of this counts as 32-bit. The products run on the tensor cores (mma.sync m16n8k16) with every float x split into three bfloat16
+// numbers h + m + l = x (8 bits each, nothing left), six of the nine products of the parts (the others are below 2^-24), smallest
+// first, in an accumulator that starts from zero for every 16 terms and is then added in float, so that no sum is longer than 16
+// terms before a rounded addition. Measured against 64 bits, read-outs and states are about 1e-7 off (2-norms), as the walk's are.
+// What bounds them now: the walk's step of 1.9 us is 1,250 cycles of the tensor pipe a scheduler and as many of shared memory (each 16
+// rows of [W; Q'] cross it once a block), one after the other, and two barriers; the preparation issues 29,000 instructions a block with two blocks
+// an SM (three, in 80 registers, spill: 76 us). 2,048 tokens, 16 heads of 128 x 128, gated delta rule: 120 us for the walk, 67 for the
+// preparation (as plain multiply-adds, bound by shared-memory reads, 209 and 105; token by token 704). A chunk's matrices come as one
+// bulk copy: 22 cp.async a thread held the products' own reads up (208 us), 32 small bulk copies for the rows of V' cost their warp
+// 1,700 cycles a step (163 us), so those rows come through registers, a chunk ahead.
+// A number that is not finite has no parts to multiply (0 times infinity would reach back to earlier tokens): a chunk that meets one
+// in its matrices, in S or in U takes plain multiply-adds instead, over the same operands.
 #include "chunked_recurrence.h"
 
 #include "common.cuh"
+#include "tcgen05_ops.cuh"
 
 using namespace sb;
+typedef __nv_bfloat16 bf16;
 
 namespace {
 
 constexpr int CH = 32;                 // tokens of a chunk
 constexpr int VC = 16;                 // columns of S a block of the walk takes
 constexpr int THREADS = 256;
-constexpr int TP = CH + 4;             // pitch of a [row][token] tile
+constexpr int TP = CH + 4;             // pitch of a [row][token] tile of floats
+constexpr int PP = CH + 8;             // pitch of the parts of P
 enum { MODE_DECAY = 0, MODE_SSM = 1, MODE_DELTA = 2, MODE_WKV = 3, MODE_GLA = 4, MODE_RET = 5 };
 
-// floats of one (chunk, head) in the work space: Q' and K'' (and W) [32][DKT], P [32][32], c [2][DKT]: the float nearest to the product
-// of the decays and what that leaves (a fixed decay's c is off the same way in every chunk, which would add up)
-__host__ __device__ constexpr int part_floats(int dkt, bool delta) { return (delta ? 3 : 2) * CH * dkt + CH * CH + 2 * dkt; }
+// What the preparation leaves of a (chunk, head), as the walk's shared memory holds it: the three parts of [W; Q'] (or Q'), of K'' and
+// of P, each row 16 bytes longer than it is; c as the float nearest to the product of the decays and what that leaves (a fixed
+// decay's c is off the same way in every chunk, which would add up); four ints, the first not zero if something is not finite.
+template <int DKT, bool DELTA>
+struct Part {
+  static constexpr int ROWS = DELTA ? 2 * CH : CH, AP = DKT + 8;
+  static constexpr int K_OFF = 3 * ROWS * AP, P_OFF = K_OFF + 3 * CH * AP, C_OFF = P_OFF + 3 * CH * PP;      // bf16 numbers
+  static constexpr int BYTES = C_OFF * 2 + 2 * DKT * 4 + 16;
+};
+__host__ __device__ constexpr long long part_bytes(int dkt, bool delta) {
+  return dkt == 64 ? (delta ? Part<64, true>::BYTES : Part<64, false>::BYTES) : (delta ? Part<128, true>::BYTES : Part<128, false>::BYTES);
+}
 
 struct Place { int row, t0, n, n_chunks; long long slot; };
+
+// Two numbers in three parts each (the first in the low halves), h + m + l = x exactly. A float beyond the largest bfloat16 leaves more to
+// m; of one that is not finite m is not finite.
+__device__ __forceinline__ float2 unpack(uint32_t u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t packed(float x, float y) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
+  constexpr float MOST = 3.3895313892515355e38f;
+  p[0] = packed(fminf(fmaxf(x, -MOST), MOST), fminf(fmaxf(y, -MOST), MOST));
+  const float2 h = unpack(p[0]);
+  x -= h.x;
+  y -= h.y;
+  p[1] = packed(x, y);
+  const float2 m = unpack(p[1]);
+  p[2] = packed(x - m.x, y - m.y);
+}
+__device__ __forceinline__ float whole(float h, float m, float l) { return fabsf(m) < INFINITY ? h + (m + l) : m; }
+// the two numbers whose parts lie ``plane`` apart from p on
+__device__ __forceinline__ float2 joined2(const bf16* p, int plane) {
+  const float2 h = unpack(*reinterpret_cast<const uint32_t*>(p)), m = unpack(*reinterpret_cast<const uint32_t*>(p + plane)),
+               l = unpack(*reinterpret_cast<const uint32_t*>(p + 2 * plane));
+  return make_float2(whole(h.x, m.x, l.x), whole(h.y, m.y, l.y));
+}
+__device__ __forceinline__ float joined(const bf16* p, int plane) {
+  return whole(__bfloat162float(p[0]), __bfloat162float(p[plane]), __bfloat162float(p[2 * plane]));
+}
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) < INFINITY; }
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// acc[n] += the product of 32 terms, in two slices of 16 with sums of their own: 2 NT chains of six products side by side.
+// b[..][..][2 n, 2 n + 1]: columns n.
+template <int NT>
+__device__ __forceinline__ void product32(float (&acc)[NT][4], const uint32_t (&a)[2][3][4], const uint32_t (&b)[2][3][2 * NT]) {
+  float t[2][NT][4] = {};
+  constexpr int LEFT[6] = {2, 0, 1, 1, 0, 0}, RIGHT[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+  for (int i = 0; i < 6; ++i)
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+      for (int n = 0; n < NT; ++n) mma(t[k][n], a[k][LEFT[i]], b[k][RIGHT[i]][2 * n], b[k][RIGHT[i]][2 * n + 1]);
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[n][e] += t[k][n][e];
+}
 
 // Where entry i's chunk c lies: false if there is none (the whole block). The chunks of the entries before it are counted by the block.
 __device__ __forceinline__ bool find_chunk(const SbChunkedWalk& a, int i, int c, Place& p, int* red) {
@@ -62,36 +146,28 @@ __device__ __forceinline__ bool find_chunk(const SbChunkedWalk& a, int i, int c,
 }
 
 template <int DKT>
-constexpr int prep_floats(bool vec) { return (vec ? 3 : 2) * DKT * TP + 8 * CH * (CH + 1) + CH * TP + CH * (CH + 1) + 3 * CH; }
+constexpr int rows_smem() { return (3 * DKT * TP + 8 * CH * (CH + 1) + CH * TP + CH) * 4; }
 
-// grid (chunk, head, list entry). VEC: a decay per row of S; else one for all of it.
-template <int DKT, bool VEC, int MODE>
-__global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk a, float* __restrict__ u_rows) {
+// A decay per row of S: it sits inside the products of P and A, so those are multiply-adds here. grid (chunk, head, list entry).
+template <int DKT, int MODE>
+__global__ void __launch_bounds__(THREADS) chunk_prep_rows_kernel(const SbChunkedWalk a, float* __restrict__ u_rows) {
   constexpr bool DELTA = MODE == MODE_DELTA, WKV = MODE == MODE_WKV;
+  typedef Part<DKT, DELTA> L;
   extern __shared__ __align__(16) float sm[];
   __shared__ int red_i[8];
   float* kT = sm;                                  // [DKT][TP]
   float* qT = kT + DKT * TP;
-  float* gT = qT + DKT * TP;                       // VEC only
-  float* part = gT + (VEC ? DKT * TP : 0);         // [8 warps][CH][CH + 1]
-  float* At = part + 8 * CH * (CH + 1);            // [CH][TP]
-  float* Dm = At + CH * TP;                        // [CH][CH + 1]: product of the decays s + 1 .. t (scalar decays)
-  float* g1 = Dm + CH * (CH + 1);                  // [CH] decays, factors, products up to t (scalar decays)
-  float* fac = g1 + CH;
-  float* gam = fac + CH;
+  float* gT = qT + DKT * TP;
+  float* part = gT + DKT * TP;                     // [8 warps][CH][CH + 1]
+  float* At = part + 8 * CH * (CH + 1);            // [s][TP]: A_ts
+  float* fac = At + CH * TP;                       // [CH] beta or the bonus sum
   Place p;
   if (!find_chunk(a, blockIdx.z, blockIdx.x, p, red_i)) return;
   const int h = blockIdx.y, hq = h / (a.H / a.Hqk);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool live = lane < p.n;
   const size_t tok = (size_t)(p.t0 + lane);
-  const float f = live ? a.sc[tok * a.H + h] : 0.f;              // beta, dt or the bonus sum of token ``lane``
-  if (warp == 0) {
-    float g = 1.f;
-    if (!VEC && live) g = a.head_rate ? a.af[(tok * a.H + h) * a.dkp] : a.dec[tok * a.H + h];
-    g1[lane] = g;
-    fac[lane] = f;
-  }
+  if (warp == 0) fac[lane] = live ? a.sc[tok * a.H + h] : 0.f;
   // lane = token: the rows are read 16 bytes at a time and turned, [row of S][token]
 #pragma unroll 4
   for (int c = warp * 4; c < DKT; c += 32) {
@@ -99,24 +175,13 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
     if (live && c < a.dkp) {
       k = *reinterpret_cast<const float4*>(a.kf + (tok * a.Hqk + hq) * a.dkp + c);
       q = *reinterpret_cast<const float4*>(a.qf + (tok * a.Hqk + hq) * a.dkp + c);
-      if (VEC) g = *reinterpret_cast<const float4*>(a.af + (tok * a.H + h) * a.dkp + c);
+      g = *reinterpret_cast<const float4*>(a.af + (tok * a.H + h) * a.dkp + c);
     }
-    if (MODE == MODE_SSM) { k.x *= f; k.y *= f; k.z *= f; k.w *= f; }          // S += (dt k) v^T
     kT[c * TP + lane] = k.x; kT[(c + 1) * TP + lane] = k.y; kT[(c + 2) * TP + lane] = k.z; kT[(c + 3) * TP + lane] = k.w;
     qT[c * TP + lane] = q.x; qT[(c + 1) * TP + lane] = q.y; qT[(c + 2) * TP + lane] = q.z; qT[(c + 3) * TP + lane] = q.w;
-    if (VEC) { gT[c * TP + lane] = g.x; gT[(c + 1) * TP + lane] = g.y; gT[(c + 2) * TP + lane] = g.z; gT[(c + 3) * TP + lane] = g.w; }
+    gT[c * TP + lane] = g.x; gT[(c + 1) * TP + lane] = g.y; gT[(c + 2) * TP + lane] = g.z; gT[(c + 3) * TP + lane] = g.w;
   }
   __syncthreads();
-  if (!VEC && warp == 0) {
-    double d = 1.0, up = 1.0;                     // (products of equal factors in float would all lean the same way)
-    for (int t = 0; t < CH; ++t) {                // lane = s
-      const double g = (double)g1[t];
-      up *= g;
-      if (t > lane) d *= g;
-      Dm[t * (CH + 1) + lane] = (float)d;
-      if (lane == 0) gam[t] = (float)up;
-    }
-  }
   // lane = t, a warp takes DKT / 8 rows of S: q_t . k_s and k_t . k_s with the decays between s and t
   {
     float aq[CH], ak[DELTA ? CH : 1];
@@ -132,15 +197,15 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
       for (int s4 = CH - 4; s4 >= 0; s4 -= 4) {
         const float4 k4 = *reinterpret_cast<const float4*>(kT + c * TP + s4);
         const float kk[4] = {k4.x, k4.y, k4.z, k4.w};
-        float gg[4] = {1.f, 1.f, 1.f, 1.f};
-        if (VEC) { const float4 g4 = *reinterpret_cast<const float4*>(gT + c * TP + s4); gg[0] = g4.x; gg[1] = g4.y; gg[2] = g4.z; gg[3] = g4.w; }
+        const float4 g4 = *reinterpret_cast<const float4*>(gT + c * TP + s4);
+        const float gg[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
         for (int u = 3; u >= 0; --u) {
           const int s = s4 + u;                     // (sums of s beyond t are left out below)
-          const float x = VEC ? kk[u] * d : kk[u];
+          const float x = kk[u] * d;
           aq[s] = fmaf(qt, x, aq[s]);
           if (DELTA) ak[s] = fmaf(kt, x, ak[s]);
-          if (VEC && (WKV ? s < lane : s <= lane)) d *= gg[u];
+          if (WKV ? s < lane : s <= lane) d *= gg[u];
         }
       }
     }
@@ -155,7 +220,6 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
         float x = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) x += part[(w * CH + t) * (CH + 1) + s];
-        if (!VEC) x *= Dm[t * (CH + 1) + s];
         At[s * TP + t] = s < t ? fac[t] * x : 0.f;
       }
       __syncthreads();
@@ -164,24 +228,29 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
     for (int s = 0; s < CH; ++s) mine[s] = aq[s];
   }
   __syncthreads();
-  float* dst = a.work + ((p.slot + blockIdx.x) * a.H + h) * (long long)part_floats(DKT, DELTA);
-  float* dst_p = dst + (DELTA ? 3 : 2) * CH * DKT;
-  {
-    const float skip = MODE != MODE_SSM ? 0.f : a.skip_dtype == SB_DTYPE_F32 ? ((const float*)a.skip)[h] : to_float(((const __nv_bfloat16*)a.skip)[h]);
+  unsigned char* image = reinterpret_cast<unsigned char*>(a.work) + ((p.slot + blockIdx.x) * a.H + h) * (long long)L::BYTES;
+  bf16* img = reinterpret_cast<bf16*>(image);
+  float* img_c = reinterpret_cast<float*>(img + L::C_OFF);
+  bool bad = false;                                // something this thread leaves is not finite
+  auto leave = [&](int off, int plane, float x) {
+    uint32_t parts[3];
+    split3(x, 0.f, parts);
 #pragma unroll
-    for (int e = tid; e < CH * CH; e += THREADS) {
-      const int t = e >> 5, s = e & 31;
-      float x = 0.f;
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<unsigned short*>(img + off + i * plane) = (unsigned short)parts[i];
+    bad |= !finite(x);
+  };
 #pragma unroll
-      for (int w = 0; w < 8; ++w) x += part[(w * CH + t) * (CH + 1) + s];
-      if (!VEC) x *= Dm[t * (CH + 1) + s];
-      if (s == t) x = WKV ? fac[t] : x + skip;
-      dst_p[e] = s <= t ? x : 0.f;
-    }
+  for (int e = tid; e < CH * CH; e += THREADS) {
+    const int t = e >> 5, s = e & 31;
+    float x = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x += part[(w * CH + t) * (CH + 1) + s];
+    if (WKV && s == t) x = fac[t];
+    leave(L::P_OFF + t * PP + s, CH * PP, s <= t ? x : 0.f);
   }
   // a thread a row of S: Q' forwards with the running product of the decays, K'' backwards
   if (tid < DKT) {
-    const float *q = qT + tid * TP, *g = VEC ? gT + tid * TP : g1;
+    const float *q = qT + tid * TP, *g = gT + tid * TP;
     double up = 1.0;
 #pragma unroll
     for (int t4 = 0; t4 < CH; t4 += 4) {
@@ -190,15 +259,16 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (!WKV) up *= (double)gg[u];
-        dst[(t4 + u) * DKT + tid] = qq[u] * (float)up;
+        leave(((DELTA ? CH : 0) + t4 + u) * L::AP + tid, L::ROWS * L::AP, qq[u] * (float)up);
         if (WKV) up *= (double)gg[u];
       }
     }
-    dst_p[CH * CH + tid] = (float)up;
-    dst_p[CH * CH + DKT + tid] = (float)(up - (double)(float)up);
+    img_c[tid] = (float)up;
+    img_c[DKT + tid] = finite((float)up) ? (float)(up - (double)(float)up) : 0.f;
+    bad |= !finite((float)up);
   } else if (tid < 2 * DKT) {
     const int i = tid - DKT;
-    const float *k = kT + i * TP, *g = VEC ? gT + i * TP : g1;
+    const float *k = kT + i * TP, *g = gT + i * TP;
     double down = 1.0;
 #pragma unroll
     for (int t4 = CH - 4; t4 >= 0; t4 -= 4) {
@@ -206,7 +276,7 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
       const float kk[4] = {k4.x, k4.y, k4.z, k4.w}, gg[4] = {g4.x, g4.y, g4.z, g4.w};
 #pragma unroll
       for (int u = 3; u >= 0; --u) {
-        dst[CH * DKT + (t4 + u) * DKT + i] = kk[u] * (float)down;
+        leave(L::K_OFF + (t4 + u) * L::AP + i, CH * L::AP, kk[u] * (float)down);
         down *= (double)gg[u];
       }
     }
@@ -220,8 +290,8 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
 #pragma unroll
     for (int t = 0; t < CH; ++t) {
       if (is_k) {
-        if (VEC) up *= (double)gT[c * TP + t];
-        x[t] = fac[t] * ((VEC ? (float)up : gam[t]) * kT[c * TP + t]);
+        up *= (double)gT[c * TP + t];
+        x[t] = fac[t] * ((float)up * kT[c * TP + t]);
       } else {
         x[t] = t < p.n ? fac[t] * a.vf[((size_t)(p.t0 + t) * a.H + h) * a.dvp + j] : 0.f;
       }
@@ -239,191 +309,453 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_kernel(const SbChunkedWalk
     }
 #pragma unroll
     for (int t = 0; t < CH; ++t) {
-      if (is_k) dst[2 * CH * DKT + t * DKT + c] = x[t];
+      if (is_k) leave(t * L::AP + c, L::ROWS * L::AP, x[t]);
       else if (t < p.n) u_rows[((size_t)(p.t0 + t) * a.H + h) * a.dvp + j] = x[t];
     }
   }
+  const int any = __syncthreads_or(bad);
+  if (tid == 0) reinterpret_cast<int*>(image)[L::BYTES / 4 - 4] = any;
 }
 
-__device__ __forceinline__ void cp16(float* smem, const float* g, bool valid) {
-  const int n = valid ? 16 : 0;                    // 0: nothing is read, the 16 bytes are zeros
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g), "r"(n));
+template <int DKT>
+constexpr int head_smem() { return 6 * CH * (DKT + 8) * 2 + (CH * TP + CH * (CH + 1) + 4 * CH) * 4; }
+
+// One decay for all of S. grid (chunk, head, list entry). P and A are products of q and k as they are, the decays between the
+// two tokens a factor of each element.
+template <int DKT, int MODE>
+__global__ void __launch_bounds__(THREADS, 2) chunk_prep_head_kernel(const SbChunkedWalk a, float* __restrict__ u_rows) {
+  constexpr bool DELTA = MODE == MODE_DELTA;
+  typedef Part<DKT, DELTA> L;
+  constexpr int AP = L::AP, PL = CH * AP;          // pitch and distance of the parts of q and k
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ int red_i[8];
+  bf16 *qp = reinterpret_cast<bf16*>(raw), *kp = qp + 3 * PL;      // [3][CH][AP]
+  float* At = reinterpret_cast<float*>(kp + 3 * PL);               // [s][TP]: A_ts
+  float* Dm = At + CH * TP;                        // [CH][CH + 1]: product of the decays s + 1 .. t
+  float* g1 = Dm + CH * (CH + 1);                  // [CH] decays, factors, products up to t and from t + 1 on
+  float *fac = g1 + CH, *gup = fac + CH, *gdn = gup + CH;
+  Place p;
+  if (!find_chunk(a, blockIdx.z, blockIdx.x, p, red_i)) return;
+  const int h = blockIdx.y, hq = h / (a.H / a.Hqk);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long c_row = (long long)p.t0 * a.H + h;               // (token, head) rows are a.H apart
+  // the values this thread's column of the substitution needs: under way while everything else is made
+  float x[CH];
+  if (DELTA) {
+    const int j = tid - DKT;
+#pragma unroll
+    for (int t = 0; t < CH; ++t) x[t] = (j >= 0 && j < a.dvp && t < p.n) ? a.vf[(c_row + (long long)t * a.H) * a.dvp + j] : 0.f;
+  }
+  if (warp == 0) {
+    const bool live = lane < p.n;
+    const long long r = c_row + (long long)lane * a.H;
+    g1[lane] = !live ? 1.f : (a.head_rate ? a.af[r * a.dkp] : a.dec[r]);
+    fac[lane] = live ? a.sc[r] : 0.f;
+  }
+  // rows of q and k in parts: DKT / 4 lanes a token
+  constexpr int LPT = DKT / 4;
+#pragma unroll
+  for (int u = 0; u < CH * LPT / THREADS; ++u) {
+    const int e = tid + u * THREADS, t = e / LPT, c = (e - t * LPT) * 4;
+    float4 k = make_float4(0.f, 0.f, 0.f, 0.f), q = k;
+    if (t < p.n && c < a.dkp) {
+      const long long at = ((long long)(p.t0 + t) * a.Hqk + hq) * a.dkp + c;
+      k = *reinterpret_cast<const float4*>(a.kf + at);
+      q = *reinterpret_cast<const float4*>(a.qf + at);
+      if (MODE == MODE_SSM) {                      // S += (dt k) v^T
+        const float f = a.sc[c_row + (long long)t * a.H];
+        k.x *= f; k.y *= f; k.z *= f; k.w *= f;
+      }
+    }
+    uint32_t lo[3], hi[3];
+    split3(q.x, q.y, lo);
+    split3(q.z, q.w, hi);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(qp + i * PL + t * AP + c) = make_uint2(lo[i], hi[i]);
+    split3(k.x, k.y, lo);
+    split3(k.z, k.w, hi);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(kp + i * PL + t * AP + c) = make_uint2(lo[i], hi[i]);
+  }
+  __syncthreads();
+  // warps 0 .. 3: q k^T, 4 .. 7: k k^T (the delta rule); 16 tokens t by 16 tokens s each. Above the diagonal there is nothing to do:
+  // that warp multiplies the decays out meanwhile (in double: products of equal factors in float would all lean the same way).
+  const int m0 = (warp & 1) * 16, n0 = ((warp >> 1) & 1) * 16;
+  const bool works = n0 <= m0 && (warp < 4 || DELTA);
+  float acc[2][4] = {};
+  if (works) {
+    const bf16* left = (warp < 4 ? qp : kp) + (m0 + (lane & 15)) * AP + (lane >> 4) * 8;
+    const bf16* right = kp + (n0 + (lane >> 4) * 8 + (lane & 7)) * AP + ((lane >> 3) & 1) * 8;
+#pragma unroll 1
+    for (int kk = 0; kk < DKT; kk += 32) {
+      uint32_t av[2][3][4], bv[2][3][4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) { ldsm4(av[k][i], left + i * PL + kk + k * 16); ldsm4(bv[k][i], right + i * PL + kk + k * 16); }
+      product32(acc, av, bv);
+    }
+  } else if (warp == 2) {
+    double d = 1.0, up = 1.0, dn = 1.0;
+    for (int t = 0; t < CH; ++t) {                 // lane = s
+      const double g = (double)g1[t];
+      up *= g;
+      if (t > lane) d *= g;
+      Dm[t * (CH + 1) + lane] = (float)d;
+      if (lane == t) gup[t] = (float)up;
+      if (t > lane) dn *= g;
+    }
+    gdn[lane] = (float)dn;
+    if (lane == 0) {
+      g1[0] = (float)up;                           // c (the decays themselves are not needed any more)
+      g1[1] = finite((float)up) ? (float)(up - (double)(float)up) : 0.f;
+    }
+  }
+  __syncthreads();
+  unsigned char* image = reinterpret_cast<unsigned char*>(a.work) + ((p.slot + blockIdx.x) * a.H + h) * (long long)L::BYTES;
+  bf16* img = reinterpret_cast<bf16*>(image);
+  bool bad = false;                                // something this thread leaves is not finite
+  auto leave2 = [&](int off, int plane, float u, float v) {
+    uint32_t parts[3];
+    split3(u, v, parts);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(img + off + i * plane) = parts[i];
+    bad |= !finite(u) || !finite(v);
+  };
+  {
+    const float skip = MODE != MODE_SSM ? 0.f : a.skip_dtype == SB_DTYPE_F32 ? ((const float*)a.skip)[h] : to_float(((const bf16*)a.skip)[h]);
+    const int g = lane >> 2, c2 = (lane & 3) * 2;
+    if (warp < 4 || DELTA) {
+#pragma unroll
+      for (int n = 0; n < 2; ++n)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int t = m0 + g + 8 * r, s = n0 + n * 8 + c2;
+          const float u = acc[n][2 * r] * Dm[t * (CH + 1) + s], v = acc[n][2 * r + 1] * Dm[t * (CH + 1) + s + 1];
+          if (warp < 4) {
+            leave2(L::P_OFF + t * PP + s, CH * PP, s <= t ? (s == t ? u + skip : u) : 0.f, s + 1 <= t ? (s + 1 == t ? v + skip : v) : 0.f);
+          } else {
+            At[s * TP + t] = s < t ? fac[t] * u : 0.f;
+            At[(s + 1) * TP + t] = s + 1 < t ? fac[t] * v : 0.f;
+          }
+        }
+    }
+  }
+  // Q' and K'': two neighbouring rows of S a thread, the tokens shared out
+  constexpr int GROUPS = THREADS / (DKT / 2);
+  {
+    const int c = (tid % (DKT / 2)) * 2, first = tid / (DKT / 2) * (CH / GROUPS);
+#pragma unroll 4
+    for (int t = first; t < first + CH / GROUPS; ++t) {
+      const float2 q = joined2(qp + t * AP + c, PL), k = joined2(kp + t * AP + c, PL);
+      leave2(((DELTA ? CH : 0) + t) * AP + c, L::ROWS * AP, q.x * gup[t], q.y * gup[t]);
+      leave2(L::K_OFF + t * AP + c, CH * AP, k.x * gdn[t], k.y * gdn[t]);
+    }
+  }
+  if (tid < DKT) {
+    float* img_c = reinterpret_cast<float*>(img + L::C_OFF);
+    img_c[tid] = g1[0];
+    img_c[DKT + tid] = g1[1];
+    bad |= !finite(g1[0]);
+  }
+  if constexpr (DELTA) {
+    __syncthreads();
+    // forward substitution, a thread a column of [diag(b) K' | diag(b) V]
+    for (int c = tid; c < DKT + a.dvp; c += THREADS) {
+      const bool is_k = c < DKT;                   // (a whole warp)
+      const int j = c - DKT;
+      if (c >= THREADS) {
+#pragma unroll
+        for (int t = 0; t < CH; ++t) x[t] = t < p.n ? a.vf[(c_row + (long long)t * a.H) * a.dvp + j] : 0.f;
+      }
+#pragma unroll
+      for (int t = 0; t < CH; ++t) x[t] = fac[t] * (is_k ? gup[t] * joined(kp + t * AP + c, PL) : x[t]);
+#pragma unroll
+      for (int s = 0; s < CH - 1; ++s) {           // x[s] is final: taken out of every later one (independent of one another)
+#pragma unroll
+        for (int t4 = (s + 1) & ~3; t4 < CH; t4 += 4) {
+          const float4 a4 = *reinterpret_cast<const float4*>(At + s * TP + t4);
+          if (t4 > s) x[t4] = fmaf(-a4.x, x[s], x[t4]);
+          if (t4 + 1 > s) x[t4 + 1] = fmaf(-a4.y, x[s], x[t4 + 1]);
+          if (t4 + 2 > s) x[t4 + 2] = fmaf(-a4.z, x[s], x[t4 + 2]);
+          x[t4 + 3] = fmaf(-a4.w, x[s], x[t4 + 3]);
+        }
+      }
+      if (is_k) {
+        // neighbouring columns swap every other token, so that each stores pairs
+        const bool odd = c & 1;
+#pragma unroll
+        for (int t = 0; t < CH; t += 2) {
+          const float other = __shfl_xor_sync(0xffffffffu, odd ? x[t] : x[t + 1], 1);
+          leave2((t + (odd ? 1 : 0)) * AP + (c & ~1), L::ROWS * AP, odd ? other : x[t], odd ? x[t + 1] : other);
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < CH; ++t)
+          if (t < p.n) u_rows[(c_row + (long long)t * a.H) * a.dvp + j] = x[t];
+      }
+    }
+  }
+  const int any = __syncthreads_or(bad);
+  if (tid == 0) reinterpret_cast<int*>(image)[L::BYTES / 4 - 4] = any;
 }
 
-// The state in shared memory: rows 20 floats apart, the four 16-byte pieces of a row turned by the row, so that what a warp
-// stores (rows 0, 4, 8 .. of two columns) and what it loads (a whole row at a time) both fall into different banks.
-constexpr int SP = VC + 4;
-__device__ __forceinline__ int s_at(int row, int col) { return row * SP + ((col >> 2) ^ ((row >> 3) & 3)) * 4 + (col & 3); }
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(tc::smem_u32(dst)), "l"(src), "r"(bytes), "r"(tc::smem_u32(bar)) : "memory");
+}
+
+constexpr int FETCHER = 128;           // a thread of the walk that fetches (its warp waits for no loads of its own)
+constexpr int SP = VC + 8;             // pitch of the parts of S and U: eight rows' 16-byte pieces fall into different banks
 template <int DKT, bool DELTA>
 struct Walk {
-  static constexpr int ROWS = DELTA ? 2 * CH : CH;        // rows of [W; Q']
-  static constexpr int AP = DKT + 4;                      // their pitch: eight rows' 16-byte pieces fall into different banks
-  static constexpr int SPLITS = 8 * 32 / ROWS;            // a group of ROWS threads takes DKT / SPLITS rows of S
-  static constexpr int K_OFF = ROWS * AP, P_OFF = K_OFF + CH * DKT, U_OFF = P_OFF + CH * TP, C_OFF = U_OFF + CH * VC, STAGE = C_OFF + 2 * DKT;
-  static constexpr int FLOATS = 2 * STAGE + DKT * SP + SPLITS * ROWS * VC + 2 * CH * VC;
+  typedef Part<DKT, DELTA> L;
+  static constexpr int STAGE = L::BYTES, S_OFF = 2 * STAGE, UP_OFF = S_OFF + 3 * DKT * SP * 2,
+                       PART_OFF = UP_OFF + 3 * CH * SP * 2;
+  static constexpr int US_OFF = PART_OFF + THREADS * 16, BYTES = US_OFF + CH * VC * 4;
 };
 
-// grid (ceil(dv / 16), head, list entry)
+// grid (ceil(dv / 16), head, list entry). Warps 0 .. 3 make U, 4 .. 7 read out; all of them the next S.
 template <int DKT, bool DELTA>
 __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const SbChunkedWalk a, const float* __restrict__ u_rows) {
   typedef Walk<DKT, DELTA> W;
-  extern __shared__ __align__(16) float sm[];
+  typedef Part<DKT, DELTA> L;
+  constexpr int AP = L::AP, ROWS = L::ROWS, SPL = DKT * SP, UPL = CH * SP;
+  extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int red_i[8];
-  float* Ss = sm + 2 * W::STAGE;                          // [DKT][SP]
-  float* part = Ss + DKT * SP;                            // [SPLITS][ROWS][VC]
-  float* Us = part + W::SPLITS * W::ROWS * VC;            // [CH][VC]
-  float* Rs = Us + CH * VC;                               // [CH][VC]: Q' S
+  __shared__ __align__(8) uint64_t full[2];
+  __shared__ int gave_up;
+  bf16* Sp = reinterpret_cast<bf16*>(raw + W::S_OFF);              // [3][DKT][SP]
+  bf16* Up = reinterpret_cast<bf16*>(raw + W::UP_OFF);             // [3][CH][SP]
+  float4* part = reinterpret_cast<float4*>(raw + W::PART_OFF);     // [warp][lane]: what the warp's neighbour adds to its sums
+  float* Us = reinterpret_cast<float*>(raw + W::US_OFF);           // [CH][VC]: U
   Place p;
   if (!find_chunk(a, blockIdx.z, 0, p, red_i)) return;
   const int h = blockIdx.y, j0 = blockIdx.x * VC;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, c2 = (lane & 3) * 2;
   const int n_all = a.cu_q[p.row + 1] - p.t0;
-  const float* tiles = a.work + (p.slot * a.H + h) * (long long)part_floats(DKT, DELTA);
-  const long long step = (long long)a.H * part_floats(DKT, DELTA);
+  const unsigned char* images = reinterpret_cast<const unsigned char*>(a.work) + (p.slot * a.H + h) * (long long)L::BYTES;
+  if (tid == 0) {
+    gave_up = 0;
+    tc::mbar_init(&full[0], 1);
+    tc::mbar_init(&full[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
 
-  auto fetch = [&](int c) {
-    float* st = sm + (c & 1) * W::STAGE;
-    const float* src = tiles + c * step;
-    for (int w = tid; w < W::ROWS * (DKT / 4); w += THREADS) {
-      const int r = w / (DKT / 4), i = (w - r * (DKT / 4)) * 4;
-      cp16(st + r * W::AP + i, src + (DELTA ? (r < CH ? 2 * CH * DKT + r * DKT : (r - CH) * DKT) : r * DKT) + i, true);
-    }
-    for (int w = tid; w < CH * DKT / 4; w += THREADS) cp16(st + W::K_OFF + w * 4, src + CH * DKT + w * 4, true);
-    const float* sp = src + (DELTA ? 3 : 2) * CH * DKT;
-    for (int w = tid; w < CH * CH / 4; w += THREADS) cp16(st + W::P_OFF + (w >> 3) * TP + (w & 7) * 4, sp + w * 4, true);
-    if (tid < DKT / 2) cp16(st + W::C_OFF + tid * 4, sp + CH * CH + tid * 4, true);
-    if (tid >= 128) {                                      // 32 rows of 64 bytes
-      const int t = (tid - 128) >> 2, i = (tid & 3) * 4;
-      const bool there = c * CH + t < n_all;
-      cp16(st + W::U_OFF + t * VC + i, u_rows + ((size_t)(p.t0 + (there ? c * CH + t : 0)) * a.H + h) * a.dvp + j0 + i, there);
-    }
-    asm volatile("cp.async.commit_group;");
+  auto fetch = [&](int c) {                                // (one thread) a chunk's image is one piece: one instruction
+    uint64_t* bar = &full[c & 1];
+    tc::mbar_expect_tx(bar, L::BYTES);
+    bulk_load(raw + (c & 1) * W::STAGE, images + (long long)c * a.H * L::BYTES, L::BYTES, bar);
   };
 
-  // this thread's part of S: four neighbouring rows i0 .. of one or two columns
-  constexpr int COLS = DKT == 128 ? 2 : 1;
-  const int i0 = ((lane & 7) + 8 * (warp & (DKT / 32 - 1))) * 4;
-  const int c0 = ((lane >> 3) + 4 * (warp / (DKT / 32))) * COLS;
+  // this warp's part of S, as accumulators: 16 rows i0 .. of 16 columns (128 rows) or of 8 (64 rows)
+  constexpr int NT = DKT == 128 ? 2 : 1;
+  const int i0 = (DKT == 128 ? warp : warp & 3) * 16, s0 = DKT == 128 ? 0 : (warp >> 2) * 8;
   float* S = a.state + (size_t)a.slots[p.row] * a.state_stride + (size_t)h * a.dk * a.dv;
-  float s[4][COLS];
+  float s[NT][4];
+  bool bad = false;                                        // something of S or U that this thread holds is not finite
+  auto keep = [&]() {                                      // S in parts, for the next product
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+    for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int c = 0; c < COLS; ++c) {
-      s[u][c] = (i0 + u < a.dk && j0 + c0 + c < a.dv) ? S[(size_t)(i0 + u) * a.dv + j0 + c0 + c] : 0.f;
-      Ss[s_at(i0 + u, c0 + c)] = s[u][c];
+      for (int r = 0; r < 2; ++r) {
+        uint32_t parts[3];
+        split3(s[n][2 * r], s[n][2 * r + 1], parts);
+        bad |= !finite(s[n][2 * r]) || !finite(s[n][2 * r + 1]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(Sp + i * SPL + (i0 + g + 8 * r) * SP + s0 + n * 8 + c2) = parts[i];
+      }
+  };
+  if (tid == FETCHER) fetch(0);
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + g + 8 * (e >> 1), j = j0 + s0 + n * 8 + c2 + (e & 1);
+      s[n][e] = (i < a.dk && j < a.dv) ? S[(size_t)i * a.dv + j] : 0.f;
     }
-  const int group = tid / W::ROWS, rg = lane & 7, cg = (lane >> 3) * 4, half = DELTA ? (warp & 1) * CH : 0;
-  fetch(0);
+  keep();
+  // two neighbouring warps share 16 rows of [W; Q'], each takes half of the rows of S; then each has the sums of 8 of the columns
+  const int mt = warp >> 1, half = warp & 1, n0 = half * 8;
+  const bool reads_out = mt >= 2;
+  const int t0 = (mt & 1) * 16, row0 = (DELTA ? mt : mt & 1) * 16;         // its tokens, their rows of [W; Q']
+  // rows of V' (or v) of the warps that make U, a chunk ahead in registers
+  float2 u_next[2];
+  auto fetch_u = [&](int c) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int t = c * CH + t0 + g + 8 * r;
+      u_next[r] = make_float2(0.f, 0.f);
+      if (t < n_all) u_next[r] = *reinterpret_cast<const float2*>(u_rows + ((size_t)(p.t0 + t) * a.H + h) * a.dvp + j0 + n0 + c2);
+    }
+  };
+  if (!reads_out) fetch_u(0);
   for (int c = 0; c < p.n_chunks; ++c) {
-    asm volatile("cp.async.wait_group 0;");
-    __syncthreads();                                       // the chunk's tiles and S are there; the other stage is free
-    if (c + 1 < p.n_chunks) fetch(c + 1);
-    const float* st = sm + (c & 1) * W::STAGE;
+    if (!tc::mbar_wait(&full[c & 1], (c >> 1) & 1)) gave_up = 1;
+    const bool slow_s = __syncthreads_or(bad) != 0;        // the chunk's matrices and S are there; the other stage is free
+    if (gave_up) {                                         // (all of the block; nothing else is in flight)
+      if (tid == 0) {
+        tc::mbar_wait(&full[c & 1], (c >> 1) & 1);
+        if (a.timeouts) atomicAdd(a.timeouts, 1);
+      }
+      return;
+    }
+    if (tid == FETCHER && c + 1 < p.n_chunks) fetch(c + 1);
+    const unsigned char* st = raw + (c & 1) * W::STAGE;
+    const bf16* A1 = reinterpret_cast<const bf16*>(st);
+    const bf16 *Kp = A1 + L::K_OFF, *Pp = A1 + L::P_OFF;
+    const float* cc = reinterpret_cast<const float*>(A1 + L::C_OFF);
+    const bool slow1 = slow_s || reinterpret_cast<const int*>(cc + 2 * DKT)[0] != 0;
     const int n = min(CH, n_all - c * CH);
-    {
-      float acc[4][4] = {};
-#pragma unroll 4
-      for (int k = group * (DKT / W::SPLITS); k < (group + 1) * (DKT / W::SPLITS); k += 4) {
-        float4 b[4];
+    bad = false;
+    float x[4] = {0.f, 0.f, 0.f, 0.f};
+    if (DELTA || reads_out) {
+      float acc[2][4] = {};
+      const int k0 = half * (DKT / 2);
+      if (!slow1) {
+        const bf16* left = A1 + (row0 + (lane & 15)) * AP + k0 + (lane >> 4) * 8;
+        const bf16* right = Sp + (k0 + ((lane >> 3) & 1) * 8 + (lane & 7)) * SP + (lane >> 4) * 8;
+        uint32_t av[DKT / 64][2][3][4], bv[DKT / 64][2][3][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) b[u] = *reinterpret_cast<const float4*>(Ss + s_at(k + u, cg));
+        for (int k = 0; k < DKT / 32; ++k)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 x = *reinterpret_cast<const float4*>(st + (half + rg + 8 * j) * W::AP + k);
-          acc[j][0] = fmaf(x.x, b[0].x, acc[j][0]); acc[j][1] = fmaf(x.x, b[0].y, acc[j][1]); acc[j][2] = fmaf(x.x, b[0].z, acc[j][2]); acc[j][3] = fmaf(x.x, b[0].w, acc[j][3]);
-          acc[j][0] = fmaf(x.y, b[1].x, acc[j][0]); acc[j][1] = fmaf(x.y, b[1].y, acc[j][1]); acc[j][2] = fmaf(x.y, b[1].z, acc[j][2]); acc[j][3] = fmaf(x.y, b[1].w, acc[j][3]);
-          acc[j][0] = fmaf(x.z, b[2].x, acc[j][0]); acc[j][1] = fmaf(x.z, b[2].y, acc[j][1]); acc[j][2] = fmaf(x.z, b[2].z, acc[j][2]); acc[j][3] = fmaf(x.z, b[2].w, acc[j][3]);
-          acc[j][0] = fmaf(x.w, b[3].x, acc[j][0]); acc[j][1] = fmaf(x.w, b[3].y, acc[j][1]); acc[j][2] = fmaf(x.w, b[3].z, acc[j][2]); acc[j][3] = fmaf(x.w, b[3].w, acc[j][3]);
-        }
-      }
+          for (int i = 0; i < 3; ++i) {
+            ldsm4(av[k >> 1][k & 1][i], left + i * ROWS * AP + k * 16);
+            ldsm4_t(bv[k >> 1][k & 1][i], right + i * SPL + k * 16 * SP);
+          }
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<float4*>(part + ((size_t)group * W::ROWS + half + rg + 8 * j) * VC + cg) = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
-    }
-    __syncthreads();
-    if (tid < W::ROWS * 4) {
-      const int r = tid >> 2, i = (tid & 3) * 4;
-      float4 x = *reinterpret_cast<const float4*>(part + r * VC + i);
-#pragma unroll
-      for (int g = 1; g < W::SPLITS; ++g) {
-        const float4 y = *reinterpret_cast<const float4*>(part + ((size_t)g * W::ROWS + r) * VC + i);
-        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-      }
-      if (DELTA && r < CH) {
-        const float4 v = *reinterpret_cast<const float4*>(st + W::U_OFF + r * VC + i);
-        x = r < n ? make_float4(v.x - x.x, v.y - x.y, v.z - x.z, v.w - x.w) : make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(Us + r * VC + i) = x;
+        for (int k = 0; k < DKT / 64; ++k) product32(acc, av[k], bv[k]);
       } else {
-        *reinterpret_cast<float4*>(Rs + (DELTA ? r - CH : r) * VC + i) = x;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int r = row0 + g + 8 * (e >> 1), col = m * 8 + c2 + (e & 1);
+            for (int k = k0; k < k0 + DKT / 2; ++k) acc[m][e] = fmaf(joined(A1 + r * AP + k, ROWS * AP), joined(Sp + k * SP + col, SPL), acc[m][e]);
+          }
       }
+      part[tid] = half ? make_float4(acc[0][0], acc[0][1], acc[0][2], acc[0][3]) : make_float4(acc[1][0], acc[1][1], acc[1][2], acc[1][3]);
+      asm volatile("bar.sync %0, 64;" ::"r"(mt + 1) : "memory");
+      const float4 y = part[tid ^ 32];
+      x[0] = (half ? acc[1][0] : acc[0][0]) + y.x;
+      x[1] = (half ? acc[1][1] : acc[0][1]) + y.y;
+      x[2] = (half ? acc[1][2] : acc[0][2]) + y.z;
+      x[3] = (half ? acc[1][3] : acc[0][3]) + y.w;
     }
-    __syncthreads();
-    const float* U = DELTA ? Us : st + W::U_OFF;
-    {
-      // the outputs: two columns of one token a thread; only tokens up to its own enter, whatever the later ones hold
-      const int t = tid >> 3, i = (tid & 7) * 2;
-      float2 o = *reinterpret_cast<const float2*>(Rs + t * VC + i);
-      const float* P = st + W::P_OFF + t * TP;
+    if (!reads_out) {
 #pragma unroll
-      for (int s4 = 0; s4 < CH; s4 += 4) {
-        const float4 w = *reinterpret_cast<const float4*>(P + s4);
-        const float ww[4] = {w.x, w.y, w.z, w.w};
+      for (int r = 0; r < 2; ++r) {
+        const int t = t0 + g + 8 * r;
+        float2 u = u_next[r];
+        if (DELTA) u = t < n ? make_float2(u.x - x[2 * r], u.y - x[2 * r + 1]) : make_float2(0.f, 0.f);
+        *reinterpret_cast<float2*>(Us + t * VC + n0 + c2) = u;
+        uint32_t parts[3];
+        split3(u.x, u.y, parts);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float2 v = *reinterpret_cast<const float2*>(U + (s4 + u) * VC + i);
-          if (s4 + u <= t) { o.x = fmaf(ww[u], v.x, o.x); o.y = fmaf(ww[u], v.y, o.y); }
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(Up + i * UPL + t * SP + n0 + c2) = parts[i];
+        bad |= !finite(u.x) || !finite(u.y);
+      }
+      fetch_u(c + 1);
+    }
+    const bool slow2 = __syncthreads_or(bad) != 0 || slow1;
+    bad = false;
+    uint32_t uv[2][3][4];                                  // the parts of U, 32 tokens by 16 columns
+    float add[NT][4] = {};
+    if (!slow2) {
+      const bf16* right = Up + (((lane >> 3) & 1) * 8 + (lane & 7)) * SP + (lane >> 4) * 8;
+      const bf16* left = Kp + ((lane >> 4) * 8 + (lane & 7)) * AP + i0 + ((lane >> 3) & 1) * 8;
+      uint32_t av[2][3][4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          ldsm4_t(uv[k][i], right + i * UPL + k * 16 * SP);
+          ldsm4_t(av[k][i], left + i * CH * AP + k * 16 * AP);
+        }
+      if constexpr (NT == 2) {
+        product32(add, av, uv);
+      } else {
+        uint32_t bv[2][3][2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) { bv[k][i][0] = s0 ? uv[k][i][2] : uv[k][i][0]; bv[k][i][1] = s0 ? uv[k][i][3] : uv[k][i][1]; }
+        product32(add, av, bv);
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < NT; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = i0 + g + 8 * (e >> 1), col = s0 + m * 8 + c2 + (e & 1);
+          for (int t = 0; t < CH; ++t) add[m][e] = fmaf(joined(Kp + t * AP + i, CH * AP), Us[t * VC + col], add[m][e]);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const float dc = cc[i0 + g + 8 * r], lo = cc[DKT + i0 + g + 8 * r];
+#pragma unroll
+      for (int m = 0; m < NT; ++m)
+#pragma unroll
+        for (int e = 2 * r; e < 2 * r + 2; ++e) s[m][e] = fmaf(dc, s[m][e], fmaf(lo, s[m][e], add[m][e]));
+    }
+    keep();
+    if (reads_out) {
+      if (!slow2) {
+        uint32_t av[2][3][4], bv[2][3][2];
+        float o[1][4] = {{x[0], x[1], x[2], x[3]}};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            ldsm4(av[k][i], Pp + i * CH * PP + (t0 + (lane & 15)) * PP + k * 16 + (lane >> 4) * 8);      // (zeros after the diagonal)
+            bv[k][i][0] = half ? uv[k][i][2] : uv[k][i][0];
+            bv[k][i][1] = half ? uv[k][i][3] : uv[k][i][1];
+          }
+        product32(o, av, bv);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x[e] = o[0][e];
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int t = t0 + g + 8 * (e >> 1);
+          for (int k = 0; k <= t; ++k) x[e] = fmaf(joined(Pp + t * PP + k, CH * PP), Us[k * VC + n0 + c2 + (e & 1)], x[e]);
         }
       }
-      if (t < n) {
-        float* dst = a.out + (size_t)(p.t0 + c * CH + t) * a.out_stride + (size_t)h * a.dv + j0 + i;
-        if (j0 + i < a.dv) dst[0] = o.x;
-        if (j0 + i + 1 < a.dv) dst[1] = o.y;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = t0 + g + 8 * (e >> 1), j = j0 + n0 + c2 + (e & 1);
+        if (t < n && j < a.dv) a.out[(size_t)(p.t0 + c * CH + t) * a.out_stride + (size_t)h * a.dv + j] = x[e];
       }
-    }
-    {
-      const float4 dc = *reinterpret_cast<const float4*>(st + W::C_OFF + i0), lo = *reinterpret_cast<const float4*>(st + W::C_OFF + DKT + i0);
-#pragma unroll
-      for (int v = 0; v < COLS; ++v) {
-        s[0][v] = fmaf(dc.x, s[0][v], lo.x * s[0][v]); s[1][v] = fmaf(dc.y, s[1][v], lo.y * s[1][v]);
-        s[2][v] = fmaf(dc.z, s[2][v], lo.z * s[2][v]); s[3][v] = fmaf(dc.w, s[3][v], lo.w * s[3][v]);
-      }
-#pragma unroll 8
-      for (int t = 0; t < CH; ++t) {
-        const float4 k = *reinterpret_cast<const float4*>(st + W::K_OFF + t * DKT + i0);
-#pragma unroll
-        for (int v = 0; v < COLS; ++v) {
-          const float x = U[t * VC + c0 + v];
-          s[0][v] = fmaf(k.x, x, s[0][v]); s[1][v] = fmaf(k.y, x, s[1][v]); s[2][v] = fmaf(k.z, x, s[2][v]); s[3][v] = fmaf(k.w, x, s[3][v]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < COLS; ++v) Ss[s_at(i0 + u, c0 + v)] = s[u][v];
     }
   }
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
+  for (int m = 0; m < NT; ++m)
 #pragma unroll
-    for (int v = 0; v < COLS; ++v)
-      if (i0 + u < a.dk && j0 + c0 + v < a.dv) S[(size_t)(i0 + u) * a.dv + j0 + c0 + v] = s[u][v];
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + g + 8 * (e >> 1), j = j0 + s0 + m * 8 + c2 + (e & 1);
+      if (i < a.dk && j < a.dv) S[(size_t)i * a.dv + j] = s[m][e];
+    }
 }
 
 template <int DKT, bool VEC, int MODE>
 int launch(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
   constexpr bool DELTA = MODE == MODE_DELTA;
-  float* u_rows = DELTA ? a.work + (long long)chunks * a.H * part_floats(DKT, DELTA) : nullptr;
-  const int most = (a.max_q + CH - 1) / CH;
-  {
-    auto k = chunk_prep_kernel<DKT, VEC, MODE>;
-    const int smem = prep_floats<DKT>(VEC) * (int)sizeof(float);
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k<<<dim3(most, a.H, a.n_list), THREADS, smem, stream>>>(a, u_rows);
-    SB_LAUNCH_CHECK();
+  float* u_rows = DELTA ? a.work + (long long)chunks * a.H * (part_bytes(DKT, DELTA) / 4) : nullptr;
+  const dim3 grid((a.max_q + CH - 1) / CH, a.H, a.n_list);
+  if constexpr (VEC) {
+    auto k = chunk_prep_rows_kernel<DKT, MODE>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem<DKT>());
+    k<<<grid, THREADS, rows_smem<DKT>(), stream>>>(a, u_rows);
+  } else {
+    auto k = chunk_prep_head_kernel<DKT, MODE>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, head_smem<DKT>());
+    k<<<grid, THREADS, head_smem<DKT>(), stream>>>(a, u_rows);
   }
+  SB_LAUNCH_CHECK();
   auto k = chunk_walk_kernel<DKT, DELTA>;
-  const int smem = Walk<DKT, DELTA>::FLOATS * (int)sizeof(float);
+  constexpr int smem = Walk<DKT, DELTA>::BYTES;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   k<<<dim3((a.dv + VC - 1) / VC, a.H, a.n_list), THREADS, smem, stream>>>(a, DELTA ? u_rows : a.vf);
   SB_LAUNCH_CHECK();
@@ -447,7 +779,7 @@ int launch_mode(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
 long long sb_chunked_walk_floats(int mode, int n_tokens, int chunks, int H, int dk, int dvp) {
   if (dk < 1 || dk > 128 || chunks < 1 || H < 1 || H > 65535) return -1;
   const bool delta = mode == MODE_DELTA;
-  return (long long)chunks * H * part_floats(dk <= 64 ? 64 : 128, delta) + (delta ? (long long)n_tokens * H * dvp : 0);
+  return (long long)chunks * H * (part_bytes(dk <= 64 ? 64 : 128, delta) / 4) + (delta ? (long long)n_tokens * H * dvp : 0);
 }
 
 int sb_chunked_walk(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {

@@ -19,6 +19,7 @@ struct SbChunkedWalk {
   int min_tokens;              // requests with at most this many tokens are left alone
   float* out;
   int out_stride;
+  int* timeouts;               // counts waits on a copy that ran out
   float* work;                 // sb_chunked_walk_floats() floats, 16-byte aligned
 };
 

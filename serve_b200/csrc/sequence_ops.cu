@@ -467,6 +467,7 @@ struct Chunked {
   int n_list, max_q, chunks;
   float* work;                 // null: every request is walked
   int walk_too;                // some requests are short
+  int* timeouts;               // counts waits on a copy that ran out
 };
 
 template <typename T, int MODE>
@@ -499,7 +500,7 @@ int launch_recurrence(RecArgs a, float* work, int n_rows, const Chunked& ch, cud
     c.skip = a.d_skip; c.skip_dtype = a.par_dtype;
     c.state = a.state; c.state_stride = a.state_stride; c.slots = a.slots; c.cu_q = a.cu_q;
     c.rows = ch.rows; c.n_list = ch.n_list; c.max_q = ch.max_q; c.min_tokens = a.max_walk;
-    c.out = a.out; c.out_stride = a.out_stride; c.work = ch.work;
+    c.out = a.out; c.out_stride = a.out_stride; c.work = ch.work; c.timeouts = ch.timeouts;
     const int rc = sb_chunked_walk(c, ch.chunks, stream);
     if (rc || !ch.walk_too) return rc;
   }
@@ -826,7 +827,7 @@ SB_EXPORT int sb_linear_recurrence(int mode, const void* q, int q_stride, const 
                                    const int* slots, const int* cu_q, float* out, int out_stride, int H, int Hqk, int dk, int dv,
                                    float q_scale, int n_rows, int n_tokens, float* work, long long state_stride, int dtype, float rate_scale,
                                    const int* positions, const float* inv_freq, int rot_dims, float k_scale, const int* token_row, int max_walk,
-                                   const int* rows, int n_list, int max_q, int chunks, float* chunk_work, int walk_too, cudaStream_t stream) {
+                                   const int* rows, int n_list, int max_q, int chunks, float* chunk_work, int walk_too, int* timeouts, cudaStream_t stream) {
   if (n_rows <= 0 || n_tokens <= 0) return 0;
   if (!work || !aligned16(work)) return SB_ERR_ALIGN;
   if (H <= 0 || Hqk <= 0 || H % Hqk || dk <= 0 || dv <= 0) return SB_ERR_SHAPE;
@@ -844,7 +845,7 @@ SB_EXPORT int sb_linear_recurrence(int mode, const void* q, int q_stride, const 
   a.positions = positions; a.inv_freq = inv_freq; a.rot_dims = rot_dims; a.k_scale = k_scale;
   a.token_row = token_row; a.max_walk = token_row ? max_walk : 0; a.prepare_all = 0;
   a.q_scale = q_scale; a.rate_scale = rate_scale; a.qf = a.kf = a.af = a.vf = a.sc = a.dec = nullptr;
-  const Chunked ch = {rows, n_list, max_q, chunks, a.max_walk > 0 ? chunk_work : nullptr, walk_too};
+  const Chunked ch = {rows, n_list, max_q, chunks, a.max_walk > 0 ? chunk_work : nullptr, walk_too, timeouts};
   if (dtype == SB_DTYPE_F32) {
     if (mode == MODE_DECAY) return launch_recurrence<float, MODE_DECAY>(a, work, n_rows, ch, stream);
     if (mode == MODE_SSM) return launch_recurrence<float, MODE_SSM>(a, work, n_rows, ch, stream);

@@ -1067,13 +1067,18 @@ class CudaKernels:
         shape = ctx.shape
         rows, n_list, chunks, chunk_work, walk_too = None, shape.rows, 0, None, 1
         if not max_walk and self.use_chunked_recurrence and shape.max_q > self.CHUNKS_FROM:
-            n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, self.CHUNKS_FROM)
-        if chunks and n_list * heads <= self.CHUNKS_PAIRS:
+            more_than = self.CHUNKS_FROM
+            n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, more_than)
+            if n_list * heads > self.CHUNKS_PAIRS:
+                more_than, chunks = self.CHUNKS_FROM_FULL, 0
+                if shape.max_q > more_than:
+                    n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, more_than)
+        if chunks:
             lib.sb_linear_recurrence_chunk_floats.restype = ctypes.c_longlong
             floats = lib.sb_linear_recurrence_chunk_floats(code, q.shape[0], chunks, heads, dk, dv)
             if 0 < floats <= self.CHUNK_SCRATCH_FLOATS:
                 chunk_work = torch.empty(floats, dtype=torch.float32, device=q.device)
-                max_walk, walk_too = self.CHUNKS_FROM, 1 if getattr(shape, "min_q", 1) <= self.CHUNKS_FROM else 0
+                max_walk, walk_too = more_than, 1 if getattr(shape, "min_q", 1) <= more_than else 0
                 self.launches += 1 + walk_too
         _check(lib.sb_linear_recurrence(
             code, _p(q), q.stride(0), _p(k), k.stride(0), _p(v), v.stride(0),
@@ -1083,16 +1088,20 @@ class CudaKernels:
             _p(out), out.stride(0), heads, qk_heads, dk, dv, ctypes.c_float(q_scale), ctx.shape.rows, q.shape[0], _p(work),
             ctypes.c_longlong(state.stride(0)), _DT[v.dtype], ctypes.c_float(rate_scale), _p(ctx.positions), _p(inv_freq), int(rot_dims),
             ctypes.c_float(k_scale), _p(ctx.token_row), max_walk, _p(rows), n_list, int(shape.max_q), chunks, _p(chunk_work), walk_too,
-            self._s()), "linear recurrence")
+            self._wait_flag() if chunks else None, self._s()), "linear recurrence")
 
     # Requests with more tokens than this go through the chunked kernels, where those take the layout.
     CHUNKED_FROM = 32
-    # The 32-bit chunked kernels shorten the chain of a long request; where many (request, head) pairs fill the SMs anyway the walk does
-    # fewer operations. Chunked | walked, a layer at width 2,048 (16 heads of 128 x 128), fixed decay and gated delta rule: one request of
-    # 64 tokens 47 | 49 and 57 | 53 us, of 128 54 | 67 and 65 | 76, of 1,000 167 | 308 and 218 | 411; 3 of 1,000 (48 pairs) 416 | 474 and
-    # 549 | 651; 8 of 256 (128 pairs) 263 | 287 and 392 | 396; 16 of 190 378 | 390 and 556 | 545.
+    # The 32-bit chunked kernels shorten the chain of a long request, but do more operations than the walk: where few (request, head) pairs
+    # leave SMs idle they pay from 97 tokens on, where the pairs fill the SMs from 161 on. Chunked | walked in us, a layer at width 2,048
+    # (16 heads of 128 x 128): fixed decay, gated delta rule with a decay a head, with a decay a channel. Below that:
+    #   1 request of 64 tokens 45 | 49, 48 | 53, 63 | 59; 4 of 97 (64 pairs) 81 | 78, 93 | 95, 117 | 108; 16 of 97 205 | 189, 246 | 259, 314 | 279
+    # at and above it:
+    #   1 of 97 50 | 60, 56 | 68, 69 | 73; 2 of 97 60 | 64, 67 | 77, 82 | 84; 8 of 161 172 | 192, 195 | 250, 254 | 268;
+    #   32 of 161 564 | 601, 679 | 845, 884 | 909; 8 of 256 237 | 286, 286 | 396, 387 | 428; 3 of 1,000 329 | 473, 375 | 651, 507 | 692
     CHUNKS_FROM = 96
     CHUNKS_PAIRS = 48
+    CHUNKS_FROM_FULL = 160
     CHUNK_SCRATCH_FLOATS = 1 << 28           # work space of the 32-bit chunked kernels at most (a GB); a larger step is walked
     use_chunked_recurrence = True            # tests: False keeps every request on the walking kernel
 

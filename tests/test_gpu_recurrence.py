@@ -98,6 +98,7 @@ SIZES = [
     ([40, 100, 33], 4, 2, 72, 16, torch.float32, False),                    # no list: requests in order
     ([2, 161, 5, 34], 3, 3, 16, 72, torch.bfloat16, True),
     ([300, 128], 2, 2, 100, 130, torch.float32, True),
+    ([161, 100, 170, 160], 26, 13, 16, 24, torch.bfloat16, True),          # many pairs: only the longest requests in chunks
 ]
 
 
@@ -127,10 +128,13 @@ def test_a_later_token_does_not_reach_back(K, mode):
     c.args[2][71, 5] = float("inf")                                        # a value inside the third chunk
     c.args[1][80, 7] = float("nan")
     out, _ = _run(K, c)
-    assert torch.equal(out[:71], first[:71])
+    assert torch.equal(out[:64], first[:64])
+    # the chunk that meets such a number takes its sums in another order: both orders are within the bound above of the exact sums
+    bound = 2 * (8 * 64 ** 0.5 * 2.0 ** -24 + 2e-7)
+    assert _error(out[64:71], first[64:71]) < bound
     heads, _, _, dv = c.dims
     clean = [j for j in range(dv) if j != 5]
-    assert torch.equal(out[71:80, clean], first[71:80, clean])             # the columns of S never meet
+    assert _error(out[71:80][:, clean], first[71:80][:, clean]) < bound    # the columns of S never meet
     assert not torch.isfinite(out[71, 5]) and torch.isnan(out[81, :dv]).all()
 
 
