@@ -563,9 +563,10 @@ __global__ void __launch_bounds__(128) gated_norm_kernel(const void* __restrict_
   }
 }
 
-// The same for the shape the recurrent read-outs have: float y, groups of a multiple of 4 up to 512 values that are all
-// normalised, the gate (one value an element, applied last) and the weight optional. A warp per (token, group); a lane
-// loads four neighbours at a time and keeps its share of the group in registers, so y and the gate are read once.
+// The same for the shape the recurrent read-outs have: float y, groups of a multiple of 4 up to 2,048 values that are all
+// normalised, the gate (one value an element) and the weight optional. A warp per (token, group), or a block of 128 threads for a
+// group of more than 512 values (WIDE); a lane loads four neighbours at a time and keeps its share of the group in registers, so y
+// and the gate are read once. Bound by memory: 2,048 rows that are one group of 2,048 (34 MB) 12.4 us, element by element and y twice 26.
 template <typename T> struct Vec4 { };
 template <> struct Vec4<float> {
   static __device__ __forceinline__ void load(const float* p, float (&o)[4]) { const float4 x = *(const float4*)p; o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = x.w; }
@@ -586,45 +587,63 @@ template <> struct Vec4<__nv_bfloat16> {
 };
 
 // LPG lanes a group (a power of two, at least gs / 16), so a warp takes 32 / LPG groups at once when they are short.
-template <typename T, typename W>
+template <typename T, typename W, bool WIDE, bool GATE_FIRST>
 __global__ void __launch_bounds__(128) gated_norm_vec_kernel(const float* __restrict__ y, int y_stride, const T* __restrict__ gate, int gate_stride,
                                                              int gate_act, const W* __restrict__ weight, int w_size, T* __restrict__ out,
                                                              int out_stride, int n_groups, int gs, int groups, int lpg, float eps, float scale) {
-  const int lane = threadIdx.x & 31, sub = lane & (lpg - 1);
-  const int gid = (blockIdx.x * 4 + (threadIdx.x >> 5)) * (32 / lpg) + lane / lpg;      // (token, group), groups fastest
+  __shared__ float red[WIDE ? 32 : 1];
+  const int lane = threadIdx.x & 31, sub = WIDE ? threadIdx.x : lane & (lpg - 1);
+  if (WIDE) lpg = 128;
+  const int gid = WIDE ? blockIdx.x : (blockIdx.x * 4 + (threadIdx.x >> 5)) * (32 / lpg) + lane / lpg;      // (token, group), groups fastest
   const bool live = gid < n_groups;                                   // (idle lanes still take part in the shuffles)
   const int t = live ? gid / groups : 0, c0 = live ? (gid - t * groups) * gs : 0;
   const float* yr = y + (size_t)t * y_stride + c0;
+  const T* gr = gate ? gate + (size_t)t * gate_stride + c0 : nullptr;
   float v[4][4];
   float ss = 0.f;
+  auto gate_of = [&](int c, float (&z)[4]) {
+    Vec4<T>::load(gr + c, z);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[i] = gate_act == 1 ? silu_f(z[i]) : sigmoid_f(z[i]);
+  };
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int c = (r * lpg + sub) * 4;
     if (live && c < gs) {
       Vec4<float>::load(yr + c, v[r]);
+      if (GATE_FIRST && gr) {
+        float z[4];
+        gate_of(c, z);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[r][i] *= z[i];
+      }
       ss += v[r][0] * v[r][0] + v[r][1] * v[r][1] + v[r][2] * v[r][2] + v[r][3] * v[r][3];
     }
   }
-  for (int o = lpg >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (WIDE) {
+    ss = block_sum(ss, red);
+  } else {
+    for (int o = lpg >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  }
   if (!live) return;
   const float inv = scale / sqrtf(ss / (float)gs + eps);
   const int w0 = weight ? c0 % w_size : 0;                            // (the weight's period is a multiple of the group)
-  const T* gr = gate ? gate + (size_t)t * gate_stride + c0 : nullptr;
   T* orow = out + (size_t)t * out_stride + c0;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int c = (r * lpg + sub) * 4;
     if (c < gs) {
-      float w[4] = {1.f, 1.f, 1.f, 1.f}, z[4];
+      float w[4] = {1.f, 1.f, 1.f, 1.f};
       if (weight) Vec4<W>::load(weight + w0 + c, w);
-      if (gr) {
-        Vec4<T>::load(gr + c, z);
+      if (!GATE_FIRST && gr) {
+        float z[4];
+        gate_of(c, z);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] *= gate_act == 1 ? silu_f(z[i]) : sigmoid_f(z[i]);
+        for (int i = 0; i < 4; ++i) w[i] *= z[i];
       }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) z[i] = v[r][i] * inv * w[i];
-      Vec4<T>::store(orow + c, z);
+      for (int i = 0; i < 4; ++i) w[i] *= v[r][i] * inv;
+      Vec4<T>::store(orow + c, w);
     }
   }
 }
@@ -878,9 +897,9 @@ SB_EXPORT int sb_gated_norm(const void* y, int y_dtype, int y_stride, const void
   const long long warps = (long long)n_tokens * groups;
   {   // the recurrent read-outs' shape on the kernel that moves 16 bytes a lane
     const int gs = C / groups, esz = dtype == SB_DTYPE_F32 ? 4 : 2, wsz = w_dtype == SB_DTYPE_F32 ? 4 : 2;
-    const bool fits = normalise && y_dtype == SB_DTYPE_F32 && gs <= 512 && gs % 4 == 0 && y_stride % 4 == 0 && out_stride % 4 == 0 &&
+    const bool fits = normalise && y_dtype == SB_DTYPE_F32 && gs <= 2048 && gs % 4 == 0 && y_stride % 4 == 0 && out_stride % 4 == 0 &&
                       aligned16(y) && (reinterpret_cast<uintptr_t>(out) % (4 * esz)) == 0 &&
-                      (!gate || (!gate_first && gate_cols == C && gate_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(gate) % (4 * esz)) == 0)) &&
+                      (!gate || (gate_cols == C && gate_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(gate) % (4 * esz)) == 0)) &&
                       (!weight || (w_size % gs == 0 && (reinterpret_cast<uintptr_t>(weight) % (4 * wsz)) == 0 &&
                                    (w_dtype == SB_DTYPE_F32 || w_dtype == SB_DTYPE_BF16))) &&
                       (dtype == SB_DTYPE_F32 || dtype == SB_DTYPE_BF16) && warps <= 0x7fff0000LL;
@@ -888,10 +907,13 @@ SB_EXPORT int sb_gated_norm(const void* y, int y_dtype, int y_stride, const void
       int lpg = 1;
       while (lpg * 16 < gs) lpg <<= 1;                                // four rounds of four values a lane cover the group
       const int per_block = 4 * (32 / lpg);
-      const unsigned nb = (unsigned)((warps + per_block - 1) / per_block);
-#define SB_GNV(T, W)                                                                                                            \
-  gated_norm_vec_kernel<T, W><<<nb, 128, 0, stream>>>((const float*)y, y_stride, (const T*)gate, gate_stride, gate_act, (const W*)weight, \
-                                                      weight ? w_size : gs, (T*)out, out_stride, (int)warps, gs, groups, lpg, eps, scale)
+      const bool wide = gs > 512;
+      const unsigned nb = wide ? (unsigned)warps : (unsigned)((warps + per_block - 1) / per_block);
+#define SB_GNV(T, W)                                                                                                                        \
+  (wide ? (gate_first ? gated_norm_vec_kernel<T, W, true, true> : gated_norm_vec_kernel<T, W, true, false>)                                 \
+        : (gate_first ? gated_norm_vec_kernel<T, W, false, true> : gated_norm_vec_kernel<T, W, false, false>))<<<nb, 128, 0, stream>>>(      \
+      (const float*)y, y_stride, (const T*)gate, gate_stride, gate_act, (const W*)weight, weight ? w_size : gs, (T*)out, out_stride, (int)warps, \
+      gs, groups, lpg, eps, scale)
       if (dtype == SB_DTYPE_F32) {
         if (w_dtype == SB_DTYPE_F32) SB_GNV(float, float); else SB_GNV(float, __nv_bfloat16);
       } else {
