@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(THREADS) chunk_prep_rows_kernel(const SbChunke
 }
 
 template <int DKT>
-constexpr int head_smem() { return 6 * CH * (DKT + 8) * 2 + (CH * TP + CH * (CH + 1) + 4 * CH) * 4; }
+constexpr int head_smem() { return 6 * CH * (DKT + 8) * 2 + (CH * TP + CH * (CH + 1) + 4 * CH + 2) * 4; }
 
 // One decay for all of S. grid (chunk, head, list entry). P and A are products of q and k as they are, the decays between the
 // two tokens a factor of each element.
@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_head_kernel(const SbChu
   float* Dm = At + CH * TP;                        // [CH][CH + 1]: product of the decays s + 1 .. t
   float* g1 = Dm + CH * (CH + 1);                  // [CH] decays, factors, products up to t and from t + 1 on
   float *fac = g1 + CH, *gup = fac + CH, *gdn = gup + CH;
+  float* c_all = gdn + CH;                         // [2] c and what the float leaves of it (not over g1: other lanes may still read it)
   Place p;
   if (!find_chunk(a, blockIdx.z, blockIdx.x, p, red_i)) return;
   const int h = blockIdx.y, hq = h / (a.H / a.Hqk);
@@ -407,8 +408,8 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_head_kernel(const SbChu
     }
     gdn[lane] = (float)dn;
     if (lane == 0) {
-      g1[0] = (float)up;                           // c (the decays themselves are not needed any more)
-      g1[1] = finite((float)up) ? (float)(up - (double)(float)up) : 0.f;
+      c_all[0] = (float)up;
+      c_all[1] = finite((float)up) ? (float)(up - (double)(float)up) : 0.f;
     }
   }
   __syncthreads();
@@ -454,9 +455,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_prep_head_kernel(const SbChu
   }
   if (tid < DKT) {
     float* img_c = reinterpret_cast<float*>(img + L::C_OFF);
-    img_c[tid] = g1[0];
-    img_c[DKT + tid] = g1[1];
-    bad |= !finite(g1[0]);
+    img_c[tid] = c_all[0];
+    img_c[DKT + tid] = c_all[1];
+    bad |= !finite(c_all[0]);
   }
   if constexpr (DELTA) {
     __syncthreads();

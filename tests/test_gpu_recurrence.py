@@ -148,3 +148,21 @@ def test_decays_that_vanish(K, mode):
     want, want_pool = _exact(c)
     out, pool = _run(K, c)
     assert _error(out, want) < 1e-5 and _error(pool, want_pool) < 1e-5
+
+
+@pytest.mark.parametrize("mode", ["ssm", "delta_head"])
+@pytest.mark.parametrize("dk", [64, 128])
+def test_first_decays_of_a_chunk(K, mode, dk):
+    """Decays that differ from token to token, those of a chunk's first two tokens far from the chunk's product and from the others: a lane
+    that read the product in the place of one of them would carry it into every later token."""
+    c = _case(mode, [1024, 97], 4, 2, dk, 32, torch.float32, seed=17)
+    rate = c.kw["aux" if mode == "ssm" else "rate"]
+    start = torch.arange(c.t, device=DEV)
+    start = torch.where(start < 1024, start, start - 1024) % 32
+    rate[start == 0] = -9.0
+    rate[start == 1] = 2.0
+    want, want_pool = _exact(c)
+    bound = 8 * dk ** 0.5 * 2.0 ** -24 + 2e-7              # as above
+    for _ in range(5):
+        out, pool = _run(K, c)
+        assert _error(out, want) < bound and _error(pool, want_pool) < bound
