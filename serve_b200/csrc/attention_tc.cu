@@ -370,6 +370,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
     float m_ref = -INFINITY;                             // what the exponentials are taken against (log2 domain)
     float l_run = 0.f;
     const int first_pos = p0 + tok0;                     // smallest position of the tile's rows
+    const int window_lo = p.window > 0 ? first_pos - p.window + 1 : 0;      // no row sees a key below it that is not kept
 
     for (int j = 0; j < n_tiles && !failed; ++j) {
       const int b = j & 1, kt = key_of(j);
@@ -444,17 +445,21 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
         *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
       l_run += sum0 + sum1;
-      // values of keys beyond the sequence (never written, or another tile's leftovers) must not meet a zero
-      // probability as NaN: the rows of this stage beyond hi are cleared
-      if (kt + BN > hi) {
+      // values that no row of the tile sees must not meet a zero probability as NaN (0 times infinity): the rows of this stage beyond
+      // hi (never written, or another tile's leftovers) are cleared, and so are those behind every row's window
+      if (kt + BN > hi || (kt < window_lo && kt + BN > p.keep)) {
         if (!mbar_wait(&kv_full[j % NS], (j / NS) & 1)) { failed = true; break; }
         unsigned char* vt = Vs + (size_t)(j % NS) * KV_BYTES;
-        const int first = hi - kt;                       // rows [first, BN)
-        for (int idx = (warp - 2) * 32 + lane; idx < (BN - first) * 8 * KA; idx += 128) {
-          const int a = idx / ((BN - first) * 8), rest = idx - a * (BN - first) * 8;
-          *reinterpret_cast<uint4*>(vt + (size_t)a * BN * 128 + (size_t)(first + (rest >> 3)) * 128 + ((rest & 7) << 4)) =
-              make_uint4(0u, 0u, 0u, 0u);
-        }
+        auto clear = [&](int first, int last) {          // rows [first, last) of the stage
+          const int n = last - first;
+          for (int idx = (warp - 2) * 32 + lane; idx < n * 8 * KA; idx += 128) {
+            const int a = idx / (n * 8), rest = idx - a * n * 8;
+            *reinterpret_cast<uint4*>(vt + (size_t)a * BN * 128 + (size_t)(first + (rest >> 3)) * 128 + ((rest & 7) << 4)) =
+                make_uint4(0u, 0u, 0u, 0u);
+          }
+        };
+        clear(max(0, p.keep - kt), min(BN, window_lo - kt));
+        clear(hi - kt, BN);
       }
       tc_fence_before();
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core

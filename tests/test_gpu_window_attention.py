@@ -56,3 +56,25 @@ def test_window_on_the_tensor_memory_path(K, case, d, shared):  # noqa: F811
     # own rounding on both sides
     top = float(torch.nan_to_num(s["vc"].float(), 0.0).abs().max())
     torch.testing.assert_close(out.float(), want.float(), atol=2.0 ** -8 * top, rtol=2.0 ** -7)
+
+
+@pytest.mark.parametrize("d,shared", [(64, False), (128, False), (256, True)])
+@pytest.mark.parametrize("page", [16, 64, 128])
+@pytest.mark.parametrize("keep", [0, 4])
+def test_numbers_no_query_sees_do_not_matter(K, d, shared, page, keep):  # noqa: F811
+    """Infinities and NaN at keys that lie behind every query's window and are not kept (beside the kept ones, and in the block of keys
+    where the window begins): the result is the one with other numbers there, bit for bit."""
+    heads, kv_heads, window = 8, 1 if shared else 2, 100
+    s = _paged_setup("bfloat16", heads, kv_heads, d, page, [200], [600])       # queries 400 .. 599 see keys from 301 on
+    if shared:
+        s["vc"] = s["kc"]
+    args = lambda: (s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, 1.0 / math.sqrt(d), window)
+    clean = torch.empty((200, heads * d), device=DEV, dtype=torch.bfloat16)
+    K.attention(s["qkv"], *args(), clean, s["shape"], keep_first=keep)
+    for key, number in ((4, float("nan")), (10, float("inf")), (63, float("-inf")), (256, float("nan")), (290, float("inf")), (300, float("nan"))):
+        for cache in (s["kc"], s["vc"]):
+            cache[int(s["bt"][0, key // page]), :, key % page] = number
+    out = torch.empty_like(clean)
+    K.attention(s["qkv"], *args(), out, s["shape"], keep_first=keep)
+    K.check_errors()
+    assert bool(torch.isfinite(clean).all()) and torch.equal(out, clean)
