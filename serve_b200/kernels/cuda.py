@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import bisect
 import ctypes
+import math
 import os
 from typing import Dict, Optional
 
@@ -131,6 +132,38 @@ def all_jobs():
     return (core_jobs() + [sequence_job(), experts_job(), projection_job()] + [attention_job(d) for d in SUPPORTED_HEAD_DIMS]
             + [talking_attention_job(d) for d in SUPPORTED_HEAD_DIMS]
             + [layer_run_job(d) for d in LAYER_RUN_HEAD_DIMS])
+
+
+# What a step of a linear recurrence costs, chunked and walked: (a, b, c, d) for
+#   a + hypot(b / 100 * longest request, (c * dv + d) / 100,000 * tokens * heads)   microseconds
+# the launches, the chain of the longest request, and the work of all (token, head) pairs on a full GPU. By what decays (one factor for the
+# state; one, with the delta rule; one a row, with the delta rule; one a row) and the rows of the state up to which a line holds. The
+# chunked kernels make a chain of tokens / 32 steps, but their work is that of 64 or 128 rows by 32 tokens whatever the state, so small
+# states of many requests are the walk's. Fitted to 1,400 steps of one to 16 requests of 97 to 1,024 tokens, 8 to 32 heads, 16 to 128 rows
+# by 16 to 256 columns; the choice they give is at most 1.2 times slower than the better one (0.4 % on average). Chunked | walked in us:
+#   1 request of 1,024 tokens, 16 heads of 64 x 64: 64 | 224, 85 | 312, 108 | 314, 71 | 241; of 128 x 128: 82 | 260, 112 | 366, 153 | 371, 107 | 278
+#   16 of 256, 16 heads of 64 x 64: 136 | 126, 232 | 194, 355 | 201, 166 | 170; of 128 x 128: 321 | 390, 423 | 647, 568 | 666, 390 | 547
+#   16 of 256, 16 heads of 16 x 64: 134 | 83, 231 | 104, 344 | 106, 140 | 84; 4 of 128, 32 heads of 64 x 64: 42 | 44, 67 | 65, 91 | 67, 49 | 54
+RECURRENCE_COST = {
+    "one": ((16, (11, 3.7, 1.4, 95), (6, 16.6, 0.1, 89)), (32, (12, 3.4, 1.5, 89), (6, 17.5, 0.9, 34)),
+            (64, (11, 3.3, 1.6, 95), (6, 20.5, 2.0, 40)), (128, (13, 2.5, 1.6, 290), (7, 22.6, 2.4, 290))),
+    "one, delta": ((16, (16, 3.4, 2.6, 177), (6, 19.3, 0.1, 127)), (32, (15, 4.1, 2.8, 154), (6, 22.0, 1.2, 58)),
+                   (64, (15, 3.7, 3.1, 142), (7, 29.0, 3.1, 62)), (128, (18, 3.8, 1.6, 441), (8, 33.8, 3.8, 465))),
+    "rows, delta": ((16, (20, 3.3, 2.6, 300), (6, 19.4, 0.1, 126)), (32, (20, 4.6, 2.9, 274), (6, 22.0, 1.2, 58)),
+                    (64, (19, 0.0, 3.4, 278), (7, 29.1, 3.2, 69)), (128, (23, 3.9, 1.4, 684), (9, 34.0, 4.1, 460))),
+    "rows": ((16, (12, 3.8, 1.5, 105), (6, 16.9, 0.2, 90)), (32, (13, 3.6, 1.4, 119), (6, 17.4, 0.9, 47)),
+             (64, (12, 2.9, 1.6, 139), (6, 22.3, 2.7, 57)), (128, (14, 2.4, 1.5, 415), (7, 24.1, 3.9, 318))),
+}
+
+
+def chunks_pay(mode: str, rate_per_head: bool, dk: int, dv: int, heads: int, longest: int, tokens: int) -> bool:
+    """Does a step of ``tokens`` tokens, the longest request bringing ``longest``, take less time 32 tokens at a time than walked?"""
+    kind = ("one, delta" if rate_per_head else "rows, delta") if mode == "delta" else ("rows" if mode in ("wkv", "gla") else "one")
+    for rows, chunked, walked in RECURRENCE_COST[kind]:
+        if dk <= rows:
+            cost = [a + math.hypot(b * longest / 100, (c * dv + d) * heads * tokens / 100000) for a, b, c, d in (chunked, walked)]
+            return cost[0] < 0.97 * cost[1]
+    return False
 
 
 class CudaKernels:
@@ -1048,8 +1081,10 @@ class CudaKernels:
         "retention": S = decay_h S + k v^T on q, k, v as they are, the first rot_dims elements of q and k rotated by the tokens'
         positions (pairs i, i + rot_dims / 2; inv_freq float [rot_dims / 2]), k times k_scale.
         out: float [T, heads * dv]. Long requests run chunk by chunk: "retention" in bfloat16 on the tensor cores
-        (csrc/chunked_retention.cu, more than CHUNKED_FROM tokens), otherwise a few requests of more than CHUNKS_FROM tokens with states
-        of at most 128 rows in 32-bit arithmetic (csrc/chunked_recurrence.cu). The others are walked token by token."""
+        (csrc/chunked_retention.cu, more than CHUNKED_FROM tokens), otherwise requests of more than CHUNKS_FROM tokens with states of at
+        most 128 rows in 32-bit arithmetic (csrc/chunked_recurrence.cu), in steps where that is the faster way (chunks_pay). The others
+        are walked token by token. Both ways differ from 64 bits by about 1e-7; which one a request takes depends on its portion's
+        length and on the step it is in, so these last bits do too."""
         max_walk = 0
         if mode == "retention" and self._chunked_retention(q, k, v, state, ctx, out, heads, dk, dv, decay, inv_freq, rot_dims, k_scale):
             if getattr(ctx.shape, "min_q", 1) > self.CHUNKED_FROM:
@@ -1066,13 +1101,10 @@ class CudaKernels:
         self.launches += 2
         shape = ctx.shape
         rows, n_list, chunks, chunk_work, walk_too = None, shape.rows, 0, None, 1
-        if not max_walk and self.use_chunked_recurrence and shape.max_q > self.CHUNKS_FROM:
-            more_than = self.CHUNKS_FROM
+        more_than = self.CHUNKS_FROM
+        if (not max_walk and self.use_chunked_recurrence and shape.max_q > more_than
+                and (not self.use_chunk_rule or chunks_pay(mode, rate_per_head, dk, dv, heads, shape.max_q, q.shape[0]))):
             n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, more_than)
-            if n_list * heads > self.CHUNKS_PAIRS:
-                more_than, chunks = self.CHUNKS_FROM_FULL, 0
-                if shape.max_q > more_than:
-                    n_list, rows, chunks = self._chunk_list(shape, q.shape[0], 32, more_than)
         if chunks:
             lib.sb_linear_recurrence_chunk_floats.restype = ctypes.c_longlong
             floats = lib.sb_linear_recurrence_chunk_floats(code, q.shape[0], chunks, heads, dk, dv)
@@ -1092,18 +1124,12 @@ class CudaKernels:
 
     # Requests with more tokens than this go through the chunked kernels, where those take the layout.
     CHUNKED_FROM = 32
-    # The 32-bit chunked kernels shorten the chain of a long request, but do more operations than the walk: where few (request, head) pairs
-    # leave SMs idle they pay from 97 tokens on, where the pairs fill the SMs from 161 on. Chunked | walked in us, a layer at width 2,048
-    # (16 heads of 128 x 128): fixed decay, gated delta rule with a decay a head, with a decay a channel. Below that:
-    #   1 request of 64 tokens 45 | 49, 48 | 53, 63 | 59; 4 of 97 (64 pairs) 81 | 78, 93 | 95, 117 | 108; 16 of 97 205 | 189, 246 | 259, 314 | 279
-    # at and above it:
-    #   1 of 97 50 | 60, 56 | 68, 69 | 73; 2 of 97 60 | 64, 67 | 77, 82 | 84; 8 of 161 172 | 192, 195 | 250, 254 | 268;
-    #   32 of 161 564 | 601, 679 | 845, 884 | 909; 8 of 256 237 | 286, 286 | 396, 387 | 428; 3 of 1,000 329 | 473, 375 | 651, 507 | 692
+    # Requests with more tokens than this may go through the 32-bit chunked kernels, if chunks_pay says so for the step; single requests of
+    # up to 64 tokens gain little there (45 us against 49 for a fixed decay, 63 against 59 for a decay a channel).
     CHUNKS_FROM = 96
-    CHUNKS_PAIRS = 48
-    CHUNKS_FROM_FULL = 160
     CHUNK_SCRATCH_FLOATS = 1 << 28           # work space of the 32-bit chunked kernels at most (a GB); a larger step is walked
     use_chunked_recurrence = True            # tests: False keeps every request on the walking kernel
+    use_chunk_rule = True                    # tests: False sends every request beyond CHUNKS_FROM through the chunked kernels
 
     def _chunk_list(self, shape, tokens: int, size: int, more_than: int):
         """(entries, the list or None, chunks) of the requests that bring more tokens than ``more_than``, in chunks of ``size``."""

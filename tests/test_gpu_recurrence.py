@@ -69,12 +69,13 @@ def _run(kernels, c, chunked=True, out_dtype=torch.float32):
     before = getattr(kernels, "use_chunked_recurrence", None)
     if before is not None:
         kernels.use_chunked_recurrence, kernels.use_chunked_retention, kernels.CHUNKS_FROM = chunked, False, 32
+        kernels.use_chunk_rule = False
     try:
         kernels.linear_recurrence(c.mode, *c.args, state, c.ctx, out, heads, qk_heads, dk, dv, **c.kw)
     finally:
         if before is not None:
             kernels.use_chunked_recurrence, kernels.use_chunked_retention = before, True
-            del kernels.CHUNKS_FROM                       # (the class's again)
+            del kernels.CHUNKS_FROM, kernels.use_chunk_rule                       # (the class's again)
     return out, pool
 
 
@@ -98,7 +99,7 @@ SIZES = [
     ([40, 100, 33], 4, 2, 72, 16, torch.float32, False),                    # no list: requests in order
     ([2, 161, 5, 34], 3, 3, 16, 72, torch.bfloat16, True),
     ([300, 128], 2, 2, 100, 130, torch.float32, True),
-    ([161, 100, 170, 160], 26, 13, 16, 24, torch.bfloat16, True),          # many pairs: only the longest requests in chunks
+    ([161, 100, 170, 160], 26, 13, 16, 24, torch.bfloat16, True),          # many pairs
 ]
 
 
