@@ -1109,7 +1109,11 @@ class CudaKernels:
             lib.sb_linear_recurrence_chunk_floats.restype = ctypes.c_longlong
             floats = lib.sb_linear_recurrence_chunk_floats(code, q.shape[0], chunks, heads, dk, dv)
             if 0 < floats <= self.CHUNK_SCRATCH_FLOATS:
-                chunk_work = torch.empty(floats, dtype=torch.float32, device=q.device)
+                try:
+                    chunk_work = torch.empty(floats, dtype=torch.float32, device=q.device)
+                except torch.cuda.OutOfMemoryError:
+                    chunk_work = None                    # (pages and weights fill the device: the walk needs no such room)
+            if chunk_work is not None:
                 max_walk, walk_too = more_than, 1 if getattr(shape, "min_q", 1) <= more_than else 0
                 self.launches += 1 + walk_too
         _check(lib.sb_linear_recurrence(
@@ -1127,7 +1131,9 @@ class CudaKernels:
     # Requests with more tokens than this may go through the 32-bit chunked kernels, if chunks_pay says so for the step; single requests of
     # up to 64 tokens gain little there (45 us against 49 for a fixed decay, 63 against 59 for a decay a channel).
     CHUNKS_FROM = 96
-    CHUNK_SCRATCH_FLOATS = 1 << 28           # work space of the 32-bit chunked kernels at most (a GB); a larger step is walked
+    # Work space of the 32-bit chunked kernels at most (a GB: 21,000 tokens of 16 heads of 128 x 128 with the delta rule, 106 MB for 2,048);
+    # a larger step is walked, and so is one for which the device has no such room left.
+    CHUNK_SCRATCH_FLOATS = 1 << 28
     use_chunked_recurrence = True            # tests: False keeps every request on the walking kernel
     use_chunk_rule = True                    # tests: False sends every request beyond CHUNKS_FROM through the chunked kernels
 

@@ -167,3 +167,22 @@ def test_first_decays_of_a_chunk(K, mode, dk):
     for _ in range(5):
         out, pool = _run(K, c)
         assert _error(out, want) < bound and _error(pool, want_pool) < bound
+
+
+@pytest.mark.parametrize("mode", ["decay", "delta"])
+def test_a_device_without_room_for_the_chunks(K, mode, monkeypatch):
+    """Pages and weights may fill the device: a step that cannot have the chunks' work space is walked."""
+    c = _case(mode, [150, 20], 2, 2, 64, 32, torch.bfloat16, seed=5)
+    want, want_pool = _run(K, c, chunked=False)
+    empty, asked = torch.empty, []
+
+    def full(*args, **kwargs):
+        asked.append(args)
+        if len(asked) == 2:                                                # (the first is the walk's own)
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*args, **kwargs)
+
+    monkeypatch.setattr(torch, "empty", full)
+    out, pool = _run(K, c)
+    monkeypatch.undo()
+    assert len(asked) == 2 and torch.equal(out, want) and torch.equal(pool, want_pool)
