@@ -186,3 +186,37 @@ def test_a_device_without_room_for_the_chunks(K, mode, monkeypatch):
     out, pool = _run(K, c)
     monkeypatch.undo()
     assert len(asked) == 2 and torch.equal(out, want) and torch.equal(pool, want_pool)
+
+
+def _in_steps(kernels, c, row, cuts):
+    """Request ``row`` of a case alone, its tokens brought in portions that end at ``cuts``."""
+    heads, _, dk, dv = c.dims
+    cu = c.ctx.cu_q.tolist()
+    outs, state, begin = [], c.pool[int(c.ctx.slots[row])][None].clone(), cu[row]
+    for end in [cu[row] + x for x in cuts] + [cu[row + 1]]:
+        one = types.SimpleNamespace(**vars(c))
+        n = end - begin
+        ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        shape = types.SimpleNamespace(rows=1, tokens=n, max_q=n, min_q=n, pure_decode=False, rows_by_q=ints([0]), neg_q_sorted=(-n,))
+        one.ctx = types.SimpleNamespace(shape=shape, cu_q=ints([0, n]), slots=ints([0]), positions=c.ctx.positions[begin:end].contiguous(),
+                                        token_row=ints([0] * n), memo={})
+        part = lambda x: x[begin:end] if torch.is_tensor(x) and x.dim() == 2 and x.shape[0] == c.t else x
+        one.args, one.kw = tuple(part(x) for x in c.args), {k: part(v) for k, v in c.kw.items()}
+        one.pool, one.t = state, n
+        out, state = _run(kernels, one)
+        outs.append(out)
+        begin = end
+    return torch.cat(outs), state
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_cuts_and_company_change_no_more_than_the_rounding(K, mode):
+    """A prompt whole beside others, alone, and in portions (chunks of its own, then walked tokens, then chunks that begin elsewhere): the
+    sums are added up in another order each time, so all of them are within the bound above of the exact ones, and no further."""
+    c = _case(mode, [333, 40, 5], 3, 3, 64, 48, torch.float32, seed=23)
+    n, bound = 333, 2 * (8 * 64 ** 0.5 * 2.0 ** -24 + 2e-7)
+    out, pool = _run(K, c)
+    state = pool[int(c.ctx.slots[0])][None]
+    for cuts in ([], [100], [7, 170, 180]):
+        alone, after = _in_steps(K, c, 0, cuts)
+        assert _error(alone, out[:n].double()) < bound and _error(after, state.double()) < bound
