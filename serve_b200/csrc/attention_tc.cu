@@ -27,10 +27,11 @@
 // At head_dim 256 keys and values are the same rows (latent attention), so a tile is loaded once for both products; with its
 // 256 output columns and two score buffers the kernel holds all of tensor memory.
 // Behind a window only the tiles that a row of the CTA can see are walked. 2,048 tokens, window 1,024: 16/4 heads of 128 95.2 us on
-// mma.sync -> 38.2; 16 heads over one row of 256 172.3 -> 51.5 (bound by the softmax threads: a warp a scheduler, about 1.3 us a tile
-// against 0.55 us of products).
+// mma.sync -> 46.0; 16 heads over one row of 256 172.3 -> 61.0 (bound by the softmax threads: a warp a scheduler, about 1.3 us a tile
+// against 0.55 us of products, 0.8 with both parts of the probabilities).
 // The recurrences are those of serve/kernels/attn_prefill.py:58-72 with exp2 and a folded log2(e)
-// (attn_prefill.py:330-331); probabilities are rounded to bfloat16 before the second product (attn_prefill.py:71).
+// (attn_prefill.py:330-331); probabilities are rounded to bfloat16 before the second product (attn_prefill.py:71),
+// or split into two (FINE, below).
 // Every wait is bounded; a wait that runs out raises *error and the CTA still frees its tensor memory.
 #include <cuda.h>
 
@@ -50,15 +51,31 @@ constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;
 constexpr int BM = 128;              // rows per CTA
 constexpr int BN = 64;               // keys per tile (one 128-byte row of probabilities: one k-block of P)
 constexpr int NS = 3;                // key/value stages
-constexpr int NP = 2;                // buffers of probabilities
-constexpr int BT_CACHE = 1024;       // block-table entries kept in shared memory
+constexpr int BT_CACHE = D == 256 ? 512 : 1024;       // block-table entries kept in shared memory
 constexpr int THREADS = 192;
 constexpr uint32_t TMEM_COLS = D == 256 ? 512 : 256;  // S0, S1 (BN columns each), O (D), rounded up to a power of two
 constexpr unsigned WAIT_LIMIT = 1u << 26;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int Q_BYTES = BM * D * 2, KV_BYTES = BN * D * 2, P_BYTES = BM * BN * 2;
-constexpr int TILE_BYTES = Q_BYTES + (SHARED ? 1 : 2) * NS * KV_BYTES + NP * P_BYTES;  // 96, 160 and 192 KB at head_dim 64, 128 and 256
-constexpr int SMEM_BYTES = TILE_BYTES + 256 + BT_CACHE * 4;             // + barriers + table entries; two CTAs fit an SM at head_dim 64
+
+// FINE: a probability is two bfloat16 numbers, its leading bits and what they leave, and the second product runs over both. With
+// exponentials taken against a reference that lags behind the maximum, the heaviest key of a row is not 1 but any number up to 256, so
+// its rounding (2^-9) is the result's; a kernel that follows the maximum, as attention_mma.cu does, has no error there. From 64 bits
+// (2-norms; 700 tokens, window 200, head size 128; the output's own rounding is 1.61e-3 to 1.64e-3 of it), one part | mma.sync | two
+// parts: scores of a deviation of 1 2.08e-3 | 2.00e-3 | 1.61e-3, of 2 2.10e-3 | 1.83e-3 | 1.64e-3, of 6 1.96e-3 | 1.68e-3 | 1.63e-3.
+// Following the maximum instead would rescale the accumulator in nearly every tile. What the second part costs at 2,048 tokens, window
+// 1,024: 16/4 heads of 128 35.9 -> 40.7 us (half for making it, half for its product), 16 heads over one row of 256 46.7 -> 53.4 (its
+// product). Four stages and one buffer of probabilities: 40.8 and 54.4; the second parts behind the scores of the tile after next: 48.5
+// and 62.4 (a stage comes free later, and its next load with it).
+template <bool FINE>
+struct Layout {
+  static constexpr int NP = D == 64 && FINE ? 1 : 2;    // buffers of probabilities
+  static constexpr int P_BUF = (FINE ? 2 : 1) * P_BYTES;
+  // 96 KB at head_dim 64, 160 at 128 (FINE: 192), 224 at 256
+  static constexpr int TILE_BYTES = Q_BYTES + (SHARED ? 1 : 2) * NS * KV_BYTES + NP * P_BUF;
+  static constexpr int SMEM_BYTES = TILE_BYTES + 256 + BT_CACHE * 4;    // + barriers + table entries; two CTAs fit an SM at head_dim 64
+  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of an SM");
+};
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
@@ -176,9 +193,11 @@ __device__ __forceinline__ float tanh_fast(float x) {
   return y;
 }
 
+template <bool FINE>
 __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                const __grid_constant__ CUtensorMap map_k,
                                                                const __grid_constant__ CUtensorMap map_v, const TcParams p) {
+  constexpr int NP = Layout<FINE>::NP, P_BUF = Layout<FINE>::P_BUF, TILE_BYTES = Layout<FINE>::TILE_BYTES;
   // Blocks start in the order of blockIdx.x, then y: with the heads in x, the tiles that see the most keys start first
   // for all heads. The other way round the last heads' longest tiles would start when a third of the time is over
   // and end last: 2,048 tokens, 32/8 heads took 53 us so, against 32 key tiles x ~1.1 us for the longest tile itself.
@@ -213,7 +232,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   unsigned char* Qs = base;
   unsigned char* Ks = Qs + Q_BYTES;                     // NS stages
   unsigned char* Vs = SHARED ? Ks : Ks + NS * KV_BYTES; // NS stages
-  unsigned char* Ps = Vs + NS * KV_BYTES;               // NP buffers of [128 rows][128 bytes]
+  unsigned char* Ps = Vs + NS * KV_BYTES;               // NP buffers of [128 rows][128 bytes], FINE: twice that each
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + TILE_BYTES);
   uint64_t& q_full = bars[0];
   uint64_t* kv_full = bars + 1;                         // NS: a stage's keys and values have landed
@@ -329,12 +348,23 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
         }
         tc_commit(&s_full[t & 1]);
       };
+      // O += P V: P is K-major (one block of 64 keys), FINE: both parts of it; V is MN-major, 16 keys = 2048 bytes further per step
+      auto issue_o = [&](int j) {
+        const uint32_t pa = smem_u32(Ps + (size_t)(j % NP) * P_BUF), va = smem_u32(Vs + (size_t)(j % NS) * KV_BYTES);
+#pragma unroll
+        for (int kk = 0; kk < BN / 16; ++kk) {
+          const uint64_t dv = make_desc(va + (uint32_t)(kk * 2048), BN * 128);
+          tc_mma(tmem_base + (uint32_t)(2 * BN), make_desc(pa + (uint32_t)(kk * 32), 0), dv, idesc_o, (j | kk) != 0 ? 1u : 0u);
+          if (FINE) tc_mma(tmem_base + (uint32_t)(2 * BN), make_desc(pa + (uint32_t)(P_BYTES + kk * 32), 0), dv, idesc_o, 1u);
+        }
+        tc_commit(&p_empty[j % NP]);         // also: "the products up to tile j have finished"
+        tc_commit(&kv_empty[j % NS]);
+      };
       do {
         if (!mbar_wait(&q_full, 0) || !mbar_wait(&kv_full[0], 0)) { failed = true; break; }
         tc_fence_after();
         issue_s(0);
         for (int j = 0; j < n_tiles; ++j) {
-          const int b = j % NP;
           if (j + 1 < n_tiles) {
             // the next tile's scores, as soon as its keys are there and its score buffer has been read
             const int t = j + 1;
@@ -342,19 +372,9 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
             tc_fence_after();
             issue_s(t);
           }
-          if (!mbar_wait(&p_full[b], (j / NP) & 1)) { failed = true; break; }
+          if (!mbar_wait(&p_full[j % NP], (j / NP) & 1)) { failed = true; break; }
           tc_fence_after();
-          // O += P V: P is K-major (one block of 64 keys); V is MN-major, 16 keys = 2048 bytes further per step
-          const uint32_t pa = smem_u32(Ps + (size_t)b * P_BYTES), va = smem_u32(Vs + (size_t)(j % NS) * KV_BYTES);
-          const uint32_t acc = tmem_base + (uint32_t)(2 * BN);
-#pragma unroll
-          for (int kk = 0; kk < BN / 16; ++kk) {
-            const uint64_t dp = make_desc(pa + (uint32_t)(kk * 32), 0);
-            const uint64_t dv = make_desc(va + (uint32_t)(kk * 2048), BN * 128);
-            tc_mma(acc, dp, dv, idesc_o, (j | kk) != 0 ? 1u : 0u);
-          }
-          tc_commit(&p_empty[b]);            // also: "the products up to tile j have finished"
-          tc_commit(&kv_empty[j % NS]);
+          issue_o(j);
         }
       } while (false);
     }
@@ -430,19 +450,26 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       // probabilities -> shared memory (bfloat16, the swizzled K-major layout of the second product);
       // ex2(-inf) = 0 takes care of masked entries
       float sum0 = 0.f, sum1 = 0.f;
-      unsigned char* prow = Ps + (size_t)(j % NP) * P_BYTES + (size_t)row * 128;
+      unsigned char* prow = Ps + (size_t)(j % NP) * P_BUF + (size_t)row * 128;
 #pragma unroll
       for (int c = 0; c < BN / 8; ++c) {                 // 16-byte pieces of 8 keys
-        uint32_t pk[4];
+        uint32_t pk[4], rest[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float e0 = ex2(fmaf(sv[c * 8 + 2 * i], p.scale_log2, -use));
           const float e1 = ex2(fmaf(sv[c * 8 + 2 * i + 1], p.scale_log2, -use));
           sum0 += e0;
           sum1 += e1;
-          pk[i] = pack_bf16(e0, e1);
+          if (FINE) {                                    // both parts cut off, not rounded: 2^-16 of the number is left out
+            const uint32_t u0 = __float_as_uint(e0), u1 = __float_as_uint(e1);
+            pk[i] = __byte_perm(u0, u1, 0x7632);
+            rest[i] = __byte_perm(__float_as_uint(e0 - __uint_as_float(u0 & 0xffff0000u)), __float_as_uint(e1 - __uint_as_float(u1 & 0xffff0000u)), 0x7632);
+          } else {
+            pk[i] = pack_bf16(e0, e1);
+          }
         }
         *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        if (FINE) *reinterpret_cast<uint4*>(prow + P_BYTES + ((c ^ (row & 7)) << 4)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
       }
       l_run += sum0 + sum1;
       // values that no row of the tile sees must not meet a zero probability as NaN (0 times infinity): the rows of this stage beyond
@@ -575,11 +602,20 @@ SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, 
   p.window = window; p.keep = window > 0 ? keep : 0; p.deep_group = deep_group;
   const int tok_per_tile = BM / G;
   const int m_tiles = (max_q + tok_per_tile - 1) / tok_per_tile;
-  auto k = attention_tc_kernel;
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   p.heads_in_x = m_tiles <= 65535 ? 1 : 0;
   const dim3 grid = p.heads_in_x ? dim3(Hkv, m_tiles, n_rows) : dim3(m_tiles, Hkv, n_rows);
-  SB_PDL_CHECK(launch_pdl(k, grid, dim3(THREADS), (size_t)SMEM_BYTES, stream, map_q, map_k, map_v, p));
+  auto launch = [&](auto kernel, int smem) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return launch_pdl(kernel, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p);
+  };
+  // in two parts where the mma.sync kernel would be the other choice (see the dispatch in kernels/cuda.py)
+  if constexpr (SHARED) {
+    SB_PDL_CHECK(launch(attention_tc_kernel<true>, Layout<true>::SMEM_BYTES));
+  } else if (window > 0 || kc == vc) {
+    SB_PDL_CHECK(launch(attention_tc_kernel<true>, Layout<true>::SMEM_BYTES));
+  } else {
+    SB_PDL_CHECK(launch(attention_tc_kernel<false>, Layout<false>::SMEM_BYTES));
+  }
   return 0;
 }
 

@@ -798,8 +798,8 @@ class CudaKernels:
                 scratch = self._scratch_buffer(lib, shape.rows, kv_heads, num_splits)
                 tickets = self._ticket_buffer(shape.rows * kv_heads)
         # Behind a window the tensor-memory kernel walks the window's tiles and those of the kept first keys; a cap behind a window, which
-        # no design has, stays with the exact tanh of the mma.sync kernel. 2,048 tokens, window 1,024: 95 -> 38 us at head size 128, and
-        # 172 -> 52 us for shared rows of 256, all heads of a token in one tile (any grouping of them there would load the rows again).
+        # no design has, stays with the exact tanh of the mma.sync kernel. 2,048 tokens, window 1,024: 95 -> 46 us at head size 128, and
+        # 172 -> 61 us for shared rows of 256, all heads of a token in one tile (any grouping of them there would load the rows again).
         if ((which & 1) and slopes is None and not chunk and not (window and softcap > 0.0) and self.use_tcgen05_attention
                 and self._tc_attention_takes(lib, heads, all_kv_heads, head_dim, page_size, k_cache is v_cache, qkv.stride(0))):
             # prompt portions on the tensor-memory path; what is left (decoding rows) goes to the deep shape below

@@ -78,3 +78,34 @@ def test_numbers_no_query_sees_do_not_matter(K, d, shared, page, keep):  # noqa:
     K.attention(s["qkv"], *args(), out, s["shape"], keep_first=keep)
     K.check_errors()
     assert bool(torch.isfinite(clean).all()) and torch.equal(out, clean)
+
+
+@pytest.mark.parametrize("d,shared,window", [(64, False, 200), (128, False, 200), (128, True, 200), (256, True, 0), (256, True, 200)])
+@pytest.mark.parametrize("sharp", [1.0, 6.0])
+def test_no_further_from_64_bits_than_the_mma_kernel(K, d, shared, window, sharp):  # noqa: F811
+    """Scores of about unit size and so far apart that single keys have most of the weight: the error against 64 bits is at most that of the
+    mma.sync kernel (the two round at different places, so a twentieth is allowed for)."""
+    heads, kv_heads, page = 16, 1 if shared else 4, 64
+    s = _paged_setup("bfloat16", heads, kv_heads, d, page, [700], [700])
+    if shared:
+        s["vc"] = s["kc"]
+    scale = sharp / math.sqrt(d)
+    args = (s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, scale, window)
+    q = s["qkv"][:, : heads * d].view(700, heads, d).double()
+    gather = lambda cache: cache[s["bt"][0].long()].transpose(1, 2).reshape(-1, kv_heads, d)[:700].double().repeat_interleave(heads // kv_heads, 1)
+    k, v = gather(s["kc"]), gather(s["vc"])
+    at = torch.arange(700, device=DEV)
+    seen = (at[None] <= at[:, None]) & ((at[None] > at[:, None] - window) if window else True)
+    p = (torch.einsum("qhd,khd->hqk", q, k) * scale).masked_fill(~seen[None], -math.inf).softmax(-1)
+    want = torch.einsum("hqk,khd->qhd", p, v).reshape(700, heads * d)
+    errors = []
+    for tensor_memory in (True, False):
+        out = torch.empty((700, heads * d), device=DEV, dtype=torch.bfloat16)
+        K.use_tcgen05_attention = tensor_memory
+        try:
+            K.attention(s["qkv"], *args, out, s["shape"])
+        finally:
+            K.use_tcgen05_attention = True
+        errors.append(float((out.double() - want).norm() / want.norm()))
+    K.check_errors()
+    assert errors[0] <= 1.05 * errors[1], errors
