@@ -1242,8 +1242,9 @@ class CudaKernels:
         _check(lib.sb_moe_sort(_p(idx), pairs, e, tile_rows, _p(offsets), _p(order), _p(tiles), _p(n_tiles), s), "grouping by expert")
         act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
         kind = {"swiglu": 0, "clamped_swish": 1}[activation]
+        parts = out if (top == 1 and not more) else torch.empty((pairs, n), dtype=torch.float32, device=dev)
         if tensor_rows:
-            xg = torch.empty((pairs, k), dtype=h.dtype, device=dev)          # the pairs' tokens in grouped order
+            xg = self._grouped_room(parts, out, pairs, k, h)
             self.launches += 1
             _check(lib.sb_moe_gate_up_tensor(_p(h), h.stride(0), t, _p(xg), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top,
                                              pairs, e, k, ff, 1, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha),
@@ -1252,7 +1253,6 @@ class CudaKernels:
             _check(lib.sb_moe_gate_up(_p(h), h.stride(0), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs,
                                       e, k, ff, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha), _p(act),
                                       _DT[h.dtype], s), "experts, gate and up")
-        parts = out if (top == 1 and not more) else torch.empty((pairs, n), dtype=torch.float32, device=dev)
         self._experts_down(lib, act, w_down, order, offsets, tiles, n_tiles, wts, 0 if scale_input else 1, parts, tensor_rows, s)
         if more:
             self.launches += 1
@@ -1262,6 +1262,14 @@ class CudaKernels:
         elif top > 1:
             self.launches += 1
             _check(lib.sb_moe_combine(_p(parts), top, t, n, _p(out), _DT[out.dtype], s), "sum over a token's experts")
+
+    @staticmethod
+    def _grouped_room(parts, out, pairs: int, k: int, h):
+        """Room for the pairs' tokens in grouped order: the first product reads them and nothing after it, so they lie where the second
+        one leaves its float sums (2,048 tokens, 4 experts a token, width 2,048: 34 MB that a call does not take beside them)."""
+        if parts is not out and 2 * parts.shape[1] >= k:
+            return parts
+        return torch.empty((pairs, k), dtype=h.dtype, device=h.device)
 
     def _experts_down(self, lib, act, w_down, order, offsets, tiles, n_tiles, wts, scale_output, parts, tensor_rows, s) -> None:
         e, n, ff = w_down.shape
@@ -1299,8 +1307,9 @@ class CudaKernels:
                                       table.shape[0], e, top, t, _p(idx), _p(wts), _p(self.errors_tensor()), s), "expert choice by table")
         _check(lib.sb_moe_sort(_p(idx), pairs, e, tile_rows, _p(offsets), _p(order), _p(tiles), _p(n_tiles), s), "grouping by expert")
         act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
+        parts = out if top == 1 else torch.empty((pairs, n), dtype=torch.float32, device=dev)
         if tensor_rows:
-            xg = torch.empty((pairs, k), dtype=h.dtype, device=dev)
+            xg = self._grouped_room(parts, out, pairs, k, h)
             self.launches += 1
             _check(lib.sb_moe_gate_up_tensor(_p(h), h.stride(0), t, _p(xg), _p(w_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top,
                                              pairs, e, k, ff, 0, 0, 0, ctypes.c_float(0.0), ctypes.c_float(0.0), _p(act), tile_rows,
@@ -1308,7 +1317,6 @@ class CudaKernels:
         else:
             _check(lib.sb_moe_up(_p(h), h.stride(0), _p(w_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs, e, k, ff,
                                  _p(act), _DT[h.dtype], s), "experts, up")
-        parts = out if top == 1 else torch.empty((pairs, n), dtype=torch.float32, device=dev)
         self._experts_down(lib, act, w_down, order, offsets, tiles, n_tiles, wts, 1, parts, tensor_rows, s)
         if top > 1:
             self.launches += 1

@@ -82,3 +82,22 @@ def test_ungated_expert_products(tokens, k, ff, n):
             want[t] += 0.5 * (a @ w_down[e].double().T)
             most[t] += 0.5 * (a @ w_down[e].double().abs().T)
     assert ((out.double() - want).abs() <= _bound(want, most)).all()
+
+
+def test_grouped_tokens_take_no_room_of_their_own():
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    tokens, k, ff, n = 600, 512, 64, 512
+    draw = lambda *s: torch.randn(s, device="cuda")
+    x, logits = draw(tokens, k).bfloat16(), draw(tokens, E)
+    w_gu, w_down = draw(E, 2 * ff, k).bfloat16(), draw(E, n, ff).bfloat16()
+    out = torch.empty((tokens, n), device="cuda", dtype=torch.bfloat16)
+    run = lambda: kernels.routed_experts(x, logits, w_gu, w_down, TOP, out)
+    run()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    run()
+    # float sums and activations of every pair; choices, weights and the grouping's lists are a few dozen bytes a pair
+    assert torch.cuda.max_memory_allocated() - before <= TOP * tokens * (4 * n + 2 * ff + 64) + 16384
