@@ -284,10 +284,11 @@ template <int MODE, int ACCS, typename O>
 int launch(const void* w, const void* x, int n_pairs, int E, Args a, cudaStream_t stream) {
   Maps maps;
   const uint64_t K = (uint64_t)a.K;
+  // (an encoding is host time: only what the kernel may read, which chooses among the counts of outputs for up to 16 tokens alone)
   for (int i = 0; i < UNITS; ++i) {
     int rc;
+    if (i && (ACCS == 2 || a.cap > 16 || unit_outputs(MODE, i) == unit_outputs(MODE, i - 1))) { maps.w[i] = maps.w[i - 1]; continue; }
     if (ACCS == 2) {
-      if (i) { maps.w[i] = maps.w[0]; continue; }
       rc = tc::make_map_2d(&maps.w[0], w, (uint64_t)E * a.w_rows, K, K, 128);
     } else if (MODE == GATED) {
       // [expert][group of 16 outputs][gate, up][16][k]: one box is the gate and up rows of some groups, taking turns
@@ -300,7 +301,8 @@ int launch(const void* w, const void* x, int n_pairs, int E, Args a, cudaStream_
     }
     if (rc) return rc;
   }
-  for (int i = 0; i < 3; ++i) {
+  for (int i = 2; i >= 0; --i) {                    // 128 tokens only for runs of more than 64, 64 for more than 16
+    if (a.cap <= (i == 0 ? 64 : (i == 1 ? 16 : 0))) { maps.x[i] = maps.x[i + 1]; continue; }
     const int rc = tc::make_map_2d(&maps.x[i], x, (uint64_t)n_pairs, K, K, i == 0 ? 128 : (i == 1 ? 64 : 16));
     if (rc) return rc;
   }
