@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
         __syncwarp();
       }
     }
+    // a wait that ran out: the copies under way land before the block's shared memory is given back (every other wait fails first)
+    for (int f = max(0, it - a.stages); failed && f < it; ++f) tc::mbar_wait(&full_bar[f % a.stages], (f / a.stages) & 1);
   } else if (warp == 1) {
     if (lane == 0) {
       int it = 0, local = 0;
