@@ -134,6 +134,22 @@ def all_jobs():
             + [layer_run_job(d) for d in LAYER_RUN_HEAD_DIMS])
 
 
+def short_on_mma(longest: int, group: int, keys: int, decoding_too: bool, pairs: int, places: int) -> bool:
+    """Windowed or shared-row prompt portions that the mma.sync kernel takes sooner than the tensor-memory kernel: none of more than 64 rows
+    (one tile of the former, half of one of the latter), at most ``keys`` keys a query, ``pairs`` (request, kv head) pairs (0: one row for
+    all heads), ``places`` tiles of the tensor-memory kernel on the GPU at a time."""
+    # Beside requests of the decoding shape the mma.sync kernel takes both in one call from the host, which costs 5 us less (window, requests
+    # of 12, 3 and 8 tokens: 19.9 us of host time against 14.7, 16.4 us on the device against 17.7), more than it loses while there are no
+    # more than 64 keys. With more tiles than places the tensor-memory kernel runs a second, half empty round where the mma.sync kernel's
+    # tiles still fit once (it has twice the places). Head size 128, 148 places, tensor memory | mma.sync:
+    #   6 to 16 tokens, 16 keys: 128 pairs 7.5 | 9.1 us, 160 13.2 | 10.3, 256 14.4 | 10.7, 320 19.8 | 17.3, 512 27.5 | 19.4
+    #   144 keys: 128 pairs 10.4 | 14.4, 160 17.7 | 17.3, 256 19.4 | 17.7, 320 27.2 | 31.0, 512 37.4 | 32.9;  416 keys: 256 pairs 26.4 | 28.5
+    # and at 64 (296 places), 144 keys: 296 pairs 11.2 | 12.4, 320 17.7 | 13.6. One row for all heads is never faster on mma.sync.
+    if longest * group > 64:
+        return False
+    return (decoding_too and keys <= 64) or (keys <= 256 and -(-pairs // places) > 1.75 * -(-pairs // (2 * places)))
+
+
 # What a step of a linear recurrence costs, chunked and walked: (a, b, c, d) for
 #   a + hypot(b / 100 * longest request, (c * dv + d) / 100,000 * tokens * heads)   microseconds
 # the launches, the chain of the longest request, and the work of all (token, head) pairs on a full GPU. By what decays (one factor for the
@@ -800,7 +816,12 @@ class CudaKernels:
         # Behind a window the tensor-memory kernel walks the window's tiles and those of the kept first keys; a cap behind a window, which
         # no design has, stays with the exact tanh of the mma.sync kernel. 2,048 tokens, window 1,024: 95 -> 46 us at head size 128, and
         # 172 -> 61 us for shared rows of 256, all heads of a token in one tile (any grouping of them there would load the rows again).
+        shared = k_cache is v_cache
         if ((which & 1) and slopes is None and not chunk and not (window and softcap > 0.0) and self.use_tcgen05_attention
+                and not ((window or shared) and short_on_mma(
+                    shape.max_q, group, min(shape.max_kv, window + shape.max_q + keep_first) if window else shape.max_kv, bool(which & 2),
+                    0 if shared else (n_wide if wide_rows is not None else shape.rows) * kv_heads,
+                    self.TARGET_BLOCKS * (2 if head_dim == 64 else 1)))
                 and self._tc_attention_takes(lib, heads, all_kv_heads, head_dim, page_size, k_cache is v_cache, qkv.stride(0))):
             # prompt portions on the tensor-memory path; what is left (decoding rows) goes to the deep shape below
             self.launches += 1
