@@ -415,8 +415,7 @@ __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const float* 
 
 SB_EXPORT int sb_attention_simt_head_dim() { return D; }
 
-// ``slopes`` (float [H] or null), ``chunk`` (0: none), ``softcap`` (0: none)
-// and ``sinks`` (float [H] or null).
+// Options of the scores: ``slopes`` (float [H] or null), ``chunk`` (0: none), ``softcap`` (0: none), ``sinks`` (float [H] or null)
 // and ``keep`` (0: none; with a window: the keys below it stay visible to every later query). ``n_splits`` > 1: the keys of a
 // decoding request are shared out over that many blocks; ``scratch`` then holds n_rows * Hkv * n_splits * 16 * (D + 2) floats.
 SB_EXPORT int sb_attention_simt_keep(const void* qkv, int q_stride, const void* kc, const void* vc, const int* block_table,

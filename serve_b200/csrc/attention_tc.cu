@@ -553,7 +553,7 @@ int encode4(CUtensorMap* map, const void* basep, const cuuint64_t dims[4], const
 
 }  // namespace
 
-// 1 if sb_attention_tc takes this geometry (else the caller uses the mma.sync kernel). shared: keys and values are one tensor.
+// 1 if sb_attention_tc_opts takes this geometry (else the caller uses the mma.sync kernel). shared: keys and values are one tensor.
 SB_EXPORT int sb_attention_tc_supports(int H, int Hkv, int ps, int shared, int q_stride) {
   if (H <= 0 || Hkv <= 0 || H % Hkv) return 0;
   const int G = H / Hkv;
@@ -617,13 +617,6 @@ SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, 
     SB_PDL_CHECK(launch(attention_tc_kernel<false>, Layout<false>::SMEM_BYTES));
   }
   return 0;
-}
-
-SB_EXPORT int sb_attention_tc(const void* qkv, int q_stride, int n_tokens, const void* kc, const void* vc, const int* block_table,
-                              int bt_width, const int* cu_q, const int* kv_len, int H, int Hkv, int ps, int num_pages, float scale,
-                              void* out, int n_rows, int max_q, const int* rows, int* error, cudaStream_t stream) {
-  return sb_attention_tc_opts(qkv, q_stride, n_tokens, kc, vc, block_table, bt_width, cu_q, kv_len, H, Hkv, ps, num_pages, scale, out,
-                              n_rows, max_q, rows, error, 0.f, nullptr, 0, 0, H / Hkv, stream);
 }
 
 #else

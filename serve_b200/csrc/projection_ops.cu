@@ -434,12 +434,10 @@ __global__ void __launch_bounds__(128) few_rows_batched_kernel(const __nv_bfloat
 // together) by the root mean square over their H * dim (G * dim) true elements and multiply by a float weight laid out
 // like the padded projection; rotate the first ``rot`` elements of every query and key head, element i with i + rot / 2,
 // by the angle position * inv_freq[i]; queries to q_out [T, H * D], keys and values to their page. Everything is float
-// until the one rounding at the store. The row (with its bias) and the token's cosines and sines are kept in shared
-// memory, so the sums are read from memory once (rows of up to 200 KB). With head_norm every query and key head is
-// instead divided, after its rotation, by its own root mean square over its dim true elements, without a weight. With
-// keys_are_values the row ends with the keys, [T, (H + G) * D], and the value pages take the keys as projected, before norm and
-// rotation.
-// The same for rows of whole 16-byte pieces (D a multiple of 8, rot of 8 and rot - D too) without a norm of single heads: an
+// until the one rounding at the store. With keys_are_values the row ends with the keys, [T, (H + G) * D], and the value pages take
+// the keys as projected, before norm and rotation.
+//
+// For rows of whole 16-byte pieces (D and rot multiples of 8) without a norm of single heads: an
 // item is eight elements of a head, four rotated ones and their four partners or eight plain ones, so a thread turns what it
 // has loaded itself and the row never goes through shared memory; the block meets once, for the two sums and the angles. ITEMS
 // a thread (all their loads are under way together). What bounds it is the memory: 3,072 float sums a token in, as many
@@ -537,6 +535,9 @@ __global__ void __launch_bounds__(512) qk_prepare_vec_kernel(
   }
 }
 
+// The general form: the row (with its bias) and the token's cosines and sines are kept in shared memory, so the sums are read from
+// memory once (rows of up to 200 KB). With head_norm every query and key head is divided, after its rotation, by its own root mean
+// square over its dim true elements, without a weight, instead of all of them together.
 template <typename T>
 __global__ void __launch_bounds__(512) qk_prepare_kernel(
     const float* __restrict__ sums, int stride, const float* __restrict__ bias, const int* __restrict__ positions,
@@ -818,7 +819,11 @@ SB_EXPORT int sb_qk_prepare(const float* sums, int stride, const float* bias, co
   if (head_norm == 0 && D % 8 == 0 && rot % 8 == 0 && (D - rot) % 8 == 0 && items <= 8 * 512 && stride % 4 == 0 && q_stride % 4 == 0 && aligned16(sums) &&
       aligned16(q_out) && (!bias || aligned16(bias)) && (!q_weight || aligned16(q_weight)) && (!k_weight || aligned16(k_weight)) &&
       (G == 0 || (aligned16(kc) && aligned16(vc)))) {
-    // few tokens: an item a thread; many: more items a thread and smaller blocks, whose starts and ends overlap
+    // Few tokens: an item a thread; many: more items a thread and smaller blocks, whose starts and ends overlap. With 1 | 2 | 4 | 8 items a
+    // thread, us (heads of 128, 64 turned): 8 tokens of 16/4 heads (384 items) 3.7 | 4.1 | 5.4 | 6.2, of 32/8 (768) 9.5 | 4.5 | 5.4 | 7.0,
+    // of 64/8 (1,280; one and two items need more than 512 threads: the kernel below) 13.0 | 13.2 | 5.8 | 7.4; 2,048 tokens 13.6 | 11.9 |
+    // 12.3 | 12.7, 47.1 | 24.2 | 18.2 | 21.5 and 97.8 | 97.8 | 39.0 | 44.5; 4,096 of 16/4 24.6 | 20.9 | 17.7 | 22.7. (Between 296 and 600
+    // tokens of up to 512 items one or two would be 1 us faster, beyond 1,024 items four 12 %.)
     const int per = n_tokens >= 2 * sm_count() ? (items > 1024 ? 8 : 4) : (items <= 512 ? 1 : (items <= 1024 ? 2 : 8));
     const int least = ((rot / 2 > (items + per - 1) / per ? rot / 2 : (items + per - 1) / per) + 31) & ~31;
     if (least <= 512) {

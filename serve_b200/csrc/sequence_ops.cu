@@ -818,7 +818,6 @@ SB_EXPORT int sb_causal_conv(const void* x, int x_stride, const void* w, const v
   return 0;
 }
 
-// Floats of work space sb_linear_recurrence needs for a step of n_tokens tokens.
 // Floats of chunk_work, or -1 if requests of these sizes are walked.
 SB_EXPORT long long sb_linear_recurrence_chunk_floats(int mode, int n_tokens, int chunks, int H, int dk, int dv) {
   if (dk <= 0 || dk > 128 || dv <= 0) return -1;
@@ -826,6 +825,7 @@ SB_EXPORT long long sb_linear_recurrence_chunk_floats(int mode, int n_tokens, in
   return sb_chunked_walk_floats(mode, n_tokens, chunks, H, dk, (dv + VC - 1) / VC * VC);
 }
 
+// Floats of work space sb_linear_recurrence needs for a step of n_tokens tokens.
 SB_EXPORT long long sb_linear_recurrence_work_floats(int mode, int n_tokens, int H, int Hqk, int dk, int dv) {
   if (dk <= 0 || dk > 32 * REC_RPT) return -1;
   return rec_work_floats(mode, n_tokens, H, Hqk, dk, dv);

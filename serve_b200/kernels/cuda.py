@@ -728,19 +728,17 @@ class CudaKernels:
         """``slopes`` (float [heads]): slope_h * distance is taken off every score; ``chunk`` > 0: a query sees only the keys of
         its own block of ``chunk`` positions; ``softcap`` c > 0: a scaled score s becomes c * tanh(s / c); ``sinks`` (float
         [heads]): exp(sink_h) joins the softmax's denominator; ``keep_first`` n > 0 (with a window): the sequence's first n keys
-        stay visible to every later query. In bfloat16 all run on the mma.sync kernels; cap and sink
-        also on the tensor-memory kernel (prompt portions at head sizes 64 and 128); in float32 on the plain-arithmetic kernel."""
+        stay visible to every later query. In bfloat16 prompt portions run on the tensor-memory kernel where it takes the sizes (head
+        sizes 64 and 128, and 256 where keys and values are one tensor; any window, kept keys, a sink, a cap without a window), the
+        others, slopes, chunks and decoding on the mma.sync kernels; float32 runs on the plain-arithmetic kernels, where a decoding
+        request's keys are shared out over as many blocks as the step leaves it (so the last bits depend on the step)."""
         lib = self._attention_lib(head_dim)
         softcap = float(softcap or 0.0)
         keep_first = int(keep_first or 0) if window else 0
-        opts = slopes is not None or chunk or softcap > 0.0 or sinks is not None or keep_first > 0
-        if opts and qkv.dtype == torch.bfloat16 and not self.force_simt_attention:
+        if qkv.dtype == torch.bfloat16 and not self.force_simt_attention:
             return self._attention_mma(lib, qkv, k_cache, v_cache, block_table, cu_q, kv_len, heads, kv_heads, head_dim,
                                        page_size, scale, window, out, shape, slopes=slopes, chunk=int(chunk), softcap=softcap, sinks=sinks,
                                        keep_first=keep_first)
-        if not opts and qkv.dtype == torch.bfloat16 and not self.force_simt_attention:
-            return self._attention_mma(lib, qkv, k_cache, v_cache, block_table, cu_q, kv_len, heads, kv_heads, head_dim,
-                                       page_size, scale, window, out, shape)
         group = heads // kv_heads
         # requests of at most 16 rows run in the decoding shape, the others in tiles: one launch each, as needed. The keys of the
         # former are shared out so that two blocks fit every SM.
