@@ -463,6 +463,11 @@ size_t wide_smem_bytes(bool shared_kv) { return (size_t)(64 + 2 * (shared_kv ? 1
 constexpr int DKW = D <= 64 ? 32 : 16;                    // keys per warp per step
 constexpr int DNT = DKW / 8;                              // score n-tiles per step
 constexpr int DSTAGES = 2;                                 // steps in flight per warp
+// The grid's splits are sized for the longest sequence a captured step may meet. A request whose keys one block walks in this many
+// steps of its warps is not split: the partial rows, their ticket and their merge (2 to 3 us at the end of the launch) cost more than
+// the steps that another block would save. Llama-3.2-1B decoding steps, 1 | 2 | 3 | 4 steps of 256 keys: 8 requests after 270 tokens
+// 692 | 655 | 655 | 655 us, after 510 713 | 703 | 698 | 698, after 710 742 | 742 | 707 | 707, after 1,010 the same with all.
+constexpr int SOLO = 3;
 constexpr bool DQ_IN_REGS = D <= 128;                     // query fragments live in registers
 constexpr int DCOPIES = DKW * CHUNKS / 32;                // 16-byte copies per lane per sub-tile and tensor
 
@@ -554,13 +559,18 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
   // split takes them as sub-tiles of their own, ahead of its others.
   const int keep = (OPTS && p.window > 0) ? p.keep_first : 0;
   const int keep_end = split == 0 ? min(keep, lo) : 0;
+  int splits = p.num_splits;
   {
     // the request's keys are shared out evenly over the launch's splits, in units of one step of all the block's
     // warps. The splits start at the unit boundary at or below the first key, so their size is taken from there:
     // sized from the first key itself they could end before the last one.
     constexpr int UNIT = NWARPS * DKW;
     const int base = (lo / UNIT) * UNIT;
-    const int split_size = max(UNIT, ((hi - base + p.num_splits - 1) / p.num_splits + UNIT - 1) / UNIT * UNIT);
+    if (p.tickets != nullptr && hi - base <= SOLO * UNIT) {
+      if (split > 0) { pdl_wait(); return; }
+      splits = 1;                                               // (nobody else arrives: no ticket, no merge)
+    }
+    const int split_size = max(UNIT, ((hi - base + splits - 1) / splits + UNIT - 1) / UNIT * UNIT);
     lo = max(lo, base + split * split_size);
     hi = min(hi, base + (split + 1) * split_size);
   }
@@ -572,7 +582,7 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
   if (lo >= hi) {
     pdl_launch_dependents();
     pdl_wait();
-    if (p.num_splits > 1) {
+    if (splits > 1) {
       if (tid < 16) {
         float* ml = p.part_ml + ((((size_t)r * p.Hkv + hk) * p.num_splits + split) * 16 + tid) * 2;
         ml[0] = -INFINITY; ml[1] = 0.f;
@@ -601,6 +611,7 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
     }
   }
   pdl_launch_dependents();
+  __syncthreads();                                              // table entries are in shared memory
   pdl_wait();                                                   // queries and this step's keys/values come from earlier kernels
   for (int idx = tid; idx < 16 * CHUNKS; idx += NTHR) {
     const int row = idx / CHUNKS, ch = idx - row * CHUNKS;
@@ -609,8 +620,6 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
     cp_async16(Qs + row * LDS + ch * 8, p.qkv + (size_t)(q0 + tok) * p.q_stride + (size_t)hd * D + ch * 8, ok);
   }
   cp_async_commit();
-  cp_async_wait<0>();
-  __syncthreads();                                              // queries and table entries are in shared memory
 
   const bool same_page = (p.ps % DKW) == 0;
   const int n_sub = n_keep + (hi - k_first + DKW - 1) / DKW;    // sub-tiles of the split
@@ -627,6 +636,10 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
                                           same_page, myKV + s * stage_elems, myKV + s * stage_elems + DKW * LDS, lane);
     cp_async_commit();
   }
+  // The first keys were asked for right behind the queries: one trip to memory in place of two, one after the other
+  // (batch 1 after 1,000 tokens 650 -> 643 us a Llama-3.2-1B decoding step).
+  cp_async_wait<DSTAGES - 1>();
+  __syncthreads();                                              // queries are in shared memory
   uint32_t qf[DQ_IN_REGS ? D / 16 : 1][4];
   if (DQ_IN_REGS) {
 #pragma unroll
@@ -797,7 +810,7 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
     if (row_b) { MLm[(warp * 16 + g + 8) * 2] = m_b; MLm[(warp * 16 + g + 8) * 2 + 1] = l_b; }
   }
   __syncthreads();
-  const bool last = p.num_splits == 1;
+  const bool last = splits == 1;
   for (int idx = tid; idx < M * D; idx += NTHR) {
     const int row = idx / D, d = idx - row * D;
     float mm = -INFINITY;

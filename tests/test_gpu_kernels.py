@@ -303,6 +303,26 @@ def test_decode_attention_with_a_window_over_several_splits_keeps_the_newest_key
     assert float((out.float() - 7.0).abs().max()) < 0.1
 
 
+@pytest.mark.parametrize("d,unit", [(64, 256), (128, 128), (256, 128)])
+@pytest.mark.parametrize("window", [0, 300])
+@pytest.mark.parametrize("heads", [4, 12])
+def test_decode_attention_where_one_block_takes_a_request(K, d, unit, window, heads):
+    """Requests of up to three steps of a block's warps are walked by the first split's block alone, longer ones by all splits: lengths on
+    both sides of every step's edge in one launch (a step of a captured size meets them all), groups of up to 8 and of more heads."""
+    kv_heads, page = 1, 64
+    kv_lens = [1, unit - 1, unit, unit + 1, 3 * unit - 1, 3 * unit, 3 * unit + 1, 4 * unit + 5, 2000]
+    s = _paged_setup("bfloat16", heads, kv_heads, d, page, [1] * len(kv_lens), kv_lens)
+    assert K.split_plan(len(kv_lens), kv_heads, window + 16 if window else max(kv_lens)) > 1
+    out = torch.full((len(kv_lens), heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ref = torch.empty_like(out)
+    for _ in range(2):                                # (the tickets of the split requests are zero again after a launch)
+        K.attention(s["qkv"], s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, d ** -0.5, window, out,
+                    s["shape"])
+    E.attention(s["qkv"], s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, d ** -0.5, window, ref,
+                s["shape"])
+    torch.testing.assert_close(out.float(), ref.float(), atol=2e-2, rtol=2e-2)       # (as above: bfloat16 results of size one)
+
+
 def test_refused_sizes(K):
     from serve_b200.kernels import KernelError
 
