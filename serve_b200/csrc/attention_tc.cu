@@ -4,36 +4,40 @@
 // Work is cut as in attention_mma.cu: per (request, kv head), with the G = H / Hkv query heads that share the kv
 // head folded into the row dimension: row m stands for (token m / G, head hk*G + m % G). A CTA owns 128 such
 // rows (128 / G tokens) and walks over the request's keys in tiles of 64:
-//   warp 0     one thread feeds shared memory with TMA: the query tile once (a 4-d box over the q/k/v buffer),
-//              then per tile the key and value pages named by the block table (4-d boxes over the caches,
-//              128-byte swizzle), three stages; the thread's loop is kept free of divisions, it is on the critical path;
-//   warp 1     one thread issues tcgen05.mma: S = Q K^T (128 x 64 x 64) into one of two score buffers in tensor
-//              memory, and, once the probabilities of a tile are in shared memory, O += P V (128 x 64 x 64, V read
-//              MN-major) into the output accumulator, which stays in tensor memory for the whole walk;
+//   warp 0     feeds shared memory with TMA: the query tile once (a 4-d box over the q/k/v buffer), then per tile the key and value
+//              pages named by the block table (4-d boxes over the caches, 128-byte swizzle) through a ring of stages;
+//   warp 1     issues tcgen05.mma: S = Q K^T (128 x 64) into a score buffer in tensor memory, and, once the probabilities of a tile are
+//              in tensor memory too, O += P V (V read MN-major) into the output accumulator, which stays there for the whole walk;
 //              tcgen05.commit signals the readers and frees stages and buffers;
-//   warps 2..5 one thread per row: reads its row of S from tensor memory (tcgen05.ld), scale, causal mask on
-//              the diagonal tiles, exp2 against a reference maximum, writes the probabilities as bfloat16 into the
-//              swizzled layout the second product reads (two buffers). The reference maximum only follows the
-//              running maximum when that has moved by more than 8 (a factor 256, harmless in bfloat16 and float);
-//              then, and only then, the accumulator in tensor memory is rescaled (tcgen05.ld / tcgen05.st) after
-//              the products issued so far have finished. So in the steady state nobody waits for the second
-//              product. At the end each thread divides its output row by the row's sum and stores its row.
+//   warps 2..9 two threads a row, 32 keys of a tile each: they read their part of S (tcgen05.ld), scale, causal mask on the diagonal
+//              tiles, exp2 against a reference maximum, and leave the probabilities as bfloat16 in tensor memory, the first operand
+//              of the second product. The reference maximum only follows the running maximum when that has moved by more than 8 (a
+//              factor 256, harmless in bfloat16 and float): one barrier with a vote a tile tells the two threads of a row whether it
+//              does; then, and only then, they exchange their maxima and rescale the accumulator in tensor memory after the products
+//              issued so far have finished. So in the steady state nobody waits for the second product. At the end each thread
+//              divides its half of the output row by the row's sum and stores it.
+// What bounds it: a step's latencies, not its work (head_dim 64: of 1,790 cycles a CTA's step takes, 512 are the exponentials of 128
+// rows, waits on mbarriers that are long complete 250 to 700, the pair's barrier 100). What that led to, 2,048 tokens, 32/8 heads of 64 | 16/4 of
+// 128 behind a window of 1,024 | 16 heads over a row of 256: a thread a row and one thread of a divergent warp to issue 53.9 | 45.8 | 60.5 us;
+// two threads a row and the probabilities in tensor memory 52.4 | 41.7 | 52.8; products issued from a warp that has come together, with
+// 32-bit additions in place of descriptors made anew, 50.7 | 38.3 | 49.6; waits that cost one instruction when there is nothing to wait for,
+// 48.4 | 36.0 | 49.8; copies issued like the products, a tile's page looked up a tile ahead, 47.2 | 35.2 | 48.8 (a loop of a few
+// more branches there: 52.3 | 39.0 | 49.2); two CTAs an SM at head_dim 128 (TIGHT) 28.9. No difference: two sets of softmax warps for even
+// and odd tiles, longer hardware waits, a single polling lane, packed arithmetic.
 // Two CTAs share an SM at head_dim 64 (96 KB of shared memory, 256 columns of tensor memory each).
 // At head_dim 128 an operand row is two 128-byte swizzle atoms: queries, keys and values arrive as two TMA boxes of 64
 // elements each, the first product walks over both atoms of Q and K, the second product covers the 128 output
-// columns in one instruction (the descriptor's leading byte offset names the distance between the atoms of V);
-// shared memory then holds one CTA per SM. (Two CTAs with two stages and one buffer of probabilities each, 112 KB, fit too:
-// 2,048 tokens, 24/8 heads, 81.3 us against 77.7.)
+// columns in one instruction (the descriptor's leading byte offset names the distance between the atoms of V).
 // At head_dim 256 keys and values are the same rows (latent attention), so a tile is loaded once for both products; with its
 // 256 output columns and two score buffers the kernel holds all of tensor memory.
-// Behind a window only the tiles that a row of the CTA can see are walked. 2,048 tokens, window 1,024: 16/4 heads of 128 95.2 us on
-// mma.sync -> 46.0; 16 heads over one row of 256 172.3 -> 61.0 (bound by the softmax threads: a warp a scheduler, about 1.3 us a tile
-// against 0.55 us of products, 0.8 with both parts of the probabilities).
+// Behind a window only the tiles that a row of the CTA can see are walked.
 // The recurrences are those of serve/kernels/attn_prefill.py:58-72 with exp2 and a folded log2(e)
 // (attn_prefill.py:330-331); probabilities are rounded to bfloat16 before the second product (attn_prefill.py:71),
 // or split into two (FINE, below).
 // Every wait is bounded; a wait that runs out raises *error and the CTA still frees its tensor memory.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -47,34 +51,39 @@ namespace {
 constexpr int D = SB_HEAD_DIM;
 constexpr int KA = D / 64;            // 128-byte swizzle atoms (64 elements) per operand row
 constexpr bool SHARED = D == 256;     // keys are the values (latent attention): one load a tile serves both products
-constexpr int CTAS_PER_SM = D == 64 ? 2 : 1;
 constexpr int BM = 128;              // rows per CTA
-constexpr int BN = 64;               // keys per tile (one 128-byte row of probabilities: one k-block of P)
-constexpr int NS = 3;                // key/value stages
+constexpr int BN = 64;               // keys per tile
 constexpr int BT_CACHE = D == 256 ? 512 : 1024;       // block-table entries kept in shared memory
-constexpr int THREADS = 192;
-constexpr uint32_t TMEM_COLS = D == 256 ? 512 : 256;  // S0, S1 (BN columns each), O (D), rounded up to a power of two
+constexpr int SOFTMAX_WARPS = 8;
+constexpr int THREADS = 64 + 32 * SOFTMAX_WARPS;
 constexpr unsigned WAIT_LIMIT = 1u << 26;
 constexpr float LOG2E = 1.4426950408889634f;
-constexpr int Q_BYTES = BM * D * 2, KV_BYTES = BN * D * 2, P_BYTES = BM * BN * 2;
+constexpr int Q_BYTES = BM * D * 2, KV_BYTES = BN * D * 2, P_COLS = BN / 2;      // (two probabilities a column)
 
 // FINE: a probability is two bfloat16 numbers, its leading bits and what they leave, and the second product runs over both. With
 // exponentials taken against a reference that lags behind the maximum, the heaviest key of a row is not 1 but any number up to 256, so
 // its rounding (2^-9) is the result's; a kernel that follows the maximum, as attention_mma.cu does, has no error there. From 64 bits
 // (2-norms; 700 tokens, window 200, head size 128; the output's own rounding is 1.61e-3 to 1.64e-3 of it), one part | mma.sync | two
 // parts: scores of a deviation of 1 2.08e-3 | 2.00e-3 | 1.61e-3, of 2 2.10e-3 | 1.83e-3 | 1.64e-3, of 6 1.96e-3 | 1.68e-3 | 1.63e-3.
-// Following the maximum instead would rescale the accumulator in nearly every tile. What the second part costs at 2,048 tokens, window
-// 1,024: 16/4 heads of 128 35.9 -> 40.7 us (half for making it, half for its product), 16 heads over one row of 256 46.7 -> 53.4 (its
-// product). Four stages and one buffer of probabilities: 40.8 and 54.4; the second parts behind the scores of the tile after next: 48.5
-// and 62.4 (a stage comes free later, and its next load with it).
-template <bool FINE>
+// Following the maximum instead would rescale the accumulator in nearly every tile.
+// TIGHT: the form at head_dim 128 that lets two CTAs share an SM (96 KB, 256 columns): one score buffer, two stages, and keys and values
+// with stages of their own, so that the next keys are on their way while the values are still read.
+template <bool FINE, bool TIGHT>
 struct Layout {
-  static constexpr int NP = D == 64 && FINE ? 1 : 2;    // buffers of probabilities
-  static constexpr int P_BUF = (FINE ? 2 : 1) * P_BYTES;
-  // 96 KB at head_dim 64, 160 at 128 (FINE: 192), 224 at 256
-  static constexpr int TILE_BYTES = Q_BYTES + (SHARED ? 1 : 2) * NS * KV_BYTES + NP * P_BUF;
-  static constexpr int SMEM_BYTES = TILE_BYTES + 256 + BT_CACHE * 4;    // + barriers + table entries; two CTAs fit an SM at head_dim 64
-  static_assert(SMEM_BYTES <= 227 * 1024, "shared memory of an SM");
+  static_assert(!TIGHT || D == 128, "a form of head_dim 128");
+  static constexpr int CTAS_PER_SM = D == 64 || TIGHT ? 2 : 1;
+  static constexpr bool SPLIT = TIGHT;                  // keys and values have stages of their own
+  static constexpr int NK = TIGHT ? 2 : D == 256 ? 4 : 5;     // stages of keys, and as many of values (none where the keys are the values)
+  static constexpr int NSB = TIGHT ? 1 : 2;             // score buffers
+  static constexpr uint32_t TMEM_COLS = CTAS_PER_SM == 2 ? 256 : 512;
+  static constexpr int P_BUF = (FINE ? 2 : 1) * P_COLS; // columns of tensor memory a buffer of probabilities takes
+  static constexpr int NP = NSB * BN + D + 2 * P_BUF <= (int)TMEM_COLS ? 2 : 1;     // buffers of probabilities
+  static_assert(NSB * BN + D + NP * P_BUF <= (int)TMEM_COLS, "tensor memory");
+  // 96 KB at head_dim 64 and in the tight form at 128, else 192
+  static constexpr int TILE_BYTES = Q_BYTES + (SHARED ? 1 : 2) * NK * KV_BYTES;
+  // + barriers, what the threads of a row tell one another, table entries
+  static constexpr int XCH_OFF = TILE_BYTES + 256, BT_OFF = XCH_OFF + 2 * BM * 4, SMEM_BYTES = BT_OFF + BT_CACHE * 4;
+  static_assert(SMEM_BYTES <= 227 * 1024 / CTAS_PER_SM - 1024, "shared memory of an SM");
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -87,16 +96,24 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const uint32_t addr = smem_u32(bar);
+__device__ __forceinline__ bool mbar_try(uint32_t bar, unsigned parity) {
+  uint32_t done;
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// A wait that runs out is noted in *gave_up; from then on no wait of the CTA lasts, every loop and barrier runs to its end, and what is
+// computed is not valid (*error is raised).
+__device__ __noinline__ void mbar_wait_long(uint32_t bar, unsigned parity, int* gave_up) {
   for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) return true;
+    if (mbar_try(bar, parity)) return;
+    if ((i & 1023u) == 1023u && *reinterpret_cast<volatile int*>(gave_up)) return;
   }
-  return false;
+  *reinterpret_cast<volatile int*>(gave_up) = 1;
+}
+__device__ __forceinline__ void mbar_wait(uint64_t* bar, unsigned parity, int* gave_up) {
+  const uint32_t addr = smem_u32(bar);
+  if (!mbar_try(addr, parity)) mbar_wait_long(addr, parity, gave_up);
 }
 __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
@@ -107,10 +124,26 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// A descriptor's upper half is the same for all tiles here (see desc_lo), so the issuing thread only ever adds to a 32-bit number.
+constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+      "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
+      ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(DESC_HI) : "memory");
+}
+// The same with the first operand in tensor memory: row i of it is lane i, two bfloat16 numbers to a column.
+__device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n .reg .b64 b;\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(DESC_HI) : "memory");
+}
+// One thread of a warp that has come together, always the same: the compiler then knows what is equal in all of them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(yes));
+  return yes != 0;
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 32 columns: thread i of the warp gets lane (base + i), 32 consecutive columns. No wait: several loads
@@ -139,28 +172,55 @@ __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
         "r"(u[30]), "r"(u[31])
       : "memory");
 }
+__device__ __forceinline__ void tc_store16(uint32_t taddr, const uint32_t (&u)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]),
+        "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
+      : "memory");
+}
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+// Two floats at a time: one instruction each, rounded as the single ones are.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n .reg .b64 x, y, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 w, x, y;\n mov.b64 {%0, %1}, w;\n}\n"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart; ``lbo`` is the distance between
-// 64-element swizzle atoms along the non-k dimension of an MN-major operand (not used by K-major operands).
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
+// Barriers of the 64 threads that share 32 rows (two warps); the second tells all of them whether any of them says yes.
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ bool pair_any(int id, bool yes) {
+  uint32_t any;
+  asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 q, %2, 0;\n bar.red.or.pred p, %1, 64, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(any) : "r"(id), "r"(yes ? 1u : 0u) : "memory");
+  return any != 0;
 }
+
+// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart (bits 32 .. 45), version 1 of it (46), layout type 2
+// (61 .. 63): its lower half, the address and ``lbo``, the distance between 64-element swizzle atoms along the non-k dimension of an
+// MN-major operand (not used by K-major operands), both in units of 16 bytes.
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr & 0x3FFFF) >> 4) | (lbo_bytes >> 4) << 16; }
 // kind::f16 instruction descriptor: float accumulator, bfloat16 operands; b_mn_major: the second operand has its
 // non-k dimension contiguous in shared memory (values: rows are keys, head elements contiguous)
 __host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool b_mn_major) {
@@ -193,11 +253,15 @@ __device__ __forceinline__ float tanh_fast(float x) {
   return y;
 }
 
-template <bool FINE>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
+template <bool FINE, bool TIGHT>
+__global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) attention_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                const __grid_constant__ CUtensorMap map_k,
                                                                const __grid_constant__ CUtensorMap map_v, const TcParams p) {
-  constexpr int NP = Layout<FINE>::NP, P_BUF = Layout<FINE>::P_BUF, TILE_BYTES = Layout<FINE>::TILE_BYTES;
+  typedef Layout<FINE, TIGHT> W;
+  constexpr int NP = W::NP, P_BUF = W::P_BUF, NK = W::NK, NSB = W::NSB, TILE_BYTES = W::TILE_BYTES, XCH_OFF = W::XCH_OFF, BT_OFF = W::BT_OFF;
+  constexpr uint32_t TMEM_COLS = W::TMEM_COLS;
+  constexpr bool SPLIT = W::SPLIT;
+  constexpr uint32_t O_COL = NSB * BN, P_COL = NSB * BN + D;  // the scores, O, the probabilities
   // Blocks start in the order of blockIdx.x, then y: with the heads in x, the tiles that see the most keys start first
   // for all heads. The other way round the last heads' longest tiles would start when a third of the time is over
   // and end last: 2,048 tokens, 32/8 heads took 53 us so, against 32 key tiles x ~1.1 us for the longest tile itself.
@@ -230,34 +294,38 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* base = smem;
   unsigned char* Qs = base;
-  unsigned char* Ks = Qs + Q_BYTES;                     // NS stages
-  unsigned char* Vs = SHARED ? Ks : Ks + NS * KV_BYTES; // NS stages
-  unsigned char* Ps = Vs + NS * KV_BYTES;               // NP buffers of [128 rows][128 bytes], FINE: twice that each
+  unsigned char* Ks = Qs + Q_BYTES;                     // NK stages
+  unsigned char* Vs = SHARED ? Ks : Ks + NK * KV_BYTES; // NK stages
   uint64_t* bars = reinterpret_cast<uint64_t*>(base + TILE_BYTES);
   uint64_t& q_full = bars[0];
-  uint64_t* kv_full = bars + 1;                         // NS: a stage's keys and values have landed
-  uint64_t* kv_empty = bars + 1 + NS;                   // NS: the products that read the stage have finished
-  uint64_t* s_full = bars + 1 + 2 * NS;                 // 2: a score buffer is complete
-  uint64_t* s_empty = bars + 3 + 2 * NS;                // 2: the softmax threads hold it in registers
-  uint64_t* p_full = bars + 5 + 2 * NS;                 // NP: a buffer of probabilities is written
-  uint64_t* p_empty = bars + 7 + 2 * NS;                // NP: the second product that read it has finished
-  uint32_t& tmem_base_s = *reinterpret_cast<uint32_t*>(bars + 9 + 2 * NS);
-  int* bt_s = reinterpret_cast<int*>(base + TILE_BYTES + 256);
+  uint64_t* k_full = bars + 1;                          // NK: a stage's keys have landed
+  uint64_t* k_empty = bars + 1 + NK;                    // NK: the products that read the stage have finished
+  uint64_t* v_full = SPLIT ? bars + 1 + 2 * NK : k_full;      // the same for values
+  uint64_t* v_empty = SPLIT ? bars + 1 + 3 * NK : k_empty;
+  uint64_t* s_full = bars + 1 + 4 * NK;                 // NSB: a score buffer is complete
+  uint64_t* s_empty = bars + 3 + 4 * NK;                // NSB: the softmax threads hold it in registers
+  uint64_t* p_full = bars + 5 + 4 * NK;                 // NP: a buffer of probabilities is written
+  uint64_t* p_empty = bars + 7 + 4 * NK;                // NP: the second product that read it has finished
+  uint32_t& tmem_base_s = *reinterpret_cast<uint32_t*>(bars + 9 + 4 * NK);
+  int* gave_up = reinterpret_cast<int*>(bars + 10 + 4 * NK);      // a wait of this CTA ran out
+  float* xch = reinterpret_cast<float*>(base + XCH_OFF);      // [2][BM]
+  int* bt_s = reinterpret_cast<int*>(base + BT_OFF);
   if ((smem_u32(base) & 1023u) != 0) {                  // never seen; refuse rather than compute with a wrong swizzle
     if (threadIdx.x == 0) atomicExch(p.error, 1);
     pdl_wait();
     return;
   }
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 1);
 #pragma unroll
-    for (int s = 0; s < NS; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+    for (int s = 0; s < (SPLIT ? 4 : 2) * NK; ++s) mbar_init(&k_full[s], 1);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_full[b], 1); mbar_init(&s_empty[b], 4); mbar_init(&p_full[b], 4); mbar_init(&p_empty[b], 1);
+      mbar_init(&s_full[b], 1); mbar_init(&s_empty[b], SOFTMAX_WARPS); mbar_init(&p_full[b], SOFTMAX_WARPS); mbar_init(&p_empty[b], 1);
     }
+    *gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
@@ -275,7 +343,6 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
   pdl_launch_dependents();
   pdl_wait();
   const uint32_t tmem_base = tmem_base_s;
-  bool failed = false;
 
   if (warp == 0) {
     // the table entries of the tile's keys, fetched once by the whole warp instead of one dependent load per page
@@ -286,246 +353,295 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) attention_tc_kernel(cons
       __syncwarp();
       bt = bt_s;
     }
-    if (lane == 0) {
-      // queries: box {64 elements, G heads, 1 kv head, tokens of the tile} -> rows (token, head)
+    // queries: box {64 elements, G heads, 1 kv head, tokens of the tile} -> rows (token, head)
+    if (elect_one()) {
       mbar_expect_tx(&q_full, (unsigned)(tok_per_tile * G * D * 2));
 #pragma unroll
       for (int a = 0; a < KA; ++a) tma_load_4d(Qs + (size_t)a * BM * 128, &map_q, &q_full, a * 64, 0, hk, q0 + tok0);
-      const bool big_pages = p.ps > BN;                  // a page holds several tiles (a multiple of BN keys)
-      const int pages_per_tile = big_pages ? 0 : BN / p.ps;
-      int big_blk = 0, big_at = 0;                        // big pages: the tile's page, and where in it the tile starts
-      for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % NS;
-        if (!mbar_wait(&kv_empty[s], ((j / NS) & 1) ^ 1)) { failed = true; break; }
-        const int kt = key_of(j), blk0 = (kt / BN) * pages_per_tile;   // pages tile the stage: no division in this thread's loop
-        if (big_pages && j == n_kept && skipped > 0) { big_blk = kt / p.ps; big_at = kt - big_blk * p.ps; }
-        if (big_pages) {
-          const bool there = kt < hi && big_blk < p.bt_width;
-          mbar_expect_tx(&kv_full[s], there ? (unsigned)(BN * D * 2 * (SHARED ? 1 : 2)) : 0u);
-          if (there) {
-            const int page = bt[big_blk];
-#pragma unroll
-            for (int a = 0; a < KA; ++a) {
-              const size_t off = (size_t)s * KV_BYTES + (size_t)a * BN * 128;
-              tma_load_4d(Ks + off, &map_k, &kv_full[s], a * 64, big_at, hk, page);
-              if (!SHARED) tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, big_at, hk, page);
-            }
-          }
-          big_at += BN;
-          if (big_at == p.ps) { big_at = 0; ++big_blk; }
-          continue;
-        }
-        int n_pages = 0;
-        for (int i = 0; i < pages_per_tile; ++i)
-          if (kt + i * p.ps < hi && blk0 + i < p.bt_width) ++n_pages;
-        mbar_expect_tx(&kv_full[s], (unsigned)(n_pages * p.ps * D * 2 * (SHARED ? 1 : 2)));
-        for (int i = 0; i < n_pages; ++i) {
-          const int page = bt[blk0 + i];                  // (-1, a page the window has passed: outside the map, zeros)
-#pragma unroll
-          for (int a = 0; a < KA; ++a) {
-            // atom a of a stage: 64 keys x 128 bytes; the page's keys at their rows of it
-            const size_t off = (size_t)s * KV_BYTES + (size_t)a * BN * 128 + (size_t)i * p.ps * 128;
-            tma_load_4d(Ks + off, &map_k, &kv_full[s], a * 64, 0, hk, page);
-            if (!SHARED) tma_load_4d(Vs + off, &map_v, &kv_full[s], a * 64, 0, hk, page);
-          }
-        }
+    }
+    // The loop is on the critical path: the whole warp walks it (what it computes is equal in all lanes then), no divisions, a tile's
+    // page is looked up while the tile before waits for its stage. Pages of a tile or more: a tile lies in one page, from its row ``at`` on.
+    const bool one = p.ps >= BN;
+    const int pages_per_tile = one ? 1 : BN / p.ps;
+    int blk = one ? key_of(0) / p.ps : key_of(0) / BN * pages_per_tile, at = one ? key_of(0) - blk * p.ps : 0;
+    int page = blk < p.bt_width ? bt[blk] : -1;          // the tile's first page
+    int s = 0, j = 0;
+    unsigned phase = 1;
+    for (; j < n_tiles; ++j) {
+      int n_pages = blk < p.bt_width ? 1 : 0;
+      if (!one) {
+        const int kt = key_of(j);
+        for (int i = 1; i < pages_per_tile; ++i)
+          if (kt + i * p.ps < hi && blk + i < p.bt_width) ++n_pages;
       }
+      const unsigned bytes = (unsigned)(n_pages * (one ? BN : p.ps) * D * 2);
+      // a tile of keys (or values) from its pages: atom a of a stage is 64 keys x 128 bytes, a page's keys at their rows of it
+      auto load = [&](unsigned char* stage, const CUtensorMap* map, uint64_t* full) {
+        if (n_pages > 0) {                               // (-1, a page the window has passed: outside the map, zeros)
+#pragma unroll
+          for (int a = 0; a < KA; ++a) tma_load_4d(stage + (size_t)a * BN * 128, map, full, a * 64, at, hk, page);
+        }
+        if (!one) {
+          for (int i = 1; i < n_pages; ++i) {
+            const int pg = bt[blk + i];
+#pragma unroll
+            for (int a = 0; a < KA; ++a) tma_load_4d(stage + (size_t)a * BN * 128 + (size_t)i * p.ps * 128, map, full, a * 64, 0, hk, pg);
+          }
+        }
+      };
+      mbar_wait(&k_empty[s], phase, gave_up);
+      if (*reinterpret_cast<volatile int*>(gave_up)) break;        // (no copy into a stage that may still be read)
+      __syncwarp();
+      if (elect_one()) {
+        mbar_expect_tx(&k_full[s], SPLIT || SHARED ? bytes : 2 * bytes);
+        load(Ks + (size_t)s * KV_BYTES, &map_k, &k_full[s]);
+        if (!SPLIT && !SHARED) load(Vs + (size_t)s * KV_BYTES, &map_v, &k_full[s]);
+      }
+      __syncwarp();
+      if (SPLIT) {
+        mbar_wait(&v_empty[s], phase, gave_up);
+        if (*reinterpret_cast<volatile int*>(gave_up)) { ++j; break; }
+        __syncwarp();
+        if (elect_one()) {
+          mbar_expect_tx(&v_full[s], bytes);
+          load(Vs + (size_t)s * KV_BYTES, &map_v, &v_full[s]);
+        }
+        __syncwarp();
+      }
+      // the next tile's place
+      at += BN;
+      if (at >= p.ps || !one) { at = 0; blk += pages_per_tile; }
+      if (j + 1 == n_kept && skipped > 0) {
+        const int kt = key_of(j + 1);
+        blk = one ? kt / p.ps : kt / BN * pages_per_tile;
+        at = one ? kt - blk * p.ps : 0;
+      }
+      if (j + 1 < n_tiles && blk < p.bt_width) page = bt[blk];
+      if (++s == NK) { s = 0; phase ^= 1; }
+    }
+    if (*reinterpret_cast<volatile int*>(gave_up)) {       // the copies under way land before the CTA leaves (with a limit again)
+      for (int i = max(0, j - NK); i < j; ++i) {
+        for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&k_full[i % NK]), (i / NK) & 1); ++n) {}
+        for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&v_full[i % NK]), (i / NK) & 1); ++n) {}
+      }
+      for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&q_full), 0); ++n) {}
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc(BM, BN, false);
-      constexpr uint32_t idesc_o = make_idesc(BM, D, true);
-      const uint64_t dq = make_desc(smem_u32(Qs), 0);
-      auto issue_s = [&](int t) {
-        const uint64_t dk = make_desc(smem_u32(Ks + (size_t)(t % NS) * KV_BYTES), 0);
-        const uint32_t acc = tmem_base + (uint32_t)((t & 1) * BN);
+    constexpr uint32_t idesc_s = make_idesc(BM, BN, false);
+    constexpr uint32_t idesc_o = make_idesc(BM, D, true);
+    const uint32_t dq = desc_lo(smem_u32(Qs), 0), dk0 = desc_lo(smem_u32(Ks), 0), dv0 = desc_lo(smem_u32(Vs), BN * 128);
+    int ks = 0, vs = 0;                                  // stages of the next scores and of the next values
+    unsigned kphase = 0, vphase = 0;
+    // the scores of tile t, as soon as its keys are there and its score buffer has been read
+    auto scores = [&](int t) {
+      mbar_wait(&k_full[ks], kphase, gave_up);
+      mbar_wait(&s_empty[t % NSB], ((t / NSB) & 1) ^ 1, gave_up);
+      __syncwarp();
+      tc_fence_after();
+      const uint32_t dk = dk0 + (uint32_t)(ks * (KV_BYTES >> 4)), acc = tmem_base + (uint32_t)((t % NSB) * BN);
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           // 16 k-values further: 32 bytes within an atom (4 steps), then the next atom of Q (128 rows) and K (64 rows)
-          const uint64_t qo = (uint64_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2);
-          const uint64_t ko = (uint64_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2);
-          tc_mma(acc, dq + qo, dk + ko, idesc_s, kk != 0 ? 1u : 0u);
+          tc_mma(acc, dq + (uint32_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2), dk + (uint32_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2), idesc_s,
+                 kk != 0 ? 1u : 0u);
         }
-        tc_commit(&s_full[t & 1]);
-      };
-      // O += P V: P is K-major (one block of 64 keys), FINE: both parts of it; V is MN-major, 16 keys = 2048 bytes further per step
-      auto issue_o = [&](int j) {
-        const uint32_t pa = smem_u32(Ps + (size_t)(j % NP) * P_BUF), va = smem_u32(Vs + (size_t)(j % NS) * KV_BYTES);
+        tc_commit(&s_full[t % NSB]);
+        if (SPLIT) tc_commit(&k_empty[ks]);
+      }
+      __syncwarp();
+      if (++ks == NK) { ks = 0; kphase ^= 1; }
+    };
+    mbar_wait(&q_full, 0, gave_up);
+    scores(0);
+    for (int j = 0; j < n_tiles; ++j) {
+      if (j + 1 < n_tiles) scores(j + 1);
+      mbar_wait(&p_full[j % NP], (j / NP) & 1, gave_up);
+      if (SPLIT) mbar_wait(&v_full[vs], vphase, gave_up);
+      __syncwarp();
+      tc_fence_after();
+      // O += P V: P from tensor memory (16 keys are 8 columns), FINE: both parts of it; V is MN-major, 16 keys = 2048 bytes further per step
+      const uint32_t pa = tmem_base + P_COL + (uint32_t)((j % NP) * P_BUF), dv = dv0 + (uint32_t)(vs * (KV_BYTES >> 4));
+      if (elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
-          const uint64_t dv = make_desc(va + (uint32_t)(kk * 2048), BN * 128);
-          tc_mma(tmem_base + (uint32_t)(2 * BN), make_desc(pa + (uint32_t)(kk * 32), 0), dv, idesc_o, (j | kk) != 0 ? 1u : 0u);
-          if (FINE) tc_mma(tmem_base + (uint32_t)(2 * BN), make_desc(pa + (uint32_t)(P_BYTES + kk * 32), 0), dv, idesc_o, 1u);
+          tc_mma_ts(tmem_base + O_COL, pa + (uint32_t)(kk * 8), dv + (uint32_t)(kk * (2048 >> 4)), idesc_o, (j | kk) != 0 ? 1u : 0u);
+          if (FINE) tc_mma_ts(tmem_base + O_COL, pa + (uint32_t)(P_COLS + kk * 8), dv + (uint32_t)(kk * (2048 >> 4)), idesc_o, 1u);
         }
-        tc_commit(&p_empty[j % NP]);         // also: "the products up to tile j have finished"
-        tc_commit(&kv_empty[j % NS]);
-      };
-      do {
-        if (!mbar_wait(&q_full, 0) || !mbar_wait(&kv_full[0], 0)) { failed = true; break; }
-        tc_fence_after();
-        issue_s(0);
-        for (int j = 0; j < n_tiles; ++j) {
-          if (j + 1 < n_tiles) {
-            // the next tile's scores, as soon as its keys are there and its score buffer has been read
-            const int t = j + 1;
-            if (!mbar_wait(&kv_full[t % NS], (t / NS) & 1) || !mbar_wait(&s_empty[t & 1], ((t >> 1) & 1) ^ 1)) { failed = true; break; }
-            tc_fence_after();
-            issue_s(t);
-          }
-          if (!mbar_wait(&p_full[j % NP], (j / NP) & 1)) { failed = true; break; }
-          tc_fence_after();
-          issue_o(j);
-        }
-      } while (false);
+        tc_commit(&p_empty[j % NP]);                     // also: "the products up to tile j have finished"
+        tc_commit(&v_empty[vs]);
+      }
+      __syncwarp();
+      if (++vs == NK) { vs = 0; vphase ^= 1; }
     }
   } else {
+    // Two warps share 32 rows: warps 2 .. 5 take the first 32 keys of every tile, warps 6 .. 9 the others, a thread a row. Both threads of a
+    // row hold the same reference; a barrier of the pair tells them whether either has seen a score that moves it.
     const int q = warp & 3;                              // the 32 tensor-memory lanes this warp may touch
+    const int half = (warp - 2) >> 2, pair = 1 + q;      // its half of a tile's keys; the pair's barrier
     const int row = q * 32 + lane;
     const int m = tok0 * G + row;
     const bool row_ok = row < tok_per_tile * G && m < M;
     const int tok = row_ok ? m / G : 0, head = row_ok ? hk * G + (m - tok * G) : 0;
     const int pos = row_ok ? p0 + tok : -1;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-    const uint32_t o_addr = lane_addr + (uint32_t)(2 * BN);
+    float *mine = xch + half * BM + row, *other = xch + (half ^ 1) * BM + row;
     float m_ref = -INFINITY;                             // what the exponentials are taken against (log2 domain)
-    float l_run = 0.f;
+    float l_run = 0.f;                                   // (of this thread's keys)
     const int first_pos = p0 + tok0;                     // smallest position of the tile's rows
     const int window_lo = p.window > 0 ? first_pos - p.window + 1 : 0;      // no row sees a key below it that is not kept
-
-    for (int j = 0; j < n_tiles && !failed; ++j) {
-      const int b = j & 1, kt = key_of(j);
-      if (!mbar_wait(&s_full[b], (j >> 1) & 1)) { failed = true; break; }
-      tc_fence_after();
-      // the tile reaches beyond what the first row may see, or behind the last row's window
-      const bool masked = kt + BN - 1 > first_pos || (p.window > 0 && kt <= p0 + tok_last - p.window);
-      float sv[BN];
-#pragma unroll
-      for (int c = 0; c < BN / 32; ++c) tc_load32(lane_addr + (uint32_t)(b * BN + c * 32), sv + c * 32);
-      tc_wait_ld();
-      tc_fence_before();
+    for (int j = 0; j < n_tiles; ++j) {
+      const int b = j % NSB, kt = key_of(j), k0 = kt + half * 32;
+      mbar_wait(&s_full[b], (j / NSB) & 1, gave_up);
+      // The buffer of probabilities must have been read by the product of NP tiles ago. With two buffers it has by now (these scores were
+      // issued behind that product), and the wait only keeps count of the barrier's uses.
+      if (NP == 2 && j >= NP) mbar_wait(&p_empty[j % NP], ((j - NP) / NP) & 1, gave_up);
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[b]);           // the scores are in registers: the buffer may be reused
-      if (p.cap_over_scale > 0.f) {                      // the cap comes before the mask: tanh(-inf) would be finite
-#pragma unroll
-        for (int i = 0; i < BN; ++i) sv[i] = p.cap_over_scale * tanh_fast(sv[i] * p.softcap_in);
-      }
-      if (masked) {
-#pragma unroll
-        for (int i = 0; i < BN; ++i) sv[i] = (kt + i <= pos) ? sv[i] : -INFINITY;
-        if (p.window > 0) {
-          const int from = pos - p.window + 1;            // the row's first key, the kept ones aside
-#pragma unroll
-          for (int i = 0; i < BN; ++i) sv[i] = (kt + i >= from || kt + i < p.keep) ? sv[i] : -INFINITY;
-        }
-      }
-      float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < BN; i += 4) {
-        mx0 = fmaxf(mx0, sv[i]); mx1 = fmaxf(mx1, sv[i + 1]); mx2 = fmaxf(mx2, sv[i + 2]); mx3 = fmaxf(mx3, sv[i + 3]);
-      }
-      const float m_tile = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2;
-      // the reference follows the maximum only when that has run ahead by more than 8 (or there was none yet)
-      const bool moved = m_tile > m_ref + 8.0f;           // false for m_tile = -inf; true for m_ref = -inf, m_tile finite
-      if (__any_sync(0xffffffffu, moved && m_ref != -INFINITY)) {
-        // rare: rescale the accumulator in tensor memory, once the products issued so far (up to tile j-1) are done
-        if (!mbar_wait(&p_empty[(j - 1) % NP], ((j - 1) / NP) & 1)) { failed = true; break; }
+      float sv[32];
+      float m_half;
+      {
         tc_fence_after();
-        const float f = (moved && m_ref != -INFINITY) ? ex2(m_ref - m_tile) : 1.f;
-#pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          float ov[32];
-          tc_load32(o_addr + (uint32_t)(c * 32), ov);
-          tc_wait_ld();
+        // the tile reaches beyond what the first row may see, or behind the last row's window
+        const bool masked = kt + BN - 1 > first_pos || (p.window > 0 && kt <= p0 + tok_last - p.window);
+        tc_load32(lane_addr + (uint32_t)(b * BN + half * 32), sv);
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[b]);         // the scores are in registers: the buffer may be reused
+        if (p.cap_over_scale > 0.f) {                    // the cap comes before the mask: tanh(-inf) would be finite
 #pragma unroll
-          for (int i = 0; i < 32; ++i) ov[i] *= f;
-          tc_store32(o_addr + (uint32_t)(c * 32), ov);
+          for (int i = 0; i < 32; ++i) sv[i] = p.cap_over_scale * tanh_fast(sv[i] * p.softcap_in);
         }
-        tc_wait_st();
-        l_run *= f;
-      }
-      if (moved) m_ref = m_tile;                         // (with no reference yet, accumulator and sum are still zero)
-      const float use = (m_ref == -INFINITY) ? 0.f : m_ref;
-      // the buffer of probabilities must have been read by the product of NP tiles ago
-      if (j >= NP && !mbar_wait(&p_empty[j % NP], ((j - NP) / NP) & 1)) { failed = true; break; }
-      // probabilities -> shared memory (bfloat16, the swizzled K-major layout of the second product);
-      // ex2(-inf) = 0 takes care of masked entries
-      float sum0 = 0.f, sum1 = 0.f;
-      unsigned char* prow = Ps + (size_t)(j % NP) * P_BUF + (size_t)row * 128;
+        if (masked) {
 #pragma unroll
-      for (int c = 0; c < BN / 8; ++c) {                 // 16-byte pieces of 8 keys
-        uint32_t pk[4], rest[4];
+          for (int i = 0; i < 32; ++i) sv[i] = (k0 + i <= pos) ? sv[i] : -INFINITY;
+          if (p.window > 0) {
+            const int from = pos - p.window + 1;          // the row's first key, the kept ones aside
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float e0 = ex2(fmaf(sv[c * 8 + 2 * i], p.scale_log2, -use));
-          const float e1 = ex2(fmaf(sv[c * 8 + 2 * i + 1], p.scale_log2, -use));
-          sum0 += e0;
-          sum1 += e1;
-          if (FINE) {                                    // both parts cut off, not rounded: 2^-16 of the number is left out
-            const uint32_t u0 = __float_as_uint(e0), u1 = __float_as_uint(e1);
-            pk[i] = __byte_perm(u0, u1, 0x7632);
-            rest[i] = __byte_perm(__float_as_uint(e0 - __uint_as_float(u0 & 0xffff0000u)), __float_as_uint(e1 - __uint_as_float(u1 & 0xffff0000u)), 0x7632);
-          } else {
-            pk[i] = pack_bf16(e0, e1);
+            for (int i = 0; i < 32; ++i) sv[i] = (k0 + i >= from || k0 + i < p.keep) ? sv[i] : -INFINITY;
           }
         }
-        *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        if (FINE) *reinterpret_cast<uint4*>(prow + P_BYTES + ((c ^ (row & 7)) << 4)) = make_uint4(rest[0], rest[1], rest[2], rest[3]);
+        float mx[4] = {sv[0], sv[1], sv[2], sv[3]};
+#pragma unroll
+        for (int i = 4; i < 28; i += 8)
+#pragma unroll
+          for (int u = 0; u < 4; ++u) mx[u] = max3(mx[u], sv[i + u], sv[i + 4 + u]);
+        m_half = max3(max3(mx[0], mx[1], sv[28]), max3(mx[2], mx[3], sv[29]), fmaxf(sv[30], sv[31])) * p.scale_log2;
       }
-      l_run += sum0 + sum1;
+      // the reference follows the maximum only when that has run ahead by more than 8 (or there was none yet): false for
+      // m_half = -inf, true for m_ref = -inf and m_half finite
+      if (pair_any(pair, m_half > m_ref + 8.0f)) {
+        // rare: some row's reference moves. Both threads of a row take the larger of their maxima.
+        *mine = m_half;
+        pair_sync(pair);
+        const float m_tile = fmaxf(m_half, *other);
+        const bool moves = m_tile > m_ref + 8.0f;
+        if (__any_sync(0xffffffffu, moves && m_ref != -INFINITY)) {
+          // rescale the accumulator in tensor memory, once the products issued so far (up to tile j-1) are done
+          mbar_wait(&p_empty[(j - 1) % NP], ((j - 1) / NP) & 1, gave_up);
+          __syncwarp();
+          tc_fence_after();
+          const float f = (moves && m_ref != -INFINITY) ? ex2(m_ref - m_tile) : 1.f;
+#pragma unroll 1
+          for (int c = 0; c < D / 64; ++c) {
+            const uint32_t o_addr = lane_addr + O_COL + (uint32_t)(half * (D / 2) + c * 32);
+            float ov[32];
+            tc_load32(o_addr, ov);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) ov[i] *= f;
+            tc_store32(o_addr, ov);
+          }
+          tc_wait_st();
+          l_run *= f;
+        }
+        if (moves) m_ref = m_tile;                       // (with no reference yet, accumulator and sum are still zero)
+      }
+      const float use = (m_ref == -INFINITY) ? 0.f : m_ref;
+      if (NP == 1 && j > 0) {
+        mbar_wait(&p_empty[0], (j - 1) & 1, gave_up);
+        __syncwarp();
+        tc_fence_after();
+      }
+      // probabilities -> tensor memory (bfloat16, two neighbouring keys a column); ex2(-inf) = 0 takes care of masked entries
+      float2 sum = make_float2(0.f, 0.f);
+      const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), use2 = make_float2(-use, -use);
+      const uint32_t p_addr = lane_addr + P_COL + (uint32_t)((j % NP) * P_BUF + half * 16);
+      uint32_t pk[16], rest[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float2 z = fma2(make_float2(sv[2 * i], sv[2 * i + 1]), scale2, use2);
+        const float e0 = ex2(z.x), e1 = ex2(z.y);
+        sum = add2(sum, make_float2(e0, e1));
+        if (FINE) {                                      // both parts cut off, not rounded: 2^-16 of the number is left out
+          const uint32_t u0 = __float_as_uint(e0), u1 = __float_as_uint(e1);
+          pk[i] = __byte_perm(u0, u1, 0x7632);
+          rest[i] = __byte_perm(__float_as_uint(e0 - __uint_as_float(u0 & 0xffff0000u)), __float_as_uint(e1 - __uint_as_float(u1 & 0xffff0000u)), 0x7632);
+        } else {
+          pk[i] = pack_bf16(e0, e1);
+        }
+      }
+      tc_store16(p_addr, pk);
+      if (FINE) tc_store16(p_addr + P_COLS, rest);
+      l_run += sum.x + sum.y;
       // values that no row of the tile sees must not meet a zero probability as NaN (0 times infinity): the rows of this stage beyond
       // hi (never written, or another tile's leftovers) are cleared, and so are those behind every row's window
       if (kt + BN > hi || (kt < window_lo && kt + BN > p.keep)) {
-        if (!mbar_wait(&kv_full[j % NS], (j / NS) & 1)) { failed = true; break; }
-        unsigned char* vt = Vs + (size_t)(j % NS) * KV_BYTES;
+        mbar_wait(&v_full[j % NK], (j / NK) & 1, gave_up);
+        unsigned char* vt = Vs + (size_t)(j % NK) * KV_BYTES;
         auto clear = [&](int first, int last) {          // rows [first, last) of the stage
           const int n = last - first;
-          for (int idx = (warp - 2) * 32 + lane; idx < n * 8 * KA; idx += 128) {
-            const int a = idx / (n * 8), rest = idx - a * n * 8;
-            *reinterpret_cast<uint4*>(vt + (size_t)a * BN * 128 + (size_t)(first + (rest >> 3)) * 128 + ((rest & 7) << 4)) =
+          for (int idx = (warp - 2) * 32 + lane; idx < n * 8 * KA; idx += 32 * SOFTMAX_WARPS) {
+            const int a = idx / (n * 8), rest_ = idx - a * n * 8;
+            *reinterpret_cast<uint4*>(vt + (size_t)a * BN * 128 + (size_t)(first + (rest_ >> 3)) * 128 + ((rest_ & 7) << 4)) =
                 make_uint4(0u, 0u, 0u, 0u);
           }
         };
         clear(max(0, p.keep - kt), min(BN, window_lo - kt));
         clear(hi - kt, BN);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
       }
+      tc_wait_st();
       tc_fence_before();
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[j % NP]);
     }
-    if (!failed) {
-      // all products have finished when the last one has
-      if (!mbar_wait(&p_empty[(n_tiles - 1) % NP], ((n_tiles - 1) / NP) & 1)) failed = true;
-      tc_fence_after();
-      if (!failed) {
-        if (p.sinks != nullptr && row_ok) {
-          // the sums were taken against m_ref; so is the sink (a sink far above every score makes the sum infinite and
-          // the row zero, which is its limit)
-          const float sk = p.sinks[head] * LOG2E;
-          l_run += (m_ref == -INFINITY) ? 1.f : exp2f(sk - m_ref);
-        }
-        const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-        bf16* dst = p.out + (size_t)(q0 + tok) * p.H * D + (size_t)head * D;
+    // all products have finished when the last one has
+    mbar_wait(&p_empty[(n_tiles - 1) % NP], ((n_tiles - 1) / NP) & 1, gave_up);
+    __syncwarp();
+    tc_fence_after();
+    *mine = l_run;
+    pair_sync(pair);
+    l_run = half ? *other + l_run : l_run + *other;    // (the same sum in both threads of a row)
+    {
+      if (p.sinks != nullptr && row_ok) {
+        // the sums were taken against m_ref; so is the sink (a sink far above every score makes the sum infinite and
+        // the row zero, which is its limit)
+        const float sk = p.sinks[head] * LOG2E;
+        l_run += (m_ref == -INFINITY) ? 1.f : exp2f(sk - m_ref);
+      }
+      const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
+      constexpr int COLS = D / 2;                        // output columns a thread stores
+      const int c0 = half * COLS;
+      bf16* dst = p.out + (size_t)(q0 + tok) * p.H * D + (size_t)head * D + c0;
 #pragma unroll 1
-        for (int c = 0; c < D / 64; ++c) {
-          float ov[64];
-          tc_load32(o_addr + (uint32_t)(c * 64), ov);
-          tc_load32(o_addr + (uint32_t)(c * 64 + 32), ov + 32);
-          tc_wait_ld();
-          if (row_ok) {
+      for (int c = 0; c < COLS; c += 32) {
+        float ov[32];
+        tc_load32(lane_addr + O_COL + (uint32_t)(c0 + c), ov);
+        tc_wait_ld();
+        if (row_ok) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-              *reinterpret_cast<uint4*>(dst + c * 64 + i * 8) =
-                  make_uint4(pack_bf16(ov[8 * i] * inv, ov[8 * i + 1] * inv), pack_bf16(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv),
-                             pack_bf16(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv), pack_bf16(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv));
-          }
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(dst + c + i * 8) =
+                make_uint4(pack_bf16(ov[8 * i] * inv, ov[8 * i + 1] * inv), pack_bf16(ov[8 * i + 2] * inv, ov[8 * i + 3] * inv),
+                           pack_bf16(ov[8 * i + 4] * inv, ov[8 * i + 5] * inv), pack_bf16(ov[8 * i + 6] * inv, ov[8 * i + 7] * inv));
         }
       }
     }
   }
-  if (failed) atomicExch(p.error, 1);
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *gave_up) atomicExch(p.error, 1);
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
@@ -604,19 +720,23 @@ SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, 
   const int m_tiles = (max_q + tok_per_tile - 1) / tok_per_tile;
   p.heads_in_x = m_tiles <= 65535 ? 1 : 0;
   const dim3 grid = p.heads_in_x ? dim3(Hkv, m_tiles, n_rows) : dim3(m_tiles, Hkv, n_rows);
-  auto launch = [&](auto kernel, int smem) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return launch_pdl(kernel, grid, dim3(THREADS), (size_t)smem, stream, map_q, map_k, map_v, p);
+  auto launch = [&](auto fine, auto tight) -> int {
+    constexpr bool F = SHARED || decltype(fine)::value, T = D == 128 && decltype(tight)::value;
+    auto kernel = attention_tc_kernel<F, T>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<F, T>::SMEM_BYTES);
+    SB_PDL_CHECK(launch_pdl(kernel, grid, dim3(THREADS), (size_t)Layout<F, T>::SMEM_BYTES, stream, map_q, map_k, map_v, p));
+    return 0;
   };
   // in two parts where the mma.sync kernel would be the other choice (see the dispatch in kernels/cuda.py)
-  if constexpr (SHARED) {
-    SB_PDL_CHECK(launch(attention_tc_kernel<true>, Layout<true>::SMEM_BYTES));
-  } else if (window > 0 || kc == vc) {
-    SB_PDL_CHECK(launch(attention_tc_kernel<true>, Layout<true>::SMEM_BYTES));
-  } else {
-    SB_PDL_CHECK(launch(attention_tc_kernel<false>, Layout<false>::SMEM_BYTES));
+  const bool fine = SHARED || window > 0 || kc == vc;
+  if (D == 128) {
+    // Two CTAs an SM fill one another's gaps, but each has fewer buffers and takes longer by itself: they pay once an SM would walk a
+    // second CTA after its first. 24/8 heads, whole causal prompts, one | two an SM: 600 tokens (120 CTAs) 22.8 | 26.7 us, 1,024 (200) 37.2 | 39.1,
+    // 2,048 (392) 68.7 | 56.2, 4,096 (784) 170 | 126; 16/4 heads, window 1,024: 1,024 tokens (128) 18.9 | 20.8, 2,048 (256) 35.2 | 28.9.
+    if ((long long)Hkv * m_tiles * n_rows * 2 > 3LL * sm_count())
+      return fine ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{});
   }
-  return 0;
+  return fine ? launch(std::true_type{}, std::false_type{}) : launch(std::false_type{}, std::false_type{});
 }
 
 #else

@@ -109,3 +109,31 @@ def test_no_further_from_64_bits_than_the_mma_kernel(K, d, shared, window, sharp
         errors.append(float((out.double() - want).norm() / want.norm()))
     K.check_errors()
     assert errors[0] <= 1.05 * errors[1], errors
+
+
+@pytest.mark.parametrize("d,shared", [(64, False), (128, False), (128, True), (256, True)])
+@pytest.mark.parametrize("page", [16, 64, 192, 256])
+@pytest.mark.parametrize("window", [0, 333])
+@pytest.mark.parametrize("q_lens,kv_lens", [([129, 40], [129, 400]), ([900, 850], [900, 1000])], ids=["few", "many"])
+def test_references_that_move(K, d, shared, page, window, q_lens, kv_lens):  # noqa: F811
+    """Keys that grow along the sequence, a stronger one in either half of a tile in turn: the reference of a row's exponentials moves in tile
+    after tile, seen by one of the row's two threads only, and the accumulator is rescaled with it. With many tiles of rows the form
+    of head size 128 that shares an SM is taken, with few the other one."""
+    heads, kv_heads = (16, 1) if shared else (16, 8)
+    s = _paged_setup("bfloat16", heads, kv_heads, d, page, q_lens, kv_lens)
+    for r, L in enumerate(kv_lens):
+        for key in range(0, L, 41):                        # 41 and the tile's 64 keys have no common divisor: every place of both halves
+            s["kc"][int(s["bt"][r, key // page]), :, key % page] *= 1.0 + key / 100.0
+    if shared:
+        s["vc"] = s["kc"]
+    scale, t = 1.0 / math.sqrt(d), sum(q_lens)
+    out = torch.full((t, heads * d), float("nan"), device=DEV, dtype=torch.bfloat16)
+    want = torch.empty_like(out)
+    args = (s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, scale, window)
+    K.attention(s["qkv"], *args, out, s["shape"])
+    K.check_errors()
+    E.attention(s["qkv"], *args, want, s["shape"])
+    assert bool(torch.isfinite(out).all()), "a row was not written, or NaN"
+    # as above; the reference attention's scores and weights are 32-bit, so what differs is the weights' rounding (2^-8 of each) and both outputs'
+    top = float(s["vc"].float().abs().max())
+    torch.testing.assert_close(out.float(), want.float(), atol=2.0 ** -8 * top, rtol=2.0 ** -7)
