@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
 
   constexpr bool TURNS = MODE == GATED && ACCS == 1;         // gate and up rows take turns in one accumulator
   constexpr int MOST = MODE == GATED ? 64 * ACCS : 128 * ACCS;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int stage_bytes = ACCS * W_BYTES + x_rows_of(a.cap) * BK * 2;
   const int runs = a.n_tiles[0];
   const int which = ACCS == 2 || a.cap > 16 ? 0 : pick_unit(MODE, runs, a.cols, gridDim.x);
@@ -138,7 +138,8 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
   bool failed = false;
 
   if (warp == 0) {
-    int it = 0;
+    int it = 0, s = 0;                                       // stages filled so far, the next one, its barrier's parity
+    unsigned phase = 1;                                      // (fresh barriers pass a wait on parity 1)
     for (int unit = blockIdx.x; unit < units && !failed; unit += gridDim.x) {
       const int tile = unit / col_blocks, c0 = (unit - tile * col_blocks) * unit_cols;
       const int e = a.tiles[2 * tile], row0 = a.tiles[2 * tile + 1];
@@ -150,10 +151,8 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
       const CUtensorMap* map_rest = &maps.x[rest > 64 ? 0 : (rest > 16 ? 1 : 2)];
       const unsigned bytes = w_bytes + (full * 128 + rest_rows) * BK * 2;
       for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-        const int s = it % a.stages;
-        const bool ok = tc::mbar_wait(&empty_bar[s], ((it / a.stages) & 1) ^ 1);      // (fresh barriers pass a wait on parity 1)
-        if (!__all_sync(0xffffffffu, ok)) { failed = true; break; }
-        if (lane == 0) {
+        if (!tc::warp_wait(&empty_bar[s], phase)) { failed = true; break; }
+        if (tc::elect_one()) {
           unsigned char* w_dst = ring + (size_t)s * stage_bytes;
           unsigned char* x_dst = w_dst + ACCS * W_BYTES;
           tc::mbar_expect_tx(&full_bar[s], bytes);
@@ -169,37 +168,38 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
           if (rest) tc::load_2d(x_dst + full * 128 * BK * 2, map_rest, &full_bar[s], kb * BK, row0 + full * 128);
         }
         __syncwarp();
+        if (++s == a.stages) { s = 0; phase ^= 1; }
       }
     }
     // a wait that ran out: the copies under way land before the block's shared memory is given back (every other wait fails first)
     for (int f = max(0, it - a.stages); failed && f < it; ++f) tc::mbar_wait(&full_bar[f % a.stages], (f / a.stages) & 1);
   } else if (warp == 1) {
-    if (lane == 0) {
-      int it = 0, local = 0;
-      for (int unit = blockIdx.x; unit < units && !failed; unit += gridDim.x, ++local) {
-        const int tile = unit / col_blocks;
-        const int e = a.tiles[2 * tile], row0 = a.tiles[2 * tile + 1];
-        const int n = (min(a.cap, a.offsets[e + 1] - row0) + 15) & ~15;
-        const uint32_t idesc = tc::make_idesc(128, n);
-        const int buf = bufs == 2 ? local & 1 : 0, round = bufs == 2 ? local >> 1 : local;
-        if (!tc::mbar_wait(&acc_empty[buf], (round & 1) ^ 1)) { failed = true; break; }
+    const uint32_t ring_lo = tc::desc_lo(tc::smem_u32(ring));
+    int s = 0, local = 0;
+    unsigned phase = 0;
+    for (int unit = blockIdx.x; unit < units && !failed; unit += gridDim.x, ++local) {
+      const int tile = unit / col_blocks;
+      const int e = a.tiles[2 * tile], row0 = a.tiles[2 * tile + 1];
+      const int n = (min(a.cap, a.offsets[e + 1] - row0) + 15) & ~15;
+      const uint32_t idesc = tc::make_idesc(128, n);
+      const int buf = bufs == 2 ? local & 1 : 0, round = bufs == 2 ? local >> 1 : local;
+      if (!tc::warp_wait(&acc_empty[buf], (round & 1) ^ 1)) { failed = true; break; }
+      const uint32_t acc = tmem_base + (uint32_t)(buf * 256);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!tc::warp_wait(&full_bar[s], phase)) { failed = true; break; }
         tc::fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)(buf * 256);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % a.stages;
-          if (!tc::mbar_wait(&full_bar[s], (it / a.stages) & 1)) { failed = true; break; }
-          tc::fence_after();
-          const uint32_t w_addr = tc::smem_u32(ring + (size_t)s * stage_bytes);
-          const uint64_t dx = tc::make_desc(w_addr + ACCS * W_BYTES);
+        const uint32_t dw = ring_lo + (uint32_t)(s * (stage_bytes >> 4)), dx = dw + (uint32_t)(ACCS * W_BYTES >> 4);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int j = 0; j < BK / 16; ++j)
 #pragma unroll
             for (int i = 0; i < ACCS; ++i)
-              tc::mma(acc + (uint32_t)(i * acc_cols), tc::make_desc(w_addr + i * W_BYTES) + (uint64_t)(j * 2), dx + (uint64_t)(j * 2), idesc,
-                      (kb | j) != 0 ? 1u : 0u);
+              tc::mma_lo(acc + (uint32_t)(i * acc_cols), dw + (uint32_t)((i * W_BYTES >> 4) + j * 2), dx + (uint32_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
           tc::commit(&empty_bar[s]);
+          if (kb + 1 == k_blocks) tc::commit(&acc_full[buf]);
         }
-        tc::commit(&acc_full[buf]);
+        __syncwarp();
+        if (++s == a.stages) { s = 0; phase ^= 1; }
       }
     }
   } else {

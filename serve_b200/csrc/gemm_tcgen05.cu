@@ -20,6 +20,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "tcgen05_ops.cuh"
 
 using namespace sb;
 typedef __nv_bfloat16 bf16;
@@ -61,11 +62,6 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
 // 32 lanes x 32 columns of 32-bit accumulator: thread i of the warp gets lane (base lane + i), 32 consecutive columns
 __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -78,18 +74,6 @@ __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major tile stored by TMA with the 128-byte swizzle: rows of 128 bytes,
-// 8 rows to a 1024-byte atom, atoms one after the other (stride 1024 bytes); version 1, layout type 2.
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);            // start address, 16-byte units
-  d |= (uint64_t)0 << 16;                                 // leading byte offset: not used by this layout
-  d |= (uint64_t)(1024 >> 4) << 32;                       // stride byte offset between 8-row groups
-  d |= (uint64_t)1 << 46;                                 // descriptor version of this architecture
-  d |= (uint64_t)2 << 61;                                 // 128-byte swizzle
-  return d;
 }
 
 // kind::f16 instruction descriptor: float accumulator, bfloat16 a and b, both K-major, N x M of the tile
@@ -200,7 +184,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   // the dynamic region is aligned by hand: the 128-byte swizzle wants 1024-byte aligned tiles
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // bn: accumulator columns of a tile (a multiple of 32, at most BN), chosen by the host so that the tiles
   // fill whole waves of CTAs
   const int OUT_COLS = GU ? bn / 2 : bn;             // output columns of one tile
@@ -239,52 +223,50 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   bool failed = false;
 
   // tile t of this CTA: consecutive CTAs take the row tiles of one panel of w
+  const uint32_t tiles_lo = tc::desc_lo(smem_u32(tiles));
   if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;                                      // stages issued so far, over all tiles
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
-        const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * OUT_COLS;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % NSTAGE;
-          // a fresh barrier passes a wait on parity 1: the first round finds every stage free
-          if (!mbar_wait(&empty_bar[s], ((it / NSTAGE) & 1) ^ 1)) { failed = true; break; }
-          unsigned char* a_dst = tiles + (size_t)s * STAGE_BYTES;
+    int s = 0;
+    unsigned phase = 1;                                // a fresh barrier passes a wait on parity 1: the first round finds every stage free
+    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+      const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * OUT_COLS;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!tc::warp_wait(&empty_bar[s], phase)) { failed = true; break; }
+        if (tc::elect_one()) {
+          unsigned char* a_dst = tiles + s * STAGE_BYTES;
           unsigned char* b_dst = a_dst + A_BYTES;
           mbar_expect_tx(&full_bar[s], (unsigned)(A_BYTES + bn * BK * 2));
           tma_load_2d(a_dst, &map_a, &full_bar[s], kb * BK, m0);
-          if (GU) {
-            tma_load_2d(b_dst, &map_w, &full_bar[s], kb * BK, n0);                       // 128 gate rows
-            tma_load_2d(b_dst + (size_t)(bn / 2) * BK * 2, &map_w, &full_bar[s], kb * BK, N + n0);   // their up rows
-          } else {
-            tma_load_2d(b_dst, &map_w, &full_bar[s], kb * BK, n0);
-          }
+          tma_load_2d(b_dst, &map_w, &full_bar[s], kb * BK, n0);                         // with gate_up the gate rows
+          if (GU) tma_load_2d(b_dst + bn * BK, &map_w, &full_bar[s], kb * BK, N + n0);   // and their up rows
         }
+        __syncwarp();
+        if (++s == NSTAGE) { s = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(BM, bn);
-      int it = 0, local = 0;
-      for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
-        const int buf = local & 1;
-        // the epilogue must have emptied this accumulator (first use of each: passes at once)
-        if (!mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { failed = true; break; }
+    const uint32_t idesc = make_idesc(BM, bn);
+    int s = 0, local = 0;
+    unsigned phase = 0;
+    for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
+      const int buf = local & 1;
+      // the epilogue must have emptied this accumulator (first use of each: passes at once)
+      if (!tc::warp_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { failed = true; break; }
+      const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!tc::warp_wait(&full_bar[s], phase)) { failed = true; break; }
         tc_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % NSTAGE;
-          if (!mbar_wait(&full_bar[s], (it / NSTAGE) & 1)) { failed = true; break; }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + (size_t)s * STAGE_BYTES);
-          const uint64_t da = make_desc(a_addr), db = make_desc(a_addr + A_BYTES);
+        const uint32_t da = tiles_lo + (uint32_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int j = 0; j < BK / 16; ++j) {
             // 16 k-values further along the swizzled row: 32 bytes, two 16-byte units of the start address
-            tc_mma(acc, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
+            tc::mma_lo(acc, da + (uint32_t)(j * 2), db + (uint32_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
           }
           tc_commit(&empty_bar[s]);          // the stage is free once these products have read it
+          if (kb + 1 == k_blocks) tc_commit(&acc_full[buf]);     // the accumulator is complete once all products are done
         }
-        tc_commit(&acc_full[buf]);           // the accumulator is complete once all products are done
+        __syncwarp();
+        if (++s == NSTAGE) { s = 0; phase ^= 1; }
       }
     }
   } else {
@@ -383,11 +365,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(leader_bar), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void tc_mma_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
 // arrives, once the products issued so far are done, on the barrier at this address in both CTAs of the pair
 __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -411,7 +388,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
   __shared__ uint32_t tmem_base_s;
   unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem) + 1023) & ~(uintptr_t)1023);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
@@ -451,46 +428,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
   const uint32_t tmem_base = tmem_base_s;
   bool failed = false;
 
+  const uint32_t tiles_lo = tc::desc_lo(smem_u32(tiles));
   if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;
-      for (int tile = pair; tile < total_tiles && !failed; tile += num_pairs) {
-        const int m0 = (tile % m_tiles) * 256 + (int)rank * 128, n0 = (tile / m_tiles) * OUT_COLS;
-        // with gate_up the first CTA loads the gate rows and the second their up rows: accumulator columns
-        // 0 .. half-1 are gate, half .. bn-1 are up, for the rows of both CTAs
-        const int w_row = GU ? (rank == 0 ? n0 : N + n0) : n0 + (int)rank * half;
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % PAIR_STAGES;
-          if (!mbar_wait(&empty_bar[s], ((it / PAIR_STAGES) & 1) ^ 1)) { failed = true; break; }
-          unsigned char* a_dst = tiles + (size_t)s * PAIR_STAGE_BYTES;
+    int s = 0;
+    unsigned phase = 1;
+    for (int tile = pair; tile < total_tiles && !failed; tile += num_pairs) {
+      const int m0 = (tile % m_tiles) * 256 + (int)rank * 128, n0 = (tile / m_tiles) * OUT_COLS;
+      // with gate_up the first CTA loads the gate rows and the second their up rows: accumulator columns
+      // 0 .. half-1 are gate, half .. bn-1 are up, for the rows of both CTAs
+      const int w_row = GU ? (rank == 0 ? n0 : N + n0) : n0 + (int)rank * half;
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!tc::warp_wait(&empty_bar[s], phase)) { failed = true; break; }
+        if (tc::elect_one()) {
+          unsigned char* a_dst = tiles + s * PAIR_STAGE_BYTES;
           const uint32_t leader_bar = smem_u32(&full_bar[s]) & PAIR_LEADER_MASK;
           if (rank == 0) mbar_expect_tx(&full_bar[s], (unsigned)(2 * (PAIR_A_BYTES + half * BK * 2)));
           tma_load_2d_pair(a_dst, &map_a, leader_bar, kb * BK, m0);
           tma_load_2d_pair(a_dst + PAIR_A_BYTES, &map_w, leader_bar, kb * BK, w_row);
         }
+        __syncwarp();
+        if (++s == PAIR_STAGES) { s = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      const uint32_t idesc = make_idesc(256, bn);
-      int it = 0, local = 0;
-      for (int tile = pair; tile < total_tiles && !failed; tile += num_pairs, ++local) {
-        const int buf = local & 1;
-        if (!mbar_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { failed = true; break; }
+    const uint32_t idesc = make_idesc(256, bn);
+    int s = 0, local = 0;
+    unsigned phase = 0;
+    for (int tile = pair; rank == 0 && tile < total_tiles && !failed; tile += num_pairs, ++local) {
+      const int buf = local & 1;
+      if (!tc::warp_wait(&acc_empty[buf], ((local >> 1) & 1) ^ 1)) { failed = true; break; }
+      const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (!tc::warp_wait(&full_bar[s], phase)) { failed = true; break; }
         tc_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
-        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
-          const int s = it % PAIR_STAGES;
-          if (!mbar_wait(&full_bar[s], (it / PAIR_STAGES) & 1)) { failed = true; break; }
-          tc_fence_after();
-          const uint32_t a_addr = smem_u32(tiles + (size_t)s * PAIR_STAGE_BYTES);
-          const uint64_t da = make_desc(a_addr), db = make_desc(a_addr + PAIR_A_BYTES);
+        const uint32_t da = tiles_lo + (uint32_t)(s * (PAIR_STAGE_BYTES >> 4)), db = da + (PAIR_A_BYTES >> 4);
+        if (tc::elect_one()) {
 #pragma unroll
           for (int j = 0; j < BK / 16; ++j)
-            tc_mma_pair(acc, da + (uint64_t)(j * 2), db + (uint64_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
+            tc::mma_pair_lo(acc, da + (uint32_t)(j * 2), db + (uint32_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
           tc_commit_pair(&empty_bar[s]);
+          if (kb + 1 == k_blocks) tc_commit_pair(&acc_full[buf]);
         }
-        tc_commit_pair(&acc_full[buf]);
+        __syncwarp();
+        if (++s == PAIR_STAGES) { s = 0; phase ^= 1; }
       }
     }
   } else {
