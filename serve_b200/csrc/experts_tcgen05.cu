@@ -8,15 +8,16 @@
 // A unit of work is (an expert's run of tokens, some rows of its matrix). Persistent CTAs, one an SM, take units in turn.
 // Warp 0 feeds a ring of stages of 64 k-values with TMA: weight rows, and the tokens' rows from an operand in grouped
 // order (moe_gather_kernel makes it for gate/up: fetching the rows from the activations with tile::gather4 instead took
-// 115 cycles for every four rows, and the gate/up product of 2,048 tokens 170 us). One thread of warp 1 issues the products;
+// 115 cycles for every four rows, and the gate/up product of 2,048 tokens 170 us). Warp 1 issues the products (both walk their loops
+// as whole warps, see elect_one: issued by one thread of a divergent warp, behind a division by the number of stages, 8 tokens' gate/up took
+// 44.7 us in place of 32.7);
 // sixteen warps take the finished sums out of tensor memory. The ring runs on into the next unit while sums are taken out,
 // so the weights keep streaming although a wide unit has a single set of accumulators.
 //
 // A unit with two accumulators is 256 weight rows: many tokens an expert, where the tokens' rows are what the SMs fetch
 // most. A unit with one is at most 128 rows, of a count that shares the step's rows out evenly over the SMs (pick_unit):
 // few tokens an expert, where a unit is nothing but weights and a last round of a few units would leave most SMs idle.
-// A TMA instruction costs its issuer more than a hundred cycles however little it fetches, so a stage takes as few as
-// possible: there is a map for every count of weight rows a unit may have, and maps of 128, 64 and 16 tokens.
+// Every TMA instruction costs its issuer time however little it fetches, so a stage takes as few as possible: there is a map for every count of weight rows a unit may have, and maps of 128, 64 and 16 tokens.
 //
 //   gate/up:  act[row, c] = f(g, u): with two accumulators the gate rows are one and the up rows of the same outputs the
 //             other, so a thread holds both sums; with one, 16 gate rows and the 16 up rows of the same outputs take turns
@@ -321,14 +322,15 @@ int launch(const void* w, const void* x, int n_pairs, int E, Args a, cudaStream_
 }
 
 // One accumulator a unit or two. Up to 16 tokens (a run is one group of 16 columns): what costs less for the number of
-// experts that as many uniform choices hit. Measured at width 2,048, 64 experts, 4 a token, gate/up with one | two: 1 token 18.8 |
-// 23.4 us, 4 tokens 31.4 | 24.9, 8 tokens 44.9 | 48.2 (156 units of two for 148 SMs); mma.sync tiles of 64 tokens had taken 27.8,
-// 35.2 and 50.0. More tokens: two, since the tokens' rows are then fetched half as often (64 tokens 93.7 | 71.0 us; mma.sync
-// 101.4; 2,048 tokens 113 | 108, mma.sync 261). A down unit of 256 tokens is short (ff k-values) and its sums are many: with one
-// accumulator there is room for two sets, and taking sums out overlaps the next unit's products (2,048 tokens 51.3 | 57.4 us,
-// mma.sync 152; 4,096 tokens of width 4,096, 8 a token 182 | 200, mma.sync 746).
+// experts that as many uniform choices hit. Gate/up with one | two at width 2,048, 64 experts, 4 a token: 1 token 14.2 | 17.8 us, 4 tokens 23.8 | 22.9,
+// 8 tokens 32.4 | 39.7 (156 units of two for 148 SMs), 16 tokens 45.6 | 43.9. Up to 128 tokens two: the tokens' rows are then fetched half as often
+// (64 tokens 69.6 | 68.4). With more there is room in tensor memory for two sets of sums only if a unit has one accumulator, and taking
+// sums out overlaps the next unit's products: gate/up of 256 tokens 77.2 | 79.4, 2,048 tokens 92.4 | 105.4, 4,096 tokens 118 | 146; down of 2,048
+// tokens 47.7 | 54.5. Long rows of few tokens an expert are the exception (width 4,096, 64 experts, 8 a token: gate/up of 512
+// tokens 113.9 | 110.4, of 1,024 125.2 | 127.9).
 int pick_accs(int mode, const Args& a, int n_pairs, int E) {
-  if (a.cap > 16) return mode == DOWN && a.cap == MAX_TOKENS ? 1 : 2;
+  if (a.cap > 128) return mode == GATED && a.K > 3072 && n_pairs < 100 * E ? 2 : 1;
+  if (a.cap > 16) return 2;
   float miss = 1.f;
   for (int i = 0; i < n_pairs && i < 256; ++i) miss *= 1.f - 1.f / (float)E;
   const int runs = (int)((float)E * (1.f - miss) + 0.5f), sms = sm_count();

@@ -652,11 +652,11 @@ int run_product(const void* a, const void* w, void* out, int M, int N, int K, in
     }
   }
   cudaError_t e;
-  // At equal cost the pair kernel wins only where a CTA has enough to do: starting and ending a cluster costs it about
-  // 2 us more than the one-CTA kernel (2,048 rows: q/k/v 32.5 against 29.8 us, output projection 20.5 against 18.7, but
-  // down projection, four times as many k-values, 53.3 against 54.8).
+  // At equal cost the pair kernel wins where a CTA has more than a tile or two of few k-values to do: starting and ending a cluster
+  // costs it about 1 us more than the one-CTA kernel (one CTA | pair: q/k/v, 2,048 k-values, 600 rows 12.1 | 12.2 us, 1,700 rows 25.9 | 21.6, 2,048 rows
+  // 26.7 | 23.9; gate/up to 768, 2,048 rows 20.7 | 21.3; gate/up to 8,192 of 3,072, 1,700 rows 135.6 | 126.4).
   const long long k_blocks = (K + BK - 1) / BK;
-  const bool pair_wins = cost_pair < cost_single || (cost_pair == cost_single && waves_pair * k_blocks >= 96);
+  const bool pair_wins = cost_pair < cost_single || (cost_pair == cost_single && waves_pair * k_blocks >= 64);
   if (pairs > 0 && (pair_wins || g_pair_enabled == 2)) {
     const long long m_tiles = (M + 255) / 256;
     const int bn = bn_pair;

@@ -189,43 +189,80 @@ __global__ void __launch_bounds__(128) moe_route_bias_kernel(const float* __rest
 
 constexpr int TM = 32;            // rows of a tile of the plain-arithmetic products (experts_tcgen05.cu has the others)
 
-// One block. order[offsets[e] .. offsets[e+1]) = the pairs of expert e; tiles: (expert, first row) for every TM rows
-// of an expert's group, n_tiles[0] of them.
+// One block. order[offsets[e] .. offsets[e+1]) = the pairs of expert e; tiles: (expert, first row) for every tile_rows rows
+// of an expert's group, n_tiles[0] of them. A pair's place among its expert's comes from the atomic that counts it, kept in registers
+// for up to SORT_KEEP pairs a thread (more: counted a second time); the experts' first places and tiles from one scan over the block.
+// Bound by latency: 8,192 pairs of 64 experts 13.7 -> 8.9 us, 32 pairs 6.4 -> 2.7 (one thread had walked the experts).
+constexpr int SORT_KEEP = 8;
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, int n_pairs, int E, int tile_rows,
                                                         int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ tiles,
                                                         int* __restrict__ n_tiles) {
   extern __shared__ int sh[];
   int* count = sh;            // [E]
-  int* start = sh + E;        // [E + 1]
-  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+  int* start = sh + E;        // [E]
+  __shared__ int2 warp_sums[32];
+  const int tid = threadIdx.x, n_threads = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const bool keeps = n_pairs <= SORT_KEEP * n_threads;
+  int mine[SORT_KEEP], rank[SORT_KEEP];
+#pragma unroll
+  for (int u = 0; u < SORT_KEEP; ++u) mine[u] = tid + u * n_threads < n_pairs && keeps ? idx[tid + u * n_threads] : -1;
+  for (int e = tid; e < E; e += n_threads) count[e] = 0;
   __syncthreads();
-  for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-    const int e = idx[p];
-    if (e >= 0 && e < E) atomicAdd(&count[e], 1);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int at = 0, nt = 0;
-    for (int e = 0; e < E; ++e) {
-      start[e] = at;
-      offsets[e] = at;
-      for (int r0 = 0; r0 < count[e]; r0 += tile_rows) {
-        tiles[2 * nt] = e;
-        tiles[2 * nt + 1] = at + r0;
-        ++nt;
-      }
-      at += count[e];
+  if (keeps) {
+#pragma unroll
+    for (int u = 0; u < SORT_KEEP; ++u)
+      if (mine[u] >= 0 && mine[u] < E) rank[u] = atomicAdd(&count[mine[u]], 1);
+  } else {
+    for (int p = tid; p < n_pairs; p += n_threads) {
+      const int e = idx[p];
+      if (e >= 0 && e < E) atomicAdd(&count[e], 1);
     }
-    start[E] = at;
-    offsets[E] = at;
-    n_tiles[0] = nt;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+  // a thread takes ``per`` neighbouring experts: (pairs, tiles) before them
+  const int per = (E + n_threads - 1) / n_threads, e0 = min(E, tid * per), e1 = min(E, e0 + per);
+  int pairs = 0, n = 0;
+  for (int e = e0; e < e1; ++e) { pairs += count[e]; n += (count[e] + tile_rows - 1) / tile_rows; }
+  int sp = pairs, sn = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int ap = __shfl_up_sync(0xffffffffu, sp, o), an = __shfl_up_sync(0xffffffffu, sn, o);
+    if (lane >= o) { sp += ap; sn += an; }
+  }
+  if (lane == 31) warp_sums[warp] = make_int2(sp, sn);
   __syncthreads();
-  for (int p = threadIdx.x; p < n_pairs; p += blockDim.x) {
-    const int e = idx[p];
-    if (e >= 0 && e < E) order[start[e] + atomicAdd(&count[e], 1)] = p;
+  int at = sp - pairs, nt = sn - n, all_pairs = 0, all_tiles = 0;
+  for (int w = 0; w < n_threads / 32; ++w) {
+    const int2 v = warp_sums[w];
+    if (w < warp) { at += v.x; nt += v.y; }
+    all_pairs += v.x;
+    all_tiles += v.y;
+  }
+  for (int e = e0; e < e1; ++e) {
+    const int c = count[e];
+    start[e] = at;
+    offsets[e] = at;
+    for (int r0 = 0; r0 < c; r0 += tile_rows, ++nt) {
+      tiles[2 * nt] = e;
+      tiles[2 * nt + 1] = at + r0;
+    }
+    at += c;
+    if (!keeps) count[e] = 0;
+  }
+  if (tid == 0) {
+    offsets[E] = all_pairs;
+    n_tiles[0] = all_tiles;
+  }
+  __syncthreads();
+  if (keeps) {
+#pragma unroll
+    for (int u = 0; u < SORT_KEEP; ++u)
+      if (mine[u] >= 0 && mine[u] < E) order[start[mine[u]] + rank[u]] = tid + u * n_threads;
+  } else {
+    for (int p = tid; p < n_pairs; p += n_threads) {
+      const int e = idx[p];
+      if (e >= 0 && e < E) order[start[e] + atomicAdd(&count[e], 1)] = p;
+    }
   }
 }
 
@@ -425,50 +462,81 @@ template <> __device__ __forceinline__ void moe_store4<__nv_bfloat16>(__nv_bfloa
   *reinterpret_cast<uint2*>(p) = u;
 }
 
-// VEC elements a thread (4: N and x_stride multiples of 4, every pointer 16-byte aligned; else 1).
-template <typename T, int VEC>
+// The same four elements a thread, a block a part of one token's row: the rows of four choices are under way at a time, and which choices
+// are experts is known before the loads. idx null: all are. 2,048 tokens, 4 choices, width 2,048 (84 MB): 19.5 -> 18.8 us;
+// 8 tokens 3.7 -> 3.3.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __restrict__ parts, const int* __restrict__ idx, const float* __restrict__ wts,
+                                                               int E_real, const T* __restrict__ x, int x_stride, const T* __restrict__ shared,
+                                                               const float* __restrict__ gate, int gate_stride, int top, int N, int blocks_a_row,
+                                                               T* __restrict__ out) {
+  const int t = blockIdx.x / blocks_a_row, c = ((blockIdx.x - t * blocks_a_row) * 256 + threadIdx.x) * 4;
+  if (c >= N) return;
+  float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
+  float g = 1.f;
+  if (shared) {
+    sv = moe_load4<T>(shared + (size_t)t * N + c);
+    if (gate) g = gate[(size_t)t * gate_stride];
+  }
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int k0 = 0; k0 < top; k0 += 4) {
+    float4 v[4];
+    float f[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const size_t pair = (size_t)t * top + k0 + u;
+      f[u] = 0.f;
+      if (k0 + u < top) f[u] = !idx || idx[pair] < E_real ? 1.f : wts[pair];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const size_t pair = (size_t)t * top + k0 + u;
+      if (k0 + u < top) v[u] = !idx || idx[pair] < E_real ? *reinterpret_cast<const float4*>(parts + pair * N + c) : moe_load4<T>(x + (size_t)t * x_stride + c);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k0 + u < top) {
+        s.x = fmaf(f[u], v[u].x, s.x); s.y = fmaf(f[u], v[u].y, s.y); s.z = fmaf(f[u], v[u].z, s.z); s.w = fmaf(f[u], v[u].w, s.w);
+      }
+  }
+  if (shared) {
+    if (gate) g = sigmoid_f(g);
+    s.x = fmaf(g, sv.x, s.x); s.y = fmaf(g, sv.y, s.y); s.z = fmaf(g, sv.z, s.z); s.w = fmaf(g, sv.w, s.w);
+  }
+  moe_store4<T>(out + (size_t)t * N + c, s);
+}
+
+// an element a thread, for rows that are not made of whole pieces of four
+template <typename T>
 __global__ void __launch_bounds__(256) moe_combine_more_kernel(const float* __restrict__ parts, const int* __restrict__ idx,
                                                                const float* __restrict__ wts, int E_real, const T* __restrict__ x,
                                                                int x_stride, const T* __restrict__ shared, const float* __restrict__ gate,
                                                                int gate_stride, int top, int N, long long total, T* __restrict__ out) {
-  const int nv = N / VEC;
   for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(w / nv);
-    const int c = (int)(w - (long long)t * nv) * VEC;
-    float s[VEC];
-#pragma unroll
-    for (int v = 0; v < VEC; ++v) s[v] = 0.f;
+    const int t = (int)(w / N);
+    const int c = (int)(w - (long long)t * N);
+    float s = 0.f;
     for (int k = 0; k < top; ++k) {
       const size_t pair = (size_t)t * top + k;
-      if (idx[pair] < E_real) {
-        if (VEC == 4) {
-          const float4 p4 = *reinterpret_cast<const float4*>(parts + pair * N + c);
-          s[0] += p4.x; s[1 % VEC] += p4.y; s[2 % VEC] += p4.z; s[3 % VEC] += p4.w;
-        } else {
-          s[0] += parts[pair * N + c];
-        }
-      } else {
-        const float wt = wts[pair];
-        if (VEC == 4) {
-          const float4 x4 = moe_load4<T>(x + (size_t)t * x_stride + c);
-          s[0] += wt * x4.x; s[1 % VEC] += wt * x4.y; s[2 % VEC] += wt * x4.z; s[3 % VEC] += wt * x4.w;
-        } else {
-          s[0] += wt * to_float(x[(size_t)t * x_stride + c]);
-        }
-      }
+      if (idx[pair] < E_real) s += parts[pair * N + c];
+      else s = fmaf(wts[pair], to_float(x[(size_t)t * x_stride + c]), s);
     }
-    if (shared) {
-      const float g = gate ? sigmoid_f(gate[(size_t)t * gate_stride]) : 1.f;
-      if (VEC == 4) {
-        const float4 h4 = moe_load4<T>(shared + (size_t)t * N + c);
-        s[0] += g * h4.x; s[1 % VEC] += g * h4.y; s[2 % VEC] += g * h4.z; s[3 % VEC] += g * h4.w;
-      } else {
-        s[0] += g * to_float(shared[(size_t)t * N + c]);
-      }
-    }
-    if (VEC == 4) moe_store4<T>(out + (size_t)t * N + c, make_float4(s[0], s[1 % VEC], s[2 % VEC], s[3 % VEC]));
-    else out[(size_t)t * N + c] = from_float<T>(s[0]);
+    if (shared) s = fmaf(gate ? sigmoid_f(gate[(size_t)t * gate_stride]) : 1.f, to_float(shared[(size_t)t * N + c]), s);
+    out[w] = from_float<T>(s);
   }
+}
+
+// false: the rows are not made of whole, aligned pieces of four
+template <typename T>
+bool combine_rows(const float* parts, const int* idx, const float* wts, int E_real, const void* x, int x_stride, const void* shared, const float* gate,
+                  int gate_stride, int top, int n_tokens, int N, void* out, cudaStream_t stream) {
+  const int per_row = (N / 4 + 255) / 256;
+  if (N % 4 || x_stride % 4 || !aligned16(parts) || !aligned16(x) || !aligned16(out) || (shared && !aligned16(shared)) ||
+      (long long)n_tokens * per_row > 2147483647LL)
+    return false;
+  moe_combine_rows_kernel<T><<<n_tokens * per_row, 256, 0, stream>>>(parts, idx, wts, E_real, (const T*)x, x_stride, (const T*)shared, gate, gate_stride, top,
+                                                                  N, per_row, (T*)out);
+  return true;
 }
 
 }  // namespace
@@ -492,7 +560,9 @@ SB_EXPORT int sb_moe_sort(const int* idx, int n_pairs, int E, int tile_rows, int
                           cudaStream_t stream) {
   if (n_pairs <= 0) return 0;
   if (E <= 0 || E > 4096 || tile_rows <= 0) return SB_ERR_LIMIT;
-  moe_sort_kernel<<<1, 1024, (size_t)(2 * E + 1) * sizeof(int), stream>>>(idx, n_pairs, E, tile_rows, offsets, order, tiles, n_tiles);
+  // few pairs: few warps, whose barriers are short
+  const int want = n_pairs / 4 > E ? n_pairs / 4 : E, threads = want >= 1024 ? 1024 : want <= 128 ? 128 : (want + 31) / 32 * 32;
+  moe_sort_kernel<<<1, threads, (size_t)(2 * E) * sizeof(int), stream>>>(idx, n_pairs, E, tile_rows, offsets, order, tiles, n_tiles);
   SB_LAUNCH_CHECK();
   return 0;
 }
@@ -578,12 +648,15 @@ SB_EXPORT int sb_moe_down(const void* act, const void* w_down, const int* order,
 // parts float [T * top, N] -> out [T, N]: a token's rows added in the order of its choices.
 SB_EXPORT int sb_moe_combine(const float* parts, int top, int n_tokens, int N, void* out, int dtype, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  const long long total = (long long)n_tokens * N;
-  const long long want = (total + 255) / 256;
-  const int blocks = (int)(want < sm_count() * 8 ? want : sm_count() * 8);
-  if (dtype == SB_DTYPE_F32) moe_combine_kernel<float><<<blocks, 256, 0, stream>>>(parts, top, N, total, (float*)out);
-  else if (dtype == SB_DTYPE_BF16) moe_combine_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(parts, top, N, total, (__nv_bfloat16*)out);
-  else return SB_ERR_DTYPE;
+  if (dtype != SB_DTYPE_F32 && dtype != SB_DTYPE_BF16) return SB_ERR_DTYPE;
+  const bool f32 = dtype == SB_DTYPE_F32;
+  if (!(f32 ? combine_rows<float>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream)
+            : combine_rows<__nv_bfloat16>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream))) {
+    const long long total = (long long)n_tokens * N, want = (total + 255) / 256;
+    const int blocks = (int)(want < sm_count() * 8 ? want : sm_count() * 8);
+    if (f32) moe_combine_kernel<float><<<blocks, 256, 0, stream>>>(parts, top, N, total, (float*)out);
+    else moe_combine_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(parts, top, N, total, (__nv_bfloat16*)out);
+  }
   SB_LAUNCH_CHECK();
   return 0;
 }
@@ -615,19 +688,19 @@ SB_EXPORT int sb_moe_combine_more(const float* parts, const int* idx, const floa
                                   int dtype, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (!parts || !idx || !wts || !x || top <= 0 || x_stride < N) return SB_ERR_SHAPE;
-  const bool vec = N % 4 == 0 && x_stride % 4 == 0 && aligned16(parts) && aligned16(x) && aligned16(out) && (!shared || aligned16(shared));
-  const long long total = (long long)n_tokens * (vec ? N / 4 : N);
-  const long long want = (total + 255) / 256;
-  const int blocks = (int)(want < sm_count() * 16 ? want : sm_count() * 16);
-  if (dtype == SB_DTYPE_F32) {
-    auto k = vec ? moe_combine_more_kernel<float, 4> : moe_combine_more_kernel<float, 1>;
-    k<<<blocks, 256, 0, stream>>>(parts, idx, wts, E_real, (const float*)x, x_stride, (const float*)shared, gate, gate_stride, top, N, total,
-                                  (float*)out);
-  } else if (dtype == SB_DTYPE_BF16) {
-    auto k = vec ? moe_combine_more_kernel<__nv_bfloat16, 4> : moe_combine_more_kernel<__nv_bfloat16, 1>;
-    k<<<blocks, 256, 0, stream>>>(parts, idx, wts, E_real, (const __nv_bfloat16*)x, x_stride, (const __nv_bfloat16*)shared, gate, gate_stride,
-                                  top, N, total, (__nv_bfloat16*)out);
-  } else return SB_ERR_DTYPE;
+  if (dtype != SB_DTYPE_F32 && dtype != SB_DTYPE_BF16) return SB_ERR_DTYPE;
+  const bool f32 = dtype == SB_DTYPE_F32;
+  if (!(f32 ? combine_rows<float>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream)
+            : combine_rows<__nv_bfloat16>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream))) {
+    const long long total = (long long)n_tokens * N, want = (total + 255) / 256;
+    const int blocks = (int)(want < sm_count() * 16 ? want : sm_count() * 16);
+    if (f32)
+      moe_combine_more_kernel<float><<<blocks, 256, 0, stream>>>(parts, idx, wts, E_real, (const float*)x, x_stride, (const float*)shared, gate,
+                                                                 gate_stride, top, N, total, (float*)out);
+    else
+      moe_combine_more_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(parts, idx, wts, E_real, (const __nv_bfloat16*)x, x_stride,
+                                                                         (const __nv_bfloat16*)shared, gate, gate_stride, top, N, total, (__nv_bfloat16*)out);
+  }
   SB_LAUNCH_CHECK();
   return 0;
 }

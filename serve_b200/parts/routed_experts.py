@@ -89,7 +89,12 @@ class RoutedExperts(FeedForward):
     def load(self, tensors):
         # the shared expert's gate is one more row of the router's matrix: one product gives all the float logits
         rows = [tensors[self.router_name]] + ([tensors[self.shared_gate_name]] if self.shared_gated else [])
-        self.w_router = torch.cat(rows, dim=0).contiguous()
+        w = torch.cat(rows, dim=0)
+        if not self.plain and w.shape[0] % 8:
+            # rows of zeros up to a multiple of eight, so that a row of logits is whole 16-byte pieces: the library's product of 2,048 tokens
+            # with 65 rows of 2,048 takes 17.5 us, with 72 rows 7 (nobody reads the columns beyond)
+            w = torch.cat([w, w.new_zeros((-w.shape[0] % 8, w.shape[1]))], dim=0)
+        self.w_router = w.contiguous()
         self.choice_bias = tensors[self.correction_name].float().contiguous() if self.correction else None
         if self.shared is not None:
             self.shared.load(tensors)

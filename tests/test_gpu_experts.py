@@ -101,3 +101,32 @@ def test_grouped_tokens_take_no_room_of_their_own():
     run()
     # float sums and activations of every pair; choices, weights and the grouping's lists are a few dozen bytes a pair
     assert torch.cuda.max_memory_allocated() - before <= TOP * tokens * (4 * n + 2 * ff + 64) + 16384
+
+
+@pytest.mark.parametrize("pairs,experts,rows", [(1, 1, 16), (32, 64, 16), (33, 5, 16), (1024, 64, 256), (8192, 64, 256), (8200, 64, 256), (40000, 96, 256),
+                                                (700, 1500, 32), (9000, 3000, 256)])
+def test_grouping_by_expert(pairs, experts, rows):
+    """Every pair once at a place of its expert's run, the runs in the experts' order, a tile for every ``rows`` rows of a run; choices that
+    name no expert have no place."""
+    g = torch.Generator(device="cuda").manual_seed(pairs)
+    idx = torch.randint(0, experts + 1, (pairs,), generator=g, device="cuda", dtype=torch.int32)        # ``experts`` itself: none
+    ints = lambda n: torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    offsets, order, tiles, n_tiles = ints(experts + 1), ints(pairs), ints(2 * (pairs // rows + min(experts, pairs)) + 2), ints(1)
+    import ctypes
+
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    assert kernels._moe_lib().sb_moe_sort(p(idx), pairs, experts, rows, p(offsets), p(order), p(tiles), p(n_tiles), kernels._s()) == 0
+    counts = torch.bincount(idx.long(), minlength=experts + 1)[:experts].tolist()
+    want = [0]
+    for n in counts:
+        want.append(want[-1] + n)
+    assert offsets.tolist() == want
+    got, tile = order.tolist(), []
+    for e, n in enumerate(counts):
+        assert sorted(got[want[e]: want[e + 1]]) == (idx == e).nonzero().flatten().tolist()
+        tile += [(e, want[e] + r) for r in range(0, n, rows)]
+    assert n_tiles.item() == len(tile) and tiles[: 2 * len(tile)].view(-1, 2).tolist() == [list(t) for t in tile]
+    assert got[want[-1]:] == [-7] * (pairs - want[-1])
