@@ -10,8 +10,8 @@
 // decay that underflows is simply zero.
 //   chunk_prep_*_kernel: a block a (chunk, head), all chunks at once: P, Q', K'', c; for the delta rule W = (I + A)^-1 diag(b) K' and
 //     V' = (I + A)^-1 diag(b) V by forward substitution, a thread a column, so that U = V' - W S.
-//   chunk_walk_kernel: a block a (request, head, 16 columns of S), a chain of tokens / 32 steps: [W; Q'] S, then U, then O and the
-//     next S. The matrices come through a ring of two stages; S lives in the accumulator layout in registers.
+//   chunk_walk_kernel, chunk_wide_kernel: a block a (request, head, 16 columns of S, or 32 or 64), a chain of tokens / 32 steps: [W; Q'] S,
+//     then U, then O and the next S. The matrices come through a ring of two stages; S lives in the accumulator layout in registers.
 //
 // All of this counts as 32-bit. The products run on the tensor cores (mma.sync m16n8k16) with every float x split into three bfloat16
 // numbers h + m + l = x (8 bits each, nothing left), six of the nine products of the parts (the others are below 2^-24), smallest
@@ -124,7 +124,7 @@ __device__ __forceinline__ bool find_chunk(const SbChunkedWalk& a, int i, int c,
   const int q0 = a.cu_q[r], n = a.cu_q[r + 1] - q0;
   if (n <= a.min_tokens || c * CH >= n) return false;
   int before = 0;
-  for (int u = threadIdx.x; u < i; u += THREADS) {
+  for (int u = threadIdx.x; u < i; u += blockDim.x) {
     const int ru = a.rows ? a.rows[u] : u;
     const int nu = a.cu_q[ru + 1] - a.cu_q[ru];
     if (nu > a.min_tokens) before += (nu + CH - 1) / CH;
@@ -135,7 +135,7 @@ __device__ __forceinline__ bool find_chunk(const SbChunkedWalk& a, int i, int c,
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = before;
     __syncthreads();
     before = 0;
-    for (int u = 0; u < THREADS / 32; ++u) before += red[u];
+    for (int u = 0; u < (int)blockDim.x / 32; ++u) before += red[u];
   }
   p.row = r;
   p.t0 = q0 + c * CH;
@@ -740,6 +740,350 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const SbChunkedWalk
     }
 }
 
+// The walk for many (request, head) pairs: G groups of 16 columns in a block, KS warps a group with DKT / KS rows of S each, and a warp that
+// fetches. A chunk's matrices then cross to an SM once for 16 G columns instead of once for 16, and since S lies turned over in
+// the accumulators (columns of S are the tile's rows), they are the first operand of the next product as they stand: S and U never
+// pass through shared memory, and the warps of a group meet once a step, to add their sums of W S (and Q' S) up. What bounds it: mma.sync, 16
+// cycles each on a scheduler (1,728 of them a step with 64 columns and no delta rule, 6,900 of the step's 7,900 cycles). With few pairs there
+// are not enough blocks, and chunk_walk_kernel, whose eight warps share 16 columns, has the shorter step. Eight requests of 256 tokens, 16
+// heads of 128 x 128: fixed decay 101 -> 67 us, gated delta rule 121 -> 95. (One warp for all rows of 16 columns: 91 us, registers spill;
+// the sums of Q' S a step behind those of W S, so that they hide: 107, more of them spill.)
+template <int DKT, bool DELTA, int KS, int G>
+struct Wide {
+  typedef Part<DKT, DELTA> L;
+  static constexpr int WARPS = KS * G, THREADS = 32 * (WARPS + 1);
+  static constexpr int TILES = DELTA ? 8 : 4;             // eights of rows of [W; Q'] (or Q')
+  static constexpr int XCH_OFF = 2 * L::BYTES, BYTES = XCH_OFF + (KS > 1 ? 2 * WARPS * TILES * 32 * 16 : 0);
+  static_assert(BYTES <= 226 * 1024, "shared memory of an SM");
+};
+
+__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ bool group_any(int id, int threads, bool yes) {
+  uint32_t any;
+  asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 q, %3, 0;\n bar.red.or.pred p, %1, %2, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(any) : "r"(id), "r"(threads), "r"(yes ? 1u : 0u) : "memory");
+  return any != 0;
+}
+// the parts of 16 columns (j) by 16 terms as a first operand, from two neighbouring accumulators' registers
+__device__ __forceinline__ void parts_of(uint32_t (&p)[3][4], const float (&x)[4], const float (&y)[4]) {
+  uint32_t q[4][3];
+  split3(x[0], x[1], q[0]);
+  split3(x[2], x[3], q[1]);
+  split3(y[0], y[1], q[2]);
+  split3(y[2], y[3], q[3]);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) p[i][r] = q[r][i];
+}
+
+// grid (ceil(dv / (16 G)), head, list entry).
+template <int DKT, bool DELTA, int KS, int G>
+__global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbChunkedWalk a, const float* __restrict__ u_rows) {
+  typedef Wide<DKT, DELTA, KS, G> W;
+  typedef Part<DKT, DELTA> L;
+  constexpr int AP = L::AP, ROWS = L::ROWS, TILES = W::TILES, NTS = DKT / KS / 8, OT = 4 / KS;
+  constexpr int LEFT[6] = {2, 0, 1, 1, 0, 0}, RIGHT[6] = {0, 2, 1, 0, 1, 0};      // six of the nine products of the parts, smallest first
+  extern __shared__ __align__(16) unsigned char raw[];
+  __shared__ int red_i[16];
+  __shared__ __align__(8) uint64_t full[2], empty[2];
+  __shared__ int gave_up;
+  Place p;
+  if (!find_chunk(a, blockIdx.z, 0, p, red_i)) return;
+  const int h = blockIdx.y;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int groups = min(G, (a.dv - (int)blockIdx.x * 16 * G + 15) / 16);          // (at the last columns not all have any)
+  const unsigned char* images = reinterpret_cast<const unsigned char*>(a.work) + (p.slot * a.H + h) * (long long)L::BYTES;
+  if (tid == 0) {
+    gave_up = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], groups * KS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  // A wait that runs out is noted; after it no wait lasts, every warp stays in step to the end, and what is computed is not valid.
+  auto wait = [&](uint64_t* bar, unsigned parity) {
+    if (tc::mbar_try(bar, parity)) return;
+    for (unsigned i = 0; i < tc::WAIT_LIMIT; ++i) {
+      if (tc::mbar_try(bar, parity)) return;
+      if ((i & 1023u) == 1023u && *(volatile int*)&gave_up) return;
+    }
+    *(volatile int*)&gave_up = 1;
+  };
+
+  if (warp == W::WARPS) {                                  // a chunk's matrices are one piece: one bulk copy
+    int c = 0;
+    for (; c < p.n_chunks; ++c) {
+      wait(&empty[c & 1], ((c >> 1) & 1) ^ 1);
+      if (*(volatile int*)&gave_up) break;
+      __syncwarp();
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(&full[c & 1], L::BYTES);
+        bulk_load(raw + (c & 1) * L::BYTES, images + (long long)c * a.H * L::BYTES, L::BYTES, &full[c & 1]);
+      }
+      __syncwarp();
+    }
+    if (*(volatile int*)&gave_up) {                        // copies under way land before the block leaves (with a limit again)
+      for (int i = max(0, c - 2); i < c; ++i)
+        for (unsigned n = 0; n < tc::WAIT_LIMIT && !tc::mbar_try(&full[i & 1], (i >> 1) & 1); ++n) {}
+      if (lane == 0 && a.timeouts) atomicAdd(a.timeouts, 1);
+    }
+    return;
+  }
+  const int group = warp / KS, ks = warp - group * KS;
+  if (group >= groups) return;
+  const int g = lane >> 2, c2 = (lane & 3) * 2;
+  const int j0 = ((int)blockIdx.x * G + group) * 16, i0 = ks * (DKT / KS);
+  const int n_all = a.cu_q[p.row + 1] - p.t0;
+  float* S = a.state + (size_t)a.slots[p.row] * a.state_stride + (size_t)h * a.dk * a.dv;
+  // S turned over: the tile's rows are columns j0 .. of S, its columns rows i0 .. of S. An accumulator's registers are then the first
+  // operand's of the next product, and S and U never leave the registers.
+  float s[NTS][4];
+  bool bad = false;                                        // something of S that this thread holds is not finite
+#pragma unroll
+  for (int m = 0; m < NTS; ++m)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + m * 8 + c2 + (e & 1), j = j0 + g + 8 * (e >> 1);
+      s[m][e] = (i < a.dk && j < a.dv) ? S[(size_t)i * a.dv + j] : 0.f;
+      bad |= !finite(s[m][e]);
+    }
+  // rows of V' (or v), a chunk ahead
+  float u_next[4][4];
+  auto fetch_u = [&](int c) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = c * CH + n * 8 + c2 + (e & 1);
+        u_next[n][e] = t < n_all ? u_rows[((size_t)(p.t0 + t) * a.H + h) * a.dvp + j0 + g + 8 * (e >> 1)] : 0.f;
+      }
+  };
+  fetch_u(0);
+  for (int c = 0; c < p.n_chunks; ++c) {
+    wait(&full[c & 1], (c >> 1) & 1);
+    __syncwarp();
+    const bf16* A1 = reinterpret_cast<const bf16*>(raw + (c & 1) * L::BYTES);
+    const bf16 *Kp = A1 + L::K_OFF, *Pp = A1 + L::P_OFF;
+    const float* cc = reinterpret_cast<const float*>(A1 + L::C_OFF);
+    const int n_tok = min(CH, n_all - c * CH);
+    bool slow = reinterpret_cast<const int*>(cc + 2 * DKT)[0] != 0;
+    if (KS == 1) slow |= __any_sync(0xffffffffu, bad) != 0;
+    // [W; Q'] S of this warp's rows of S
+    float x[TILES][4];
+    auto first_slow = [&]() {
+      float ls[NTS * 4];
+#pragma unroll
+      for (int m = 0; m < NTS * 4; ++m) ls[m] = s[m >> 2][m & 3];
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) x[n][0] = x[n][1] = x[n][2] = x[n][3] = 0.f;
+#pragma unroll 1
+      for (int i = 0; i < NTS * 8; ++i) {
+        const int r = (i >> 3) * 4 + (i & 1), src = (lane & ~3) | ((i & 7) >> 1);
+        const float lo = __shfl_sync(0xffffffffu, ls[r], src), hi = __shfl_sync(0xffffffffu, ls[r + 2], src);
+#pragma unroll
+        for (int n = 0; n < TILES; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float w = joined(A1 + (n * 8 + c2 + e) * AP + i0 + i, ROWS * AP);
+            x[n][e] = fmaf(w, lo, x[n][e]);
+            x[n][2 + e] = fmaf(w, hi, x[n][2 + e]);
+          }
+      }
+    };
+    if (!slow) {
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) x[n][0] = x[n][1] = x[n][2] = x[n][3] = 0.f;
+      const bf16* right = A1 + ((lane >> 4) * 8 + (lane & 7)) * AP + i0 + ((lane >> 3) & 1) * 8;
+#pragma unroll
+      for (int k = 0; k < NTS / 2; ++k) {
+        uint32_t sa[3][4];
+        parts_of(sa, s[2 * k], s[2 * k + 1]);
+#pragma unroll
+        for (int n4 = 0; n4 < TILES; n4 += 4) {
+          uint32_t b[2][3][4];
+          float t[4][4] = {};
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) ldsm4(b[u][i], right + i * ROWS * AP + (n4 * 8 + u * 16) * AP + k * 16);
+#pragma unroll
+          for (int i = 0; i < 6; ++i)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) mma(t[n], sa[LEFT[i]], b[n >> 1][RIGHT[i]][(n & 1) * 2], b[n >> 1][RIGHT[i]][(n & 1) * 2 + 1]);
+#pragma unroll
+          for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[n4 + n][e] += t[n][e];
+        }
+      }
+    } else {
+      first_slow();
+    }
+    float o[OT][4];
+    if constexpr (KS > 1) {
+      // the group's warps add their sums up, all of them W S, each its own tokens of Q' S
+      float4* xch = reinterpret_cast<float4*>(raw + W::XCH_OFF) + (size_t)((c & 1) * W::WARPS + group * KS) * TILES * 32 + lane;
+      auto leave = [&]() {
+#pragma unroll
+        for (int n = 0; n < TILES; ++n) xch[(ks * TILES + n) * 32] = make_float4(x[n][0], x[n][1], x[n][2], x[n][3]);
+      };
+      leave();
+      if (group_any(1 + group, 32 * KS, bad)) {            // (all of the group) S is not finite: once more, without parts
+        if (!slow) first_slow();
+        slow = true;
+        leave();
+        group_sync(1 + group, 32 * KS);
+      }
+      auto sum = [&](float (&y)[4], int n) {
+        float4 v[KS];
+#pragma unroll
+        for (int w = 0; w < KS; ++w) v[w] = xch[(w * TILES + n) * 32];
+        y[0] = v[0].x; y[1] = v[0].y; y[2] = v[0].z; y[3] = v[0].w;
+#pragma unroll
+        for (int w = 1; w < KS; ++w) { y[0] += v[w].x; y[1] += v[w].y; y[2] += v[w].z; y[3] += v[w].w; }
+      };
+      if (DELTA) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) sum(x[n], n);
+      }
+#pragma unroll
+      for (int n = 0; n < OT; ++n) sum(o[n], TILES - 4 + ks * OT + n);
+    } else {
+#pragma unroll
+      for (int n = 0; n < OT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = x[TILES - 4 + n][e];
+    }
+    float u[4][4];
+    bool bad_u = false;
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        u[n][e] = u_next[n][e];
+        if (DELTA) u[n][e] = n * 8 + c2 + (e & 1) < n_tok ? u[n][e] - x[n][e] : 0.f;
+        bad_u |= !finite(u[n][e]);
+      }
+    fetch_u(c + 1);
+    slow |= __any_sync(0xffffffffu, bad_u) != 0;           // (the warps of a group hold the same U)
+    uint32_t ua[2][3][4];
+    float lu[16];
+    if (!slow) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) parts_of(ua[k], u[2 * k], u[2 * k + 1]);
+    } else {
+#pragma unroll
+      for (int n = 0; n < 16; ++n) lu[n] = u[n >> 2][n & 3];
+    }
+    bad = false;
+    auto step = [&](int m, const float (&add)[4]) {        // the next S
+      const float2 dc = *reinterpret_cast<const float2*>(cc + i0 + m * 8 + c2), lo = *reinterpret_cast<const float2*>(cc + DKT + i0 + m * 8 + c2);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        s[m][e] = fmaf((e & 1) ? dc.y : dc.x, s[m][e], fmaf((e & 1) ? lo.y : lo.x, s[m][e], add[e]));
+        bad |= !finite(s[m][e]);
+      }
+    };
+    if (!slow) {
+      const bf16* right = Kp + (((lane >> 3) & 1) * 8 + (lane & 7)) * AP + i0 + (lane >> 4) * 8;
+#pragma unroll
+      for (int m = 0; m < NTS; m += 2) {
+        uint32_t b[2][3][4];
+        float t[2][2][4] = {};
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < 3; ++i) ldsm4_t(b[k][i], right + i * CH * AP + k * 16 * AP + m * 8);
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int n = 0; n < 2; ++n) mma(t[k][n], ua[k][LEFT[i]], b[k][RIGHT[i]][n * 2], b[k][RIGHT[i]][n * 2 + 1]);
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          float add[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) add[e] = t[0][n][e] + t[1][n][e];
+          step(m + n, add);
+        }
+      }
+      // O += P U: token n's eight rows of P, zeros after the diagonal (so tokens 0 .. 15 need the first 16 terms only)
+#pragma unroll
+      for (int n = 0; n < OT; ++n) {
+        const int tile = ks * OT + n;
+        uint32_t b[3][4];                                  // the 32 terms of eight tokens
+#pragma unroll
+        for (int i = 0; i < 3; ++i) ldsm4(b[i], Pp + i * CH * PP + (tile * 8 + (lane & 7)) * PP + (lane >> 3) * 8);
+        float t[2][4] = {};
+#pragma unroll
+        for (int i = 0; i < 6; ++i)
+#pragma unroll
+          for (int k = 0; k < 2; ++k) mma(t[k], ua[k][LEFT[i]], b[RIGHT[i]][k * 2], b[RIGHT[i]][k * 2 + 1]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] += t[0][e] + t[1][e];
+      }
+    } else {
+      float add[NTS][4] = {};
+#pragma unroll 1
+      for (int t = 0; t < CH; ++t) {
+        const int r = (t >> 3) * 4 + (t & 1), src = (lane & ~3) | ((t & 7) >> 1);
+        const float lo = __shfl_sync(0xffffffffu, lu[r], src), hi = __shfl_sync(0xffffffffu, lu[r + 2], src);
+#pragma unroll
+        for (int m = 0; m < NTS; ++m)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float k = joined(Kp + t * AP + i0 + m * 8 + c2 + e, CH * AP);
+            add[m][e] = fmaf(k, lo, add[m][e]);
+            add[m][2 + e] = fmaf(k, hi, add[m][2 + e]);
+          }
+#pragma unroll
+        for (int n = 0; n < OT; ++n)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int to = (ks * OT + n) * 8 + c2 + e;
+            if (t > to) continue;                          // (a later token's infinity must not reach back)
+            const float q = joined(Pp + to * PP + t, CH * PP);
+            o[n][e] = fmaf(q, lo, o[n][e]);
+            o[n][2 + e] = fmaf(q, hi, o[n][2 + e]);
+          }
+      }
+#pragma unroll
+      for (int m = 0; m < NTS; ++m) step(m, add[m]);
+    }
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(&empty[c & 1]);         // the chunk's matrices have been read
+#pragma unroll
+    for (int n = 0; n < OT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = (ks * OT + n) * 8 + c2 + (e & 1), j = j0 + g + 8 * (e >> 1);
+        if (t < n_tok && j < a.dv) a.out[(size_t)(p.t0 + c * CH + t) * a.out_stride + (size_t)h * a.dv + j] = o[n][e];
+      }
+  }
+#pragma unroll
+  for (int m = 0; m < NTS; ++m)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = i0 + m * 8 + c2 + (e & 1), j = j0 + g + 8 * (e >> 1);
+      if (i < a.dk && j < a.dv) S[(size_t)i * a.dv + j] = s[m][e];
+    }
+}
+
+template <int DKT, bool DELTA, int KS, int G>
+int launch_wide(const SbChunkedWalk& a, const float* u_rows, cudaStream_t stream) {
+  typedef Wide<DKT, DELTA, KS, G> W;
+  auto k = chunk_wide_kernel<DKT, DELTA, KS, G>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, W::BYTES);
+  k<<<dim3((a.dv + 16 * G - 1) / (16 * G), a.H, a.n_list), W::THREADS, W::BYTES, stream>>>(a, u_rows);
+  SB_LAUNCH_CHECK();
+  return 0;
+}
+
 template <int DKT, bool VEC, int MODE>
 int launch(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
   constexpr bool DELTA = MODE == MODE_DELTA;
@@ -755,10 +1099,29 @@ int launch(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
     k<<<grid, THREADS, head_smem<DKT>(), stream>>>(a, u_rows);
   }
   SB_LAUNCH_CHECK();
+  const float* u = DELTA ? u_rows : a.vf;
+  // Which walk: rounds of blocks the GPU needs times how long a step of 32 tokens takes with it (hundredths of a microsecond), the cheapest. Both
+  // sides measured, 16 heads, us (16 columns a block | 32 | 64): states of 128 x 128 with the delta rule, one request of 2,048 tokens 121 | 168,
+  // four of 512 112 | 82, sixteen of 180 179 | 126; a decay alone, one of 2,048 101 | 137 | 219, two of 1,024 103 | 73 | 112, eight of 256 101 | 79 | 67; of
+  // 64 x 64 with the delta rule, two of 512 27 | 33, four 53 | 36; a decay alone (two blocks an SM, which slow one another down), four of
+  // 512 33 | 42, eight of 256 34 | 29, sixteen 63 | 58.
+  const long long pairs = (long long)a.H * a.n_list, cols = (a.dv + 15) / 16, sms = sm_count();
+  auto cost = [&](int groups, int alone, int two) {
+    const long long blocks = pairs * ((cols + groups - 1) / groups), at_once = two > 0 && blocks > sms ? 2 * sms : sms;
+    return (blocks + at_once - 1) / at_once * (at_once > sms ? two : alone);
+  };
+  constexpr bool BIG = DKT == 128;
+  const long long one = DELTA ? cost(1, BIG ? 187 : 154, 0) : cost(1, BIG ? 157 : 133, BIG ? 0 : 205);
+  const long long two = DELTA ? cost(2, BIG ? 260 : 196, 0) : cost(2, BIG ? 213 : 246, BIG ? 0 : 340);
+  if constexpr (BIG && !DELTA) {
+    const long long four = cost(4, 342, 0);
+    if (four < one && four < two) return launch_wide<DKT, DELTA, 2, 4>(a, u, stream);
+  }
+  if (two < one) return launch_wide<DKT, DELTA, 2, 2>(a, u, stream);
   auto k = chunk_walk_kernel<DKT, DELTA>;
   constexpr int smem = Walk<DKT, DELTA>::BYTES;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  k<<<dim3((a.dv + VC - 1) / VC, a.H, a.n_list), THREADS, smem, stream>>>(a, DELTA ? u_rows : a.vf);
+  k<<<dim3((a.dv + VC - 1) / VC, a.H, a.n_list), THREADS, smem, stream>>>(a, u);
   SB_LAUNCH_CHECK();
   return 0;
 }

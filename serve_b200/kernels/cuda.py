@@ -155,20 +155,20 @@ def short_on_mma(longest: int, group: int, keys: int, decoding_too: bool, pairs:
 # the launches, the chain of the longest request, and the work of all (token, head) pairs on a full GPU. By what decays (one factor for the
 # state; one, with the delta rule; one a row, with the delta rule; one a row) and the rows of the state up to which a line holds. The
 # chunked kernels make a chain of tokens / 32 steps, but their work is that of 64 or 128 rows by 32 tokens whatever the state, so small
-# states of many requests are the walk's. Fitted to 1,400 steps of one to 16 requests of 97 to 1,024 tokens, 8 to 32 heads, 16 to 128 rows
-# by 16 to 256 columns; the choice they give is at most 1.2 times slower than the better one (0.4 % on average). Chunked | walked in us:
-#   1 request of 1,024 tokens, 16 heads of 64 x 64: 64 | 224, 85 | 312, 108 | 314, 71 | 241; of 128 x 128: 82 | 260, 112 | 366, 153 | 371, 107 | 278
-#   16 of 256, 16 heads of 64 x 64: 136 | 126, 232 | 194, 355 | 201, 166 | 170; of 128 x 128: 321 | 390, 423 | 647, 568 | 666, 390 | 547
-#   16 of 256, 16 heads of 16 x 64: 134 | 83, 231 | 104, 344 | 106, 140 | 84; 4 of 128, 32 heads of 64 x 64: 42 | 44, 67 | 65, 91 | 67, 49 | 54
+# states of many requests are the walk's. Fitted to 1,900 steps of one to 16 requests of 97 to 1,024 tokens, 8 to 32 heads, 16 to 128 rows
+# by 16 to 256 columns; the choice they give is at most 1.26 times slower than the better one (0.4 % on average). Chunked | walked in us:
+#   1 request of 1,024 tokens, 16 heads of 64 x 64: 64 | 224, 85 | 312, 109 | 314, 71 | 241; of 128 x 128: 82 | 260, 112 | 366, 154 | 371, 106 | 278
+#   16 of 256, 16 heads of 64 x 64: 133 | 127, 208 | 194, 332 | 201, 163 | 170; of 128 x 128: 246 | 390, 354 | 647, 501 | 665, 317 | 548
+#   16 of 256, 16 heads of 16 x 64: 132 | 83, 208 | 105, 322 | 105, 138 | 84; 4 of 128, 32 heads of 64 x 64: 39 | 44, 57 | 65, 81 | 67, 46 | 54
 RECURRENCE_COST = {
-    "one": ((16, (11, 3.7, 1.4, 95), (6, 16.6, 0.1, 89)), (32, (12, 3.4, 1.5, 89), (6, 17.5, 0.9, 34)),
-            (64, (11, 3.3, 1.6, 95), (6, 20.5, 2.0, 40)), (128, (13, 2.5, 1.6, 290), (7, 22.6, 2.4, 290))),
-    "one, delta": ((16, (16, 3.4, 2.6, 177), (6, 19.3, 0.1, 127)), (32, (15, 4.1, 2.8, 154), (6, 22.0, 1.2, 58)),
-                   (64, (15, 3.7, 3.1, 142), (7, 29.0, 3.1, 62)), (128, (18, 3.8, 1.6, 441), (8, 33.8, 3.8, 465))),
-    "rows, delta": ((16, (20, 3.3, 2.6, 300), (6, 19.4, 0.1, 126)), (32, (20, 4.6, 2.9, 274), (6, 22.0, 1.2, 58)),
-                    (64, (19, 0.0, 3.4, 278), (7, 29.1, 3.2, 69)), (128, (23, 3.9, 1.4, 684), (9, 34.0, 4.1, 460))),
-    "rows": ((16, (12, 3.8, 1.5, 105), (6, 16.9, 0.2, 90)), (32, (13, 3.6, 1.4, 119), (6, 17.4, 0.9, 47)),
-             (64, (12, 2.9, 1.6, 139), (6, 22.3, 2.7, 57)), (128, (14, 2.4, 1.5, 415), (7, 24.1, 3.9, 318))),
+    "one": ((16, (12, 3.5, 1.1, 105), (6, 16.6, 0.1, 89)), (32, (13, 2.9, 1.4, 73), (6, 17.5, 0.9, 34)),
+            (64, (12, 3.4, 1.4, 106), (6, 20.5, 2.0, 40)), (128, (14, 3.2, 1.1, 242), (7, 22.6, 2.4, 290))),
+    "one, delta": ((16, (16, 4.5, 1.3, 185), (6, 19.3, 0.1, 127)), (32, (16, 4.1, 1.8, 161), (6, 22.0, 1.2, 58)),
+                   (64, (16, 3.8, 2.0, 172), (7, 29.0, 3.1, 62)), (128, (18, 4.9, 3.0, 205), (8, 33.8, 3.8, 465))),
+    "rows, delta": ((16, (21, 5.1, 1.0, 297), (6, 19.4, 0.1, 126)), (32, (20, 5.5, 1.6, 268), (6, 22.0, 1.2, 58)),
+                    (64, (21, 4.1, 2.4, 290), (7, 29.1, 3.2, 69)), (128, (23, 3.9, 1.4, 684), (9, 34.0, 4.1, 460))),
+    "rows": ((16, (12, 3.5, 1.3, 112), (6, 16.9, 0.2, 90)), (32, (13, 3.2, 1.4, 105), (6, 17.4, 0.9, 47)),
+             (64, (12, 2.9, 1.6, 139), (6, 22.3, 2.7, 57)), (128, (16, 3.6, 1.4, 315), (7, 24.1, 3.9, 318))),
 }
 
 

@@ -139,6 +139,29 @@ def test_a_later_token_does_not_reach_back(K, mode):
     assert not torch.isfinite(out[71, 5]) and torch.isnan(out[81, :dv]).all()
 
 
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("dk,dv", [(128, 128), (100, 72), (64, 128), (40, 136)])
+def test_many_pairs(K, mode, dk, dv):
+    """So many (request, head) pairs that blocks walk 32 or 64 columns of S: ragged requests, part of a block's columns beyond the last, an
+    infinity in the values of one request."""
+    heads = 26
+    c = _case(mode, [161, 33, 100, 64, 40, 5], heads, 13, dk, dv, torch.bfloat16, seed=dk + dv)
+    want, want_pool = _exact(c)
+    out, pool = _run(K, c)
+    bound = 8 * dk ** 0.5 * 2.0 ** -24 + 2e-7              # as above
+    assert _error(out, want) < bound and _error(pool, want_pool) < bound
+    untouched = [i for i in range(pool.shape[0]) if i not in c.ctx.slots.tolist()]
+    assert torch.equal(pool[untouched], c.pool[untouched])
+    c.args[2][70, dv + 5] = float("inf")                   # the second head of the first request, inside its third chunk
+    later, _ = _run(K, c)
+    K.check_errors()
+    hit = torch.zeros_like(out, dtype=torch.bool)
+    hit[70:161, dv: 2 * dv] = True
+    assert _error(later[~hit], out[~hit].double()) < 2 * bound and not torch.isfinite(later[70, dv + 5])
+    others = [dv + j for j in range(dv) if j != 5]         # the columns of S never meet
+    assert _error(later[:161][:, others], out[:161][:, others].double()) < 2 * bound
+
+
 @pytest.mark.parametrize("mode", ["delta", "wkv", "gla"])
 def test_decays_that_vanish(K, mode):
     """Rates so high that products of decays underflow inside a chunk, beside rows that hardly decay."""
