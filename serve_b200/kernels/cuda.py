@@ -1052,6 +1052,7 @@ class CudaKernels:
             path = build.build_library(**job)
             self.paths[job["name"]] = path
             self._moe = ctypes.CDLL(path)
+            self._moe.sb_moe_layer_bytes.restype = ctypes.c_longlong
         return self._moe
 
     def _prep_lib(self):
@@ -1238,49 +1239,22 @@ class CudaKernels:
                      or (outputs > e and w_down.shape[1] != h.shape[1])):
             raise KernelError("routed_experts: identity experts, a choice bias and a shared expert come with weights on the outputs")
         ff, n, k = w_down.shape[2], w_down.shape[1], h.shape[1]
-        pairs = t * top
-        dev = h.device
-        tensor_rows = lib.sb_moe_tensor_rows(_DT[h.dtype], k, ff, h.stride(0), t)      # 0: not on the tensor cores
-        tile_rows = tensor_rows or lib.sb_moe_tile_rows()
-        max_tiles = pairs // tile_rows + min(e, pairs)
-        ints = torch.empty(2 * pairs + e + 1 + 2 * max_tiles + 1, dtype=torch.int32, device=dev)
-        idx, order = ints[:pairs], ints[pairs: 2 * pairs]
-        offsets = ints[2 * pairs: 2 * pairs + e + 1]
-        tiles = ints[2 * pairs + e + 1: 2 * pairs + e + 1 + 2 * max_tiles]
-        n_tiles = ints[-1:]
-        wts = torch.empty(pairs, dtype=torch.float32, device=dev)
-        s = self._s()
-        self.launches += 4
-        if more:
-            _check(lib.sb_moe_route_bias(_p(logits), logits.stride(0), outputs, top, {"sigmoid": 0, "softmax": 1}[score],
-                                         1 if renormalise else 0, ctypes.c_float(renormalise_eps), _p(choice_bias), t, _p(idx), _p(wts),
-                                         ctypes.c_float(weight_scale), int(groups), int(keep_groups), s), "expert choice")
-        else:
-            _check(lib.sb_moe_route(_p(logits), e, top, {"sigmoid": 0, "softmax": 1}[score], 1 if renormalise else 0, t, _p(idx), _p(wts), s),
-                   "expert choice")
-        _check(lib.sb_moe_sort(_p(idx), pairs, e, tile_rows, _p(offsets), _p(order), _p(tiles), _p(n_tiles), s), "grouping by expert")
-        act = torch.empty((pairs, ff), dtype=h.dtype, device=dev)
-        kind = {"swiglu": 0, "clamped_swish": 1}[activation]
-        parts = out if (top == 1 and not more) else torch.empty((pairs, n), dtype=torch.float32, device=dev)
-        if tensor_rows:
-            xg = self._grouped_room(parts, out, pairs, k, h)
-            self.launches += 1
-            _check(lib.sb_moe_gate_up_tensor(_p(h), h.stride(0), t, _p(xg), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top,
-                                             pairs, e, k, ff, 1, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha),
-                                             _p(act), tile_rows, self._wait_flag(), s), "experts, gate and up")
-        else:
-            _check(lib.sb_moe_gate_up(_p(h), h.stride(0), _p(w_gate_up), _p(order), _p(offsets), _p(tiles), _p(n_tiles), _p(wts), top, pairs,
-                                      e, k, ff, 1 if scale_input else 0, kind, ctypes.c_float(limit), ctypes.c_float(alpha), _p(act),
-                                      _DT[h.dtype], s), "experts, gate and up")
-        self._experts_down(lib, act, w_down, order, offsets, tiles, n_tiles, wts, 0 if scale_input else 1, parts, tensor_rows, s)
-        if more:
-            self.launches += 1
-            gate = logits[:, outputs:] if shared_gated else None
-            _check(lib.sb_moe_combine_more(_p(parts), _p(idx), _p(wts), e, _p(h), h.stride(0), _p(shared), _p(gate), logits.stride(0), top, t, n,
-                                           _p(out), _DT[out.dtype], s), "sum over a token's experts, identity and shared expert")
-        elif top > 1:
-            self.launches += 1
-            _check(lib.sb_moe_combine(_p(parts), top, t, n, _p(out), _DT[out.dtype], s), "sum over a token's experts")
+        x_stride, dtype = h.stride(0), _DT[h.dtype]
+        key = ("moe", t, top, e, k, ff, n, x_stride, dtype, more)
+        room = self._routes.get(key)
+        if room is None:
+            room = self._routes[key] = lib.sb_moe_layer_bytes(t, top, e, k, ff, n, x_stride, dtype, 1 if more else 0)
+        work = torch.empty(room, dtype=torch.uint8, device=h.device)
+        gate = logits.data_ptr() + 4 * outputs if shared_gated else 0
+        rc = lib.sb_moe_layer(
+            _p(logits), logits.stride(0), outputs if more else e, top, {"sigmoid": 0, "softmax": 1}[score], 1 if renormalise else 0,
+            ctypes.c_float(renormalise_eps), _p(choice_bias), ctypes.c_float(weight_scale), int(groups), int(keep_groups), 1 if more else 0,
+            _p(h), x_stride, t, _p(w_gate_up), _p(w_down), e, k, ff, n, 1 if scale_input else 0, {"swiglu": 0, "clamped_swish": 1}[activation],
+            ctypes.c_float(limit), ctypes.c_float(alpha), _p(shared), ctypes.c_void_p(gate), logits.stride(0), _p(work), _p(out), dtype,
+            _DT[out.dtype], self._wait_flag(), self._s())
+        if rc < 0:
+            _check(rc if rc > -1000 else -1000 - rc, "experts")
+        self.launches += rc
 
     @staticmethod
     def _grouped_room(parts, out, pairs: int, k: int, h):
