@@ -106,10 +106,6 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
   constexpr int MOST = MODE == GATED ? 64 * ACCS : 128 * ACCS;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int stage_bytes = ACCS * W_BYTES + x_rows_of(a.cap) * BK * 2;
-  const int runs = a.n_tiles[0];
-  const int which = ACCS == 2 || a.cap > 16 ? 0 : pick_unit(MODE, runs, a.cols, gridDim.x);
-  const int unit_cols = ACCS == 2 ? MOST : unit_outputs(MODE, which);
-  const int col_blocks = (a.cols + unit_cols - 1) / unit_cols;
   const int k_blocks = (a.K + BK - 1) / BK;
   const int acc_cols = a.cap <= 128 ? 128 : 256;             // tensor-memory columns of an accumulator
   const int bufs = ACCS * acc_cols <= 256 ? 2 : 1;           // sets of accumulators
@@ -125,7 +121,6 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
       tc::mbar_init(&acc_empty[b], EPI_WARPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w[which]) : "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(TMEM_COLS) : "memory");
@@ -134,7 +129,14 @@ __global__ void __launch_bounds__(THREADS) experts_kernel(const __grid_constant_
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
+  // set up; the runs, the tokens and the right to overwrite the output come with the end of the kernel before
+  pdl_launch_dependents();
+  pdl_wait();
   const uint32_t tmem_base = tmem_base_s;
+  const int runs = a.n_tiles[0];
+  const int which = ACCS == 2 || a.cap > 16 ? 0 : pick_unit(MODE, runs, a.cols, gridDim.x);
+  const int unit_cols = ACCS == 2 ? MOST : unit_outputs(MODE, which);
+  const int col_blocks = (a.cols + unit_cols - 1) / unit_cols;
   const int units = runs * col_blocks;
   bool failed = false;
 
@@ -316,8 +318,7 @@ int launch(const void* w, const void* x, int n_pairs, int E, Args a, cudaStream_
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const long long units = (long long)(n_pairs / a.cap + (E < n_pairs ? E : n_pairs)) * ((a.cols + 15) / 16);      // (at most)
   const int sms = sm_count();
-  k<<<(unsigned)(units < sms ? units : sms), THREADS, smem, stream>>>(maps, a);
-  SB_LAUNCH_CHECK();
+  SB_PDL_CHECK(launch_pdl(k, dim3((unsigned)(units < sms ? units : sms)), dim3(THREADS), smem, stream, maps, a));
   return 0;
 }
 
@@ -347,6 +348,8 @@ int launch_accs(const void* w, const void* x, int n_pairs, int E, const Args& a,
 __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ x, int x_stride, const int* __restrict__ order, const int* __restrict__ offsets,
                                                          int E, int top, int K, bf16* __restrict__ xg) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i >= offsets[E]) return;                      // (choices that name no expert have no place)
   const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)(order[i] / top) * x_stride);
   uint4* dst = reinterpret_cast<uint4*>(xg + (size_t)i * K);
@@ -380,8 +383,7 @@ SB_EXPORT int sb_moe_gate_up_tensor(const void* x, int x_stride, int n_tokens, v
   if (n_pairs <= 0) return 0;
   if (tile_rows != sb_moe_tensor_rows(SB_DTYPE_BF16, K, ff, x_stride, n_tokens) || tile_rows == 0 || top <= 0 || E <= 0) return SB_ERR_SHAPE;
   if (!aligned16(x) || !aligned16(w) || !aligned16(xg) || !error) return SB_ERR_ALIGN;
-  moe_gather_kernel<<<(n_pairs + 7) / 8, 256, 0, stream>>>((const bf16*)x, x_stride, order, offsets, E, top, K, (bf16*)xg);
-  SB_LAUNCH_CHECK();
+  SB_PDL_CHECK(launch_pdl(moe_gather_kernel, dim3((n_pairs + 7) / 8), dim3(256), 0, stream, (const bf16*)x, x_stride, order, offsets, E, top, K, (bf16*)xg));
   Args a = {};
   a.order = order; a.offsets = offsets; a.tiles = tiles; a.n_tiles = n_tiles; a.wts = wts; a.out = act; a.error = error;
   a.K = K; a.cols = ff; a.w_rows = gated ? 2 * ff : ff; a.cap = tile_rows; a.scale = gated && scale_input;

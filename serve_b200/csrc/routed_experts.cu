@@ -32,6 +32,8 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
                                                         int n_tokens, int* __restrict__ idx, float* __restrict__ wts) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_launch_dependents();
+  pdl_wait();
   if (t >= n_tokens) return;
   const float* z = logits + (size_t)t * E;
   float mine[ROUTE_PER_LANE];
@@ -99,6 +101,8 @@ __global__ void __launch_bounds__(128) moe_route_bias_kernel(const float* __rest
                                                              int n_groups, int keep_groups) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+  pdl_launch_dependents();
+  pdl_wait();
   if (t >= n_tokens) return;
   const float* z = logits + (size_t)t * stride;
   float score[PER_LANE], pick[PER_LANE];
@@ -203,6 +207,8 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
   __shared__ int2 warp_sums[32];
   const int tid = threadIdx.x, n_threads = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const bool keeps = n_pairs <= SORT_KEEP * n_threads;
+  pdl_launch_dependents();
+  pdl_wait();
   int mine[SORT_KEEP], rank[SORT_KEEP];
 #pragma unroll
   for (int u = 0; u < SORT_KEEP; ++u) mine[u] = tid + u * n_threads < n_pairs && keeps ? idx[tid + u * n_threads] : -1;
@@ -471,6 +477,8 @@ __global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __re
                                                                const float* __restrict__ gate, int gate_stride, int top, int N, int blocks_a_row,
                                                                T* __restrict__ out) {
   const int t = blockIdx.x / blocks_a_row, c = ((blockIdx.x - t * blocks_a_row) * 256 + threadIdx.x) * 4;
+  pdl_launch_dependents();
+  pdl_wait();
   if (c >= N) return;
   float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
   float g = 1.f;
@@ -529,13 +537,14 @@ __global__ void __launch_bounds__(256) moe_combine_more_kernel(const float* __re
 // false: the rows are not made of whole, aligned pieces of four
 template <typename T>
 bool combine_rows(const float* parts, const int* idx, const float* wts, int E_real, const void* x, int x_stride, const void* shared, const float* gate,
-                  int gate_stride, int top, int n_tokens, int N, void* out, cudaStream_t stream) {
+                  int gate_stride, int top, int n_tokens, int N, void* out, cudaStream_t stream, cudaError_t& e) {
   const int per_row = (N / 4 + 255) / 256;
+  e = cudaSuccess;
   if (N % 4 || x_stride % 4 || !aligned16(parts) || !aligned16(x) || !aligned16(out) || (shared && !aligned16(shared)) ||
       (long long)n_tokens * per_row > 2147483647LL)
     return false;
-  moe_combine_rows_kernel<T><<<n_tokens * per_row, 256, 0, stream>>>(parts, idx, wts, E_real, (const T*)x, x_stride, (const T*)shared, gate, gate_stride, top,
-                                                                  N, per_row, (T*)out);
+  e = launch_pdl(moe_combine_rows_kernel<T>, dim3(n_tokens * per_row), dim3(256), 0, stream, parts, idx, wts, E_real, (const T*)x, x_stride, (const T*)shared,
+                 gate, gate_stride, top, N, per_row, (T*)out);
   return true;
 }
 
@@ -550,8 +559,7 @@ SB_EXPORT int sb_moe_route(const float* logits, int E, int top, int score_kind, 
                            cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
   if (E <= 0 || top <= 0 || top > E || top > ROUTE_MAX_TOP || E > 32 * ROUTE_PER_LANE) return SB_ERR_LIMIT;
-  moe_route_kernel<<<(n_tokens + 3) / 4, 128, 0, stream>>>(logits, E, top, score_kind, renorm, n_tokens, idx, wts);
-  SB_LAUNCH_CHECK();
+  SB_PDL_CHECK(launch_pdl(moe_route_kernel, dim3((n_tokens + 3) / 4), dim3(128), 0, stream, logits, E, top, score_kind, renorm, n_tokens, idx, wts));
   return 0;
 }
 
@@ -562,8 +570,8 @@ SB_EXPORT int sb_moe_sort(const int* idx, int n_pairs, int E, int tile_rows, int
   if (E <= 0 || E > 4096 || tile_rows <= 0) return SB_ERR_LIMIT;
   // few pairs: few warps, whose barriers are short
   const int want = n_pairs / 4 > E ? n_pairs / 4 : E, threads = want >= 1024 ? 1024 : want <= 128 ? 128 : (want + 31) / 32 * 32;
-  moe_sort_kernel<<<1, threads, (size_t)(2 * E) * sizeof(int), stream>>>(idx, n_pairs, E, tile_rows, offsets, order, tiles, n_tiles);
-  SB_LAUNCH_CHECK();
+  SB_PDL_CHECK(launch_pdl(moe_sort_kernel, dim3(1), dim3(threads), (size_t)(2 * E) * sizeof(int), stream, idx, n_pairs, E, tile_rows, offsets, order, tiles,
+                          n_tiles));
   return 0;
 }
 
@@ -650,13 +658,15 @@ SB_EXPORT int sb_moe_combine(const float* parts, int top, int n_tokens, int N, v
   if (n_tokens <= 0) return 0;
   if (dtype != SB_DTYPE_F32 && dtype != SB_DTYPE_BF16) return SB_ERR_DTYPE;
   const bool f32 = dtype == SB_DTYPE_F32;
-  if (!(f32 ? combine_rows<float>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream)
-            : combine_rows<__nv_bfloat16>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream))) {
+  cudaError_t e;
+  if (!(f32 ? combine_rows<float>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream, e)
+            : combine_rows<__nv_bfloat16>(parts, nullptr, nullptr, 0, out, 4, nullptr, nullptr, 0, top, n_tokens, N, out, stream, e))) {
     const long long total = (long long)n_tokens * N, want = (total + 255) / 256;
     const int blocks = (int)(want < sm_count() * 8 ? want : sm_count() * 8);
     if (f32) moe_combine_kernel<float><<<blocks, 256, 0, stream>>>(parts, top, N, total, (float*)out);
     else moe_combine_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(parts, top, N, total, (__nv_bfloat16*)out);
   }
+  if (e != cudaSuccess) return (int)e;
   SB_LAUNCH_CHECK();
   return 0;
 }
@@ -674,9 +684,8 @@ SB_EXPORT int sb_moe_route_bias(const float* logits, int stride, int E, int top,
   if (n_groups <= 0 || E % n_groups || keep_groups <= 0 || keep_groups > n_groups || (long long)top > (long long)keep_groups * (E / n_groups)) return SB_ERR_SHAPE;
   auto k = E <= 64 ? moe_route_bias_kernel<2> : E <= 128 ? moe_route_bias_kernel<4> : E <= 256 ? moe_route_bias_kernel<8>
                                                                                                : moe_route_bias_kernel<ROUTE_PER_LANE>;
-  k<<<(n_tokens + 3) / 4, 128, 0, stream>>>(logits, stride, E, top, score_kind, renorm, sum_eps, bias, n_tokens, idx, wts, weight_scale,
-                                            n_groups, keep_groups);
-  SB_LAUNCH_CHECK();
+  SB_PDL_CHECK(launch_pdl(k, dim3((n_tokens + 3) / 4), dim3(128), 0, stream, logits, stride, E, top, score_kind, renorm, sum_eps, bias, n_tokens, idx, wts,
+                          weight_scale, n_groups, keep_groups));
   return 0;
 }
 
@@ -690,8 +699,9 @@ SB_EXPORT int sb_moe_combine_more(const float* parts, const int* idx, const floa
   if (!parts || !idx || !wts || !x || top <= 0 || x_stride < N) return SB_ERR_SHAPE;
   if (dtype != SB_DTYPE_F32 && dtype != SB_DTYPE_BF16) return SB_ERR_DTYPE;
   const bool f32 = dtype == SB_DTYPE_F32;
-  if (!(f32 ? combine_rows<float>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream)
-            : combine_rows<__nv_bfloat16>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream))) {
+  cudaError_t e;
+  if (!(f32 ? combine_rows<float>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream, e)
+            : combine_rows<__nv_bfloat16>(parts, idx, wts, E_real, x, x_stride, shared, gate, gate_stride, top, n_tokens, N, out, stream, e))) {
     const long long total = (long long)n_tokens * N, want = (total + 255) / 256;
     const int blocks = (int)(want < sm_count() * 16 ? want : sm_count() * 16);
     if (f32)
@@ -701,6 +711,7 @@ SB_EXPORT int sb_moe_combine_more(const float* parts, const int* idx, const floa
       moe_combine_more_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(parts, idx, wts, E_real, (const __nv_bfloat16*)x, x_stride,
                                                                          (const __nv_bfloat16*)shared, gate, gate_stride, top, N, total, (__nv_bfloat16*)out);
   }
+  if (e != cudaSuccess) return (int)e;
   SB_LAUNCH_CHECK();
   return 0;
 }
