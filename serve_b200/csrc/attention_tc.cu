@@ -23,7 +23,8 @@
 // 32-bit additions in place of descriptors made anew, 50.7 | 38.3 | 49.6; waits that cost one instruction when there is nothing to wait for,
 // 48.4 | 36.0 | 49.8; copies issued like the products, a tile's page looked up a tile ahead, 47.2 | 35.2 | 48.8 (a loop of a few
 // more branches there: 52.3 | 39.0 | 49.2); two CTAs an SM at head_dim 128 (TIGHT) 28.9. No difference: two sets of softmax warps for even
-// and odd tiles, longer hardware waits, a single polling lane, packed arithmetic.
+// and odd tiles, longer hardware waits, a single polling lane, packed arithmetic, a tile's page looked up still earlier. Slower: tiles of 128
+// keys (one buffer each of scores and probabilities: eight prompts of 256 26 us against 24; 55.7 over rows of 256).
 // Two CTAs share an SM at head_dim 64 (96 KB of shared memory, 256 columns of tensor memory each).
 // At head_dim 128 an operand row is two 128-byte swizzle atoms: queries, keys and values arrive as two TMA boxes of 64
 // elements each, the first product walks over both atoms of Q and K, the second product covers the 128 output
@@ -731,8 +732,9 @@ SB_EXPORT int sb_attention_tc_opts(const void* qkv, int q_stride, int n_tokens, 
   const bool fine = SHARED || window > 0 || kc == vc;
   if (D == 128) {
     // Two CTAs an SM fill one another's gaps, but each has fewer buffers and takes longer by itself: they pay once an SM would walk a
-    // second CTA after its first. 24/8 heads, whole causal prompts, one | two an SM: 600 tokens (120 CTAs) 22.8 | 26.7 us, 1,024 (200) 37.2 | 39.1,
-    // 2,048 (392) 68.7 | 56.2, 4,096 (784) 170 | 126; 16/4 heads, window 1,024: 1,024 tokens (128) 18.9 | 20.8, 2,048 (256) 35.2 | 28.9.
+    // second CTA after its first. 24/8 heads, whole causal prompts, one | two an SM: 600 tokens (120 CTAs) 22.1 | 25.3 us, 1,024 (200) 30.6 | 32.5,
+    // 1,300 (248) 39.3 | 41.3, 1,500 (288) 42.5 | 41.9, 2,048 (392) 62.2 | 49.9, 4,096 (784) 168 | 125; 16/4 heads, window 1,024: 1,024 tokens (128)
+    // 19.2 | 20.9, 1,600 (200) 24.6 | 26.6, 1,800 (228) 30.4 | 27.7, 2,048 (256) 35.5 | 28.9.
     if ((long long)Hkv * m_tiles * n_rows * 2 > 3LL * sm_count())
       return fine ? launch(std::true_type{}, std::true_type{}) : launch(std::false_type{}, std::true_type{});
   }

@@ -164,7 +164,7 @@ RECURRENCE_COST = {
     "one": ((16, (12, 3.5, 1.1, 105), (6, 16.6, 0.1, 89)), (32, (13, 2.9, 1.4, 73), (6, 17.5, 0.9, 34)),
             (64, (12, 3.4, 1.4, 106), (6, 20.5, 2.0, 40)), (128, (14, 3.2, 1.1, 242), (7, 22.6, 2.4, 290))),
     "one, delta": ((16, (16, 4.5, 1.3, 185), (6, 19.3, 0.1, 127)), (32, (16, 4.1, 1.8, 161), (6, 22.0, 1.2, 58)),
-                   (64, (16, 3.8, 2.0, 172), (7, 29.0, 3.1, 62)), (128, (18, 4.9, 3.0, 205), (8, 33.8, 3.8, 465))),
+                   (64, (16, 3.8, 2.1, 172), (7, 29.0, 3.1, 62)), (128, (18, 4.9, 3.0, 205), (8, 33.8, 3.8, 465))),
     "rows, delta": ((16, (21, 5.1, 1.0, 297), (6, 19.4, 0.1, 126)), (32, (20, 5.5, 1.6, 268), (6, 22.0, 1.2, 58)),
                     (64, (21, 4.1, 2.4, 290), (7, 29.1, 3.2, 69)), (128, (23, 3.9, 1.4, 684), (9, 34.0, 4.1, 460))),
     "rows": ((16, (12, 3.5, 1.3, 112), (6, 16.9, 0.2, 90)), (32, (13, 3.2, 1.4, 105), (6, 17.4, 0.9, 47)),
