@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         clear(max(0, p.keep - kt), min(BN, window_lo - kt));
         clear(hi - kt, BN);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
+        __syncwarp();
       }
       tc_wait_st();
       tc_fence_before();
