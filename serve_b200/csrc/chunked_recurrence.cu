@@ -27,6 +27,7 @@
 // in its matrices, in S or in U takes plain multiply-adds instead, over the same operands.
 #include "chunked_recurrence.h"
 
+#include "bounded_wait.h"
 #include "common.cuh"
 #include "tcgen05_ops.cuh"
 
@@ -777,6 +778,14 @@ __device__ __forceinline__ void parts_of(uint32_t (&p)[3][4], const float (&x)[4
     for (int r = 0; r < 4; ++r) p[i][r] = q[r][i];
 }
 
+// what its waits leave (bounded_wait.h)
+struct Notes {
+  int *gave_up, *timeouts;
+  __device__ __forceinline__ bool raise() { return atomicExch(gave_up, 1) == 0; }
+  __device__ __forceinline__ bool raised() const { return *(volatile int*)gave_up != 0; }
+  __device__ __forceinline__ void count() { if (timeouts) atomicAdd(timeouts, 1); }
+};
+
 // grid (ceil(dv / (16 G)), head, list entry).
 template <int DKT, bool DELTA, int KS, int G>
 __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbChunkedWalk a, const float* __restrict__ u_rows) {
@@ -804,33 +813,24 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // A wait that runs out is noted; after it no wait lasts, every warp stays in step to the end, and what is computed is not valid.
+  Notes notes{&gave_up, a.timeouts};
   auto wait = [&](uint64_t* bar, unsigned parity) {
-    if (tc::mbar_try(bar, parity)) return;
-    for (unsigned i = 0; i < tc::WAIT_LIMIT; ++i) {
-      if (tc::mbar_try(bar, parity)) return;
-      if ((i & 1023u) == 1023u && *(volatile int*)&gave_up) return;
-    }
-    *(volatile int*)&gave_up = 1;
+    if (!tc::mbar_try(bar, parity)) wait_in_step([&] { return tc::mbar_try(bar, parity); }, notes, tc::WAIT_LIMIT);
   };
 
   if (warp == W::WARPS) {                                  // a chunk's matrices are one piece: one bulk copy
     int c = 0;
     for (; c < p.n_chunks; ++c) {
       wait(&empty[c & 1], ((c >> 1) & 1) ^ 1);
-      if (*(volatile int*)&gave_up) break;
-      __syncwarp();
+      if (__any_sync(0xffffffffu, notes.raised())) break;
       if (tc::elect_one()) {
         tc::mbar_expect_tx(&full[c & 1], L::BYTES);
         bulk_load(raw + (c & 1) * L::BYTES, images + (long long)c * a.H * L::BYTES, L::BYTES, &full[c & 1]);
       }
       __syncwarp();
     }
-    if (*(volatile int*)&gave_up) {                        // copies under way land before the block leaves (with a limit again)
-      for (int i = max(0, c - 2); i < c; ++i)
-        for (unsigned n = 0; n < tc::WAIT_LIMIT && !tc::mbar_try(&full[i & 1], (i >> 1) & 1); ++n) {}
-      if (lane == 0 && a.timeouts) atomicAdd(a.timeouts, 1);
-    }
+    for (int i = max(0, c - 2); i < c; ++i)                // copies under way land before the block may leave
+      wait_landed([&] { return tc::mbar_try(&full[i & 1], (i >> 1) & 1); }, notes, tc::WAIT_LIMIT);
     return;
   }
   const int group = warp / KS, ks = warp - group * KS;
@@ -1065,6 +1065,7 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
         if (t < n_tok && j < a.dv) a.out[(size_t)(p.t0 + c * CH + t) * a.out_stride + (size_t)h * a.dv + j] = o[n][e];
       }
   }
+  if (notes.raised()) return;                              // (the state stays the one before this step)
 #pragma unroll
   for (int m = 0; m < NTS; ++m)
 #pragma unroll
