@@ -148,8 +148,10 @@ __device__ __forceinline__ bool elect_one() {
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 32 columns: thread i of the warp gets lane (base + i), 32 consecutive columns. No wait: several loads
-// may be in flight; tc_wait_ld() before the registers are read.
+// may be in flight; tc_wait_ld() before the registers are read. Loads and stores, and the wait for stores, are the warp's instructions:
+// lanes that a branch before them has parted meet first.
 __device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
+  __syncwarp();
   uint32_t* u = reinterpret_cast<uint32_t*>(r);
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -162,6 +164,7 @@ __device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
       : "r"(taddr));
 }
 __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
+  __syncwarp();
   const uint32_t* u = reinterpret_cast<const uint32_t*>(r);
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -174,13 +177,18 @@ __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
       : "memory");
 }
 __device__ __forceinline__ void tc_store16(uint32_t taddr, const uint32_t (&u)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]),
         "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
       : "memory");
 }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_wait_st() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool any_lane(int yes) { return __any_sync(0xffffffffu, yes) != 0; }
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -209,10 +217,15 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// Barriers of the 64 threads that share 32 rows (two warps); the second tells all of them whether any of them says yes.
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+// Barriers of the 64 threads that share 32 rows (two warps, each of which comes as a whole); the second tells all of them whether any of
+// them says yes.
+__device__ __forceinline__ void pair_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
 __device__ __forceinline__ bool pair_any(int id, bool yes) {
   uint32_t any;
+  __syncwarp();
   asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 q, %2, 0;\n bar.red.or.pred p, %1, 64, q;\n selp.u32 %0, 1, 0, p;\n}\n"
                : "=r"(any) : "r"(id), "r"(yes ? 1u : 0u) : "memory");
   return any != 0;
@@ -391,8 +404,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         }
       };
       mbar_wait(&k_empty[s], phase, gave_up);
-      if (*reinterpret_cast<volatile int*>(gave_up)) break;        // (no copy into a stage that may still be read)
-      __syncwarp();
+      if (any_lane(*reinterpret_cast<volatile int*>(gave_up))) break;        // (no copy into a stage that may still be read)
       if (elect_one()) {
         mbar_expect_tx(&k_full[s], SPLIT || SHARED ? bytes : 2 * bytes);
         load(Ks + (size_t)s * KV_BYTES, &map_k, &k_full[s]);
@@ -401,8 +413,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       __syncwarp();
       if (SPLIT) {
         mbar_wait(&v_empty[s], phase, gave_up);
-        if (*reinterpret_cast<volatile int*>(gave_up)) { ++j; break; }
-        __syncwarp();
+        if (any_lane(*reinterpret_cast<volatile int*>(gave_up))) { ++j; break; }
         if (elect_one()) {
           mbar_expect_tx(&v_full[s], bytes);
           load(Vs + (size_t)s * KV_BYTES, &map_v, &v_full[s]);
@@ -601,7 +612,6 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         clear(max(0, p.keep - kt), min(BN, window_lo - kt));
         clear(hi - kt, BN);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
-        __syncwarp();
       }
       tc_wait_st();
       tc_fence_before();

@@ -63,7 +63,9 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // 32 lanes x 32 columns of 32-bit accumulator: thread i of the warp gets lane (base lane + i), 32 consecutive columns
+// (the warp's instruction: lanes that a branch before it has parted meet first)
 __device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
     for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
       const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * OUT_COLS;
       const int buf = local & 1;
-      if (!mbar_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
+      if (!tc::warp_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
@@ -483,7 +485,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
     for (int tile = pair; tile < total_tiles && !failed; tile += num_pairs, ++local) {
       const int m0 = (tile % m_tiles) * 256 + (int)rank * 128, n0 = (tile / m_tiles) * OUT_COLS;
       const int buf = local & 1;
-      if (!mbar_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
+      if (!tc::warp_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
       tc_fence_after();
       const int row = m0 + q * 32 + lane;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);

@@ -78,6 +78,7 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
+  __syncwarp();                      // the warp's instruction: lanes that a branch before it has parted meet first
   uint32_t* u = reinterpret_cast<uint32_t*>(r);
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(64 + EPI * 32, 2) scores_tc_kernel(const __gri
     const float two_in = p.cap_in * (2.f * LOG2E), cap_log2 = p.cap * LOG2E, scale_log2 = p.scale * LOG2E;
     const int tiles_pitch = p.pitch / BN;
     for (int j = set; j < n_steps && !failed; j += 2) {
-      if (!mbar_wait(&s_full[set], (j >> 1) & 1)) { failed = true; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[set], (j >> 1) & 1))) { failed = true; break; }
       tc_fence_after();
       const int kt = kt_first + j * BN;
       float v[BN];
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
     for (int j = 0; j < n_tiles && !failed; j = (j == 0 && n_tiles > 1) ? n_tiles - 1 : n_tiles) {
       int head, tail;
       if (!edges(j, head, tail)) continue;
-      if (!mbar_wait(&landed, clears & 1)) { failed = true; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(&landed, clears & 1))) { failed = true; break; }
       ++clears;
       unsigned char* vt = Vs + (size_t)(j % NS_V) * V_BYTES;
       const int gone = head + (BN - tail);
@@ -444,7 +445,7 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&cleared);
     }
-    if (!failed && !mbar_wait(&o_full, 0)) failed = true;
+    if (!failed && !__all_sync(0xffffffffu, mbar_wait(&o_full, 0))) failed = true;
     tc_fence_after();
     if (!failed) {
       const int q = warp & 3, row = q * 32 + lane, tok = row / p.per;

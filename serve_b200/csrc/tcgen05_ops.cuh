@@ -62,8 +62,9 @@ __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t desc_a, uint64_t d
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 // 32 lanes x 32 columns of 32-bit accumulator: thread i of the warp gets lane (base lane + i), 32 consecutive columns
-// (wait_loads() before the registers are used)
+// (wait_loads() before the registers are used). The instruction is the warp's: lanes that a branch before it has parted meet first.
 __device__ __forceinline__ void load32(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
