@@ -344,9 +344,9 @@ int launch_accs(const void* w, const void* x, int n_pairs, int E, const Args& a,
   return pick_accs(MODE, a, n_pairs, E) == 2 ? launch<MODE, 2, O>(w, x, n_pairs, E, a, stream) : launch<MODE, 1, O>(w, x, n_pairs, E, a, stream);
 }
 
-// xg[i] = x[order[i] / top]: a warp a row, 16 bytes a lane and step.
-__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict__ x, int x_stride, const int* __restrict__ order, const int* __restrict__ offsets,
-                                                         int E, int top, int K, bf16* __restrict__ xg) {
+// xg[i] = x[order[i] / top]: a warp a row, 16 bytes a lane and step. Like the kernels of routed_experts.cu it may begin before the kernel
+// that writes what it reads has ended, so it reads with plain loads (no __ldg, no __restrict__: both say that nobody writes meanwhile).
+__global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* x, int x_stride, const int* order, const int* offsets, int E, int top, int K, bf16* xg) {
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   pdl_launch_dependents();
   pdl_wait();
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const bf16* __restrict_
     uint4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (c + 32 * u < K / 8) v[u] = __ldg(src + c + 32 * u);
+      if (c + 32 * u < K / 8) v[u] = src[c + 32 * u];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (c + 32 * u < K / 8) dst[c + 32 * u] = v[u];

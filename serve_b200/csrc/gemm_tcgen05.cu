@@ -140,11 +140,12 @@ __device__ __forceinline__ void rope_store_chunk(const RopeEpilogue& ra, const u
   uint32_t packed[16];
   const bool turns = head < ra.H + ra.Hkv;
   // the table is [pair][row]: the 32 rows of a warp read 256 consecutive bytes per pair. All loads first, so that
-  // their latencies overlap (a warp alone on its scheduler has nothing else to run meanwhile).
+  // their latencies overlap (a warp alone on its scheduler has nothing else to run meanwhile). Plain loads: the angles are made in the
+  // same step, by a kernel that need not have ended when this one begins.
   float2 a[16];
   const float2* angles = ra.cos_sin + (size_t)(d0 >> 1) * M + row;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) a[i] = (turns && d0 + 2 * i < ra.rot) ? __ldg(angles + (size_t)i * M) : make_float2(1.f, 0.f);
+  for (int i = 0; i < 16; ++i) a[i] = (turns && d0 + 2 * i < ra.rot) ? angles[(size_t)i * M] : make_float2(1.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     const float x = to_float(__float2bfloat16_rn(__uint_as_float(v[2 * i]))), y = to_float(__float2bfloat16_rn(__uint_as_float(v[2 * i + 1])));

@@ -24,12 +24,15 @@ __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + expf(-
 
 constexpr int ROUTE_MAX_TOP = 16;
 
+// The kernels of a layer may begin before the ones before them have ended (common.cuh), so what those write is read with plain loads behind
+// pdl_wait(): no __ldg and no __restrict__, which say that nobody writes the data while the kernel runs.
+//
 // A warp per token: lane l holds the logits of experts l, l + 32, ... (at most ROUTE_PER_LANE of them); the best of
 // what is left is found `top` times by a shuffle tree over (logit, index), lower index first on equal logits.
 constexpr int ROUTE_PER_LANE = 32;      // so at most 1024 experts
 
-__global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict__ logits, int E, int top, int score_kind, int renorm,
-                                                        int n_tokens, int* __restrict__ idx, float* __restrict__ wts) {
+__global__ void __launch_bounds__(128) moe_route_kernel(const float* logits, int E, int top, int score_kind, int renorm,
+                                                        int n_tokens, int* idx, float* wts) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
   pdl_launch_dependents();
@@ -95,9 +98,9 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float* __restrict_
 // a group is as good as its best output, and only outputs of the keep_groups best groups can be chosen. E counts every output the router scores; an index at or beyond
 // the number of real experts means "the token itself" to the kernels after this one.
 template <int PER_LANE>
-__global__ void __launch_bounds__(128) moe_route_bias_kernel(const float* __restrict__ logits, int stride, int E, int top, int score_kind,
-                                                             int renorm, float sum_eps, const float* __restrict__ bias, int n_tokens,
-                                                             int* __restrict__ idx, float* __restrict__ wts, float weight_scale,
+__global__ void __launch_bounds__(128) moe_route_bias_kernel(const float* logits, int stride, int E, int top, int score_kind,
+                                                             int renorm, float sum_eps, const float* bias, int n_tokens,
+                                                             int* idx, float* wts, float weight_scale,
                                                              int n_groups, int keep_groups) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -198,9 +201,9 @@ constexpr int TM = 32;            // rows of a tile of the plain-arithmetic prod
 // for up to SORT_KEEP pairs a thread (more: counted a second time); the experts' first places and tiles from one scan over the block.
 // Bound by latency: 8,192 pairs of 64 experts 13.7 -> 8.9 us, 32 pairs 6.4 -> 2.7 (one thread had walked the experts).
 constexpr int SORT_KEEP = 8;
-__global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, int n_pairs, int E, int tile_rows,
-                                                        int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ tiles,
-                                                        int* __restrict__ n_tiles) {
+__global__ void __launch_bounds__(1024) moe_sort_kernel(const int* idx, int n_pairs, int E, int tile_rows,
+                                                        int* offsets, int* order, int* tiles,
+                                                        int* n_tiles) {
   extern __shared__ int sh[];
   int* count = sh;            // [E]
   int* start = sh + E;        // [E]
@@ -472,10 +475,10 @@ template <> __device__ __forceinline__ void moe_store4<__nv_bfloat16>(__nv_bfloa
 // are experts is known before the loads. idx null: all are. 2,048 tokens, 4 choices, width 2,048 (84 MB): 19.5 -> 18.8 us;
 // 8 tokens 3.7 -> 3.3.
 template <typename T>
-__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* __restrict__ parts, const int* __restrict__ idx, const float* __restrict__ wts,
-                                                               int E_real, const T* __restrict__ x, int x_stride, const T* __restrict__ shared,
-                                                               const float* __restrict__ gate, int gate_stride, int top, int N, int blocks_a_row,
-                                                               T* __restrict__ out) {
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const float* parts, const int* idx, const float* wts,
+                                                               int E_real, const T* x, int x_stride, const T* shared,
+                                                               const float* gate, int gate_stride, int top, int N, int blocks_a_row,
+                                                               T* out) {
   const int t = blockIdx.x / blocks_a_row, c = ((blockIdx.x - t * blocks_a_row) * 256 + threadIdx.x) * 4;
   pdl_launch_dependents();
   pdl_wait();

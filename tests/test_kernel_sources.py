@@ -35,3 +35,20 @@ def test_lanes_that_load_from_tensor_memory_give_up_together(name):
         block = text[:m.start()]
         single = max(block.rfind("if (lane == 0) {"), block.rfind("if (lane == 0 && "))
         assert single > block.rfind("} else {\n"), text[m.start():m.end()]
+
+
+# file -> what is read with __ldg: weights, which no kernel of a step writes
+WEIGHTS = {"projection_ops.cu": ["reinterpret_cast<const uint32_t*>(wr"], "decode_stack.cu": ["reinterpret_cast<const float4*>(weight)", "reinterpret_cast<const uint2*>(weight)"],
+           "talking_attention.cu": ["a)", "a +", "ta +", "tb +"]}
+EARLY_EXPERTS = ["moe_route_kernel", "moe_route_bias_kernel", "moe_sort_kernel", "moe_combine_rows_kernel", "moe_gather_kernel"]
+
+
+def test_only_weights_are_read_as_unchanging():
+    """A kernel that begins before its predecessors have ended must not tell the compiler that nobody writes what they leave it."""
+    for name, text in SOURCES.items():
+        for m in re.finditer(r"__ldg\(([^\n]*)", text):
+            assert any(m.group(1).startswith(w) for w in WEIGHTS.get(name, [])), (name, m.group(0))
+    for kernel in EARLY_EXPERTS:
+        text = SOURCES["experts_tcgen05.cu" if kernel == "moe_gather_kernel" else "routed_experts.cu"]
+        signature = re.search(r"__global__ void [^;{]*?\b" + kernel + r"\([^{]*\{", text).group(0)
+        assert "__restrict__" not in signature and "pdl_wait();" in text[text.index(signature):][:1200], kernel
