@@ -464,9 +464,14 @@ constexpr int DKW = D <= 64 ? 32 : 16;                    // keys per warp per s
 constexpr int DNT = DKW / 8;                              // score n-tiles per step
 constexpr int DSTAGES = 2;                                 // steps in flight per warp
 // The grid's splits are sized for the longest sequence a captured step may meet. A request whose keys one block walks in this many
-// steps of its warps is not split: the partial rows, their ticket and their merge (2 to 3 us at the end of the launch) cost more than
-// the steps that another block would save. Llama-3.2-1B decoding steps, 1 | 2 | 3 | 4 steps of 256 keys: 8 requests after 270 tokens
-// 692 | 655 | 655 | 655 us, after 510 713 | 703 | 698 | 698, after 710 742 | 742 | 707 | 707, after 1,010 the same with all.
+// steps of its warps is not split: the partial rows, their ticket and their merge (2 to 5 us at the end of the launch) cost more than
+// the steps that another block would save. A captured layer, always split | one block up to 2 | 3 | 4 steps, us: head size 64 (steps of 256 keys),
+// eight requests of 200 keys 14.35 | 11.4 | 11.4 | 11.4, of 380 14.7 | 12.7 | 12.6 | 12.7, of 700 16.6 | 16.5 | 14.7 | 14.7, of 900 16.9 | 16.8 | 16.9 | 15.7, one of 700
+// 13.75 | 13.6 | 12.8 | 12.7; head size 128 (steps of 128 keys), one of 200 22.5 | 20.1 | 19.6 | 20.1, of 380 22.6 | 22.6 | 20.7 | 21.7, eight of 380 26.7 | 26.7 | 24.5 | 24.7, of
+// 500 27.2 | 27.3 | 27.1 | 26.2; behind a window of 256, eight of 1,500 23.4 | 23.3 | 21.3 | 21.4; rows of 256, eight of 130 28.0 | 24.2 | 24.2 | 24.2, of 380 28.8 | 28.7 |
+// 27.55 | 27.5, one of 500 27.6 | 27.1 | 27.8 | 28.7 (steps of one variant are 0.1 to 0.7 apart from run to run there). Three is nowhere behind two, four
+// is behind three for one request. The blocks left over wait and leave: that they let the next kernel begin first changed nothing (one request
+// of head size 128 at 3,072 columns took 1 us longer: 17.7 against 18.8).
 constexpr int SOLO = 3;
 constexpr bool DQ_IN_REGS = D <= 128;                     // query fragments live in registers
 constexpr int DCOPIES = DKW * CHUNKS / 32;                // 16-byte copies per lane per sub-tile and tensor
@@ -611,7 +616,13 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
     }
   }
   pdl_launch_dependents();
-  __syncthreads();                                              // table entries are in shared memory
+  // The first keys are asked for right behind the queries where those live in registers: one trip to memory in place of two, one after the
+  // other (attention layers in a captured step, before | behind: one request of 1,000 keys, head size 64 13.82 | 13.41 us, eight of 2,000
+  // 19.17 | 18.87, head size 128 34.2 | 34.05). Longer rows read their queries from shared memory in every step and their first keys are few:
+  // there the keys follow the queries (latent layer, rows of 256, eight requests of 2,048 tokens, window 1,024: 32.87 | 33.05 us, of 500 28.3 | 28.55,
+  // one of 100 22.5 | 22.7; without the rule of SOLO, too, 32.76 | 32.87).
+  constexpr bool KEYS_AT_ONCE = DQ_IN_REGS;
+  if (KEYS_AT_ONCE) __syncthreads();                            // table entries are in shared memory
   pdl_wait();                                                   // queries and this step's keys/values come from earlier kernels
   for (int idx = tid; idx < 16 * CHUNKS; idx += NTHR) {
     const int row = idx / CHUNKS, ch = idx - row * CHUNKS;
@@ -621,6 +632,10 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
   }
   cp_async_commit();
 
+  if (!KEYS_AT_ONCE) {
+    cp_async_wait<0>();
+    __syncthreads();                                            // queries and table entries are in shared memory
+  }
   const bool same_page = (p.ps % DKW) == 0;
   const int n_sub = n_keep + (hi - k_first + DKW - 1) / DKW;    // sub-tiles of the split
   // sub-tile n of the split: its first key, and the range of keys it fetches
@@ -636,10 +651,10 @@ __global__ void __launch_bounds__(NWARPS * 32) attention_deep_kernel(const Param
                                           same_page, myKV + s * stage_elems, myKV + s * stage_elems + DKW * LDS, lane);
     cp_async_commit();
   }
-  // The first keys were asked for right behind the queries: one trip to memory in place of two, one after the other
-  // (batch 1 after 1,000 tokens 650 -> 643 us a Llama-3.2-1B decoding step).
-  cp_async_wait<DSTAGES - 1>();
-  __syncthreads();                                              // queries are in shared memory
+  if (KEYS_AT_ONCE) {
+    cp_async_wait<DSTAGES - 1>();
+    __syncthreads();                                            // queries are in shared memory
+  }
   uint32_t qf[DQ_IN_REGS ? D / 16 : 1][4];
   if (DQ_IN_REGS) {
 #pragma unroll
