@@ -390,10 +390,14 @@ __global__ void __launch_bounds__(256) add_bias_kernel(float* __restrict__ x, co
 }
 
 // The same in pieces of four, a block a part of the columns of ADD_ROWS rows: the bias is read once for them, their loads go out together and no
-// index is divided. 2,048 x 2,048 (34 MB, most of it in the L2 cache behind the product) 9.4 -> 4.8 us.
-constexpr int ADD_ROWS = 8;
-__global__ void __launch_bounds__(256) add_bias_rows_kernel(float* __restrict__ x, const float* __restrict__ bias, int n_rows, int cols) {
-  const int c = (blockIdx.x * 256 + threadIdx.x) * 4, r0 = blockIdx.y * ADD_ROWS;
+// index is divided. 2,048 x 2,048 (34 MB, most of it in the L2 cache behind the product) 8.4 -> 4.0 us. (One, four and eight rows a block: 4.25,
+// 3.9 and 4.3, but 1.5, 1.75 and 2.1 us against 1.55 with two for 32 to 256 rows: a thread's rows come one behind the other.)
+constexpr int ADD_ROWS = 2;
+// Up to this many numbers the element-wise kernel's many short threads are the faster way: eight rows of 2,048 1.4 | 1.55 us (in a windowed layer's
+// decoding step 27.9 | 28.1 us), 64 rows 1.5 | 1.6, 128 rows 1.9 | 1.6; of 1,024 128 rows 1.55 | 1.55; of 4,096 32 rows 1.55 | 1.6, 64 rows 1.9 | 1.6.
+constexpr size_t ADD_FEW = 1 << 17;
+__global__ void __launch_bounds__(256) add_bias_rows_kernel(float* __restrict__ x, const float* __restrict__ bias, int n_rows, int cols, int blocks_a_row) {
+  const int at_row = blockIdx.x / blocks_a_row, c = ((blockIdx.x - at_row * blocks_a_row) * 256 + threadIdx.x) * 4, r0 = at_row * ADD_ROWS;
   if (c >= cols) return;
   const float4 b = *reinterpret_cast<const float4*>(bias + c);
   float4* at = reinterpret_cast<float4*>(x + (size_t)r0 * cols + c);
@@ -804,13 +808,14 @@ SB_EXPORT int sb_activation(const void* x, const float* bias, void* out, int n_r
 
 SB_EXPORT int sb_add_bias(float* x, const float* bias, int n_rows, int cols, cudaStream_t stream) {
   if (n_rows <= 0 || cols <= 0) return 0;
-  const int row_blocks = (n_rows + ADD_ROWS - 1) / ADD_ROWS;
-  if (cols % 4 == 0 && aligned16(x) && aligned16(bias) && row_blocks <= 65535) {
-    add_bias_rows_kernel<<<dim3((cols + 1023) / 1024, row_blocks), 256, 0, stream>>>(x, bias, n_rows, cols);
+  const size_t total = (size_t)n_rows * cols, want = (total + 255) / 256;
+  const int per_row = (int)(((long long)cols + 1023) / 1024);
+  const long long pieces = ((long long)n_rows + ADD_ROWS - 1) / ADD_ROWS * per_row;
+  if (total > ADD_FEW && cols % 4 == 0 && aligned16(x) && aligned16(bias) && pieces <= 2147483647LL) {
+    add_bias_rows_kernel<<<(unsigned)pieces, 256, 0, stream>>>(x, bias, n_rows, cols, per_row);
     SB_LAUNCH_CHECK();
     return 0;
   }
-  const size_t total = (size_t)n_rows * cols, want = (total + 255) / 256;
   const int blocks = (int)(want < (size_t)sm_count() * 16 ? want : (size_t)sm_count() * 16);
   add_bias_kernel<<<blocks, 256, 0, stream>>>(x, bias, total, cols);
   SB_LAUNCH_CHECK();

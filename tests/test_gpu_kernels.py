@@ -766,3 +766,17 @@ def test_attention_tensor_memory_path_rescales_when_the_maximum_runs_ahead(K, d)
     K.check_errors()
     E.attention(s["qkv"], s["kc"], s["vc"], s["bt"], s["cu"], s["kv"], s["row"], s["pos"], heads, kv_heads, d, page, 1.0, 0, ref, s["shape"])
     torch.testing.assert_close(out.float(), ref.float(), atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("rows,cols,offset", [(1, 1, 0), (3, 4, 0), (8, 2048, 0), (128, 1024, 0), (129, 1024, 0), (33, 4100, 0), (130, 1028, 0), (67, 2050, 0),
+                                              (200, 1024, 1), (2, 70000, 0), (2049, 2048, 0)])
+def test_bias_on_float_sums(K, rows, cols, offset):
+    """Around the number of sums from which rows are taken in pairs and pieces of four: odd rows, columns beyond a block's 1,024, columns that are
+    no pieces of four, sums that begin off a 16-byte boundary. One float addition each, so the same numbers as torch's."""
+    g = torch.Generator(device=DEV).manual_seed(rows + cols)
+    room = torch.randn(rows * cols + 8 + offset, generator=g, device=DEV)
+    bias = torch.randn(cols, generator=g, device=DEV)
+    x = room[4 + offset: 4 + offset + rows * cols].view(rows, cols)
+    want, around = x + bias, (room[: 4 + offset].clone(), room[4 + offset + rows * cols:].clone())
+    K.add_bias(x, bias)
+    assert torch.equal(x, want) and torch.equal(room[: 4 + offset], around[0]) and torch.equal(room[4 + offset + rows * cols:], around[1])
