@@ -149,9 +149,9 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 32 columns: thread i of the warp gets lane (base + i), 32 consecutive columns. No wait: several loads
 // may be in flight; tc_wait_ld() before the registers are read. Loads and stores, and the wait for stores, are the warp's instructions:
-// lanes that a branch before them has parted meet first.
-__device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
-  __syncwarp();
+// lanes that a branch before them has parted meet first, or (_met) have just met and taken no branch of their own since (meeting
+// again for each of them cost a windowed prompt 1.2 %).
+__device__ __forceinline__ void tc_load32_met(uint32_t taddr, float* r) {
   uint32_t* u = reinterpret_cast<uint32_t*>(r);
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -162,6 +162,10 @@ __device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
         "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]),
         "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
       : "r"(taddr));
+}
+__device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
+  __syncwarp();
+  tc_load32_met(taddr, r);
 }
 __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
   __syncwarp();
@@ -176,18 +180,14 @@ __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
         "r"(u[30]), "r"(u[31])
       : "memory");
 }
-__device__ __forceinline__ void tc_store16(uint32_t taddr, const uint32_t (&u)[16]) {
-  __syncwarp();
+__device__ __forceinline__ void tc_store16_met(uint32_t taddr, const uint32_t (&u)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]), "r"(u[8]), "r"(u[9]),
         "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15])
       : "memory");
 }
-__device__ __forceinline__ void tc_wait_st() {
-  __syncwarp();
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
+__device__ __forceinline__ void tc_wait_st_met() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ bool any_lane(int yes) { return __any_sync(0xffffffffu, yes) != 0; }
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         tc_fence_after();
         // the tile reaches beyond what the first row may see, or behind the last row's window
         const bool masked = kt + BN - 1 > first_pos || (p.window > 0 && kt <= p0 + tok_last - p.window);
-        tc_load32(lane_addr + (uint32_t)(b * BN + half * 32), sv);
+        tc_load32_met(lane_addr + (uint32_t)(b * BN + half * 32), sv);
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
             for (int i = 0; i < 32; ++i) ov[i] *= f;
             tc_store32(o_addr, ov);
           }
-          tc_wait_st();
+          tc_wait_st_met();
           l_run *= f;
         }
         if (moves) m_ref = m_tile;                       // (with no reference yet, accumulator and sum are still zero)
@@ -593,8 +593,8 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
           pk[i] = pack_bf16(e0, e1);
         }
       }
-      tc_store16(p_addr, pk);
-      if (FINE) tc_store16(p_addr + P_COLS, rest);
+      tc_store16_met(p_addr, pk);
+      if (FINE) tc_store16_met(p_addr + P_COLS, rest);
       l_run += sum.x + sum.y;
       // values that no row of the tile sees must not meet a zero probability as NaN (0 times infinity): the rows of this stage beyond
       // hi (never written, or another tile's leftovers) are cleared, and so are those behind every row's window
@@ -612,8 +612,9 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         clear(max(0, p.keep - kt), min(BN, window_lo - kt));
         clear(hi - kt, BN);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
+        __syncwarp();
       }
-      tc_wait_st();
+      tc_wait_st_met();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&p_full[j % NP]);

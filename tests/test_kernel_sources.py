@@ -9,22 +9,30 @@ from serve_b200.kernels.build import CSRC
 SOURCES = {f: open(os.path.join(CSRC, f)).read() for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh"))}
 
 
-def _body_before(text, at):
-    """What stands between the opening brace of the function that holds position ``at`` and that position."""
-    start = max(m.end() for m in re.finditer(r"^__device__ __forceinline__ [^;]*?\{", text[:at], re.M | re.S))
-    assert text.find("\n}", start) > at, "an instruction outside a function of its own"
-    return text[start:at]
+def _function(text, at):
+    """(name, what stands between its opening brace and ``at``) of the function that holds position ``at``."""
+    start = max(re.finditer(r"^__device__ __forceinline__ \w+ (\w+)\([^;]*?\{", text[:at], re.M | re.S), key=lambda m: m.end())
+    assert text.find("\n}", start.end()) > at or text.find("}\n", start.end()) > at, "an instruction outside a function of its own"
+    return start.group(1), text[start.end():at]
 
 
 @pytest.mark.parametrize("name", [f for f, s in SOURCES.items() if "tcgen05.ld" in s])
 def test_a_warp_meets_before_its_tensor_memory_instructions(name):
     """tcgen05.ld, .st, the wait for stores and barriers are ``.aligned``: all lanes execute them together. Branches that rows beyond the last
-    and lanes that wait alone take stand before them, so the functions that issue them begin with the warp's meeting."""
+    and lanes that wait alone take stand before them, so the functions that issue them begin with the warp's meeting. Those named _met do
+    not: before their calls no lane has gone its own way since the warp met last."""
     text = SOURCES[name]
     found = list(re.finditer(r'"(\{\\n .reg .pred p, q;\\n setp[^;]*;\\n )?(tcgen05\.(ld|st|wait::st)\.sync\.aligned|bar\.(sync|red))', text))
     assert found
     for m in found:
-        assert "__syncwarp();" in _body_before(text, m.start()), text[m.start():m.end()]
+        name, before = _function(text, m.start())
+        assert "__syncwarp();" in before or name.endswith("_met"), name
+    for m in re.finditer(r"(?<!void )\b\w+_met\(", text):
+        if "__forceinline__" in text[text.rfind("\n", 0, text.rfind("\n", 0, m.start())):m.start()]:
+            continue                                        # (a function that is a meeting and such a call)
+        met = max(text.rfind(s, 0, m.start()) for s in ("__syncwarp();", "pair_any(", " tc_load32(", " tc_store32("))
+        between = text[met + 1:m.start()]
+        assert met > 0 and not re.search(r"mbar_|if \(lane|row_ok|\breturn\b", between), between
 
 
 @pytest.mark.parametrize("name", [f for f, s in SOURCES.items() if "tcgen05.ld" in s])
