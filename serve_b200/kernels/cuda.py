@@ -155,20 +155,22 @@ def short_on_mma(longest: int, group: int, keys: int, decoding_too: bool, pairs:
 # the launches, the chain of the longest request, and the work of all (token, head) pairs on a full GPU. By what decays (one factor for the
 # state; one, with the delta rule; one a row, with the delta rule; one a row) and the rows of the state up to which a line holds. The
 # chunked kernels make a chain of tokens / 32 steps, but their work is that of 64 or 128 rows by 32 tokens whatever the state, so small
-# states of many requests are the walk's. Fitted to 1,900 steps of one to 16 requests of 97 to 1,024 tokens, 8 to 32 heads, 16 to 128 rows
-# by 16 to 256 columns; the choice they give is at most 1.26 times slower than the better one (0.4 % on average). Chunked | walked in us:
-#   1 request of 1,024 tokens, 16 heads of 64 x 64: 64 | 224, 85 | 312, 109 | 314, 71 | 241; of 128 x 128: 82 | 260, 112 | 366, 154 | 371, 106 | 278
-#   16 of 256, 16 heads of 64 x 64: 133 | 127, 208 | 194, 332 | 201, 163 | 170; of 128 x 128: 246 | 390, 354 | 647, 501 | 665, 317 | 548
-#   16 of 256, 16 heads of 16 x 64: 132 | 83, 208 | 105, 322 | 105, 138 | 84; 4 of 128, 32 heads of 64 x 64: 39 | 44, 57 | 65, 81 | 67, 46 | 54
+# states of many requests are the walk's, and so are requests of hardly more than 32 tokens. Fitted to 9,800 steps of one to 16 requests of 33 to
+# 2,048 tokens, alike and ragged, 4 to 32 heads, 16 to 128 rows by 16 to 256 columns. Of 1,400 other steps the choice is the slower one by
+# more than 5 % in 4.7 % of them, by more than 10 % in 2.9 %; 0.7 % on average, 1.29 times at most. Chunked | walked in us (one, one with the
+# delta rule, one a row with the delta rule, one a row):
+#   1 request of 1,024 tokens, 16 heads of 64 x 64: 66 | 226, 80 | 308, 107 | 311, 70 | 248; of 128 x 128: 79 | 257, 106 | 362, 145 | 365, 97 | 281
+#   16 of 256, 16 heads of 64 x 64: 125 | 131, 193 | 181, 325 | 195, 144 | 162; of 128 x 128: 240 | 382, 342 | 634, 484 | 645, 288 | 521
+#   16 of 256, 16 heads of 16 x 64: 121 | 84, 195 | 90, 317 | 104, 128 | 89
 RECURRENCE_COST = {
-    "one": ((16, (12, 3.5, 1.1, 105), (6, 16.6, 0.1, 89)), (32, (13, 2.9, 1.4, 73), (6, 17.5, 0.9, 34)),
-            (64, (12, 3.4, 1.4, 106), (6, 20.5, 2.0, 40)), (128, (14, 3.2, 1.1, 242), (7, 22.6, 2.4, 290))),
-    "one, delta": ((16, (16, 4.5, 1.3, 185), (6, 19.3, 0.1, 127)), (32, (16, 4.1, 1.8, 161), (6, 22.0, 1.2, 58)),
-                   (64, (16, 3.8, 2.1, 172), (7, 29.0, 3.1, 62)), (128, (18, 4.9, 3.0, 205), (8, 33.8, 3.8, 465))),
-    "rows, delta": ((16, (21, 5.1, 1.0, 297), (6, 19.4, 0.1, 126)), (32, (20, 5.5, 1.6, 268), (6, 22.0, 1.2, 58)),
-                    (64, (21, 4.1, 2.4, 290), (7, 29.1, 3.2, 69)), (128, (23, 3.9, 1.4, 684), (9, 34.0, 4.1, 460))),
-    "rows": ((16, (12, 3.5, 1.3, 112), (6, 16.9, 0.2, 90)), (32, (13, 3.2, 1.4, 105), (6, 17.4, 0.9, 47)),
-             (64, (12, 2.9, 1.6, 139), (6, 22.3, 2.7, 57)), (128, (16, 3.6, 1.4, 315), (7, 24.1, 3.9, 318))),
+    "one": ((16, (15, 3.6, 0.8, 92), (6, 16.8, 0.0, 91)), (32, (16, 2.9, 0.9, 71), (7, 17.1, 0.8, 44)),
+            (64, (18, 1.9, 1.2, 71), (8, 20.5, 1.7, 44)), (128, (18, 3.2, 2.3, 115), (7, 24.3, 3.8, 59))),
+    "one, delta": ((16, (17, 5.5, 1.3, 151), (8, 19.2, 0.2, 91)), (32, (19, 3.2, 1.8, 135), (7, 23.4, 1.1, 44)),
+                   (64, (22, 1.4, 2.3, 105), (7, 30.3, 3.0, 49)), (128, (27, 2.5, 3.5, 138), (9, 32.3, 7.0, 47))),
+    "rows, delta": ((16, (26, 5.0, 1.5, 274), (8, 20.2, 0.3, 107)), (32, (26, 4.4, 1.6, 271), (10, 22.0, 1.0, 71)),
+                    (64, (29, 4.7, 2.1, 242), (8, 31.2, 2.8, 122)), (128, (35, 4.1, 3.6, 261), (12, 34.6, 6.5, 67))),
+    "rows": ((16, (17, 3.6, 0.6, 112), (8, 16.9, 0.2, 97)), (32, (17, 2.3, 0.9, 116), (8, 18.2, 0.8, 74)),
+             (64, (20, 2.0, 1.1, 129), (9, 22.4, 2.3, 68)), (128, (24, 2.1, 2.1, 194), (9, 26.8, 5.4, 76))),
 }
 
 
