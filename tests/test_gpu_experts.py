@@ -1,5 +1,6 @@
 """The experts' tensor-core products at the edges of their tiles: runs of 1 to more than 256 tokens an expert, counts that are no
-multiple of 16, 64 or 128, outputs that end inside a unit, k that ends inside a stage, experts without tokens, every epilogue."""
+multiple of 16, 64 or 128, outputs that end inside a unit, k that ends inside a stage, experts without tokens, every epilogue. The widest two:
+long rows of few tokens an expert have two accumulators that fill tensor memory, and blocks that hand them over to a second unit."""
 import pytest
 import torch
 
@@ -41,7 +42,8 @@ def _bound(want, most):
 
 @pytest.mark.parametrize("kind", ["swiglu", "clamped_swish"])
 @pytest.mark.parametrize("tokens,k,ff,n", [(1, 64, 32, 40), (7, 96, 160, 64), (16, 2080, 96, 200), (17, 64, 128, 136), (33, 160, 64, 129), (65, 128, 416, 128),
-                                           (129, 32, 96, 257), (200, 64, 64, 64), (257, 96, 32, 72), (700, 128, 224, 300)])
+                                           (129, 32, 96, 257), (200, 64, 64, 64), (257, 96, 32, 72), (700, 128, 224, 300),
+                                           (200, 3104, 4832, 64), (249, 3136, 4768, 40)])
 def test_expert_products(tokens, k, ff, n, kind):
     from serve_b200.kernels import load_kernels
 
@@ -59,6 +61,44 @@ def test_expert_products(tokens, k, ff, n, kind):
     kernels.check_errors()
     want, most = _reference(x, logits, w_gu, w_down, kind)
     assert ((out.double() - want).abs() <= _bound(want, most)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,k,ff", [(1, 64, 32), (19, 256, 96), (300, 96, 64)])
+@pytest.mark.parametrize("gated,identity", [(True, 0), (False, 2)])
+def test_one_choice_beside_a_shared_expert(tokens, k, ff, gated, identity, dtype):
+    """A single choice a token has no sums of its own to add up, but its output still meets the shared expert's (or is the token itself)."""
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    g = torch.Generator(device="cuda").manual_seed(tokens + ff)
+    draw = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, shared = draw(tokens, k).to(dtype), draw(tokens, k).to(dtype)
+    outputs = E + identity
+    logits = draw(tokens, 8)                                # columns beyond the outputs and the gate are not read
+    w_gu, w_down = (draw(E, 2 * ff, k) / k ** 0.5).to(dtype), (draw(E, k, ff) / ff ** 0.5).to(dtype)
+    bias = draw(outputs) * 0.1
+    out = torch.full((tokens, k), float("nan"), device="cuda", dtype=dtype)
+    kernels.routed_experts(x, logits, w_gu, w_down, 1, out, score="sigmoid", scale_input=False, activation="swiglu", outputs=outputs,
+                           choice_bias=bias, shared=shared, shared_gated=gated)
+    kernels.check_errors()
+    score = torch.sigmoid(logits[:, :outputs].double())
+    idx = (score + bias.double()).argmax(-1)
+    want = shared.double() * (torch.sigmoid(logits[:, outputs].double())[:, None] if gated else 1.0)
+    most = want.abs()
+    for t in range(tokens):
+        e, w = int(idx[t]), score[t, idx[t]]
+        if e >= E:
+            want[t] += w * x[t].double()
+            most[t] += w * x[t].double().abs()
+        else:
+            a = x[t].double() @ w_gu[e, :ff].double().T
+            a = a * torch.sigmoid(a) * (x[t].double() @ w_gu[e, ff:].double().T)
+            want[t] += w * (a @ w_down[e].double().T)
+            most[t] += w * (a.abs() @ w_down[e].double().abs().T)
+    # float: sums of k and ff terms, each off by at most 2^-24 of the absolute terms a step
+    bound = _bound(want, most) if dtype == torch.bfloat16 else (k + ff + 8) * 2.0 ** -24 * (most + want.abs()) + 1e-30
+    assert ((out.double() - want).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("tokens,k,ff,n", [(3, 64, 32, 48), (20, 96, 160, 130), (300, 64, 96, 72)])

@@ -13,10 +13,18 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("bias,activation,residual", [(True, "silu", False), (False, "none", True)])
-@pytest.mark.parametrize("lengths,channels", [([1, 9, 2, 1000, 3, 8, 16, 1, 1, 2007], 2048), ([4096], 1032), ([5, 6], 64)])
-def test_convolution_over_runs_of_tokens(K, taps, bias, activation, residual, lengths, channels):  # noqa: F811
+@pytest.mark.parametrize("lengths,channels,runs", [([1, 9, 2, 1000, 3, 8, 16, 1, 1, 2007], 2048, None), ([1, 9, 2, 700, 3, 8, 16, 1, 1, 0], 2048, True),
+                                                   ([1, 1, 13, 2, 0], 1032, True), ([4096], 1032, None), ([5, 6], 64, False)])
+def test_convolution_over_runs_of_tokens(K, taps, bias, activation, residual, lengths, channels, runs):  # noqa: F811
     """Requests that begin inside a run of eight tokens, ones shorter than the filter, a count of tokens that is no multiple of a run; the state's
-    inputs before the first tokens. Few tokens take a thread each."""
+    inputs before the first tokens. Few tokens take a thread each. Whether a step is taken in runs depends on the GPU's size: a last request of 0
+    tokens stands for as many as make it one that is, all but a token of a run."""
+    wide, places = -(-channels // 1024), 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    if lengths[-1] == 0:
+        lengths = lengths[:-1] + [8 * (places * 9 // 10 // wide) - 1 - sum(lengths)]
+    blocks = -(-sum(lengths) // 8) * wide
+    if runs is not None:                                                # (the rule of sb_causal_conv)
+        assert (blocks * 10 >= -(-blocks // places) * places * 7) == runs
     g = torch.Generator(device=DEV).manual_seed(taps + channels)
     rn = lambda *s: torch.randn(s, generator=g, device=DEV)
     t, r = sum(lengths), len(lengths)
