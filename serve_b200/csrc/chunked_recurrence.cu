@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const SbChunkedWalk
     }
 }
 
-// The walk for many (request, head) pairs: G groups of 16 columns in a block, KS warps a group with DKT / KS rows of S each, and a warp that
+// The walk for many (request, head) pairs: G groups of 16 columns in a block, KS = 2 warps a group with half of the rows of S each, and a warp that
 // fetches. A chunk's matrices then cross to an SM once for 16 G columns instead of once for 16, and since S lies turned over in
 // the accumulators (columns of S are the tile's rows), they are the first operand of the next product as they stand: S and U never
 // pass through shared memory, and the warps of a group meet once a step, to add their sums of W S (and Q' S) up. What bounds it: mma.sync, 16
@@ -749,12 +749,13 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const SbChunkedWalk
 // are not enough blocks, and chunk_walk_kernel, whose eight warps share 16 columns, has the shorter step. Eight requests of 256 tokens, 16
 // heads of 128 x 128: fixed decay 101 -> 67 us, gated delta rule 121 -> 95. (One warp for all rows of 16 columns: 91 us, registers spill;
 // the sums of Q' S a step behind those of W S, so that they hide: 107, more of them spill.)
-template <int DKT, bool DELTA, int KS, int G>
+template <int DKT, bool DELTA, int G>
 struct Wide {
   typedef Part<DKT, DELTA> L;
+  static constexpr int KS = 2;
   static constexpr int WARPS = KS * G, THREADS = 32 * (WARPS + 1);
   static constexpr int TILES = DELTA ? 8 : 4;             // eights of rows of [W; Q'] (or Q')
-  static constexpr int XCH_OFF = 2 * L::BYTES, BYTES = XCH_OFF + (KS > 1 ? 2 * WARPS * TILES * 32 * 16 : 0);
+  static constexpr int XCH_OFF = 2 * L::BYTES, BYTES = XCH_OFF + 2 * WARPS * TILES * 32 * 16;
   static_assert(BYTES <= 226 * 1024, "shared memory of an SM");
 };
 
@@ -787,11 +788,11 @@ struct Notes {
 };
 
 // grid (ceil(dv / (16 G)), head, list entry).
-template <int DKT, bool DELTA, int KS, int G>
-__global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbChunkedWalk a, const float* __restrict__ u_rows) {
-  typedef Wide<DKT, DELTA, KS, G> W;
+template <int DKT, bool DELTA, int G>
+__global__ void __launch_bounds__(Wide<DKT, DELTA, G>::THREADS) chunk_wide_kernel(const SbChunkedWalk a, const float* __restrict__ u_rows) {
+  typedef Wide<DKT, DELTA, G> W;
   typedef Part<DKT, DELTA> L;
-  constexpr int AP = L::AP, ROWS = L::ROWS, TILES = W::TILES, NTS = DKT / KS / 8, OT = 4 / KS;
+  constexpr int AP = L::AP, ROWS = L::ROWS, TILES = W::TILES, KS = W::KS, NTS = DKT / KS / 8, OT = 4 / KS;
   constexpr int LEFT[6] = {2, 0, 1, 1, 0, 0}, RIGHT[6] = {0, 2, 1, 0, 1, 0};      // six of the nine products of the parts, smallest first
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int red_i[16];
@@ -871,7 +872,6 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
     const float* cc = reinterpret_cast<const float*>(A1 + L::C_OFF);
     const int n_tok = min(CH, n_all - c * CH);
     bool slow = reinterpret_cast<const int*>(cc + 2 * DKT)[0] != 0;
-    if (KS == 1) slow |= __any_sync(0xffffffffu, bad) != 0;
     // [W; Q'] S of this warp's rows of S
     float x[TILES][4];
     auto first_slow = [&]() {
@@ -924,40 +924,33 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
       first_slow();
     }
     float o[OT][4];
-    if constexpr (KS > 1) {
-      // the group's warps add their sums up, all of them W S, each its own tokens of Q' S
-      float4* xch = reinterpret_cast<float4*>(raw + W::XCH_OFF) + (size_t)((c & 1) * W::WARPS + group * KS) * TILES * 32 + lane;
-      auto leave = [&]() {
+    // the group's warps add their sums up, all of them W S, each its own tokens of Q' S
+    float4* xch = reinterpret_cast<float4*>(raw + W::XCH_OFF) + (size_t)((c & 1) * W::WARPS + group * KS) * TILES * 32 + lane;
+    auto leave = [&]() {
 #pragma unroll
-        for (int n = 0; n < TILES; ++n) xch[(ks * TILES + n) * 32] = make_float4(x[n][0], x[n][1], x[n][2], x[n][3]);
-      };
+      for (int n = 0; n < TILES; ++n) xch[(ks * TILES + n) * 32] = make_float4(x[n][0], x[n][1], x[n][2], x[n][3]);
+    };
+    leave();
+    if (group_any(1 + group, 32 * KS, bad)) {            // (all of the group) S is not finite: once more, without parts
+      if (!slow) first_slow();
+      slow = true;
       leave();
-      if (group_any(1 + group, 32 * KS, bad)) {            // (all of the group) S is not finite: once more, without parts
-        if (!slow) first_slow();
-        slow = true;
-        leave();
-        group_sync(1 + group, 32 * KS);
-      }
-      auto sum = [&](float (&y)[4], int n) {
-        float4 v[KS];
-#pragma unroll
-        for (int w = 0; w < KS; ++w) v[w] = xch[(w * TILES + n) * 32];
-        y[0] = v[0].x; y[1] = v[0].y; y[2] = v[0].z; y[3] = v[0].w;
-#pragma unroll
-        for (int w = 1; w < KS; ++w) { y[0] += v[w].x; y[1] += v[w].y; y[2] += v[w].z; y[3] += v[w].w; }
-      };
-      if (DELTA) {
-#pragma unroll
-        for (int n = 0; n < 4; ++n) sum(x[n], n);
-      }
-#pragma unroll
-      for (int n = 0; n < OT; ++n) sum(o[n], TILES - 4 + ks * OT + n);
-    } else {
-#pragma unroll
-      for (int n = 0; n < OT; ++n)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[n][e] = x[TILES - 4 + n][e];
+      group_sync(1 + group, 32 * KS);
     }
+    auto sum = [&](float (&y)[4], int n) {
+      float4 v[KS];
+#pragma unroll
+      for (int w = 0; w < KS; ++w) v[w] = xch[(w * TILES + n) * 32];
+      y[0] = v[0].x; y[1] = v[0].y; y[2] = v[0].z; y[3] = v[0].w;
+#pragma unroll
+      for (int w = 1; w < KS; ++w) { y[0] += v[w].x; y[1] += v[w].y; y[2] += v[w].z; y[3] += v[w].w; }
+    };
+    if (DELTA) {
+#pragma unroll
+      for (int n = 0; n < 4; ++n) sum(x[n], n);
+    }
+#pragma unroll
+    for (int n = 0; n < OT; ++n) sum(o[n], TILES - 4 + ks * OT + n);
     float u[4][4];
     bool bad_u = false;
 #pragma unroll
@@ -1012,7 +1005,7 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
           step(m + n, add);
         }
       }
-      // O += P U: token n's eight rows of P, zeros after the diagonal (so tokens 0 .. 15 need the first 16 terms only)
+      // O += P U: token n's eight rows of P, zeros after the diagonal
 #pragma unroll
       for (int n = 0; n < OT; ++n) {
         const int tile = ks * OT + n;
@@ -1075,10 +1068,10 @@ __global__ void __launch_bounds__(32 * (KS * G + 1)) chunk_wide_kernel(const SbC
     }
 }
 
-template <int DKT, bool DELTA, int KS, int G>
+template <int DKT, bool DELTA, int G>
 int launch_wide(const SbChunkedWalk& a, const float* u_rows, cudaStream_t stream) {
-  typedef Wide<DKT, DELTA, KS, G> W;
-  auto k = chunk_wide_kernel<DKT, DELTA, KS, G>;
+  typedef Wide<DKT, DELTA, G> W;
+  auto k = chunk_wide_kernel<DKT, DELTA, G>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, W::BYTES);
   k<<<dim3((a.dv + 16 * G - 1) / (16 * G), a.H, a.n_list), W::THREADS, W::BYTES, stream>>>(a, u_rows);
   SB_LAUNCH_CHECK();
@@ -1116,9 +1109,9 @@ int launch(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
   const long long two = DELTA ? cost(2, BIG ? 260 : 196, 0) : cost(2, BIG ? 213 : 246, BIG ? 0 : 340);
   if constexpr (BIG && !DELTA) {
     const long long four = cost(4, 342, 0);
-    if (four < one && four < two) return launch_wide<DKT, DELTA, 2, 4>(a, u, stream);
+    if (four < one && four < two) return launch_wide<DKT, DELTA, 4>(a, u, stream);
   }
-  if (two < one) return launch_wide<DKT, DELTA, 2, 2>(a, u, stream);
+  if (two < one) return launch_wide<DKT, DELTA, 2>(a, u, stream);
   auto k = chunk_walk_kernel<DKT, DELTA>;
   constexpr int smem = Walk<DKT, DELTA>::BYTES;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

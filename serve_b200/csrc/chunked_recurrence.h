@@ -8,7 +8,7 @@ struct SbChunkedWalk {
   const float *qf, *kf, *af, *vf, *sc, *dec;
   int n_tokens, H, Hqk, dk, dv, dkp, dvp;
   int mode;                    // as in sequence_ops.cu
-  int head_rate;               // af holds one decay a head, repeated over its rows
+  int head_rate;               // af holds one decay a head: the first of its dkp numbers is read, the others need not be there
   const void* skip;            // SSM: D of every head, float or bfloat16 (skip_dtype, as in common.cuh)
   int skip_dtype;
   float* state;
