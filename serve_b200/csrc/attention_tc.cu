@@ -41,6 +41,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "tcgen05_ops.cuh"
 
 #if SB_HEAD_DIM == 64 || SB_HEAD_DIM == 128 || SB_HEAD_DIM == 256
 
@@ -57,7 +58,6 @@ constexpr int BN = 64;               // keys per tile
 constexpr int BT_CACHE = D == 256 ? 512 : 1024;       // block-table entries kept in shared memory
 constexpr int SOFTMAX_WARPS = 8;
 constexpr int THREADS = 64 + 32 * SOFTMAX_WARPS;
-constexpr unsigned WAIT_LIMIT = 1u << 26;
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr int Q_BYTES = BM * D * 2, KV_BYTES = BN * D * 2, P_COLS = BN / 2;      // (two probabilities a column)
 
@@ -87,86 +87,28 @@ struct Layout {
   static_assert(SMEM_BYTES <= 227 * 1024 / CTAS_PER_SM - 1024, "shared memory of an SM");
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, unsigned parity) {
-  uint32_t done;
-  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
-}
 // A wait that runs out is noted in *gave_up; from then on no wait of the CTA lasts, every loop and barrier runs to its end, and what is
 // computed is not valid (*error is raised).
 __device__ __noinline__ void mbar_wait_long(uint32_t bar, unsigned parity, int* gave_up) {
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    if (mbar_try(bar, parity)) return;
+  for (unsigned i = 0; i < tc::WAIT_LIMIT; ++i) {
+    if (tc::mbar_try(bar, parity)) return;
     if ((i & 1023u) == 1023u && *reinterpret_cast<volatile int*>(gave_up)) return;
   }
   *reinterpret_cast<volatile int*>(gave_up) = 1;
 }
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, unsigned parity, int* gave_up) {
-  const uint32_t addr = smem_u32(bar);
-  if (!mbar_try(addr, parity)) mbar_wait_long(addr, parity, gave_up);
+  const uint32_t addr = tc::smem_u32(bar);
+  if (!tc::mbar_try(addr, parity)) mbar_wait_long(addr, parity, gave_up);
 }
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// A descriptor's upper half is the same for all tiles here (see desc_lo), so the issuing thread only ever adds to a 32-bit number.
-constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(DESC_HI) : "memory");
-}
-// The same with the first operand in tensor memory: row i of it is lane i, two bfloat16 numbers to a column.
+// A product whose first operand lies in tensor memory: row i of it is lane i, two bfloat16 numbers to a column.
 __device__ __forceinline__ void tc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n .reg .b64 b;\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(DESC_HI) : "memory");
+      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(idesc), "r"(accumulate), "n"(tc::DESC_HI) : "memory");
 }
-// One thread of a warp that has come together, always the same: the compiler then knows what is equal in all of them.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t yes;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(yes));
-  return yes != 0;
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// 32 lanes x 32 columns: thread i of the warp gets lane (base + i), 32 consecutive columns. No wait: several loads
-// may be in flight; tc_wait_ld() before the registers are read. Loads and stores, and the wait for stores, are the warp's instructions:
-// lanes that a branch before them has parted meet first, or (_met) have just met and taken no branch of their own since (meeting
-// again for each of them cost a windowed prompt 1.2 %).
-__device__ __forceinline__ void tc_load32_met(uint32_t taddr, float* r) {
-  uint32_t* u = reinterpret_cast<uint32_t*>(r);
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
-        "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]),
-        "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]),
-        "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
-  __syncwarp();
-  tc_load32_met(taddr, r);
-}
+// Stores and the wait for them, as loads, are the warp's instructions: lanes that a branch before them has parted meet first, or (_met) have
+// just met and taken no branch of their own since (meeting again for each of them cost a windowed prompt 1.2 %).
 __device__ __forceinline__ void tc_store32(uint32_t taddr, const float* r) {
   __syncwarp();
   const uint32_t* u = reinterpret_cast<const uint32_t*>(r);
@@ -229,16 +171,6 @@ __device__ __forceinline__ bool pair_any(int id, bool yes) {
   asm volatile("{\n .reg .pred p, q;\n setp.ne.b32 q, %2, 0;\n bar.red.or.pred p, %1, 64, q;\n selp.u32 %0, 1, 0, p;\n}\n"
                : "=r"(any) : "r"(id), "r"(yes ? 1u : 0u) : "memory");
   return any != 0;
-}
-
-// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart (bits 32 .. 45), version 1 of it (46), layout type 2
-// (61 .. 63): its lower half, the address and ``lbo``, the distance between 64-element swizzle atoms along the non-k dimension of an
-// MN-major operand (not used by K-major operands), both in units of 16 bytes.
-__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr & 0x3FFFF) >> 4) | (lbo_bytes >> 4) << 16; }
-// kind::f16 instruction descriptor: float accumulator, bfloat16 operands; b_mn_major: the second operand has its
-// non-k dimension contiguous in shared memory (values: rows are keys, head elements contiguous)
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 struct TcParams {
@@ -324,7 +256,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
   int* gave_up = reinterpret_cast<int*>(bars + 10 + 4 * NK);      // a wait of this CTA ran out
   float* xch = reinterpret_cast<float*>(base + XCH_OFF);      // [2][BM]
   int* bt_s = reinterpret_cast<int*>(base + BT_OFF);
-  if ((smem_u32(base) & 1023u) != 0) {                  // never seen; refuse rather than compute with a wrong swizzle
+  if ((tc::smem_u32(base) & 1023u) != 0) {                  // never seen; refuse rather than compute with a wrong swizzle
     if (threadIdx.x == 0) atomicExch(p.error, 1);
     pdl_wait();
     return;
@@ -332,12 +264,12 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    mbar_init(&q_full, 1);
+    tc::mbar_init(&q_full, 1);
 #pragma unroll
-    for (int s = 0; s < (SPLIT ? 4 : 2) * NK; ++s) mbar_init(&k_full[s], 1);
+    for (int s = 0; s < (SPLIT ? 4 : 2) * NK; ++s) tc::mbar_init(&k_full[s], 1);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&s_full[b], 1); mbar_init(&s_empty[b], SOFTMAX_WARPS); mbar_init(&p_full[b], SOFTMAX_WARPS); mbar_init(&p_empty[b], 1);
+      tc::mbar_init(&s_full[b], 1); tc::mbar_init(&s_empty[b], SOFTMAX_WARPS); tc::mbar_init(&p_full[b], SOFTMAX_WARPS); tc::mbar_init(&p_empty[b], 1);
     }
     *gave_up = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -346,13 +278,13 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
-  tc_fence_after();
+  tc::fence_after();
   // set up; queries, this step's keys and values, and the right to overwrite out come with the end of the kernel before
   pdl_launch_dependents();
   pdl_wait();
@@ -368,10 +300,10 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       bt = bt_s;
     }
     // queries: box {64 elements, G heads, 1 kv head, tokens of the tile} -> rows (token, head)
-    if (elect_one()) {
-      mbar_expect_tx(&q_full, (unsigned)(tok_per_tile * G * D * 2));
+    if (tc::elect_one()) {
+      tc::mbar_expect_tx(&q_full, (unsigned)(tok_per_tile * G * D * 2));
 #pragma unroll
-      for (int a = 0; a < KA; ++a) tma_load_4d(Qs + (size_t)a * BM * 128, &map_q, &q_full, a * 64, 0, hk, q0 + tok0);
+      for (int a = 0; a < KA; ++a) tc::load_4d(Qs + (size_t)a * BM * 128, &map_q, &q_full, a * 64, 0, hk, q0 + tok0);
     }
     // The loop is on the critical path: the whole warp walks it (what it computes is equal in all lanes then), no divisions, a tile's
     // page is looked up while the tile before waits for its stage. Pages of a tile or more: a tile lies in one page, from its row ``at`` on.
@@ -393,20 +325,20 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       auto load = [&](unsigned char* stage, const CUtensorMap* map, uint64_t* full) {
         if (n_pages > 0) {                               // (-1, a page the window has passed: outside the map, zeros)
 #pragma unroll
-          for (int a = 0; a < KA; ++a) tma_load_4d(stage + (size_t)a * BN * 128, map, full, a * 64, at, hk, page);
+          for (int a = 0; a < KA; ++a) tc::load_4d(stage + (size_t)a * BN * 128, map, full, a * 64, at, hk, page);
         }
         if (!one) {
           for (int i = 1; i < n_pages; ++i) {
             const int pg = bt[blk + i];
 #pragma unroll
-            for (int a = 0; a < KA; ++a) tma_load_4d(stage + (size_t)a * BN * 128 + (size_t)i * p.ps * 128, map, full, a * 64, 0, hk, pg);
+            for (int a = 0; a < KA; ++a) tc::load_4d(stage + (size_t)a * BN * 128 + (size_t)i * p.ps * 128, map, full, a * 64, 0, hk, pg);
           }
         }
       };
       mbar_wait(&k_empty[s], phase, gave_up);
       if (any_lane(*reinterpret_cast<volatile int*>(gave_up))) break;        // (no copy into a stage that may still be read)
-      if (elect_one()) {
-        mbar_expect_tx(&k_full[s], SPLIT || SHARED ? bytes : 2 * bytes);
+      if (tc::elect_one()) {
+        tc::mbar_expect_tx(&k_full[s], SPLIT || SHARED ? bytes : 2 * bytes);
         load(Ks + (size_t)s * KV_BYTES, &map_k, &k_full[s]);
         if (!SPLIT && !SHARED) load(Vs + (size_t)s * KV_BYTES, &map_v, &k_full[s]);
       }
@@ -414,8 +346,8 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       if (SPLIT) {
         mbar_wait(&v_empty[s], phase, gave_up);
         if (any_lane(*reinterpret_cast<volatile int*>(gave_up))) { ++j; break; }
-        if (elect_one()) {
-          mbar_expect_tx(&v_full[s], bytes);
+        if (tc::elect_one()) {
+          tc::mbar_expect_tx(&v_full[s], bytes);
           load(Vs + (size_t)s * KV_BYTES, &map_v, &v_full[s]);
         }
         __syncwarp();
@@ -433,15 +365,15 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
     }
     if (*reinterpret_cast<volatile int*>(gave_up)) {       // the copies under way land before the CTA leaves (with a limit again)
       for (int i = max(0, j - NK); i < j; ++i) {
-        for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&k_full[i % NK]), (i / NK) & 1); ++n) {}
-        for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&v_full[i % NK]), (i / NK) & 1); ++n) {}
+        for (unsigned n = 0; n < tc::WAIT_LIMIT && !tc::mbar_try(&k_full[i % NK], (i / NK) & 1); ++n) {}
+        for (unsigned n = 0; n < tc::WAIT_LIMIT && !tc::mbar_try(&v_full[i % NK], (i / NK) & 1); ++n) {}
       }
-      for (unsigned n = 0; n < WAIT_LIMIT && !mbar_try(smem_u32(&q_full), 0); ++n) {}
+      for (unsigned n = 0; n < tc::WAIT_LIMIT && !tc::mbar_try(&q_full, 0); ++n) {}
     }
   } else if (warp == 1) {
-    constexpr uint32_t idesc_s = make_idesc(BM, BN, false);
-    constexpr uint32_t idesc_o = make_idesc(BM, D, true);
-    const uint32_t dq = desc_lo(smem_u32(Qs), 0), dk0 = desc_lo(smem_u32(Ks), 0), dv0 = desc_lo(smem_u32(Vs), BN * 128);
+    constexpr uint32_t idesc_s = tc::make_idesc(BM, BN, false);
+    constexpr uint32_t idesc_o = tc::make_idesc(BM, D, true);
+    const uint32_t dq = tc::desc_lo(tc::smem_u32(Qs)), dk0 = tc::desc_lo(tc::smem_u32(Ks)), dv0 = tc::desc_lo(tc::smem_u32(Vs), BN * 128);
     int ks = 0, vs = 0;                                  // stages of the next scores and of the next values
     unsigned kphase = 0, vphase = 0;
     // the scores of tile t, as soon as its keys are there and its score buffer has been read
@@ -449,17 +381,17 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       mbar_wait(&k_full[ks], kphase, gave_up);
       mbar_wait(&s_empty[t % NSB], ((t / NSB) & 1) ^ 1, gave_up);
       __syncwarp();
-      tc_fence_after();
+      tc::fence_after();
       const uint32_t dk = dk0 + (uint32_t)(ks * (KV_BYTES >> 4)), acc = tmem_base + (uint32_t)((t % NSB) * BN);
-      if (elect_one()) {
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           // 16 k-values further: 32 bytes within an atom (4 steps), then the next atom of Q (128 rows) and K (64 rows)
-          tc_mma(acc, dq + (uint32_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2), dk + (uint32_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2), idesc_s,
+          tc::mma_lo(acc, dq + (uint32_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2), dk + (uint32_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2), idesc_s,
                  kk != 0 ? 1u : 0u);
         }
-        tc_commit(&s_full[t % NSB]);
-        if (SPLIT) tc_commit(&k_empty[ks]);
+        tc::commit(&s_full[t % NSB]);
+        if (SPLIT) tc::commit(&k_empty[ks]);
       }
       __syncwarp();
       if (++ks == NK) { ks = 0; kphase ^= 1; }
@@ -471,17 +403,17 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       mbar_wait(&p_full[j % NP], (j / NP) & 1, gave_up);
       if (SPLIT) mbar_wait(&v_full[vs], vphase, gave_up);
       __syncwarp();
-      tc_fence_after();
+      tc::fence_after();
       // O += P V: P from tensor memory (16 keys are 8 columns), FINE: both parts of it; V is MN-major, 16 keys = 2048 bytes further per step
       const uint32_t pa = tmem_base + P_COL + (uint32_t)((j % NP) * P_BUF), dv = dv0 + (uint32_t)(vs * (KV_BYTES >> 4));
-      if (elect_one()) {
+      if (tc::elect_one()) {
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk) {
           tc_mma_ts(tmem_base + O_COL, pa + (uint32_t)(kk * 8), dv + (uint32_t)(kk * (2048 >> 4)), idesc_o, (j | kk) != 0 ? 1u : 0u);
           if (FINE) tc_mma_ts(tmem_base + O_COL, pa + (uint32_t)(P_COLS + kk * 8), dv + (uint32_t)(kk * (2048 >> 4)), idesc_o, 1u);
         }
-        tc_commit(&p_empty[j % NP]);                     // also: "the products up to tile j have finished"
-        tc_commit(&v_empty[vs]);
+        tc::commit(&p_empty[j % NP]);                     // also: "the products up to tile j have finished"
+        tc::commit(&v_empty[vs]);
       }
       __syncwarp();
       if (++vs == NK) { vs = 0; vphase ^= 1; }
@@ -512,14 +444,14 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       float sv[32];
       float m_half;
       {
-        tc_fence_after();
+        tc::fence_after();
         // the tile reaches beyond what the first row may see, or behind the last row's window
         const bool masked = kt + BN - 1 > first_pos || (p.window > 0 && kt <= p0 + tok_last - p.window);
-        tc_load32_met(lane_addr + (uint32_t)(b * BN + half * 32), sv);
-        tc_wait_ld();
-        tc_fence_before();
+        tc::load32_met(lane_addr + (uint32_t)(b * BN + half * 32), sv);
+        tc::wait_loads();
+        tc::fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[b]);         // the scores are in registers: the buffer may be reused
+        if (lane == 0) tc::mbar_arrive(&s_empty[b]);         // the scores are in registers: the buffer may be reused
         if (p.cap_over_scale > 0.f) {                    // the cap comes before the mask: tanh(-inf) would be finite
 #pragma unroll
           for (int i = 0; i < 32; ++i) sv[i] = p.cap_over_scale * tanh_fast(sv[i] * p.softcap_in);
@@ -552,14 +484,14 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
           // rescale the accumulator in tensor memory, once the products issued so far (up to tile j-1) are done
           mbar_wait(&p_empty[(j - 1) % NP], ((j - 1) / NP) & 1, gave_up);
           __syncwarp();
-          tc_fence_after();
+          tc::fence_after();
           const float f = (moves && m_ref != -INFINITY) ? ex2(m_ref - m_tile) : 1.f;
 #pragma unroll 1
           for (int c = 0; c < D / 64; ++c) {
             const uint32_t o_addr = lane_addr + O_COL + (uint32_t)(half * (D / 2) + c * 32);
             float ov[32];
-            tc_load32(o_addr, ov);
-            tc_wait_ld();
+            tc::load32(o_addr, ov);
+            tc::wait_loads();
 #pragma unroll
             for (int i = 0; i < 32; ++i) ov[i] *= f;
             tc_store32(o_addr, ov);
@@ -573,7 +505,7 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       if (NP == 1 && j > 0) {
         mbar_wait(&p_empty[0], (j - 1) & 1, gave_up);
         __syncwarp();
-        tc_fence_after();
+        tc::fence_after();
       }
       // probabilities -> tensor memory (bfloat16, two neighbouring keys a column); ex2(-inf) = 0 takes care of masked entries
       float2 sum = make_float2(0.f, 0.f);
@@ -615,14 +547,14 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
         __syncwarp();
       }
       tc_wait_st_met();
-      tc_fence_before();
+      tc::fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[j % NP]);
+      if (lane == 0) tc::mbar_arrive(&p_full[j % NP]);
     }
     // all products have finished when the last one has
     mbar_wait(&p_empty[(n_tiles - 1) % NP], ((n_tiles - 1) / NP) & 1, gave_up);
     __syncwarp();
-    tc_fence_after();
+    tc::fence_after();
     *mine = l_run;
     pair_sync(pair);
     l_run = half ? *other + l_run : l_run + *other;    // (the same sum in both threads of a row)
@@ -640,8 +572,8 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
 #pragma unroll 1
       for (int c = 0; c < COLS; c += 32) {
         float ov[32];
-        tc_load32(lane_addr + O_COL + (uint32_t)(c0 + c), ov);
-        tc_wait_ld();
+        tc::load32(lane_addr + O_COL + (uint32_t)(c0 + c), ov);
+        tc::wait_loads();
         if (row_ok) {
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -652,29 +584,20 @@ __global__ void __launch_bounds__(THREADS, Layout<FINE, TIGHT>::CTAS_PER_SM) att
       }
     }
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *gave_up) atomicExch(p.error, 1);
   if (warp == 1) {
-    tc_fence_after();
+    tc::fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn g_encode = nullptr;
-
 int encode4(CUtensorMap* map, const void* basep, const cuuint64_t dims[4], const cuuint64_t strides[3], const cuuint32_t box[4]) {
-  if (!g_encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn) return -300;
-    g_encode = (EncodeTiledFn)fn;
-  }
+  const tc::EncodeTiledFn encode = tc::encode_fn();
+  if (!encode) return -300;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult rc = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(basep), dims, strides, box, estr,
+  const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(basep), dims, strides, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS ? 0 : -301 - (int)rc;

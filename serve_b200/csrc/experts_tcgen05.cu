@@ -17,7 +17,8 @@
 // A unit with two accumulators is 256 weight rows: many tokens an expert, where the tokens' rows are what the SMs fetch
 // most. A unit with one is at most 128 rows, of a count that shares the step's rows out evenly over the SMs (pick_unit):
 // few tokens an expert, where a unit is nothing but weights and a last round of a few units would leave most SMs idle.
-// Every TMA instruction costs its issuer time however little it fetches, so a stage takes as few as possible: there is a map for every count of weight rows a unit may have, and maps of 128, 64 and 16 tokens.
+// Every TMA instruction costs its issuer time however little it fetches, so a stage takes as few as possible: there is a map for every
+// count of weight rows a unit may have, and maps of 128, 64 and 16 tokens.
 //
 //   gate/up:  act[row, c] = f(g, u): with two accumulators the gate rows are one and the up rows of the same outputs the
 //             other, so a thread holds both sums; with one, 16 gate rows and the 16 up rows of the same outputs take turns

@@ -30,58 +30,9 @@ namespace {
 constexpr int BM = 128, BN = 256, BK = 64;      // accumulator tile and k-values per stage
 constexpr int NSTAGE = 4;
 constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int EPI_WARPS = 16;                    // two warps per quarter of the tensor-memory lanes: even and odd column chunks
-constexpr int THREADS = 64 + 32 * EPI_WARPS;     // warp 0: TMA, warp 1: MMA + tensor memory, warps 2..9: epilogue
-constexpr unsigned WAIT_LIMIT = 1u << 26;
+constexpr int EPI_WARPS = 16;                    // four warps per quarter of the tensor-memory lanes
+constexpr int THREADS = 64 + 32 * EPI_WARPS;     // warp 0: TMA, warp 1: MMA + tensor memory, warps 2..17: epilogue
 constexpr uint32_t TMEM_COLS = 512;              // two accumulators of BN columns
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// 32 lanes x 32 columns of 32-bit accumulator: thread i of the warp gets lane (base lane + i), 32 consecutive columns
-// (the warp's instruction: lanes that a branch before it has parted meet first)
-__device__ __forceinline__ void tc_load32(uint32_t taddr, uint32_t (&r)[32]) {
-  __syncwarp();
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// kind::f16 instruction descriptor: float accumulator, bfloat16 a and b, both K-major, N x M of the tile
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
 
 constexpr int EPI_STORE = 0, EPI_GATE_UP = 1, EPI_ROPE = 2;
 
@@ -198,26 +149,26 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int s = 0; s < NSTAGE; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      tc::mbar_init(&full_bar[s], 1);
+      tc::mbar_init(&empty_bar[s], 1);
     }
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], EPI_WARPS);       // one arrival per epilogue warp
+      tc::mbar_init(&acc_full[b], 1);
+      tc::mbar_init(&acc_empty[b], EPI_WARPS);       // one arrival per epilogue warp
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
-  tc_fence_after();
+  tc::fence_after();
   // barriers, tensor memory and descriptors are ready; the activations (and the right to overwrite out) come with
   // the end of the kernel before this one
   pdl_launch_dependents();
@@ -226,7 +177,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
   bool failed = false;
 
   // tile t of this CTA: consecutive CTAs take the row tiles of one panel of w
-  const uint32_t tiles_lo = tc::desc_lo(smem_u32(tiles));
+  const uint32_t tiles_lo = tc::desc_lo(tc::smem_u32(tiles));
   if (warp == 0) {
     int s = 0;
     unsigned phase = 1;                                // a fresh barrier passes a wait on parity 1: the first round finds every stage free
@@ -237,17 +188,17 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
         if (tc::elect_one()) {
           unsigned char* a_dst = tiles + s * STAGE_BYTES;
           unsigned char* b_dst = a_dst + A_BYTES;
-          mbar_expect_tx(&full_bar[s], (unsigned)(A_BYTES + bn * BK * 2));
-          tma_load_2d(a_dst, &map_a, &full_bar[s], kb * BK, m0);
-          tma_load_2d(b_dst, &map_w, &full_bar[s], kb * BK, n0);                         // with gate_up the gate rows
-          if (GU) tma_load_2d(b_dst + bn * BK, &map_w, &full_bar[s], kb * BK, N + n0);   // and their up rows
+          tc::mbar_expect_tx(&full_bar[s], (unsigned)(A_BYTES + bn * BK * 2));
+          tc::load_2d(a_dst, &map_a, &full_bar[s], kb * BK, m0);
+          tc::load_2d(b_dst, &map_w, &full_bar[s], kb * BK, n0);                         // with gate_up the gate rows
+          if (GU) tc::load_2d(b_dst + bn * BK, &map_w, &full_bar[s], kb * BK, N + n0);   // and their up rows
         }
         __syncwarp();
         if (++s == NSTAGE) { s = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    const uint32_t idesc = make_idesc(BM, bn);
+    const uint32_t idesc = tc::make_idesc(BM, bn);
     int s = 0, local = 0;
     unsigned phase = 0;
     for (int tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x, ++local) {
@@ -257,7 +208,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
       const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!tc::warp_wait(&full_bar[s], phase)) { failed = true; break; }
-        tc_fence_after();
+        tc::fence_after();
         const uint32_t da = tiles_lo + (uint32_t)(s * (STAGE_BYTES >> 4)), db = da + (A_BYTES >> 4);
         if (tc::elect_one()) {
 #pragma unroll
@@ -265,8 +216,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
             // 16 k-values further along the swizzled row: 32 bytes, two 16-byte units of the start address
             tc::mma_lo(acc, da + (uint32_t)(j * 2), db + (uint32_t)(j * 2), idesc, (kb | j) != 0 ? 1u : 0u);
           }
-          tc_commit(&empty_bar[s]);          // the stage is free once these products have read it
-          if (kb + 1 == k_blocks) tc_commit(&acc_full[buf]);     // the accumulator is complete once all products are done
+          tc::commit(&empty_bar[s]);          // the stage is free once these products have read it
+          if (kb + 1 == k_blocks) tc::commit(&acc_full[buf]);     // the accumulator is complete once all products are done
         }
         __syncwarp();
         if (++s == NSTAGE) { s = 0; phase ^= 1; }
@@ -283,7 +234,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
       const int m0 = (tile % m_tiles) * BM, n0 = (tile / m_tiles) * OUT_COLS;
       const int buf = local & 1;
       if (!tc::warp_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
-      tc_fence_after();
+      tc::fence_after();
       const int row = m0 + q * 32 + lane;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
       int pos = 0;
@@ -296,7 +247,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
       for (int c = c_first; c < OUT_COLS; c += 32 * (EPI_WARPS / 4)) {
         if (n0 + c >= N) break;
         uint32_t v[32];
-        tc_load32(acc + (uint32_t)c, v);
+        tc::load32(acc + (uint32_t)c, v);
+        if (!GU) tc::wait_loads();
         if (EPI == EPI_ROPE) {
           if (row < M) rope_store_chunk(ra, v, row, n0 + c, M, N, slot, out);
           continue;
@@ -304,7 +256,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
         uint32_t packed[16];
         if (GU) {
           uint32_t u[32];
-          tc_load32(acc + (uint32_t)(OUT_COLS + c), u);
+          tc::load32(acc + (uint32_t)(OUT_COLS + c), u);
+          tc::wait_loads();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             // both halves rounded to the activation type first, as the unfused path stores them
@@ -335,16 +288,16 @@ __global__ void __launch_bounds__(THREADS) gemm_tcgen05_kernel(const __grid_cons
         }
       }
       // this warp has read its part of the accumulator: the next tile but one may overwrite it
-      tc_fence_before();
+      tc::fence_before();
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[buf])) : "memory");
+      if (lane == 0) tc::mbar_arrive(&acc_empty[buf]);
     }
   }
   if (failed) atomicExch(error, 1);
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   if (warp == 1) {
-    tc_fence_after();
+    tc::fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
@@ -366,12 +319,12 @@ constexpr uint32_t PAIR_LEADER_MASK = 0xFEFFFFFFu;   // clears the bit of a shar
 
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t leader_bar, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(map), "r"(leader_bar), "r"(x), "r"(y) : "memory");
+               ::"r"(tc::smem_u32(dst)), "l"(map), "r"(leader_bar), "r"(x), "r"(y) : "memory");
 }
 // arrives, once the products issued so far are done, on the barrier at this address in both CTAs of the pair
 __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"((unsigned short)3) : "memory");
+               ::"r"(tc::smem_u32(bar)), "h"((unsigned short)3) : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all_threads() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -404,13 +357,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int s = 0; s < PAIR_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      tc::mbar_init(&full_bar[s], 1);
+      tc::mbar_init(&empty_bar[s], 1);
     }
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], 2 * EPI_WARPS);   // one arrival per epilogue warp of both CTAs
+      tc::mbar_init(&acc_full[b], 1);
+      tc::mbar_init(&acc_empty[b], 2 * EPI_WARPS);   // one arrival per epilogue warp of both CTAs
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
@@ -418,20 +371,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
   }
   if (warp == 1) {
     // the same warp of both CTAs allocates: the accumulators get the same address in both tensor memories
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(TMEM_COLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   cluster_sync_all_threads();            // the other CTA's barriers exist before anything arrives on them
-  tc_fence_after();
+  tc::fence_after();
   pdl_launch_dependents();
   pdl_wait();                            // as in the one-CTA kernel
   const uint32_t tmem_base = tmem_base_s;
   bool failed = false;
 
-  const uint32_t tiles_lo = tc::desc_lo(smem_u32(tiles));
+  const uint32_t tiles_lo = tc::desc_lo(tc::smem_u32(tiles));
   if (warp == 0) {
     int s = 0;
     unsigned phase = 1;
@@ -444,8 +397,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
         if (!tc::warp_wait(&empty_bar[s], phase)) { failed = true; break; }
         if (tc::elect_one()) {
           unsigned char* a_dst = tiles + s * PAIR_STAGE_BYTES;
-          const uint32_t leader_bar = smem_u32(&full_bar[s]) & PAIR_LEADER_MASK;
-          if (rank == 0) mbar_expect_tx(&full_bar[s], (unsigned)(2 * (PAIR_A_BYTES + half * BK * 2)));
+          const uint32_t leader_bar = tc::smem_u32(&full_bar[s]) & PAIR_LEADER_MASK;
+          if (rank == 0) tc::mbar_expect_tx(&full_bar[s], (unsigned)(2 * (PAIR_A_BYTES + half * BK * 2)));
           tma_load_2d_pair(a_dst, &map_a, leader_bar, kb * BK, m0);
           tma_load_2d_pair(a_dst + PAIR_A_BYTES, &map_w, leader_bar, kb * BK, w_row);
         }
@@ -454,7 +407,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
       }
     }
   } else if (warp == 1) {
-    const uint32_t idesc = make_idesc(256, bn);
+    const uint32_t idesc = tc::make_idesc(256, bn);
     int s = 0, local = 0;
     unsigned phase = 0;
     for (int tile = pair; rank == 0 && tile < total_tiles && !failed; tile += num_pairs, ++local) {
@@ -463,7 +416,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
       const uint32_t acc = tmem_base + (uint32_t)(buf * BN);
       for (int kb = 0; kb < k_blocks; ++kb) {
         if (!tc::warp_wait(&full_bar[s], phase)) { failed = true; break; }
-        tc_fence_after();
+        tc::fence_after();
         const uint32_t da = tiles_lo + (uint32_t)(s * (PAIR_STAGE_BYTES >> 4)), db = da + (PAIR_A_BYTES >> 4);
         if (tc::elect_one()) {
 #pragma unroll
@@ -481,13 +434,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
     uint32_t leader_acc_empty[2];
 #pragma unroll
     for (int b = 0; b < 2; ++b)
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(leader_acc_empty[b]) : "r"(smem_u32(&acc_empty[b])), "r"(0u));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(leader_acc_empty[b]) : "r"(tc::smem_u32(&acc_empty[b])), "r"(0u));
     int local = 0;
     for (int tile = pair; tile < total_tiles && !failed; tile += num_pairs, ++local) {
       const int m0 = (tile % m_tiles) * 256 + (int)rank * 128, n0 = (tile / m_tiles) * OUT_COLS;
       const int buf = local & 1;
       if (!tc::warp_wait(&acc_full[buf], (local >> 1) & 1)) { failed = true; break; }
-      tc_fence_after();
+      tc::fence_after();
       const int row = m0 + q * 32 + lane;
       const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN);
       int pos = 0;
@@ -500,7 +453,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
       for (int c = c_first; c < OUT_COLS; c += 32 * (EPI_WARPS / 4)) {
         if (n0 + c >= N) break;
         uint32_t v[32];
-        tc_load32(acc + (uint32_t)c, v);
+        tc::load32(acc + (uint32_t)c, v);
+        if (!GU) tc::wait_loads();
         if (EPI == EPI_ROPE) {
           if (row < M) rope_store_chunk(ra, v, row, n0 + c, M, N, slot, out);
           continue;
@@ -508,7 +462,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
         uint32_t packed[16];
         if (GU) {
           uint32_t u[32];
-          tc_load32(acc + (uint32_t)(OUT_COLS + c), u);
+          tc::load32(acc + (uint32_t)(OUT_COLS + c), u);
+          tc::wait_loads();
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float g0 = to_float(__float2bfloat16_rn(__uint_as_float(v[2 * i]))), g1 = to_float(__float2bfloat16_rn(__uint_as_float(v[2 * i + 1])));
@@ -537,40 +492,31 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
           }
         }
       }
-      tc_fence_before();
+      tc::fence_before();
       __syncwarp();
       if (lane == 0)
         asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_acc_empty[buf]) : "memory");
     }
   }
   if (failed) atomicExch(error, 1);
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   cluster_sync_all_threads();            // neither CTA leaves, or frees tensor memory, while the other may still use it
   if (warp == 1) {
-    tc_fence_after();
+    tc::fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn g_encode = nullptr;
-
 // rows x cols bfloat16, row-major; box of box_rows x 64 columns, 128-byte swizzle, zero fill outside
 int make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  if (!g_encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn) return -300;
-    g_encode = (EncodeTiledFn)fn;
-  }
+  const tc::EncodeTiledFn encode = tc::encode_fn();
+  if (!encode) return -300;
   const cuuint64_t dims[2] = {cols, rows};
   const cuuint64_t strides[1] = {cols * 2};
   const cuuint32_t box[2] = {(cuuint32_t)BK, box_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : -301 - (int)r;

@@ -15,6 +15,7 @@
 #include <cuda.h>
 
 #include "talking_attention.cuh"
+#include "tcgen05_ops.cuh"
 
 using namespace sb;
 
@@ -32,7 +33,6 @@ constexpr int RUN = 16, RUN_FEW = 8;  // score steps (of 64 keys) a CTA takes; t
                                       // measured: a CTA's start costs about three steps)
 constexpr int NS_S = 2, NS_V = 3;     // stages (two CTAs of either kernel share an SM)
 constexpr int BT_CACHE = 512;         // block-table entries kept in shared memory
-constexpr unsigned WAIT_LIMIT = 1u << 26;
 constexpr int LDE = 36;               // staging row stride (floats): 32 and 16 bytes of padding
 constexpr int Q_BYTES = BM * D * 2, K_BYTES = BN * D * 2, W_BYTES = BM * BN * 2, V_BYTES = BN * D * 2;
 constexpr int EPI = 8;                // epilogue warps of the scores
@@ -43,72 +43,10 @@ constexpr int V_SMEM = V_TILES + 256 + BT_CACHE * 4;
 constexpr uint32_t S_COLS = 2 * BN, V_COLS = D;
 static_assert(S_SMEM <= 113 * 1024 && V_SMEM <= 113 * 1024, "two CTAs an SM");
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
-  const uint32_t addr = smem_u32(bar);
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2), "r"(c3) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-               ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_load32(uint32_t taddr, float* r) {
-  __syncwarp();                      // the warp's instruction: lanes that a branch before it has parted meet first
-  uint32_t* u = reinterpret_cast<uint32_t*>(r);
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]), "=r"(u[9]),
-        "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]), "=r"(u[16]), "=r"(u[17]), "=r"(u[18]),
-        "=r"(u[19]), "=r"(u[20]), "=r"(u[21]), "=r"(u[22]), "=r"(u[23]), "=r"(u[24]), "=r"(u[25]), "=r"(u[26]), "=r"(u[27]),
-        "=r"(u[28]), "=r"(u[29]), "=r"(u[30]), "=r"(u[31])
-      : "r"(taddr));
-}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
 }
-// Shared-memory matrix descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart; ``lbo`` is the distance between 64-element
-// swizzle atoms along the non-k dimension of an MN-major operand (not used by K-major operands).
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
 // tanh by its Taylor series, for |z| <= SERIES_LIMIT (the first term left out is below 2^-24 of z): no special-function unit, whose
 // two calls per score (three with the exponential) bound the scores otherwise.
 constexpr float SERIES_LIMIT = 0.3f;
@@ -179,7 +117,7 @@ __device__ __forceinline__ int load_keys(const Params& p, const CUtensorMap* map
     if (bar) {
       const int page = bt[blk - bt_first];
 #pragma unroll
-      for (int a = 0; a < KA; ++a) tma_load_4d(dst + (size_t)a * atom + (size_t)(k - kt) * 128, map, bar, a * 64, k - blk * p.ps, hk, page);
+      for (int a = 0; a < KA; ++a) tc::load_4d(dst + (size_t)a * atom + (size_t)(k - kt) * 128, map, bar, a * 64, k - blk * p.ps, hk, page);
     }
     ++n;
   }
@@ -203,26 +141,26 @@ __global__ void __launch_bounds__(64 + EPI * 32, 2) scores_tc_kernel(const __gri
   const int run = blockIdx.y % n_runs;
   const int n_steps_all = (w.hi - w.kt0 + BN - 1) / BN, step0 = run * run_steps, n_steps = min(n_steps_all - step0, run_steps);
   if (n_steps <= 0) return;
-  if ((smem_u32(smem) & 1023u) != 0) {                        // never seen; refuse rather than compute with a wrong swizzle
+  if ((tc::smem_u32(smem) & 1023u) != 0) {                        // never seen; refuse rather than compute with a wrong swizzle
     if (threadIdx.x == 0) atomicExch(error, 1);
     return;
   }
   const int kt_first = w.kt0 + step0 * BN;
   if (threadIdx.x == 0) {
-    mbar_init(&q_full, 1);
+    tc::mbar_init(&q_full, 1);
 #pragma unroll
-    for (int s = 0; s < NS_S; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
+    for (int s = 0; s < NS_S; ++s) { tc::mbar_init(&k_full[s], 1); tc::mbar_init(&k_empty[s], 1); }
 #pragma unroll
-    for (int b = 0; b < 2; ++b) { mbar_init(&s_full[b], 1); mbar_init(&s_empty[b], EPI / 2); }
+    for (int b = 0; b < 2; ++b) { tc::mbar_init(&s_full[b], 1); tc::mbar_init(&s_empty[b], EPI / 2); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(S_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(S_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
-  tc_fence_after();
+  tc::fence_after();
   const uint32_t tmem_base = tmem_base_s;
   const int tpt = BM / p.per;
   bool failed = false;
@@ -231,35 +169,35 @@ __global__ void __launch_bounds__(64 + EPI * 32, 2) scores_tc_kernel(const __gri
     int bt_first;
     const int* bt = table_of(p, w, max(kt_first, w.lo), min(kt_first + n_steps * BN, w.hi), bt_s, lane, bt_first);
     if (lane == 0) {
-      mbar_expect_tx(&q_full, (unsigned)(tpt * p.per * D * 2));
+      tc::mbar_expect_tx(&q_full, (unsigned)(tpt * p.per * D * 2));
 #pragma unroll
-      for (int a = 0; a < KA; ++a) tma_load_4d(Qs + (size_t)a * BM * 128, &map_q, &q_full, a * 64, 0, w.hk, w.q0 + w.tok0);
+      for (int a = 0; a < KA; ++a) tc::load_4d(Qs + (size_t)a * BM * 128, &map_q, &q_full, a * 64, 0, w.hk, w.q0 + w.tok0);
       const unsigned box = (unsigned)((p.ps < BN ? p.ps : BN) * D * 2);
       for (int j = 0; j < n_steps; ++j) {
         const int s = j % NS_S, kt = kt_first + j * BN;
-        if (!mbar_wait(&k_empty[s], ((j / NS_S) & 1) ^ 1)) { failed = true; break; }
-        mbar_expect_tx(&k_full[s], load_keys(p, &map_k, bt, bt_first, w.hk, kt, w.lo, w.hi, nullptr, 0, nullptr) * box);
+        if (!tc::mbar_wait(&k_empty[s], ((j / NS_S) & 1) ^ 1)) { failed = true; break; }
+        tc::mbar_expect_tx(&k_full[s], load_keys(p, &map_k, bt, bt_first, w.hk, kt, w.lo, w.hi, nullptr, 0, nullptr) * box);
         load_keys(p, &map_k, bt, bt_first, w.hk, kt, w.lo, w.hi, Ks + (size_t)s * K_BYTES, BN * 128, &k_full[s]);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, BN, false);
-      const uint64_t dq = make_desc(smem_u32(Qs), 0);
-      failed = !mbar_wait(&q_full, 0);
+      constexpr uint32_t idesc = tc::make_idesc(BM, BN, false);
+      const uint32_t dq = tc::desc_lo(tc::smem_u32(Qs));
+      failed = !tc::mbar_wait(&q_full, 0);
       for (int j = 0; j < n_steps && !failed; ++j) {
-        if (!mbar_wait(&k_full[j % NS_S], (j / NS_S) & 1) || !mbar_wait(&s_empty[j & 1], ((j >> 1) & 1) ^ 1)) { failed = true; break; }
-        tc_fence_after();
-        const uint64_t dk = make_desc(smem_u32(Ks + (size_t)(j % NS_S) * K_BYTES), 0);
+        if (!tc::mbar_wait(&k_full[j % NS_S], (j / NS_S) & 1) || !tc::mbar_wait(&s_empty[j & 1], ((j >> 1) & 1) ^ 1)) { failed = true; break; }
+        tc::fence_after();
+        const uint32_t dk = tc::desc_lo(tc::smem_u32(Ks + (size_t)(j % NS_S) * K_BYTES));
         const uint32_t acc = tmem_base + (uint32_t)((j & 1) * BN);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           // 16 k-values further: 32 bytes within an atom (4 steps), then the next atom of Q (128 rows) and K (64 rows)
-          const uint64_t qo = (uint64_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2), ko = (uint64_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2);
-          tc_mma(acc, dq + qo, dk + ko, idesc, kk != 0 ? 1u : 0u);
+          const uint32_t qo = (uint32_t)((kk >> 2) * (BM * 128 >> 4) + (kk & 3) * 2), ko = (uint32_t)((kk >> 2) * (BN * 128 >> 4) + (kk & 3) * 2);
+          tc::mma_lo(acc, dq + qo, dk + ko, idesc, kk != 0 ? 1u : 0u);
         }
-        tc_commit(&s_full[j & 1]);
-        tc_commit(&k_empty[j % NS_S]);
+        tc::commit(&s_full[j & 1]);
+        tc::commit(&k_empty[j % NS_S]);
       }
     }
   } else {
@@ -274,16 +212,16 @@ __global__ void __launch_bounds__(64 + EPI * 32, 2) scores_tc_kernel(const __gri
     const float two_in = p.cap_in * (2.f * LOG2E), cap_log2 = p.cap * LOG2E, scale_log2 = p.scale * LOG2E;
     const int tiles_pitch = p.pitch / BN;
     for (int j = set; j < n_steps && !failed; j += 2) {
-      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[set], (j >> 1) & 1))) { failed = true; break; }
-      tc_fence_after();
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&s_full[set], (j >> 1) & 1))) { failed = true; break; }
+      tc::fence_after();
       const int kt = kt_first + j * BN;
       float v[BN];
-      tc_load32(lane_addr, v);
-      tc_load32(lane_addr + 32u, v + 32);
-      tc_wait_ld();
-      tc_fence_before();
+      tc::load32(lane_addr, v);
+      tc::load32(lane_addr + 32u, v + 32);
+      tc::wait_loads();
+      tc::fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s_empty[set]);              // the scores are in registers: the buffer may be used again
+      if (lane == 0) tc::mbar_arrive(&s_empty[set]);              // the scores are in registers: the buffer may be used again
       const bool live = kt <= pos;                            // the row reads keys of this tile (its first key is never behind it)
       if (!__any_sync(0xffffffffu, live)) continue;
       if (p.cap > 0.f) {
@@ -341,10 +279,10 @@ __global__ void __launch_bounds__(64 + EPI * 32, 2) scores_tc_kernel(const __gri
     }
   }
   if (failed) atomicExch(error, 1);
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   if (warp == 1) {
-    tc_fence_after();
+    tc::fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S_COLS) : "memory");
   }
 }
@@ -362,26 +300,26 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
   pdl_wait();
   Tile w;
   if (!find_tile(p, blockIdx.y, w)) return;
-  if ((smem_u32(smem) & 1023u) != 0) {
+  if ((tc::smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0) atomicExch(error, 1);
     return;
   }
   const int n_tiles = (w.hi - w.kt0 + BN - 1) / BN;
   if (threadIdx.x == 0) {
 #pragma unroll
-    for (int s = 0; s < NS_V; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    mbar_init(&landed, 1);
-    mbar_init(&cleared, 4);
-    mbar_init(&o_full, 1);
+    for (int s = 0; s < NS_V; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
+    tc::mbar_init(&landed, 1);
+    tc::mbar_init(&cleared, 4);
+    tc::mbar_init(&o_full, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(V_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(&tmem_base_s)), "r"(V_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
-  tc_fence_after();
+  tc::fence_after();
   const uint32_t tmem_base = tmem_base_s;
   const int tpt = BM / p.per;
   bool failed = false;
@@ -399,41 +337,41 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
       const unsigned box = (unsigned)((p.ps < BN ? p.ps : BN) * D * 2);
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % NS_V, kt = w.kt0 + j * BN;
-        if (!mbar_wait(&empty[s], ((j / NS_V) & 1) ^ 1)) { failed = true; break; }
+        if (!tc::mbar_wait(&empty[s], ((j / NS_V) & 1) ^ 1)) { failed = true; break; }
         const int n = load_keys(p, &map_v, bt, bt_first, w.hk, kt, w.lo, w.hi, nullptr, 0, nullptr);
-        mbar_expect_tx(&full[s], n * box + (unsigned)(tpt * p.per * BN * 2));
-        tma_load_4d(Ws + (size_t)s * W_BYTES, &map_w, &full[s], j * BN, 0, w.hk, w.q0 + w.tok0 - p.t_lo);
+        tc::mbar_expect_tx(&full[s], n * box + (unsigned)(tpt * p.per * BN * 2));
+        tc::load_4d(Ws + (size_t)s * W_BYTES, &map_w, &full[s], j * BN, 0, w.hk, w.q0 + w.tok0 - p.t_lo);
         load_keys(p, &map_v, bt, bt_first, w.hk, kt, w.lo, w.hi, Vs + (size_t)s * V_BYTES, BN * 128, &full[s]);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, D, true);
+      constexpr uint32_t idesc = tc::make_idesc(BM, D, true);
       unsigned clears = 0;
       for (int j = 0; j < n_tiles; ++j) {
         const int s = j % NS_V;
-        if (!mbar_wait(&full[s], (j / NS_V) & 1)) { failed = true; break; }
+        if (!tc::mbar_wait(&full[s], (j / NS_V) & 1)) { failed = true; break; }
         int head, tail;
         if (edges(j, head, tail)) {
-          mbar_arrive(&landed);
-          if (!mbar_wait(&cleared, clears & 1)) { failed = true; break; }
+          tc::mbar_arrive(&landed);
+          if (!tc::mbar_wait(&cleared, clears & 1)) { failed = true; break; }
           ++clears;
         }
-        tc_fence_after();
-        const uint32_t wa = smem_u32(Ws + (size_t)s * W_BYTES), va = smem_u32(Vs + (size_t)s * V_BYTES);
+        tc::fence_after();
+        const uint32_t wa = tc::smem_u32(Ws + (size_t)s * W_BYTES), va = tc::smem_u32(Vs + (size_t)s * V_BYTES);
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)
-          tc_mma(tmem_base, make_desc(wa + (uint32_t)(kk * 32), 0), make_desc(va + (uint32_t)(kk * 2048), BN * 128), idesc, (j | kk) != 0 ? 1u : 0u);
-        tc_commit(&empty[s]);
+          tc::mma_lo(tmem_base, tc::desc_lo(wa + (uint32_t)(kk * 32)), tc::desc_lo(va + (uint32_t)(kk * 2048), BN * 128), idesc, (j | kk) != 0 ? 1u : 0u);
+        tc::commit(&empty[s]);
       }
-      tc_commit(&o_full);
+      tc::commit(&o_full);
     }
   } else {
     unsigned clears = 0;
     for (int j = 0; j < n_tiles && !failed; j = (j == 0 && n_tiles > 1) ? n_tiles - 1 : n_tiles) {
       int head, tail;
       if (!edges(j, head, tail)) continue;
-      if (!__all_sync(0xffffffffu, mbar_wait(&landed, clears & 1))) { failed = true; break; }
+      if (!__all_sync(0xffffffffu, tc::mbar_wait(&landed, clears & 1))) { failed = true; break; }
       ++clears;
       unsigned char* vt = Vs + (size_t)(j % NS_V) * V_BYTES;
       const int gone = head + (BN - tail);
@@ -443,16 +381,16 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // these writes are read by the tensor core
       __syncwarp();
-      if (lane == 0) mbar_arrive(&cleared);
+      if (lane == 0) tc::mbar_arrive(&cleared);
     }
-    if (!failed && !__all_sync(0xffffffffu, mbar_wait(&o_full, 0))) failed = true;
-    tc_fence_after();
+    if (!failed && !__all_sync(0xffffffffu, tc::mbar_wait(&o_full, 0))) failed = true;
+    tc::fence_after();
     if (!failed) {
       const int q = warp & 3, row = q * 32 + lane, tok = row / p.per;
       float o[D];
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) tc_load32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), o + c * 32);
-      tc_wait_ld();
+      for (int c = 0; c < D / 32; ++c) tc::load32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * 32), o + c * 32);
+      tc::wait_loads();
       if (row < tpt * p.per && w.tok0 + tok < w.tok1) {
         bf16* dst = (bf16*)p.out + ((size_t)(w.q0 + w.tok0 + tok) * p.H + w.hk * p.per + (row - tok * p.per)) * D;
 #pragma unroll
@@ -463,28 +401,19 @@ __global__ void __launch_bounds__(192, 2) values_tc_kernel(const __grid_constant
     }
   }
   if (failed) atomicExch(error, 1);
-  tc_fence_before();
+  tc::fence_before();
   __syncthreads();
   if (warp == 1) {
-    tc_fence_after();
+    tc::fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(V_COLS) : "memory");
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn g_encode = nullptr;
-
 int encode4(CUtensorMap* map, const void* basep, const cuuint64_t (&dims)[4], const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4]) {
-  if (!g_encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess || !fn) return -300;
-    g_encode = (EncodeTiledFn)fn;
-  }
+  const tc::EncodeTiledFn encode = tc::encode_fn();
+  if (!encode) return -300;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult rc = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(basep), dims, strides, box, estr,
+  const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(basep), dims, strides, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return rc == CUDA_SUCCESS ? 0 : -301 - (int)rc;

@@ -20,22 +20,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_try(uint32_t bar_addr, unsigned parity) {
   uint32_t done;
   asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+               : "=r"(done) : "r"(bar_addr), "r"(parity) : "memory");
   return done != 0;
 }
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, unsigned parity) { return mbar_try(smem_u32(bar), parity); }
 // false: the wait ran out (the caller gives up and says so)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   const uint32_t addr = smem_u32(bar);
-  for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) return true;
-  }
+  for (unsigned i = 0; i < WAIT_LIMIT; ++i)
+    if (mbar_try(addr, parity)) return true;
   return false;
 }
 // the same for a whole warp: all lanes get the same answer
@@ -47,6 +43,10 @@ __device__ __forceinline__ void load_2d(void* dst, const CUtensorMap* map, uint6
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void load_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int u) {
+  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+               ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u) : "memory");
+}
 __device__ __forceinline__ void load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int u, int v) {
   asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
                ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(u), "r"(v) : "memory");
@@ -56,15 +56,10 @@ __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::aft
 __device__ __forceinline__ void commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
 // 32 lanes x 32 columns of 32-bit accumulator: thread i of the warp gets lane (base lane + i), 32 consecutive columns
-// (wait_loads() before the registers are used). The instruction is the warp's: lanes that a branch before it has parted meet first.
-__device__ __forceinline__ void load32(uint32_t taddr, uint32_t (&r)[32]) {
-  __syncwarp();
+// (wait_loads() before the registers are used). The instruction is the warp's: lanes that a branch before it has parted meet first, or
+// (_met) have just met and taken no branch of their own since.
+__device__ __forceinline__ void load32_met(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -75,18 +70,22 @@ __device__ __forceinline__ void load32(uint32_t taddr, uint32_t (&r)[32]) {
         "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
 }
+__device__ __forceinline__ void load32_met(uint32_t taddr, float* r) { load32_met(taddr, reinterpret_cast<uint32_t*>(r)); }
+template <typename T>
+__device__ __forceinline__ void load32(uint32_t taddr, T* r) {
+  __syncwarp();
+  load32_met(taddr, r);
+}
 __device__ __forceinline__ void wait_loads() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor, 128-byte swizzle: rows of 128 bytes, 8 rows to a 1024-byte atom, atoms one after the
-// other (stride 1024 bytes); version 1, layout type 2; a K-major operand.
-__device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
-}
-
-// Its upper half, the same for all tiles, and its lower half: the thread that issues the products then only ever adds to a 32-bit
-// number (the address in units of 16 bytes) instead of making a descriptor anew for each.
+// other (stride 1024 bytes); version 1, layout type 2; a K-major operand. Its upper half is the same for all tiles, its lower half the
+// address in units of 16 bytes: the thread that issues the products only ever adds to a 32-bit number instead of making a descriptor
+// anew for each.
 constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr) { return (smem_addr & 0x3FFFF) >> 4; }
+// ... of an MN-major operand: ``lbo``, the distance between 64-element swizzle atoms along the non-k dimension
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return desc_lo(smem_addr) | (lbo_bytes >> 4) << 16; }
 __device__ __forceinline__ void mma_lo(uint32_t tmem_d, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %5};\n mov.b64 b, {%2, %5};\n setp.ne.b32 p, %4, 0;\n"
@@ -108,9 +107,10 @@ __device__ __forceinline__ bool elect_one() {
   return yes != 0;
 }
 
-// kind::f16 instruction descriptor: float accumulator, bfloat16 a and b, N x M of the tile; both K-major
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+// kind::f16 instruction descriptor: float accumulator, bfloat16 a and b, N x M of the tile; a K-major, and b too unless its non-k dimension
+// is the contiguous one in shared memory (values: rows are keys, head elements contiguous)
+__host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool b_mn_major = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

@@ -16,26 +16,30 @@ def _function(text, at):
     return start.group(1), text[start.end():at]
 
 
-@pytest.mark.parametrize("name", [f for f, s in SOURCES.items() if "tcgen05.ld" in s])
+TENSOR_MEMORY = [f for f, s in SOURCES.items() if "tcgen05." in s]
+
+
+@pytest.mark.parametrize("name", TENSOR_MEMORY)
 def test_a_warp_meets_before_its_tensor_memory_instructions(name):
     """tcgen05.ld, .st, the wait for stores and barriers are ``.aligned``: all lanes execute them together. Branches that rows beyond the last
     and lanes that wait alone take stand before them, so the functions that issue them begin with the warp's meeting. Those named _met do
     not: before their calls no lane has gone its own way since the warp met last."""
     text = SOURCES[name]
     found = list(re.finditer(r'"(\{\\n .reg .pred p, q;\\n setp[^;]*;\\n )?(tcgen05\.(ld|st|wait::st)\.sync\.aligned|bar\.(sync|red))', text))
-    assert found
+    assert found or name not in ("tcgen05_ops.cuh", "attention_tc.cu")
     for m in found:
-        name, before = _function(text, m.start())
-        assert "__syncwarp();" in before or name.endswith("_met"), name
+        function, before = _function(text, m.start())
+        assert "__syncwarp();" in before or function.endswith("_met"), function
     for m in re.finditer(r"(?<!void )\b\w+_met\(", text):
-        if "__forceinline__" in text[text.rfind("\n", 0, text.rfind("\n", 0, m.start())):m.start()]:
-            continue                                        # (a function that is a meeting and such a call)
-        met = max(text.rfind(s, 0, m.start()) for s in ("__syncwarp();", "pair_any(", " tc_load32(", " tc_store32("))
+        line = text[text.rfind("\n", 0, m.start()) + 1:m.start()]
+        if "__forceinline__" in line or "__syncwarp();\n" in text[m.start() - 60:m.start()]:
+            continue                                        # (one that hands on to another, or a meeting and such a call)
+        met = max(text.rfind(s, 0, m.start()) for s in ("__syncwarp();", "pair_any(", "tc::load32(", "tc_store32("))
         between = text[met + 1:m.start()]
         assert met > 0 and not re.search(r"mbar_|if \(lane|row_ok|\breturn\b", between), between
 
 
-@pytest.mark.parametrize("name", [f for f, s in SOURCES.items() if "tcgen05.ld" in s])
+@pytest.mark.parametrize("name", TENSOR_MEMORY)
 def test_lanes_that_load_from_tensor_memory_give_up_together(name):
     """A lane that left such a loop by itself would not come to the next meeting: only single-lane loops may leave on one lane's wait."""
     text = SOURCES[name]
