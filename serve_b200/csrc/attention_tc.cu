@@ -16,14 +16,15 @@
 //              does; then, and only then, they exchange their maxima and rescale the accumulator in tensor memory after the products
 //              issued so far have finished. So in the steady state nobody waits for the second product. At the end each thread
 //              divides its half of the output row by the row's sum and stores it.
-// What bounds it: a step's latencies, not its work (head_dim 64: of 1,790 cycles a CTA's step takes, 512 are the exponentials of 128
-// rows, waits on mbarriers that are long complete 250 to 700, the pair's barrier 100). What that led to, 2,048 tokens, 32/8 heads of 64 | 16/4 of
-// 128 behind a window of 1,024 | 16 heads over a row of 256: a thread a row and one thread of a divergent warp to issue 53.9 | 45.8 | 60.5 us;
+// What bounds it: a step's latencies, not its work (head_dim 64, 2,048 tokens: of 1,860 cycles a tile takes, 390 wait for the scores, 300 load them
+// and take the maximum, 80 are the pair's vote, 120 moved references, 780 the exponentials and their stores, of which the exp2 unit itself
+// needs 512 for the rows of a CTA, 180 the wait for the stores and the arrival; tensor pipe active 19 % of the time). What
+// that led to, 2,048 tokens, 32/8 heads of 64 | 16/4 of 128 behind a window of 1,024 | 16 heads over a row of 256: a thread a row and one thread of a divergent warp to issue 53.9 | 45.8 | 60.5 us;
 // two threads a row and the probabilities in tensor memory 52.4 | 41.7 | 52.8; products issued from a warp that has come together, with
 // 32-bit additions in place of descriptors made anew, 50.7 | 38.3 | 49.6; waits that cost one instruction when there is nothing to wait for,
 // 48.4 | 36.0 | 49.8; copies issued like the products, a tile's page looked up a tile ahead, 47.2 | 35.2 | 48.8 (a loop of a few
-// more branches there: 52.3 | 39.0 | 49.2); two CTAs an SM at head_dim 128 (TIGHT) 28.9. No difference: two sets of softmax warps for even
-// and odd tiles, longer hardware waits, a single polling lane, packed arithmetic, a tile's page looked up still earlier. Slower: tiles of 128
+// more branches there: 52.3 | 39.0 | 49.2); two CTAs an SM at head_dim 128 (TIGHT) 28.9. Packed
+// arithmetic (fma2, add2, max3): a whole layer 77.3 -> 76.35 | 84.8 -> 84.3 | 106.45 -> 106.2. No difference: two sets of softmax warps for even and odd tiles, longer hardware waits, a single polling lane. Slower: tiles of 128
 // keys (one buffer each of scores and probabilities: eight prompts of 256 26 us against 24; 55.7 over rows of 256).
 // Two CTAs share an SM at head_dim 64 (96 KB of shared memory, 256 columns of tensor memory each).
 // At head_dim 128 an operand row is two 128-byte swizzle atoms: queries, keys and values arrive as two TMA boxes of 64

@@ -745,7 +745,8 @@ __global__ void __launch_bounds__(THREADS) chunk_walk_kernel(const SbChunkedWalk
 // fetches. A chunk's matrices then cross to an SM once for 16 G columns instead of once for 16, and since S lies turned over in
 // the accumulators (columns of S are the tile's rows), they are the first operand of the next product as they stand: S and U never
 // pass through shared memory, and the warps of a group meet once a step, to add their sums of W S (and Q' S) up. What bounds it: mma.sync, 16
-// cycles each on a scheduler (1,728 of them a step with 64 columns and no delta rule, 6,900 of the step's 7,900 cycles). With few pairs there
+// cycles each on a scheduler by timing (1,728 of them a step with 64 columns and no delta rule: 6,900 of the step's 7,800 cycles; the tensor pipe's
+// counter calls it active in half of those). With few pairs there
 // are not enough blocks, and chunk_walk_kernel, whose eight warps share 16 columns, has the shorter step. Eight requests of 256 tokens, 16
 // heads of 128 x 128: fixed decay 101 -> 67 us, gated delta rule 121 -> 95. (One warp for all rows of 16 columns: 91 us, registers spill;
 // the sums of Q' S a step behind those of W S, so that they hide: 107, more of them spill.)
