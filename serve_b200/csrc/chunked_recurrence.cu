@@ -30,6 +30,7 @@
 #include "bounded_wait.h"
 #include "common.cuh"
 #include "tcgen05_ops.cuh"
+#include "walk_rule.h"
 
 using namespace sb;
 typedef __nv_bfloat16 bf16;
@@ -1095,24 +1096,11 @@ int launch(const SbChunkedWalk& a, int chunks, cudaStream_t stream) {
   }
   SB_LAUNCH_CHECK();
   const float* u = DELTA ? u_rows : a.vf;
-  // Which walk: rounds of blocks the GPU needs times how long a step of 32 tokens takes with it (hundredths of a microsecond), the cheapest. Both
-  // sides measured, 16 heads, us (16 columns a block | 32 | 64): states of 128 x 128 with the delta rule, one request of 2,048 tokens 121 | 168,
-  // four of 512 112 | 82, sixteen of 180 179 | 126; a decay alone, one of 2,048 101 | 137 | 219, two of 1,024 103 | 73 | 112, eight of 256 101 | 79 | 67; of
-  // 64 x 64 with the delta rule, two of 512 27 | 33, four 53 | 36; a decay alone (two blocks an SM, which slow one another down), four of
-  // 512 33 | 42, eight of 256 34 | 29, sixteen 63 | 58.
-  const long long pairs = (long long)a.H * a.n_list, cols = (a.dv + 15) / 16, sms = sm_count();
-  auto cost = [&](int groups, int alone, int two) {
-    const long long blocks = pairs * ((cols + groups - 1) / groups), at_once = two > 0 && blocks > sms ? 2 * sms : sms;
-    return (blocks + at_once - 1) / at_once * (at_once > sms ? two : alone);
-  };
-  constexpr bool BIG = DKT == 128;
-  const long long one = DELTA ? cost(1, BIG ? 187 : 154, 0) : cost(1, BIG ? 157 : 133, BIG ? 0 : 205);
-  const long long two = DELTA ? cost(2, BIG ? 260 : 196, 0) : cost(2, BIG ? 213 : 246, BIG ? 0 : 340);
-  if constexpr (BIG && !DELTA) {
-    const long long four = cost(4, 342, 0);
-    if (four < one && four < two) return launch_wide<DKT, DELTA, 4>(a, u, stream);
+  const int groups = walk_groups(DELTA, DKT == 128, a.H, (a.dv + 15) / 16, chunks, (a.max_q + CH - 1) / CH, sm_count());
+  if constexpr (DKT == 128 && !DELTA) {
+    if (groups == 4) return launch_wide<DKT, DELTA, 4>(a, u, stream);
   }
-  if (two < one) return launch_wide<DKT, DELTA, 2>(a, u, stream);
+  if (groups == 2) return launch_wide<DKT, DELTA, 2>(a, u, stream);
   auto k = chunk_walk_kernel<DKT, DELTA>;
   constexpr int smem = Walk<DKT, DELTA>::BYTES;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -157,7 +157,7 @@ def short_on_mma(longest: int, group: int, keys: int, decoding_too: bool, pairs:
 # chunked kernels make a chain of tokens / 32 steps, but their work is that of 64 or 128 rows by 32 tokens whatever the state, so small
 # states of many requests are the walk's, and so are requests of hardly more than 32 tokens. Fitted to 9,800 steps of one to 16 requests of 33 to
 # 2,048 tokens, alike and ragged, 4 to 32 heads, 16 to 128 rows by 16 to 256 columns. Of 1,400 other steps the choice is the slower one by
-# more than 5 % in 4.7 % of them, by more than 10 % in 2.9 %; 0.7 % on average, 1.29 times at most. Chunked | walked in us (one, one with the
+# more than 5 % in 4.5 % of them, by more than 10 % in 2.8 %; 0.65 % on average, 1.29 times at most. Chunked | walked in us (one, one with the
 # delta rule, one a row with the delta rule, one a row):
 #   1 request of 1,024 tokens, 16 heads of 64 x 64: 66 | 226, 80 | 308, 107 | 311, 70 | 248; of 128 x 128: 79 | 257, 106 | 362, 145 | 365, 97 | 281
 #   16 of 256, 16 heads of 64 x 64: 125 | 131, 193 | 181, 325 | 195, 144 | 162; of 128 x 128: 240 | 382, 342 | 634, 484 | 645, 288 | 521

@@ -140,7 +140,7 @@ def test_a_later_token_does_not_reach_back(K, mode):
 
 
 @pytest.mark.parametrize("mode", MODES)
-@pytest.mark.parametrize("dk,dv", [(128, 128), (100, 72), (64, 128), (40, 136)])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (100, 72), (100, 40), (64, 128), (40, 136)])
 def test_many_pairs(K, mode, dk, dv):
     """So many (request, head) pairs that blocks walk 32 or 64 columns of S: ragged requests, part of a block's columns beyond the last, an
     infinity in the values of one request."""
