@@ -170,3 +170,32 @@ def test_grouping_by_expert(pairs, experts, rows):
         tile += [(e, want[e] + r) for r in range(0, n, rows)]
     assert n_tiles.item() == len(tile) and tiles[: 2 * len(tile)].view(-1, 2).tolist() == [list(t) for t in tile]
     assert got[want[-1]:] == [-7] * (pairs - want[-1])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,n,top", [(1, 4, 1), (33, 64, 3), (70, 1000, 5), (9, 924, 4), (7, 1100, 2), (5, 1024, 9), (3, 1924, 4), (4, 30, 2), (2, 2048, 3)])
+def test_sum_over_a_tokens_choices(tokens, n, top, dtype):
+    """Rows that fill the blocks a block takes a part of one in, rows that do not, rows of no whole pieces of four;
+    choices that are the token itself, a gated shared expert, an input with a stride of its own."""
+    import ctypes
+
+    from serve_b200.kernels import load_kernels
+
+    kernels = load_kernels("cuda:0")
+    g = torch.Generator(device="cuda").manual_seed(n + top)
+    draw = lambda *s: torch.randn(s, generator=g, device="cuda")
+    parts, x = draw(tokens * top, n), draw(tokens, n + 4).to(dtype)[:, :n]
+    shared, logits, weights = draw(tokens, n).to(dtype), draw(tokens, 3), draw(tokens * top)
+    idx = torch.randint(0, 6, (tokens * top,), generator=g, device="cuda", dtype=torch.int32)
+    room = torch.full((tokens * n + 8,), 7.0, device="cuda", dtype=dtype)
+    out = room[: tokens * n].view(tokens, n)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    code = 1 if dtype == torch.bfloat16 else 0
+    assert kernels._moe_lib().sb_moe_combine_more(p(parts), p(idx), p(weights), 4, p(x), x.stride(0), p(shared), ctypes.c_void_p(logits.data_ptr() + 8), 3,
+                                                  top, tokens, n, p(out), code, kernels._s()) == 0
+    rows = torch.where(idx[:, None] < 4, parts.double(), weights.double()[:, None] * x.double().repeat_interleave(top, 0)).view(tokens, top, n)
+    want = rows.sum(1) + torch.sigmoid(logits[:, 2:].double()) * shared.double()
+    most = rows.abs().sum(1) + shared.double().abs()
+    # top + 1 float additions, the sigmoid's few roundings, and the output's own
+    assert ((out.double() - want).abs() <= (top + 8) * 2.0 ** -24 * most + (2.0 ** -8 * want.abs() if code else 0.0)).all()
+    assert (room[tokens * n:] == 7.0).all()
