@@ -510,10 +510,24 @@ __global__ void __launch_bounds__(REC_THREADS) recurrence_prep_vec_kernel(RecArg
   }
 }
 
+// Is it the faster way? Up to 128 rows a warp takes four tokens one behind the other, which pays once there is more than a round of warps:
+// below 8,192 (token, head) pairs a warp a pair is 1 to 3 us faster (decoding, 64 requests, 16 heads of 64, a warp a pair | in pieces: fixed decay
+// 14.6 | 17.6 us of recurrence, delta rule 18.7 | 21.2, a decay a row 17.1 | 19.6; 8 requests of 128 rows 12.6 | 14.6, 15.1 | 16.9, 14.1 | 15.5). Above, few rows leave
+// most lanes of a warp without a piece, the longer the more each number costs: 32,768 pairs of 64 rows 1.2 us slower with a fixed decay (three
+// silu), 3 to 9 faster in the other modes; of 32 rows 4.4 slower with a fixed decay, 1.4 with a decay a row, of 128 rows 3.4 to 13.7 faster in all. Rows
+// of more than 128 are faster in pieces at any count (256: 0 to 14 us with a fixed decay, whose 192 are 1 to 3 slower, to 94 with a decay a row).
+template <int MODE>
+bool pieces_pay(const RecArgs& a) {
+  if (a.dk > 128) return MODE != MODE_DECAY || a.dk > 192;
+  const int heads = a.H > a.Hqk ? a.H : a.Hqk;
+  if ((long long)a.n_tokens * heads < 8192) return false;
+  return a.dk >= (MODE == MODE_DECAY ? 96 : MODE == MODE_GLA || (MODE == MODE_DELTA && !a.rate_per_head) ? 48 : 1);
+}
+
 // May recurrence_prep_vec_kernel take these rows? (The work space is made of whole pieces: dkp and dvp are multiples of four.)
 template <typename T, int MODE>
 bool prep_in_pieces(const RecArgs& a) {
-  if (MODE == MODE_RET || MODE == MODE_WKV) return false;
+  if (MODE == MODE_RET || MODE == MODE_WKV || !pieces_pay<MODE>(a)) return false;
   auto piece = [](const void* p, int dtype) { return ((uintptr_t)p & (dtype == SB_DTYPE_F32 ? 15u : 7u)) == 0; };
   const int td = sizeof(T) == 4 ? SB_DTYPE_F32 : SB_DTYPE_BF16;
   if ((a.dk | a.dv | a.q_stride | a.k_stride | a.v_stride | a.dkp | a.dvp) % 4 || !piece(a.q, td) || !piece(a.k, td) || !piece(a.v, td) ||

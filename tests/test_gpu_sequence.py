@@ -57,3 +57,17 @@ def test_what_the_walk_reads(K, mode, dk, dtype):  # noqa: F811
     out, pool = _run(K, c, chunked=False)
     bound = 8 * dk ** 0.5 * 2.0 ** -24 + 2e-7              # (see the chunks' test)
     assert _error(out, want) < bound and _error(pool, want_pool) < bound
+
+
+@pytest.mark.parametrize("mode", ["decay", "ssm", "delta", "delta_head", "gla"])
+@pytest.mark.parametrize("dk", [16, 48, 100, 128])
+def test_what_the_walk_reads_of_many_tokens(K, mode, dk):  # noqa: F811
+    """From 8,192 (token, head) pairs on a warp takes four tokens of up to 128 rows: requests that begin inside such a run, a last run of one."""
+    lengths = [100, 1, 150, 6]
+    c = _case(mode, lengths, 32, 32, dk, 40, torch.bfloat16, seed=dk)
+    assert sum(lengths) * 32 >= 8192 and sum(lengths) % 4 == 1
+    want, want_pool = _exact(c)
+    bound = 8 * dk ** 0.5 * 2.0 ** -24 + 2e-7              # (see the chunks' test)
+    for chunked in (False, True):                          # walked; the two longer requests in chunks
+        out, pool = _run(K, c, chunked=chunked)
+        assert _error(out, want) < bound and _error(pool, want_pool) < bound
