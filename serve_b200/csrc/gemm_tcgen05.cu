@@ -601,11 +601,13 @@ int run_product(const void* a, const void* w, void* out, int M, int N, int K, in
     }
   }
   cudaError_t e;
-  // At equal cost the pair kernel wins where a CTA has more than a tile or two of few k-values to do: starting and ending a cluster
-  // costs it about 1 us more than the one-CTA kernel (one CTA | pair: q/k/v, 2,048 k-values, 600 rows 12.1 | 12.2 us, 1,700 rows 25.9 | 21.6, 2,048 rows
-  // 26.7 | 23.9; gate/up to 768, 2,048 rows 20.7 | 21.3; gate/up to 8,192 of 3,072, 1,700 rows 135.6 | 126.4).
+  // At equal cost the pair kernel wins where a CTA has more than a tile of 32 blocks of k-values or more to do: starting and ending a
+  // cluster costs it about 1 us more than the one-CTA kernel, and with shorter rows its tiles' ends come too often (one CTA | pair: q/k/v, 2,048
+  // k-values, 600 rows 12.1 | 12.2 us, 1,700 rows 25.9 | 21.6, 2,048 rows 26.7 | 23.9; gate/up to 768, 2,048 rows 20.7 | 21.3; gate/up to 8,192 of 3,072, 1,700 rows
+  // 135.6 | 126.4; of 1,024 k-values, gate/up to 4,096, 2,048 rows 33.1 | 35.2, to 8,192, 4,096 rows 109.9 | 116.4, of 1,536 to 2,048, 4,096 rows 42.3 | 43.3; one tile of
+  // 4,096, gate/up to 768, 1,000 rows 44.4 | 45.7).
   const long long k_blocks = (K + BK - 1) / BK;
-  const bool pair_wins = cost_pair < cost_single || (cost_pair == cost_single && waves_pair * k_blocks >= 64);
+  const bool pair_wins = cost_pair < cost_single || (cost_pair == cost_single && k_blocks >= 32 && waves_pair * k_blocks >= (waves_pair > 1 ? 64 : 96));
   if (pairs > 0 && (pair_wins || g_pair_enabled == 2)) {
     const long long m_tiles = (M + 255) / 256;
     const int bn = bn_pair;
